@@ -14,6 +14,8 @@ KB_MAX_WORLD = 16
 KB_OK, KB_ERR_CUDA, KB_ERR_ARG, KB_ERR_TIMEOUT, KB_ERR_IO, KB_ERR_UNSUPPORTED = range(6)
 BACKEND_HOST, BACKEND_VMM, BACKEND_IPC = 0, 1, 2
 GEMM_PLAIN, GEMM_RS, GEMM_AG = 0, 1, 2
+LOCAL_DENSE, LOCAL_ROWS, LOCAL_CONTRACT = 0, 1, 2
+ACTS = {None: 0, "gelu": 1, "relu": 2, "silu": 3}
 
 DEV_CODES = {0: "ok", 1: "pipeline barrier timeout", 2: "peer flag timeout", 3: "index out of bounds"}
 
@@ -61,6 +63,34 @@ class GemmArgs(C.Structure):
         ("wait_limit_ns", C.c_uint64),
         ("num_ctas", C.c_int),
         ("mc_base", C.c_void_p),
+    ]
+
+
+class LocalGemmArgs(C.Structure):
+    _fields_ = [
+        ("kind", C.c_int),
+        ("M", C.c_int),
+        ("N", C.c_int),
+        ("K", C.c_int),
+        ("a_mn", C.c_int),
+        ("b_mn", C.c_int),
+        ("groups", C.c_int),
+        ("row_start", C.c_void_p),
+        ("row_count", C.c_void_p),
+        ("A", C.c_void_p),
+        ("B", C.c_void_p),
+        ("bias", C.c_void_p),
+        ("bias_scale", C.c_float),
+        ("out", C.c_void_p),
+        ("act", C.c_int),
+        ("pre_out", C.c_void_p),
+        ("pre_in", C.c_void_p),
+        ("status", C.c_void_p),
+        ("wait_limit_ns", C.c_uint64),
+        ("num_ctas", C.c_int),
+        ("pair", C.c_int),
+        ("bn", C.c_int),
+        ("split", C.c_int),
     ]
 
 
@@ -126,6 +156,11 @@ def _declare(lib: C.CDLL) -> None:
         "kb_wait_flags": (i, [vp, i, i, u32, u64, vp, vp]),
         "kb_device_barrier": (i, [C.POINTER(vp), u64, i, i, u32, u64, vp, vp]),
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
+        "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
+        "kb_gemm_local_config": (i, [i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
+        "kb_moe_permute": (i, [vp, vp, i, i, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
+        "kb_moe_combine": (i, [vp, vp, vp, i, i, i, vp, vp]),
+        "kb_moe_grad_rows": (i, [vp, vp, vp, vp, i, i, i, i, vp, vp, vp, vp, vp, vp]),
         "kb_gemm_schedule": (i, [i, i, i, i, i, i, i, C.POINTER(i), C.POINTER(i)]),
         "kb_gemm_rs_data_bytes": (u64, [i, i, i]),
         "kb_gemm_rs_flag_bytes": (u64, [i, i, i]),

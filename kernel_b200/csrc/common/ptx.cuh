@@ -107,6 +107,10 @@ __device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uin
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void st_shared_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 // ----------------------------------------------------------------- TMA ----
 // 2-D tiled load global -> shared of one box, completion on an mbarrier.
 // Plain (single-CTA) form only.  x is the innermost coordinate and must keep
@@ -116,6 +120,28 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
+}
+// 3-D forms (innermost coordinate x, then y, z).  kPair: the completion is counted on
+// the mbarrier at cluster address `bar` (the leader of a CTA pair); otherwise `bar` is
+// the shared-memory address of one of this CTA's own barriers.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y, int32_t z) {
+  if constexpr (kPair) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+  } else {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+  }
+}
+__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_src, int32_t x, int32_t y, int32_t z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
@@ -269,6 +295,49 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
 __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
                : "memory");
+}
+
+// Warp-converged forms: every lane of the warp calls them with the same arguments and
+// one elected lane issues.  With the loop around them free of divergence the compiler
+// keeps addresses and descriptors in uniform registers, where tcgen05 wants its
+// operands; issued from inside an `if (lane == 0)` the same instructions cost a move
+// per operand register, which made the issuing thread the bottleneck of the mainloop
+// (640 instead of 512 cycles per 64-wide k block of a 256 x 256 pair tile).
+//
+// Four consecutive K steps (64 elements) of D (+)= A * B; the descriptors advance by
+// `a_step` / `b_step` 16-byte units per step.
+template <bool kPair>
+__device__ __forceinline__ void umma_f16_x4(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                            uint32_t a_step, uint32_t b_step, uint32_t idesc, uint32_t accumulate) {
+#define KB_UMMA_X4(GROUP)                                                                                          \
+  asm volatile(                                                                                                    \
+      "{\n\t.reg .pred q, p;\n\t.reg .b32 al, bl;\n\t.reg .b64 da, db;\n\t"                                             \
+      "elect.sync _|q, 0xffffffff;\n\t"                                                                            \
+      "setp.ne.b32 p, %8, 0;\n\t"                                                                                  \
+      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"                                                        \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %7, p;\n\t"                                     \
+      "add.u32 al, %1, %5;\n\tadd.u32 bl, %3, %6;\n\tmov.b64 da, {al, %2};\n\tmov.b64 db, {bl, %4};\n\t"        \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %7, 1;\n\t"                                     \
+      "add.u32 al, al, %5;\n\tadd.u32 bl, bl, %6;\n\tmov.b64 da, {al, %2};\n\tmov.b64 db, {bl, %4};\n\t"        \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %7, 1;\n\t"                                     \
+      "add.u32 al, al, %5;\n\tadd.u32 bl, bl, %6;\n\tmov.b64 da, {al, %2};\n\tmov.b64 db, {bl, %4};\n\t"        \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %7, 1;\n\t}"                                    \
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(a_step), "r"(b_step), "r"(idesc), "r"(accumulate) \
+      : "memory")
+  if constexpr (kPair) KB_UMMA_X4("2");
+  else KB_UMMA_X4("1");
+#undef KB_UMMA_X4
+}
+// Commit of the elected lane; `bar`: shared-memory address (cluster address for a pair).
+template <bool kPair>
+__device__ __forceinline__ void umma_commit_warp(uint32_t bar) {
+  if constexpr (kPair) {
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+  } else {
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+  }
 }
 
 // Shared-memory operand descriptor for a K-major bf16 tile stored as rows of

@@ -118,6 +118,37 @@ typedef struct KbGemmArgs {
 } KbGemmArgs;
 
 int kb_gemm(const KbGemmArgs* args, void* stream);
+
+// Products whose operands are all on this GPU (kernels/gemm_local.cu).
+enum KbLocalKind {
+  KB_LOCAL_DENSE = 0,     // out[M,N] = A * B^T
+  KB_LOCAL_ROWS = 1,      // group e: out[rows of e][N] = A[rows of e][K] * B[e]^T
+  KB_LOCAL_CONTRACT = 2,  // group e: out[e][M,N] = A[rows of e][M]^T * B[rows of e][N]
+};
+enum KbAct { KB_ACT_NONE = 0, KB_ACT_GELU = 1, KB_ACT_RELU = 2, KB_ACT_SILU = 3 };
+typedef struct KbLocalGemmArgs {
+  int kind;
+  int M, N, K;          // ROWS: M = rows of A and out; CONTRACT: K = rows of A and B
+  int a_mn, b_mn;       // 0: operand contiguous along K ([M,K], [N,K]); 1: along M / N ([K,M], [K,N]); CONTRACT: both 1
+  int groups;           // ROWS, CONTRACT
+  const int32_t* row_start;  // device [groups]; CONTRACT: rows between a group's last row and the next multiple of
+  const int32_t* row_count;  // 64 rows after its start must hold zeros in A or B and finite values in the other
+  const void* A;
+  const void* B;        // ROWS: [groups] matrices
+  const void* bias;     // bf16 [N] or NULL; not with groups
+  float bias_scale;
+  void* out;            // DENSE [M,N], ROWS [M,N], CONTRACT [groups][M,N]
+  int act;              // activation of the bf16-rounded result ...
+  void* pre_out;        // ... which is stored here too when not NULL (same shape as out)
+  const void* pre_in;   // not NULL: out = product * act'(pre_in) instead
+  uint32_t* status;
+  uint64_t wait_limit_ns;
+  int num_ctas;         // 0 = one per SM
+  int pair, bn, split;  // tile configuration; -1 / 0 / 0: chosen from the sizes (pair 2: 512-row tiles)
+} KbLocalGemmArgs;
+int kb_gemm_local(const KbLocalGemmArgs* args, void* stream);
+// The configuration kb_gemm_local picks for a dense product on `sms` SMs (tests of the rule).
+int kb_gemm_local_config(int M, int N, int K, int b_mn, int sms, int* pair, int* bn, int* split);
 // The fused modes (RS, AG) run by a CPU rank over a KB_BACKEND_HOST heap: same
 // schedule, staging layouts, flags and rounding points as the kernel (symm/gemm_host.cpp).
 int kb_gemm_host(const KbGemmArgs* args, int timeout_ms);
@@ -129,6 +160,18 @@ uint64_t kb_gemm_rs_flag_bytes(int M, int N, int world);
 uint64_t kb_gemm_ag_data_bytes(int M, int K);
 uint64_t kb_gemm_ag_flag_bytes(int M, int world);
 uint64_t kb_gemm_ag_counter_bytes(int M, int world);
+
+// ---- MoE rows on one rank (kernels/moe_rows.cu), bf16 rows of `hidden` elements ----
+// permute: copy of token t for its choice j -> rows[slots[t*k + j]], experts in ascending order, an expert's rows in
+// token order, each expert starting at a multiple of `pad` rows (the rows in between are zeroed).
+int kb_moe_permute(const void* x, const int32_t* indices, int T, int k, int experts, int hidden, int pad, void* rows,
+                   int32_t* slots, int32_t* row_start, int32_t* row_count, int32_t* row_padded, uint32_t* status, void* stream);
+// combine: out[t] = sum_j weights[t,j] * y[slots[t*k + j]] (weights NULL: ones).
+int kb_moe_combine(const void* y, const int32_t* slots, const float* weights, int T, int k, int hidden, void* out, void* stream);
+// grad_rows: dyr[slot] = weight * dy[t], dw[t,j] = <dy[t], y[slot]>; padding rows of dyr are zeroed.
+int kb_moe_grad_rows(const void* dy, const void* y, const int32_t* slots, const float* weights, int T, int k, int experts,
+                     int hidden, void* dyr, float* dw, const int32_t* row_start, const int32_t* row_count,
+                     const int32_t* row_padded, void* stream);
 
 // ---- MoE dispatch / combine ----------------------------------------------------
 typedef struct KbA2aArgs {

@@ -1,6 +1,6 @@
-// Persistent, warp-specialised bf16 GEMM for sm_100a in three modes:
+// Persistent, warp-specialised bf16 GEMM for sm_100a fused with a collective, in two
+// modes (without a collective: gemm_local.cu):
 //
-//   PLAIN  out = A * B^T (+ bias)
 //   RS     GEMM fused with reduce-scatter.  Every rank computes its K-shard's
 //          partial product tile by tile into its OWN half of a parity-buffered
 //          [M, N] bf16 staging matrix in the symmetric heap and, per tile,
@@ -22,7 +22,7 @@
 // Mainloop: one TMA producer thread fills a ring of 128x64 (A) and 256x64 (B)
 // K-major tiles with 128-byte swizzle; one thread issues tcgen05.mma into one of
 // two 256-column TMEM accumulators; four epilogue warps drain the other
-// accumulator.  Two epilogue variants: "tma" (PLAIN and AG only) goes tcgen05.ld ->
+// accumulator.  Two epilogue variants: "tma" (AG only) goes tcgen05.ld ->
 // bf16 -> 128-byte-swizzled shared memory -> cp.async.bulk.tensor store issued
 // by one lane per warp, two staging boxes per warp; "direct" stores 16-byte
 // vectors straight from the registers tcgen05.ld filled (a lane owns a row, so a
@@ -76,8 +76,7 @@ constexpr int OUT_BOX_BYTES = OUT_BOX_ROWS * OUT_BOX_COLS * 2;  // 4 KB
 constexpr int TMEM_COLS = 512;
 constexpr int BAR_BYTES = 256;
 constexpr int SMEM_BYTES = 1024 + 7 * 32768 + BAR_BYTES;  // 6 pair stages + staging = 4 single stages + staging = 7 pair stages
-constexpr int THREADS_BASE = 256;             // warps 0..3 control, 4..7 epilogue
-constexpr int THREADS_COMM = 384;             // + warps 8..11: all-gather pushers or reduce-scatter reducers
+constexpr int THREADS_COMM = 384;             // warps 0..3 control, 4..7 epilogue, 8..11 all-gather pushers or reduce-scatter reducers
 constexpr int SCHED_RING = 4;                 // AG: claimed tile positions in flight between the claimer and the other roles
 constexpr int AG_TILE_CLAIM = 128;            // AG: two words of the counter block (one per epoch parity) that hand out tile positions
 constexpr int RS_ROW_GROUP = 64;              // rows of one reduction unit
@@ -87,7 +86,7 @@ struct alignas(64) GemmParams {
   CUtensorMap tmA;
   CUtensorMap tmB;
   CUtensorMap tmOwn;  // AG: this rank's own rows, read in place
-  CUtensorMap tmOut;  // PLAIN/AG: the output, written with TMA stores
+  CUtensorMap tmOut;  // AG: the output, written with TMA stores
   int mode, M, N, K;
   int MB, NB, KB;
   const bf16* bias;
@@ -299,7 +298,7 @@ __device__ __forceinline__ void stage_box(uint32_t taddr, uint8_t* box, int lane
 }
 
 template <int kMode, bool kPair, bool kDirect>
-__global__ void __launch_bounds__(kMode == KB_GEMM_PLAIN ? THREADS_BASE : THREADS_COMM, 1)
+__global__ void __launch_bounds__(THREADS_COMM, 1)
 gemm_kernel(const __grid_constant__ GemmParams p) {
   constexpr bool kAG = (kMode == KB_GEMM_AG);
   constexpr bool kRS = (kMode == KB_GEMM_RS);
@@ -998,12 +997,31 @@ extern "C" int kb_gemm(const KbGemmArgs* a, void* stream_v) {
     }
   }
 
+  if (!dist) {  // one rank: nothing to exchange
+    KbLocalGemmArgs l;
+    memset(&l, 0, sizeof(l));
+    l.kind = KB_LOCAL_DENSE;
+    l.M = a->M;
+    l.N = a->N;
+    l.K = a->K;
+    l.A = a->A;
+    l.B = a->B;
+    l.bias = a->bias;
+    l.bias_scale = a->bias_scale;
+    l.out = a->out;
+    l.status = a->status;
+    l.wait_limit_ns = a->wait_limit_ns;
+    l.num_ctas = a->num_ctas & ~(1 << 30);
+    l.pair = (a->num_ctas & (1 << 30)) != 0 ? 0 : -1;
+    return kb_gemm_local(&l, stream_v);
+  }
+
   // CTA pairs need 256-row scheduling blocks that do not straddle two ranks.
   // num_ctas bit 30 forces the single-CTA kernel (tests, comparisons).
   const EnvConfig& env = env_config();
   const bool forbid_pair = (a->num_ctas & (1 << 30)) != 0 || env.no_pair;
   const int req_ctas = a->num_ctas & ~(1 << 30);
-  bool pair = !forbid_pair && a->M >= 256 && (!dist || (rpo % 256) == 0);
+  bool pair = !forbid_pair && a->M >= 256 && (rpo % 256) == 0;
   int dev = 0, sms = 0;
   KB_CUDA_OK(cudaGetDevice(&dev));
   {
@@ -1024,7 +1042,7 @@ extern "C" int kb_gemm(const KbGemmArgs* a, void* stream_v) {
 
   GemmParams p;
   memset(&p, 0, sizeof(p));
-  fill_schedule(p, a->mode, a->M, a->N, dist ? a->rank : 0, dist ? a->world : 1, pair);
+  fill_schedule(p, a->mode, a->M, a->N, a->rank, a->world, pair);
   p.K = a->K;
   p.KB = (a->K + BK - 1) / BK;
   p.bias = static_cast<const bf16*>(a->bias);
@@ -1037,19 +1055,15 @@ extern "C" int kb_gemm(const KbGemmArgs* a, void* stream_v) {
   p.flag_off = a->flag_off;
   p.counter_off = a->counter_off;
   p.timing = env.timing ? 1 : 0;
-  p.own_lo_mb = 0;
-  p.own_hi_mb = p.MB - 1;
   const void* a_ptr = a->A;
-  if (dist) {
-    for (int r = 0; r < a->world; ++r) p.peer_base[r] = static_cast<char*>(a->peer_base[r]);
-    p.mc_base = static_cast<char*>(a->mc_base);
-    p.own_lo_mb = (a->rank * rpo) / BM;
-    p.own_hi_mb = ((a->rank + 1) * rpo - 1) / BM;
-    if (a->mode == KB_GEMM_AG) {
-      p.a_local = static_cast<const bf16*>(a->A);
-      const uint32_t parity = a->epoch & 1u;
-      a_ptr = p.peer_base[a->rank] + a->data_off + (uint64_t)parity * a->M * a->K * 2;
-    }
+  for (int r = 0; r < a->world; ++r) p.peer_base[r] = static_cast<char*>(a->peer_base[r]);
+  p.mc_base = static_cast<char*>(a->mc_base);
+  p.own_lo_mb = (a->rank * rpo) / BM;
+  p.own_hi_mb = ((a->rank + 1) * rpo - 1) / BM;
+  if (a->mode == KB_GEMM_AG) {
+    p.a_local = static_cast<const bf16*>(a->A);
+    const uint32_t parity = a->epoch & 1u;
+    a_ptr = p.peer_base[a->rank] + a->data_off + (uint64_t)parity * a->M * a->K * 2;
   }
 
   int rc = make_tmap(&p.tmA, a_ptr, a->M, a->K, BK, BM);
@@ -1067,28 +1081,24 @@ extern "C" int kb_gemm(const KbGemmArgs* a, void* stream_v) {
     if (rc != KB_OK) return rc;
   }
 
-  const int total_units = p.MBQ * p.NB * (pair ? 2 : 1);
-  if (p.mode == KB_GEMM_PLAIN && grid > total_units) grid = total_units;  // the fused modes keep every CTA: their extra warps share the transfers
-
-  const int threads = p.mode == KB_GEMM_PLAIN ? THREADS_BASE : THREADS_COMM;
-  const void* fns[2][2][3] = {
-      {{(const void*)gemm_kernel<KB_GEMM_PLAIN, false, false>, nullptr, (const void*)gemm_kernel<KB_GEMM_AG, false, false>},
-       {(const void*)gemm_kernel<KB_GEMM_PLAIN, false, true>, (const void*)gemm_kernel<KB_GEMM_RS, false, true>,
-        (const void*)gemm_kernel<KB_GEMM_AG, false, true>}},
-      {{(const void*)gemm_kernel<KB_GEMM_PLAIN, true, false>, nullptr, (const void*)gemm_kernel<KB_GEMM_AG, true, false>},
-       {(const void*)gemm_kernel<KB_GEMM_PLAIN, true, true>, (const void*)gemm_kernel<KB_GEMM_RS, true, true>,
-        (const void*)gemm_kernel<KB_GEMM_AG, true, true>}}};
-  const void* fn = fns[pair ? 1 : 0][direct ? 1 : 0][p.mode];
+  // Every CTA is launched however few the tiles: the extra warps share the transfers.
+  const bool ag = a->mode == KB_GEMM_AG;
+  const void* fns[2][3] = {{(const void*)gemm_kernel<KB_GEMM_RS, false, true>, (const void*)gemm_kernel<KB_GEMM_AG, false, true>,
+                            (const void*)gemm_kernel<KB_GEMM_AG, false, false>},
+                           {(const void*)gemm_kernel<KB_GEMM_RS, true, true>, (const void*)gemm_kernel<KB_GEMM_AG, true, true>,
+                            (const void*)gemm_kernel<KB_GEMM_AG, true, false>}};
+  const int variant = !ag ? 0 : direct ? 1 : 2;
+  const void* fn = fns[pair ? 1 : 0][variant];
   {
-    static bool attr_set[64][2][2][3] = {};
-    if (dev < 0 || dev >= 64 || !attr_set[dev][pair ? 1 : 0][direct ? 1 : 0][p.mode]) {
+    static bool attr_set[64][2][3] = {};
+    if (dev < 0 || dev >= 64 || !attr_set[dev][pair ? 1 : 0][variant]) {
       KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      if (dev >= 0 && dev < 64) attr_set[dev][pair ? 1 : 0][direct ? 1 : 0][p.mode] = true;
+      if (dev >= 0 && dev < 64) attr_set[dev][pair ? 1 : 0][variant] = true;
     }
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
+  cfg.blockDim = dim3(THREADS_COMM);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from ..ops.dispatch_combine import MoEAllToAll
-from ..ops.gemm import gemm
+from ..ops.local import ROW_ALIGN, ExpertRows, contract_product, rows_product
 
 
 class MoELayer:
@@ -31,20 +31,20 @@ class MoELayer:
         a2a = self.a2a
         if not x.is_cuda and not a2a.host_heap:
             return self._dense(x, indices, weights)
+        if _all_local(a2a, x):
+            a2a._validate(x, indices, weights)
+            er = ExpertRows(x, indices, a2a.E, status=a2a.status)
+            h = rows_product(er.rows, self.w_up, er.start, er.count, act="silu")
+            return er.combine(rows_product(h, self.w_down, er.start, er.count), weights)
         counts, recv = a2a.dispatch(x, indices)
-        # the segment lengths size the GEMMs (one sync per layer call); the rows of
+        # the segment lengths size the buffers (one sync per layer call); the rows of
         # one expert, from all sources, are gathered into one block per expert
         rows_idx, n_e = _expert_major_rows(counts.cpu(), a2a.cap)
         rows_idx = rows_idx.to(x.device)
+        start, count, _, _ = _group_table(n_e, 1, x.device)
         X = recv.view(-1, a2a.H)[rows_idx]
-        Y = torch.empty_like(X)
-        o = 0
-        for le, n in enumerate(n_e):
-            if n:
-                h = torch.nn.functional.silu(_gemm(X[o:o + n], self.w_up[le]))
-                gemm(h, self.w_down[le], out=Y[o:o + n], pair=False)
-            o += n
-        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = Y
+        h = rows_product(X, self.w_up, start, count, act="silu")
+        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = rows_product(h, self.w_down, start, count)
         return a2a.combine(x, indices, weights)
 
     def _dense(self, x, indices, weights) -> torch.Tensor:
@@ -78,26 +78,55 @@ def _expert_major_rows(counts_h: torch.Tensor, cap: int):
     return idx, c.sum(0).tolist()
 
 
-def _pad8_t(rows: torch.Tensor) -> torch.Tensor:
-    """``rows[n, A]`` -> contiguous ``[A, n8]`` (n rounded up to a multiple of 8 with
-    zero columns): the K-major operand layout of the GEMM kernel, whose K must be a
-    multiple of 8."""
-    n, A = rows.shape
-    n8 = (n + 7) // 8 * 8
-    out = rows.new_zeros((A, n8))
-    out[:, :n] = rows.t()
-    return out
+def _all_local(a2a: MoEAllToAll, x: torch.Tensor) -> bool:
+    """One rank on a GPU: no row leaves it, so the layer permutes rows instead of
+    sending them, and no count has to reach the host."""
+    return x.is_cuda and a2a.world == 1
 
 
-def _gemm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
-    """GEMMs whose row or reduction count is a per-step token count: a fixed tile
-    configuration instead of the per-shape tuning of ``gemm`` (which would time
-    both configurations again for every new count)."""
-    return gemm(a, b, pair=False)
+def _group_table(n_e, pad: int, device):
+    """Group table of compact expert-major rows with each expert padded to a multiple of
+    ``pad``: ``(start, padded count, positions of the real rows, total rows)``."""
+    n = torch.tensor(n_e, dtype=torch.long)
+    padded = (n + pad - 1) // pad * pad
+    start = padded.cumsum(0) - padded
+    first = n.cumsum(0) - n
+    pos = torch.repeat_interleave(start - first, n) + torch.arange(int(n.sum()))
+    return (start.to(torch.int32).to(device), padded.to(torch.int32).to(device), pos.to(device), int(padded.sum()))
+
+
+class _LocalMoEFn(torch.autograd.Function):
+    """The block on one GPU: eight launches forward and backward together besides the
+    two of the combine passes, none of which waits for the host.  Experts start at
+    multiples of 64 rows with zero rows in between, so the weight gradients can
+    contract over whole k blocks."""
+
+    @staticmethod
+    def forward(ctx, x, weights, w_up, w_down, layer, indices):
+        a2a = layer.a2a
+        a2a._validate(x, indices, weights)
+        er = ExpertRows(x, indices, a2a.E, pad=ROW_ALIGN, status=a2a.status)
+        pre = torch.empty((er.rows.shape[0], w_up.shape[1]), dtype=x.dtype, device=x.device)
+        h = rows_product(er.rows, w_up, er.start, er.padded, act="silu", pre_out=pre)
+        Y = rows_product(h, w_down, er.start, er.padded)
+        ctx.er = er
+        ctx.save_for_backward(weights, w_up, w_down, pre, h, Y)
+        return er.combine(Y, weights)
+
+    @staticmethod
+    def backward(ctx, dy):
+        er = ctx.er
+        weights, w_up, w_down, pre, h, Y = ctx.saved_tensors
+        dYs, dweights = er.grad_rows(dy.contiguous(), Y, weights)
+        dpre = rows_product(dYs, w_down, er.start, er.padded, b_t=True, act="silu", pre_in=pre)
+        dw_down = contract_product(dYs, h, er.start, er.count)
+        dw_up = contract_product(dpre, er.rows, er.start, er.count)
+        dX = rows_product(dpre, w_up, er.start, er.padded, b_t=True)
+        return er.combine(dX, None), dweights, dw_up, dw_down, None, None
 
 
 class _MoEFn(torch.autograd.Function):
-    """Expert-parallel MoE block with a backward pass built from the same two
+    """Expert-parallel MoE block with a backward pass built from the same two exchange
     kernels: the gradient of combine is a dispatch (of ``dy``) and the gradient of
     dispatch is a combine (of the experts' input gradients, with unit weights).
     The routing weight of every received row, which the expert-side gradients
@@ -111,25 +140,22 @@ class _MoEFn(torch.autograd.Function):
         counts, recv = a2a.dispatch(x, indices)
         rows_idx_h, n_e = _expert_major_rows(counts.cpu(), a2a.cap)
         rows_idx = rows_idx_h.to(x.device)
-        X = recv.view(-1, a2a.H)[rows_idx]                              # expert-major copy of the received rows
-        pre = torch.empty((X.shape[0], w_up.shape[1]), dtype=x.dtype, device=x.device)
-        Y = torch.empty_like(X)
-        o = 0
-        for le, n in enumerate(n_e):
-            if n:
-                pre[o:o + n] = _gemm(X[o:o + n], w_up[le])
-                Y[o:o + n] = _gemm(torch.nn.functional.silu(pre[o:o + n]), w_down[le])
-            o += n
-        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = Y
+        start, padded, pos, total = _group_table(n_e, ROW_ALIGN, x.device)
+        X = torch.zeros((total, a2a.H), dtype=x.dtype, device=x.device)
+        X[pos] = recv.view(-1, a2a.H)[rows_idx]                         # expert-major copy of the received rows
+        pre = torch.empty((total, w_up.shape[1]), dtype=x.dtype, device=x.device)
+        h = rows_product(X, w_up, start, padded, act="silu", pre_out=pre)
+        Y = rows_product(h, w_down, start, padded)
+        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = Y[pos]
         out = a2a.combine(x, indices, weights)
         ctx.layer, ctx.n_e = layer, n_e
-        ctx.save_for_backward(indices, weights, w_up, w_down, X, pre, Y, rows_idx)
+        ctx.save_for_backward(indices, weights, w_up, w_down, X, pre, h, Y, rows_idx, start, padded, pos)
         return out
 
     @staticmethod
     def backward(ctx, dy):
         layer, n_e = ctx.layer, ctx.n_e
-        indices, weights, w_up, w_down, X, pre, Y, rows_idx = ctx.saved_tensors
+        indices, weights, w_up, w_down, X, pre, h, Y, rows_idx, start, padded, pos = ctx.saved_tensors
         a2a, meta = layer.a2a, layer.meta
         k, dev = a2a.k, dy.device
         dy = dy.contiguous()
@@ -146,30 +172,20 @@ class _MoEFn(torch.autograd.Function):
         j = (M[:, k:2 * k] == row_expert.unsqueeze(1).float()).float().argmax(1)   # which of the token's k choices this row is
         w_row = M.gather(1, j.unsqueeze(1))                                        # its routing weight
         # d weights[t, j] = <dy[t], y_row>: returned as one-hot rows, summed over k by a unit-weight combine
-        g = (dYr.float() * Y.float()).sum(1, keepdim=True)
+        g = (dYr.float() * Y[pos].float()).sum(1, keepdim=True)
         back = torch.zeros((M.shape[0], meta.H), dtype=torch.float32, device=dev)
         back.scatter_(1, j.unsqueeze(1), g)
         meta.expert_output_buffer().view(-1, meta.H)[rows_idx] = back
         ones = torch.ones((T, k), dtype=torch.float32, device=dev)
         dweights = meta.combine(info, indices, ones)[:, :k].contiguous()
         # expert backward on dY = w_row * dy
-        dYs = (dYr.float() * w_row).to(dy.dtype)
-        dX = torch.empty_like(X)
-        dw_up, dw_down = torch.zeros_like(w_up), torch.zeros_like(w_down)
-        o = 0
-        for le, n in enumerate(n_e):
-            if n:
-                sl = slice(o, o + n)
-                p32 = pre[sl].float()
-                sig = torch.sigmoid(p32)
-                h = (p32 * sig).to(dy.dtype)
-                dw_down[le] = _gemm(_pad8_t(dYs[sl]), _pad8_t(h))                     # [H, F]
-                dh = _gemm(dYs[sl], w_down[le].t().contiguous())                      # [n, F]
-                dpre = (dh.float() * (sig * (1 + p32 * (1 - sig)))).to(dy.dtype)
-                dw_up[le] = _gemm(_pad8_t(dpre), _pad8_t(X[sl]))                      # [F, H]
-                dX[sl] = _gemm(dpre, w_up[le].t().contiguous())                       # [n, H]
-            o += n
-        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = dX
+        dYs = torch.zeros_like(Y)
+        dYs[pos] = (dYr.float() * w_row).to(dy.dtype)
+        dpre = rows_product(dYs, w_down, start, padded, b_t=True, act="silu", pre_in=pre)
+        dw_down = contract_product(dYs, h, start, padded)
+        dw_up = contract_product(dpre, X, start, padded)
+        dX = rows_product(dpre, w_up, start, padded, b_t=True)
+        a2a.expert_output_buffer().view(-1, a2a.H)[rows_idx] = dX[pos]
         dx = a2a.combine(dy, indices, ones)
         return dx, dweights, dw_up, dw_down, None, None
 
@@ -178,8 +194,8 @@ class TrainableMoELayer(torch.nn.Module):
     """``MoELayer`` with parameters and a backward pass (see ``_MoEFn``).  Gradients
     flow to the tokens, the routing weights and both expert matrices; every GEMM of
     both passes is the tcgen05 kernel and every exchange one of the two fused
-    all-to-all kernels.  ``forward`` synchronises with the host once (the segment
-    lengths size the GEMMs)."""
+    all-to-all kernels.  With several ranks ``forward`` synchronises with the host once
+    (the segment lengths size the buffers); on one GPU it does not."""
 
     def __init__(self, num_experts: int, topk: int, hidden: int, ffn: int, max_tokens: int, group=None, device=None):
         super().__init__()
@@ -194,7 +210,8 @@ class TrainableMoELayer(torch.nn.Module):
         torch.nn.init.normal_(self.w_down, std=ffn ** -0.5)
 
     def forward(self, x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor) -> torch.Tensor:
-        return _MoEFn.apply(x, weights, self.w_up, self.w_down, self, indices)
+        fn = _LocalMoEFn if _all_local(self.a2a, x) else _MoEFn
+        return fn.apply(x, weights, self.w_up, self.w_down, self, indices)
 
     def close(self) -> None:
         for c in (self.a2a, self.meta):

@@ -41,6 +41,38 @@ def _launch(args: N.GemmArgs, device: torch.device) -> None:
     launch_count += 1
 
 
+def _local_args(status: Optional[torch.Tensor]) -> N.LocalGemmArgs:
+    """Argument block of a product whose operands are all on this GPU."""
+    args = N.LocalGemmArgs()
+    args.kind, args.pair, args.bias_scale = N.LOCAL_DENSE, -1, 1.0
+    args.status = status.data_ptr() if status is not None else None
+    args.wait_limit_ns = _WAIT_LIMIT_NS
+    return args
+
+
+def _launch_local(args: N.LocalGemmArgs, device: torch.device) -> None:
+    global launch_count
+    index = device.index
+    code = N.lib().kb_gemm_local(C.byref(args), torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index))
+    if code:
+        N.check(code)
+    launch_count += 1
+
+
+def _run_local(ctx, a: torch.Tensor, w: torch.Tensor, bias, bias_scale: float, out: torch.Tensor) -> torch.Tensor:
+    """The fused ops on one rank: nothing to exchange, a dense product.  The argument
+    block is kept with the context; a call refreshes what changes."""
+    args = ctx._hot
+    if args is None:
+        args = ctx._hot = _local_args(ctx.status)
+    (args.M, args.K), args.N = a.shape, out.shape[1]
+    args.A, args.B, args.out = a.data_ptr(), w.data_ptr(), out.data_ptr()
+    args.bias = bias.data_ptr() if bias is not None else None
+    args.bias_scale = bias_scale
+    _launch_local(args, a.device)
+    return out
+
+
 def _cpu_heap_path() -> bool:
     """CPU ranks run the kernels' protocol over a memfd-backed symmetric heap
     (``csrc/symm/gemm_host.cpp``) unless ``KB200_GEMM_CPU_PATH=collectives`` selects
@@ -76,44 +108,6 @@ def _host_args(ctx, mode: int, M: int, Nn: int, K: int, a, w, bias, bias_scale: 
 def _rows_bad(rpo: int) -> bool:
     """The tile schedule needs the rows per rank to divide, or be a multiple of, the 128-row block."""
     return rpo <= 0 or (rpo % 128 != 0 and 128 % rpo != 0)
-
-
-_NO_PAIR_BIT = 1 << 30
-_pair_choice: dict = {}  # (M, N, K) -> True if the CTA-pair kernel is the faster one on this device
-
-
-def _tuned_pair(args: N.GemmArgs, device: torch.device) -> bool:
-    """Single-rank calls pick between the two tile configurations by timing both
-    once per shape (three alternating launches each, CUDA events); which one wins depends on
-    the shape (pairs win at K around 4096, the single-CTA kernel at very large K)."""
-    key = (args.M, args.N, args.K)
-    hit = _pair_choice.get(key)
-    if hit is not None:
-        return hit
-    if args.M < 256 or os.environ.get("KB200_GEMM_NO_PAIR") == "1":
-        _pair_choice[key] = False
-        return False
-    base = args.num_ctas & ~_NO_PAIR_BIT
-    times = {True: 0.0, False: 0.0}
-
-    def run(use_pair: bool) -> None:
-        args.num_ctas = base | (0 if use_pair else _NO_PAIR_BIT)
-        _launch(args, device)
-
-    for use_pair in (True, False, True, False):  # warm up both; the clocks settle under load
-        run(use_pair)
-    # Alternate the two so that neither is measured on a cooler, faster-clocked GPU.
-    for _ in range(3):
-        for use_pair in (True, False):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            run(use_pair)
-            e1.record()
-            e1.synchronize()
-            times[use_pair] += e0.elapsed_time(e1)
-    args.num_ctas = base
-    _pair_choice[key] = times[True] <= times[False]
-    return _pair_choice[key]
 
 
 class _HostPipeline:
@@ -185,8 +179,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
     """``out[M,N] = a[M,K] @ b[N,K]^T (+ bias_scale * bias)`` in bf16 with fp32 accumulation.
 
     ``pair=True`` uses clusters of two CTAs sharing 256x256 tiles (``cta_group::2``,
-    M >= 256), ``pair=False`` the single-CTA 128x256 kernel, ``None`` times both
-    once per shape and keeps the faster."""
+    more than 128 rows), ``pair=False`` tiles of one CTA, ``None`` lets the launcher pick
+    the tile shape from the sizes (``choose_config`` in ``csrc/kernels/gemm_local.cu``)."""
     _check_bf16_2d(a, "a")
     _check_bf16_2d(b, "b")
     M, K = a.shape
@@ -204,20 +198,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
         return res
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
-    args = N.GemmArgs()
-    args.mode = N.GEMM_PLAIN
+    args = _local_args(status)
     args.M, args.N, args.K = M, Nn, K
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     args.bias = bias.data_ptr() if bias is not None else None
     args.bias_scale = bias_scale
-    args.rank, args.world, args.epoch = 0, 1, 1
-    args.status = status.data_ptr() if status is not None else None
-    args.wait_limit_ns = _WAIT_LIMIT_NS
     args.num_ctas = num_ctas
-    if pair is None:
-        pair = _tuned_pair(args, a.device)
-    args.num_ctas = num_ctas | (0 if pair else _NO_PAIR_BIT)
-    _launch(args, a.device)
+    args.pair = -1 if pair is None else int(pair)
+    _launch_local(args, a.device)
     return out
 
 
@@ -285,6 +273,8 @@ class GemmRS:
         if out is None:
             out = torch.empty((rows, self.N), dtype=torch.bfloat16, device=a.device)
         self.epoch += 1
+        if self.world == 1:
+            return _run_local(self, a, w, bias, bias_scale, out)
         args = self._hot
         if args is None:  # built once; calls only refresh pointers, K and the epoch
             args = self._hot = N.GemmArgs()
@@ -302,9 +292,6 @@ class GemmRS:
         args.bias = bias.data_ptr() if bias is not None else None
         args.bias_scale = bias_scale
         args.epoch = self.epoch
-        if self.world == 1:
-            args.num_ctas = 0
-            args.num_ctas = 0 if _tuned_pair(args, a.device) else _NO_PAIR_BIT
         _launch(args, a.device)
         return out
 
@@ -441,6 +428,8 @@ class AGGemm:
         if out is None:
             out = torch.empty((self.M, Nl), dtype=torch.bfloat16, device=a_local.device)
         self.epoch += 1
+        if self.world == 1:
+            return _run_local(self, a_local, w, bias, 1.0, out)
         args = self._hot
         if args is None:
             args = self._hot = N.GemmArgs()
@@ -458,9 +447,6 @@ class AGGemm:
         args.A, args.B, args.out = a_local.data_ptr(), w.data_ptr(), out.data_ptr()
         args.bias = bias.data_ptr() if bias is not None else None
         args.epoch = self.epoch
-        if self.world == 1:
-            args.num_ctas = 0
-            args.num_ctas = 0 if _tuned_pair(args, a_local.device) else _NO_PAIR_BIT
         _launch(args, a_local.device)
         return out
 

@@ -1,0 +1,178 @@
+"""Products whose operands are all on this GPU, and the row movement of a MoE layer
+whose experts are all on this GPU: front-ends of ``csrc/kernels/gemm_local.cu`` and
+``csrc/kernels/moe_rows.cu``.
+
+``product`` is the dense one; an operand may be given transposed (``a_t``, ``b_t``),
+which the kernel reads as it lies in memory.  ``rows_product`` multiplies groups of
+rows by their group's own matrix, ``contract_product`` contracts over the rows of each
+group (weight gradients); both take the group table from device memory.  CPU tensors
+take a plain fp32 torch formulation with the same rounding points, so that the layers
+built on them are testable without a GPU.
+"""
+from __future__ import annotations
+
+import ctypes as C
+from typing import Optional
+
+import torch
+
+from .. import _native as N
+
+ROW_ALIGN = 64  # rows of a group in a table made for contract_product start at multiples of the kernel's k block
+
+_ACTS = {
+    "gelu": lambda x: torch.nn.functional.gelu(x, approximate="tanh"),
+    "relu": torch.relu,
+    "silu": torch.nn.functional.silu,
+}
+
+
+def _slope(act: str, pre: torch.Tensor) -> torch.Tensor:
+    with torch.enable_grad():
+        x = pre.float().detach().requires_grad_(True)
+        return torch.autograd.grad(_ACTS[act](x).sum(), x)[0]
+
+
+def _finish(res: torch.Tensor, act, pre_out, pre_in, out) -> torch.Tensor:
+    """The kernel's epilogue on an fp32 product."""
+    if pre_in is not None:
+        res = (res * _slope(act, pre_in)).to(torch.bfloat16)
+    else:
+        res = res.to(torch.bfloat16)
+        if pre_out is not None:
+            pre_out.copy_(res)
+        if act is not None:
+            res = _ACTS[act](res.float()).to(torch.bfloat16)
+    if out is None:
+        return res
+    out.copy_(res)
+    return out
+
+
+def _ptr(t: Optional[torch.Tensor]):
+    return t.data_ptr() if t is not None else None
+
+
+def _stream(device: torch.device) -> int:
+    return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
+
+
+def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
+    from . import gemm as G  # launch accounting of the GEMM front-ends
+
+    code = N.lib().kb_gemm_local(C.byref(args), _stream(device))
+    if code:
+        N.check(code)
+    G.launch_count += 1
+
+
+def product(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = False, act: Optional[str] = None,
+            pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
+            out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``A @ B^T`` in bf16 with fp32 accumulation, ``A`` being ``a[M, K]`` (``a_t``: ``a[K, M]``)
+    and ``B`` being ``b[N, K]`` (``b_t``: ``b[K, N]``); ``a_t`` needs ``b_t``.
+
+    ``act``: the activation of the rounded product, which ``pre_out`` also receives;
+    with ``pre_in`` the product is multiplied by the activation's slope there."""
+    K, M = a.shape if a_t else a.shape[::-1]
+    Nn = b.shape[1] if b_t else b.shape[0]
+    if not a.is_cuda:
+        A, B = a.float(), b.float()
+        return _finish((A.t() if a_t else A) @ (B if b_t else B.t()), act, pre_out, pre_in, out)
+    if out is None:
+        out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
+    args = N.LocalGemmArgs()
+    args.kind, args.M, args.N, args.K = N.LOCAL_DENSE, M, Nn, K
+    args.a_mn, args.b_mn = a_t, b_t
+    args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    args.act, args.pre_out, args.pre_in = N.ACTS[act], _ptr(pre_out), _ptr(pre_in)
+    args.pair = -1
+    _launch(args, a.device)
+    return out
+
+
+def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor, *, b_t: bool = False,
+                 act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
+                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Rows ``start[e] .. start[e] + count[e]`` of ``a[R, K]`` times ``b[e]`` transposed
+    (``b[E, N, K]``, ``b_t``: ``b[E, K, N]``).  Rows outside every group are left alone."""
+    R, K = a.shape
+    E = b.shape[0]
+    Nn = b.shape[2] if b_t else b.shape[1]
+    if out is None:
+        out = torch.empty((R, Nn), dtype=torch.bfloat16, device=a.device)
+    if R == 0:
+        return out
+    if not a.is_cuda:
+        for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+            if n:
+                B = b[e].float()
+                sl = slice(s, s + n)
+                _finish(a[sl].float() @ (B if b_t else B.t()), act, None if pre_out is None else pre_out[sl],
+                        None if pre_in is None else pre_in[sl], out[sl])
+        return out
+    args = N.LocalGemmArgs()
+    args.kind, args.M, args.N, args.K = N.LOCAL_ROWS, R, Nn, K
+    args.b_mn, args.groups = b_t, E
+    args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
+    args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    args.act, args.pre_out, args.pre_in = N.ACTS[act], _ptr(pre_out), _ptr(pre_in)
+    args.pair = -1
+    _launch(args, a.device)
+    return out
+
+
+def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor) -> torch.Tensor:
+    """``out[e] = a[rows of e]^T @ b[rows of e]`` for ``a[R, M]``, ``b[R, N]``.  Groups start at
+    multiples of ``ROW_ALIGN``; rows between a group's last and the next multiple are
+    zero in one operand and finite in the other."""
+    (R, M), Nn, E = a.shape, b.shape[1], start.shape[0]
+    if not a.is_cuda or R == 0:
+        out = torch.zeros((E, M, Nn), dtype=torch.bfloat16, device=a.device)
+        for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+            out[e] = (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)
+        return out
+    out = torch.empty((E, M, Nn), dtype=torch.bfloat16, device=a.device)
+    args = N.LocalGemmArgs()
+    args.kind, args.M, args.N, args.K = N.LOCAL_CONTRACT, M, Nn, R
+    args.groups = E
+    args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
+    args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    args.pair = -1
+    _launch(args, a.device)
+    return out
+
+
+class ExpertRows:
+    """Expert-major copies of a batch's token rows on one GPU, one row per (token, choice).
+
+    ``rows[R, H]``; group table ``start``, ``count`` (``padded``: count rounded up to
+    ``pad`` rows, zero rows in between); ``slots[T, k]`` maps a choice to its row.
+    ``R`` is the capacity ``T * k + E * (pad - 1)``: no count travels to the host."""
+
+    def __init__(self, x: torch.Tensor, indices: torch.Tensor, experts: int, pad: int = 1, status: Optional[torch.Tensor] = None):
+        (T, H), k, dev = x.shape, indices.shape[1], x.device
+        self.T, self.k, self.E, self.H = T, k, experts, H
+        self.rows = torch.empty((T * k + experts * (pad - 1), H), dtype=torch.bfloat16, device=dev)
+        table = torch.empty(3 * experts + T * k, dtype=torch.int32, device=dev)
+        self.start, self.count, self.padded = table[:experts], table[experts:2 * experts], table[2 * experts:3 * experts]
+        self.slots = table[3 * experts:].view(T, k)
+        N.check(N.lib().kb_moe_permute(x.data_ptr(), indices.data_ptr(), T, k, experts, H, pad, self.rows.data_ptr(),
+                                       self.slots.data_ptr(), self.start.data_ptr(), self.count.data_ptr(), self.padded.data_ptr(),
+                                       _ptr(status), _stream(dev)))
+
+    def combine(self, y: torch.Tensor, weights: Optional[torch.Tensor]) -> torch.Tensor:
+        """``out[t] = sum_j weights[t, j] * y[slots[t, j]]`` (``None``: unit weights)."""
+        out = torch.empty((self.T, self.H), dtype=torch.bfloat16, device=y.device)
+        N.check(N.lib().kb_moe_combine(y.data_ptr(), self.slots.data_ptr(), _ptr(weights), self.T, self.k, self.H, out.data_ptr(),
+                                       _stream(y.device)))
+        return out
+
+    def grad_rows(self, dy: torch.Tensor, y: torch.Tensor, weights: torch.Tensor):
+        """Backward of ``combine``: ``(dY rows, d weights)``."""
+        dyr = torch.empty_like(y)
+        dw = torch.empty((self.T, self.k), dtype=torch.float32, device=dy.device)
+        N.check(N.lib().kb_moe_grad_rows(dy.data_ptr(), y.data_ptr(), self.slots.data_ptr(), weights.data_ptr(), self.T, self.k, self.E,
+                                         self.H, dyr.data_ptr(), dw.data_ptr(), self.start.data_ptr(), self.count.data_ptr(),
+                                         self.padded.data_ptr(), _stream(dy.device)))
+        return dyr, dw
