@@ -684,6 +684,7 @@ __global__ void __launch_bounds__(A2A_THREADS) a2a_combine_kernel(const A2aParam
 
 #include "a2a_dedup.cuh"
 #include "a2a_ll.cuh"
+#include "a2a_local.cuh"
 
 // All three phases in one cooperative launch (every CTA is resident, so CTAs may
 // wait for one another).  The last CTA of the grid is the poller: it moves no
@@ -1035,6 +1036,14 @@ extern "C" int kb_a2a_round_trip(const KbA2aArgs* a, void* stream) {
   rc = fill_params(a, &p, sms);
   if (rc != KB_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // One rank: nothing to exchange.  A traced call runs the general kernel, whose phases the stamps describe.
+  if (p.world == 1 && p.trace == nullptr) {
+    switch (a->dtype) {
+      case 0: return launch_local<__nv_bfloat16>(p, sms, st);
+      case 1: return launch_local<__half>(p, sms, st);
+      case 2: return launch_local<float>(p, sms, st);
+    }
+  }
   // The choice must be the same on every rank, so it depends on the context's capacity, not on this call's tokens.
   if (p.ll_off != 0 && p.ll_tmax >= p.tmax && p.tmax <= LL_MAX_TOKENS && p.T <= p.ll_tmax) {
     switch (a->dtype) {

@@ -100,6 +100,7 @@ class MoEAllToAll:
             self._trace = None
             self._hot_args = None
             self._lib = lib
+            self._round_trip = lib.kb_a2a_round_trip
             if os.environ.get("KB200_TRACE", "0") == "1":
                 self.enable_trace()
 
@@ -154,12 +155,13 @@ class MoEAllToAll:
         return out
 
     def _validate(self, x, indices, weights) -> None:
-        T = x.shape[0]
-        if x.dtype != self.dtype or x.shape[1] != self.H or not x.is_contiguous():
+        T, H = x.shape
+        if x.dtype != self.dtype or H != self.H or not x.is_contiguous():
             raise ValueError("x must be contiguous [T, hidden] in the context dtype")
-        if indices.dtype != torch.int32 or tuple(indices.shape) != (T, self.k) or not indices.is_contiguous():
+        Tk = (T, self.k)  # a torch.Size compares equal to a tuple
+        if indices.dtype != torch.int32 or indices.shape != Tk or not indices.is_contiguous():
             raise ValueError("indices must be contiguous int32 [T, k]")
-        if weights is not None and (weights.dtype != torch.float32 or tuple(weights.shape) != (T, self.k) or not weights.is_contiguous()):
+        if weights is not None and (weights.dtype != torch.float32 or weights.shape != Tk or not weights.is_contiguous()):
             raise ValueError("weights must be contiguous float32 [T, k]")
         if T > self.max_tokens:
             raise ValueError("more tokens than max_num_tokens")
@@ -196,8 +198,8 @@ class MoEAllToAll:
         st = torch._C._cuda_getCurrentRawStream(self._dev_index)  # the raw handle, without building a Stream object
         lib = self._lib
         if self._fused:
-            code = lib.kb_a2a_round_trip(self._hot_ref, st)
-            if code == N.KB_OK:
+            code = self._round_trip(self._hot_ref, st)
+            if code == 0:
                 launch_count += 1
                 return out
             if code != N.KB_ERR_UNSUPPORTED:
