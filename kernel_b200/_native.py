@@ -157,7 +157,7 @@ def _declare(lib: C.CDLL) -> None:
         "kb_device_barrier": (i, [C.POINTER(vp), u64, i, i, u32, u64, vp, vp]),
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
         "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
-        "kb_gemm_local_config": (i, [i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
+        "kb_gemm_local_config": (i, [i, i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
         "kb_moe_permute": (i, [vp, vp, i, i, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
         "kb_moe_combine": (i, [vp, vp, vp, i, i, i, vp, vp]),
         "kb_moe_grad_rows": (i, [vp, vp, vp, vp, i, i, i, i, vp, vp, vp, vp, vp, vp]),

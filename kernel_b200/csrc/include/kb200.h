@@ -148,7 +148,7 @@ typedef struct KbLocalGemmArgs {
 } KbLocalGemmArgs;
 int kb_gemm_local(const KbLocalGemmArgs* args, void* stream);
 // The configuration kb_gemm_local picks for a dense product on `sms` SMs (tests of the rule).
-int kb_gemm_local_config(int M, int N, int K, int b_mn, int sms, int* pair, int* bn, int* split);
+int kb_gemm_local_config(int M, int N, int K, int a_mn, int b_mn, int sms, int* pair, int* bn, int* split);
 // The fused modes (RS, AG) run by a CPU rank over a KB_BACKEND_HOST heap: same
 // schedule, staging layouts, flags and rounding points as the kernel (symm/gemm_host.cpp).
 int kb_gemm_host(const KbGemmArgs* args, int timeout_ms);

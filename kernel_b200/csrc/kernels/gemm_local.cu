@@ -4,12 +4,17 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+#include <mutex>
+
 namespace {
 
 using namespace kbl;
 
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
 // bf16 tensor [d2][d1][d0], contiguous, d0 innermost.
-int make_tmap3(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box0, uint32_t box1, bool swizzle64) {
+int make_tmap3(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box0, uint32_t box1) {
   static auto encode = KB_DRV(cuTensorMapEncodeTiled);
   if (encode == nullptr) return KB_ERR_UNSUPPORTED;
   cuuint64_t dims[3] = {d0, d1, d2};
@@ -17,7 +22,7 @@ int make_tmap3(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint
   cuuint32_t box[3] = {box0, box1, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     kb::set_error("cuTensorMapEncodeTiled failed: CUresult %d (ptr %p dims %llu %llu %llu)", (int)r, ptr, (unsigned long long)d0,
@@ -42,13 +47,23 @@ const Env& env() {
   return e;
 }
 
-int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 struct Config {
   bool pair;
   int bn, split;
   bool tall = false;  // pair with 256 rows per CTA
 };
+
+// Ring stages of a configuration and whether the partial tiles of a split fit the ring.
+int ring_stages(int a_slot, int b_slot, int tables) {
+  const int n = (SMEM_MAX - 1024 - BAR_BYTES - tables) / (a_slot + b_slot);
+  return n > MAX_STAGES ? MAX_STAGES : n;
+}
+bool exchange_fits(int a_rows, bool pair, int bn, int split) {
+  const int a_slot = a_rows * BK * 2, b_slot = (pair ? bn / 2 : bn) * BK * 2;
+  const int slot_rows = pair ? 128 : ceil_div(a_rows, 32) * 32;
+  return ceil_div(bn / CHUNK_COLS, split) * (split - 1) * slot_rows * CHUNK_COLS * 4 <= ring_stages(a_slot, b_slot, 4) * (a_slot + b_slot);
+}
 
 // Columns a tile may have: multiples of 32; an operand that is contiguous along N
 // comes in boxes of 64 columns per CTA.
@@ -57,23 +72,55 @@ bool bn_ok(int bn, bool pair, bool b_mn) {
   return b_mn ? per_cta % 64 == 0 : bn % 32 == 0;
 }
 
-Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, int sms, int shape) {
-  (void)a_mn;
+// Clusters of 1 to 8 CTAs that are resident at a time ([0] unused).  Clusters do not
+// cross a group of SMs that share a GPC, so large ones leave SMs idle (148 SMs: 74
+// pairs, but 33 clusters of 4 and 15 of 8).
+struct Capacity {
+  int clusters[9];
+};
+
+// Picks the tile shape (one CTA, pair, 512-row pair), its columns and the split of K.
+//
+// Model of the kernel's time in ns, constants fitted to 190 shapes x all configurations
+// on a B200 (M 2 to 16000, N and K 1000 to 29000; all three operand layouts; launches
+// back to back in a graph): the picked configuration is 1.8 % slower than the best one
+// on average.
+//   k block   the tensor pipe needs 300 for 256 columns, tiles narrower than about 190
+//             columns do not get faster (the operands of a single CTA's MMAs take
+//             a third more shared-memory bandwidth); operand bytes arrive at 95 per ns
+//             and SM, a little slower in the many small boxes of M/N-contiguous tensors
+//   wave      2000 between the tiles of a CTA, the epilogue's last part is exposed
+//             once, with 512-row tiles (no second accumulator) in every wave
+//   split     one barrier more and the exchange of (split - 1) / split of a tile
+//   memory    everything read and written once at 6.5 TB/s
+// The configurations differ most where few tiles leave SMs idle: 64 x 7168 x 18432 takes
+// 114 us with 256-column tiles and no split (28 of 148 SMs), 48 with the pick; 256 x 4096 x 14336 76
+// and 33 us; 2048 x 2880 x 2880 39 and 32 us.  512-row tiles move 25 % fewer operand bytes
+// per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).
+Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape) {
   Config best = {false, 256, 1};
   double best_t = 1e30;
   const int KB = ceil_div(K, BK);
+  const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
   for (int s = 0; s < 3; ++s) {
-    if (shape >= 0 ? s != shape : s != 0 && M <= 128) continue;
+    if (shape >= 0 ? s != shape : s != 0 && (M <= 128 || cap.clusters[2] < 1)) continue;
     const bool pair = s > 0, tall = s == 2;
-    const int units = pair ? sms / 2 : sms;
+    const int rows = tall ? 256 : (!pair && !a_mn && M < 128) ? ceil_div(M, 8) * 8 : 128;  // rows of A per stage
     for (int bn = 64; bn <= 256; bn += 32) {
       if (!bn_ok(bn, pair, b_mn) || (tall && bn != 256)) continue;
-      const int tiles = ceil_div(M, 128 << s) * ceil_div(N, bn);
+      const double tiles = static_cast<double>(ceil_div(M, 128 << s)) * ceil_div(N, bn);
+      const double mma = 300.0 * (bn < 190 ? 190 : bn) / 256.0 * (tall ? 2.0 : pair ? 1.0 : 1.33);
+      const double load = 128.0 * (rows + (pair ? bn / 2 : bn)) / 95.0 * (b_mn ? 1.07 : 1.0);
+      const double k_block = mma > load ? mma : load;
+      const double epilogue = 2000.0 * bn / 256.0 * (tall ? 2.0 : 1.0);
       for (int split = 1; split <= (tall ? 1 : pair ? 4 : 8); ++split) {
-        if (split > 1 && (tiles * split > units || KB < 4 * split)) break;
-        const int waves = ceil_div(tiles * split, units);
-        const double kb_ns = (tall ? 2 : 1) * (290.0 * (bn < 96 ? 96 : bn) / 256.0 + (pair ? 0 : 20));
-        const double t = waves * (ceil_div(KB, split) * kb_ns) + 1500.0 + (split > 1 ? 2500.0 : 0.0);
+        const int units = cap.clusters[(pair ? 2 : 1) * split];
+        if (split > 1 && (tiles > units || KB < 4 * split || !exchange_fits(rows, pair, bn, split))) continue;
+        const double waves = units > 0 ? static_cast<double>((static_cast<long long>(tiles) + units - 1) / units) : 1e9;
+        double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 2000.0) + epilogue + (pair ? 1000.0 : 0.0);
+        if (tall) t += 1.25 * waves * epilogue;
+        if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
+        if (t < memory) t = memory;
         if (t < best_t) {
           best_t = t;
           best = {pair, bn, split, tall};
@@ -99,19 +146,116 @@ int device_info(int* dev_out, int* sms_out) {
   return KB_OK;
 }
 
-template <Kind kKind, bool kAMn, bool kBMn>
+// Without a device to ask: what a B200 reports, scaled.
+Capacity estimated_capacity(int sms) {
+  static const int on_148[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  Capacity c;
+  for (int i = 0; i < 9; ++i) c.clusters[i] = on_148[i] * sms / 148;
+  return c;
+}
+
+template <Kind kKind, bool kAMn, bool kBMn, Epi kEpi>
 const void* kernel_of(const Config& c) {
   if constexpr (kKind == DENSE) {
-    if (c.tall) return (const void*)gemm_local_kernel<kKind, true, kAMn, kBMn, 2>;
+    if (c.tall) return (const void*)gemm_local_kernel<kKind, true, kAMn, kBMn, 2, kEpi>;
   }
-  return c.pair ? (const void*)gemm_local_kernel<kKind, true, kAMn, kBMn, 1> : (const void*)gemm_local_kernel<kKind, false, kAMn, kBMn, 1>;
+  return c.pair ? (const void*)gemm_local_kernel<kKind, true, kAMn, kBMn, 1, kEpi>
+                : (const void*)gemm_local_kernel<kKind, false, kAMn, kBMn, 1, kEpi>;
+}
+
+// The kernels that exist: an activation follows a product whose weights are
+// contiguous along K (forward), a slope one whose weights are contiguous along N
+// (backward); row 3 * variant + epilogue of the attribute cache.
+const void* find_kernel(int kind, bool a_mn, bool b_mn, int epi, const Config& c, int* row) {
+  const int variant = kind == ROWS ? (b_mn ? 4 : 3) : kind == CONTRACT ? 5 : a_mn ? 2 : b_mn ? 1 : 0;
+  *row = 3 * variant + epi;
+  switch (*row) {
+    case 0: return kernel_of<DENSE, false, false, EPI_PLAIN>(c);
+    case 1: return kernel_of<DENSE, false, false, EPI_ACT>(c);
+    case 3: return kernel_of<DENSE, false, true, EPI_PLAIN>(c);
+    case 5: return kernel_of<DENSE, false, true, EPI_SLOPE>(c);
+    case 6: return kernel_of<DENSE, true, true, EPI_PLAIN>(c);
+    case 9: return kernel_of<ROWS, false, false, EPI_PLAIN>(c);
+    case 10: return kernel_of<ROWS, false, false, EPI_ACT>(c);
+    case 12: return kernel_of<ROWS, false, true, EPI_PLAIN>(c);
+    case 14: return kernel_of<ROWS, false, true, EPI_SLOPE>(c);
+    case 15: return kernel_of<CONTRACT, true, true, EPI_PLAIN>(c);
+  }
+  return nullptr;
 }
 
 }  // namespace
 
-extern "C" int kb_gemm_local_config(int M, int N, int K, int b_mn, int sms, int* pair, int* bn, int* split) {
+namespace {
+
+// Asked once per device.
+int device_capacity(int dev, int sms, Capacity* out) {
+  static Capacity cached_clusters[64];
+  static std::atomic<int> known[64];
+  const bool keep = dev >= 0 && dev < 64;
+  if (keep && known[dev].load(std::memory_order_acquire)) {
+    *out = cached_clusters[dev];
+    return KB_OK;
+  }
+  Capacity c = {{0, sms}};
+  const void* fn = (const void*)gemm_local_kernel<DENSE, false, false, false, 1, EPI_PLAIN>;
+  KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+  for (int size = 2; size <= 8; ++size) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(size * sms);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM_MAX;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    KB_CUDA_OK(cudaOccupancyMaxActiveClusters(&n, fn, &cfg));
+    c.clusters[size] = n;
+  }
+  if (keep) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!known[dev].load(std::memory_order_relaxed)) {
+      cached_clusters[dev] = c;
+      known[dev].store(1, std::memory_order_release);
+    }
+  }
+  *out = c;
+  return KB_OK;
+}
+
+// The choice depends on the sizes alone and a program calls with the same ones again
+// and again: a small table per thread remembers it (the search takes about 2 us).
+struct Remembered {
+  int M, N, K, key, dev;
+  Config c;
+};
+int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, Config* out) {
+  thread_local Remembered table[64] = {};
+  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+  const uint32_t h = (static_cast<uint32_t>(M) * 0x9e3779b1u) ^ (static_cast<uint32_t>(N) * 0x85ebca6bu) ^
+                     (static_cast<uint32_t>(K) * 0xc2b2ae35u) ^ static_cast<uint32_t>(key);
+  Remembered& e = table[(h ^ (h >> 15)) & 63u];
+  if (e.M != M || e.N != N || e.K != K || e.key != key || e.dev != dev) {
+    Capacity have;
+    const int rc = device_capacity(dev, sms, &have);
+    if (rc != KB_OK) return rc;
+    for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
+    e = {M, N, K, key, dev, choose_config(M, N, K, a_mn, b_mn, have, shape)};
+  }
+  *out = e.c;
+  return KB_OK;
+}
+
+}  // namespace
+
+extern "C" int kb_gemm_local_config(int M, int N, int K, int a_mn, int b_mn, int sms, int* pair, int* bn, int* split) {
   if (M <= 0 || N <= 0 || K <= 0 || sms < 2 || !pair || !bn || !split) return KB_ERR_ARG;
-  const Config c = choose_config(M, N, K, false, b_mn != 0, sms, -1);
+  const Config c = choose_config(M, N, K, a_mn != 0, b_mn != 0, estimated_capacity(sms), -1);
   *pair = c.tall ? 2 : c.pair ? 1 : 0;
   *bn = c.bn;
   *split = c.split;
@@ -142,6 +286,10 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     kb::set_error("kb_gemm_local: A contiguous along M is built only with B contiguous along N");
     return KB_ERR_UNSUPPORTED;
   }
+  if ((a->pre_in != nullptr || a->pre_out != nullptr) && a->act == KB_ACT_NONE) {
+    kb::set_error("kb_gemm_local: pre_in and pre_out belong to an activation");
+    return KB_ERR_ARG;
+  }
   auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) != 0; };
   if (a->A == nullptr || a->B == nullptr || a->out == nullptr || misaligned(a->A) || misaligned(a->B) || misaligned(a->out) ||
       misaligned(a->bias) || misaligned(a->pre_out) || misaligned(a->pre_in)) {
@@ -159,7 +307,8 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   Config c;
   if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    c = choose_config(a->M, a->N, a->K, a_mn, b_mn, cap, shape);
+    rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &c);
+    if (rc != KB_OK) return rc;
   } else {
     // Rows per group decide: with fewer than about 1.5 tiles of 256 rows per group a pair
     // would work mostly on padding.
@@ -204,23 +353,20 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.a_slot = p.a_rows * BK * 2;
   p.b_slot = (c.pair ? c.bn / 2 : c.bn) * BK * 2;
   const int tables = grouped ? (3 * groups + 1) * 4 : 4;
-  int stages = (SMEM_MAX - 1024 - EPI_BYTES - BAR_BYTES - tables) / (p.a_slot + p.b_slot);
-  if (stages > MAX_STAGES) stages = MAX_STAGES;
-  p.stages = stages;
+  p.stages = ring_stages(p.a_slot, p.b_slot, tables);
   // the last A slot is read up to 128 rows far: the B slots behind it cover that
   if (p.stages < 2 || p.stages * p.b_slot < 16384) {
     kb::set_error("kb_gemm_local: operand ring too small");
     return KB_ERR_ARG;
   }
-  if (c.split > 1) {
-    const int chunks = c.bn / CHUNK_COLS;
-    const int need = ceil_div(chunks, c.split) * (c.split - 1) * BM * CHUNK_COLS * 4;
-    if (need > p.stages * (p.a_slot + p.b_slot) + EPI_BYTES) {
-      kb::set_error("kb_gemm_local: partial tiles do not fit the operand ring");
-      return KB_ERR_ARG;
-    }
+  p.slot_rows = c.pair ? 128 : ceil_div(p.a_rows, 32) * 32;
+  if (c.split > 1 && !exchange_fits(p.a_rows, c.pair, c.bn, c.split)) {
+    kb::set_error("kb_gemm_local: partial tiles do not fit the operand ring");
+    return KB_ERR_ARG;
   }
-  p.box_cols = c.bn % 64 == 0 ? 64 : 32;
+  const int epi = a->pre_in != nullptr ? EPI_SLOPE : a->act != ACT_NONE ? EPI_ACT : EPI_PLAIN;
+  auto wide = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0; };
+  p.wide = a->N % 16 == 0 && wide(a->out) && wide(a->pre_out) ? 1 : 0;
   p.act = a->act;
   p.bias = static_cast<const bf16*>(a->bias);
   p.bias_scale = a->bias_scale;
@@ -233,19 +379,12 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.limit_ns = a->wait_limit_ns ? a->wait_limit_ns : 2000000000ull;
   p.timing = env().timing ? 1 : 0;
 
-  const uint64_t bz = a->kind == KB_LOCAL_ROWS ? groups : 1, oz = contract ? groups : 1;
-  rc = a_mn ? make_tmap3(&p.tmA, a->A, a->M, a->K, 1, 64, BK, false) : make_tmap3(&p.tmA, a->A, a->K, a->M, 1, BK, p.a_rows, false);
+  const uint64_t bz = a->kind == KB_LOCAL_ROWS ? groups : 1;
+  rc = a_mn ? make_tmap3(&p.tmA, a->A, a->M, a->K, 1, 64, BK) : make_tmap3(&p.tmA, a->A, a->K, a->M, 1, BK, p.a_rows);
   if (rc != KB_OK) return rc;
-  rc = b_mn ? make_tmap3(&p.tmB, a->B, a->N, a->K, bz, 64, BK, false)
-            : make_tmap3(&p.tmB, a->B, a->K, a->N, bz, BK, c.pair ? c.bn / 2 : c.bn, false);
+  rc = b_mn ? make_tmap3(&p.tmB, a->B, a->N, a->K, bz, 64, BK)
+            : make_tmap3(&p.tmB, a->B, a->K, a->N, bz, BK, c.pair ? c.bn / 2 : c.bn);
   if (rc != KB_OK) return rc;
-  rc = make_tmap3(&p.tmOut, a->out, a->N, a->M, oz, p.box_cols, BOX_ROWS, p.box_cols == 32);
-  if (rc != KB_OK) return rc;
-  if (p.pre_out != nullptr) {
-    rc = make_tmap3(&p.tmPre, a->pre_out, a->N, a->M, oz, p.box_cols, BOX_ROWS, p.box_cols == 32);
-    if (rc != KB_OK) return rc;
-  }
-
   const int cluster = (c.pair ? 2 : 1) * c.split;
   int grid;
   if (c.split > 1) {
@@ -257,21 +396,17 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     if (grid > blocks * p.NB * cluster) grid = static_cast<int>(blocks * p.NB * cluster);
   }
 
-  const int variant = a->kind == KB_LOCAL_ROWS ? (b_mn ? 4 : 3) : contract ? 5 : a_mn ? 2 : b_mn ? 1 : 0;
-  const void* fn = nullptr;
-  switch (variant) {
-    case 0: fn = kernel_of<DENSE, false, false>(c); break;
-    case 1: fn = kernel_of<DENSE, false, true>(c); break;
-    case 2: fn = kernel_of<DENSE, true, true>(c); break;
-    case 3: fn = kernel_of<ROWS, false, false>(c); break;
-    case 4: fn = kernel_of<ROWS, false, true>(c); break;
-    default: fn = kernel_of<CONTRACT, true, true>(c); break;
+  int kernel_row = 0;
+  const void* fn = find_kernel(a->kind, a_mn, b_mn, epi, c, &kernel_row);
+  if (fn == nullptr) {
+    kb::set_error("kb_gemm_local: no kernel for kind %d, layouts %d %d, epilogue %d", a->kind, (int)a_mn, (int)b_mn, epi);
+    return KB_ERR_UNSUPPORTED;
   }
-  const int attr_row = c.tall ? 2 : c.pair ? 1 : 0;
-  static bool attr_set[64][3][6] = {};
-  if (dev < 0 || dev >= 64 || !attr_set[dev][attr_row][variant]) {
+  const int shape_row = c.tall ? 2 : c.pair ? 1 : 0;
+  static bool attr_set[64][3][18] = {};
+  if (dev < 0 || dev >= 64 || !attr_set[dev][shape_row][kernel_row]) {
     KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-    if (dev >= 0 && dev < 64) attr_set[dev][attr_row][variant] = true;
+    if (dev >= 0 && dev < 64) attr_set[dev][shape_row][kernel_row] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);

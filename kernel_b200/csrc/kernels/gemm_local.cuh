@@ -14,7 +14,7 @@
 // descriptors of the MMA differ.
 //
 // Warp 0 is the TMA producer, warp 1 the MMA issuer, warp 2 owns the TMEM
-// allocation, warps 4 to 7 are the epilogue.  Two 256-column accumulators: the
+// allocation, warps 4 to 11 are the epilogue.  Two 256-column accumulators: the
 // epilogue of a tile runs under the mainloop of the next one.
 //
 // A tile has 128 rows (one CTA) or 256 rows (CTA pair, cta_group::2) and `bn`
@@ -45,22 +45,23 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int ACC_COLS = 256;  // TMEM columns of one accumulator
 constexpr int TMEM_COLS = 512;
-constexpr int THREADS = 256;
+constexpr int THREADS = 384;
+constexpr int EPI_WARPS = 8;  // two per TMEM lane quadrant
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_GROUPS = 1024;
-constexpr int BOX_ROWS = 32;
-constexpr int EPI_WARP_BYTES = 8192;  // two staging boxes of 32 rows x up to 64 columns
-constexpr int EPI_BYTES = 4 * EPI_WARP_BYTES;
 constexpr int BAR_BYTES = 256;
 constexpr int MN_BLOCK_BYTES = BK * 128;  // M/N-contiguous operand: one box of 64 k rows x 64 elements
 constexpr int SMEM_MAX = 232448;
 constexpr int CHUNK_COLS = 32;            // split: columns are exchanged in chunks of 32
 
 enum Kind { DENSE = 0, ROWS = 1, CONTRACT = 2 };
+// What the epilogue does besides the bias: nothing; the activation (runtime kind), with
+// the value before it kept if asked for; the product with the activation's slope.
+enum Epi { EPI_PLAIN = 0, EPI_ACT = 1, EPI_SLOPE = 2 };
 enum Act { ACT_NONE = 0, ACT_GELU = 1, ACT_RELU = 2, ACT_SILU = 3 };
 
 struct alignas(64) Params {
-  CUtensorMap tmA, tmB, tmOut, tmPre;
+  CUtensorMap tmA, tmB;
   int M, N, K;
   int MBQ, NB, KB;   // scheduling blocks (128 or 256 rows), column blocks, k blocks of the whole contraction
   int bn;            // tile columns
@@ -69,7 +70,8 @@ struct alignas(64) Params {
   int split;         // members of a cluster that share a tile
   int stages, a_slot, b_slot;  // operand ring: bytes per stage
   int a_rows;        // rows of A a stage brings in (128 per half, or fewer when M or the groups are smaller)
-  int box_cols;      // columns of an output box: 64, or 32 when bn is an odd multiple of 32
+  int slot_rows;     // split: rows of an exchange slot (128, or fewer when M is smaller)
+  int wide;          // rows of the output start at multiples of 32 bytes: whole-sector stores
   int act;           // applied to the rounded result, or, with pre_in, its derivative at pre_in
   const bf16* bias;
   float bias_scale;
@@ -109,59 +111,99 @@ __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.0f, 1.0f
 // tanh form of GELU: x * sigmoid(2u), u = sqrt(2/pi) * (x + 0.044715 x^3)
 constexpr float GELU_C = 2.0f * 0.7978845608028654f;
 constexpr float GELU_A = 0.044715f;
-__device__ __forceinline__ float act_value(int act, float x) {
-  if (act == ACT_GELU) return x * sigmoid(GELU_C * x * (1.0f + GELU_A * x * x));
-  if (act == ACT_SILU) return x * sigmoid(x);
-  return x < 0.0f ? 0.0f : x;
+template <int kAct>
+__device__ __forceinline__ float act_value(float x) {
+  if constexpr (kAct == ACT_GELU) return x * sigmoid(GELU_C * x * (1.0f + GELU_A * x * x));
+  else if constexpr (kAct == ACT_SILU) return x * sigmoid(x);
+  else return x < 0.0f ? 0.0f : x;
 }
-__device__ __forceinline__ float act_slope(int act, float x) {
-  if (act == ACT_GELU) {
+template <int kAct>
+__device__ __forceinline__ float act_slope(float x) {
+  if constexpr (kAct == ACT_GELU) {
     const float s = sigmoid(GELU_C * x * (1.0f + GELU_A * x * x));
     return s + x * s * (1.0f - s) * GELU_C * (1.0f + 3.0f * GELU_A * x * x);
-  }
-  if (act == ACT_SILU) {
+  } else if constexpr (kAct == ACT_SILU) {
     const float s = sigmoid(x);
     return s * (1.0f + x * (1.0f - s));
+  } else {
+    return x > 0.0f ? 1.0f : 0.0f;
   }
-  return x > 0.0f ? 1.0f : 0.0f;
+}
+template <int kAct>
+__device__ __forceinline__ void act32(const uint4* pre, uint4* out) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float s[8];
+    unpack8(pre[i], s);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = act_value<kAct>(s[e]);
+    out[i] = pack8(s);
+  }
+}
+template <int kAct>
+__device__ __forceinline__ void slope32(const uint4* at, float* f) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float s[8];
+    unpack8(at[i], s);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[8 * i + e] *= act_slope<kAct>(s[e]);
+  }
 }
 
-// Eight accumulator values of one row -> bf16: (+ bias, one rounding), then the
-// activation of the rounded value, or the product with the slope at `pre_in`.
-struct Out8 {
-  uint4 out, pre;
-};
-__device__ __forceinline__ Out8 finish8(const Params& p, const float* acc, int row, int col, bool live) {
-  float f[8];
+// 32 accumulator values of one row -> bf16: (+ bias, one rounding), then the activation
+// of the rounded value, or the product with the slope at `pre_in`.  A scheduler has two
+// epilogue warps at most, so latency counts: all loads of the 32 columns are issued
+// together and the arithmetic is straight-line, branches are taken once per 32 columns
+// (branching per 8 values cost 250 cycles each: 11000 cycles for a 128 x 256 tile).
+template <Epi kEpi>
+__device__ __forceinline__ void finish32(const Params& p, float* f, int row, int col, bool row_ok, uint4* out, uint4* pre) {
+  if (p.bias != nullptr) {
+    uint4 b[4];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) f[e] = acc[e];
-  if (p.bias != nullptr && col < p.N) {
-    float b[8];
-    unpack8(*reinterpret_cast<const uint4*>(p.bias + col), b);  // the same 16 bytes for every lane
+    for (int i = 0; i < 4; ++i) b[i] = col + 8 * i < p.N ? __ldg(reinterpret_cast<const uint4*>(p.bias + col) + i) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] += p.bias_scale * b[e];
+    for (int i = 0; i < 4; ++i) {
+      float t[8];
+      unpack8(b[i], t);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[8 * i + e] += p.bias_scale * t[e];
+    }
   }
-  Out8 o;
-  if (p.pre_in != nullptr) {
-    float s[8];
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (live) v = *reinterpret_cast<const uint4*>(p.pre_in + static_cast<size_t>(row) * p.N + col);
-    unpack8(v, s);
+  if constexpr (kEpi == EPI_SLOPE) {
+    uint4 at[4];
+    const uint4* src = reinterpret_cast<const uint4*>(p.pre_in + static_cast<size_t>(row) * p.N + col);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] *= act_slope(p.act, s[e]);
-    o.out = pack8(f);
-    return o;
+    for (int i = 0; i < 4; ++i) at[i] = row_ok && col + 8 * i < p.N ? src[i] : make_uint4(0, 0, 0, 0);
+    if (p.act == ACT_SILU) slope32<ACT_SILU>(at, f);
+    else if (p.act == ACT_GELU) slope32<ACT_GELU>(at, f);
+    else slope32<ACT_RELU>(at, f);
   }
-  o.pre = pack8(f);
-  o.out = o.pre;
-  if (p.act != ACT_NONE) {
-    float s[8];
-    unpack8(o.pre, s);
+  uint4* rounded = kEpi == EPI_ACT ? pre : out;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) s[e] = act_value(p.act, s[e]);
-    o.out = pack8(s);
+  for (int i = 0; i < 4; ++i) rounded[i] = pack8(f + 8 * i);
+  if constexpr (kEpi == EPI_ACT) {
+    if (p.act == ACT_SILU) act32<ACT_SILU>(pre, out);
+    else if (p.act == ACT_GELU) act32<ACT_GELU>(pre, out);
+    else act32<ACT_RELU>(pre, out);
   }
-  return o;
+}
+// 32 values of a lane's row, straight from the registers.  A lane's 32-byte store is a
+// whole L2 sector, so the 32 rows a warp touches per instruction cost no partial
+// writes; against staging through shared memory and TMA stores this saves a fence, a
+// store issue and the wait for the store engine to read the box (about 1000 cycles per
+// box with two epilogue warps per scheduler), and the staging memory is another
+// pipeline stage.
+__device__ __forceinline__ void store_row32(bf16* base, size_t at, int col, int n, bool wide, const uint4* v) {
+  if (wide && col + 32 <= n) {
+    kb::st_global_v8(base + at, v[0], v[1]);
+    kb::st_global_v8(base + at + 16, v[2], v[3]);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (col + 8 * i < n) *reinterpret_cast<uint4*>(base + at + 8 * i) = v[i];
+  }
 }
 
 // Shared-memory descriptor of an M/N-contiguous operand with the 128-byte swizzle:
@@ -179,21 +221,21 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 
 // kHalves: 128-row blocks per CTA and tile.  2 (pairs only): a 512-row tile whose two
 // halves fill both accumulators.
-template <Kind kKind, bool kPair, bool kAMn, bool kBMn, int kHalves>
+template <Kind kKind, bool kPair, bool kAMn, bool kBMn, int kHalves, Epi kEpi>
 __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sm_a = base;
   uint8_t* sm_b = sm_a + p.stages * p.a_slot;
-  uint8_t* sm_epi = sm_b + p.stages * p.b_slot;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sm_epi + EPI_BYTES);
+  uint8_t* sm_bar = sm_b + p.stages * p.b_slot;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm_bar);
   uint64_t* empty = full + MAX_STAGES;
   uint64_t* tfull = empty + MAX_STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   static_assert((2 * MAX_STAGES + 4) * 8 + 8 <= BAR_BYTES, "barrier block too small");
-  int32_t* pref = reinterpret_cast<int32_t*>(sm_epi + EPI_BYTES + BAR_BYTES);  // [groups + 1] row blocks before a group
+  int32_t* pref = reinterpret_cast<int32_t*>(sm_bar + BAR_BYTES);  // [groups + 1] row blocks before a group
   int32_t* g_start = pref + p.groups + 1;                                      // [groups]
   int32_t* g_count = g_start + p.groups;                                       // [groups]
 
@@ -215,17 +257,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
   const int block_rows = (kKind == ROWS && !kPair) ? p.a_rows : TILE_ROWS;
   const int b_cols = kPair ? p.bn / 2 : p.bn;  // columns of B this CTA stages
 
-  if (tid == 0) {
-    for (int s = 0; s < p.stages; ++s) {
-      kb::mbar_init(&full[s], 1);
-      kb::mbar_init(&empty[s], 1);
+  if (warp == 0) {
+    if (lane < p.stages) {
+      kb::mbar_init(&full[lane], 1);
+      kb::mbar_init(&empty[lane], 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      kb::mbar_init(&tfull[a], 1);
-      kb::mbar_init(&tempty[a], kPair ? 8 : 4);
+    if (lane < 2) {
+      kb::mbar_init(&tfull[lane], 1);
+      kb::mbar_init(&tempty[lane], kPair ? 2 * EPI_WARPS : EPI_WARPS);
     }
-    *abort_flag = 0;
+    if (lane == 0) *abort_flag = 0;
     kb::mbar_fence_init();
+    __syncwarp();
   }
   if (warp == 2) {
     if constexpr (kPair) {
@@ -239,7 +282,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
   if (warp == 3 && lane == 0) {
     kb::tma_prefetch_desc(&p.tmA);
     kb::tma_prefetch_desc(&p.tmB);
-    kb::tma_prefetch_desc(&p.tmOut);
   }
   if constexpr (kKind != DENSE) {
     for (int e = tid; e < p.groups; e += THREADS) {
@@ -266,11 +308,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       }
     }
   }
-  kb::tc_fence_before_sync();
-  __syncthreads();
-  if (kPair || p.split > 1) kb::cluster_sync_all();  // the other CTAs' barriers exist before anything signals them
-  kb::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  // A pair's CTAs signal each other's barriers: both must have initialised theirs.
+  // Otherwise the producer warp, which needs only the barriers it has just made,
+  // goes ahead: its first loads are under way while the tensor memory is allocated.
+  if constexpr (kPair) {
+    kb::tc_fence_before_sync();
+    __syncthreads();
+    kb::cluster_sync_all();
+    kb::tc_fence_after_sync();
+  } else if (kKind == DENSE && warp == 0) {
+    asm volatile("bar.arrive 1, %0;" ::"n"(THREADS) : "memory");
+  } else {
+    kb::tc_fence_before_sync();
+    if constexpr (kKind == DENSE) asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    else __syncthreads();
+    kb::tc_fence_after_sync();
+  }
+  const uint32_t tmem_base = (kPair || kKind != DENSE || warp != 0) ? *tmem_slot : 0u;
 
   const int total_tiles = kKind == DENSE ? p.MBQ * p.NB : kKind == ROWS ? pref[p.groups] * p.NB : p.groups * p.MBQ * p.NB;
 
@@ -451,94 +505,74 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     __syncwarp();
   } else if (warp >= 4 && p.split == 1) {
     // ---------------------------------------------------------- epilogue ----
-    const int q = warp - 4;
-    uint8_t* warp_epi = sm_epi + q * EPI_WARP_BYTES;
+    // Warps q and q + 4 of the role drain lane quadrant q, 64 columns in turn.
+    const int q = warp & 3;
+    const int turn = (warp - 4) >> 2;
     uint32_t it = 0;
-    int box = 0;  // next staging box
     for (int pos = sched_id; pos < total_tiles; pos += sched_n, ++it) {
       const Tile t = tile_at(pos);
+      const size_t out0 = kKind == CONTRACT ? static_cast<size_t>(t.group) * p.M * p.N : 0;
+      const int cols = min(p.bn, p.N - t.n0);
 #pragma unroll 1
       for (int hb = 0; hb < kHalves; ++hb) {
-      const uint32_t acc = kHalves == 2 ? static_cast<uint32_t>(hb) : it & 1u;
-      const uint32_t aph = (kHalves == 2 ? it : it >> 1) & 1u;
-      if (*abort_flag == 0 && !kb::mbar_wait_bounded(&tfull[acc], aph, p.limit_ns, 2000)) {
-        kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, SITE_TFULL, (uint32_t)pos, 0);
-        *abort_flag = 1;
-      }
-      kb::tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * ACC_COLS;
-      const int gr0 = t.row0 + hb * BM + q * 32;
-      const int row = gr0 + lane;
-      const bool row_ok = row < t.row_end;
-      // A box leaves through TMA unless it would reach into the next group's rows.
-      const bool tma_ok = kKind != ROWS || gr0 + BOX_ROWS <= t.row_end;
-      const int cols = min(p.bn, p.N - t.n0);
-      const int oz = kKind == CONTRACT ? t.group : 0;
-      if (gr0 < t.row_end) {
-#pragma unroll 1
-        for (int c = 0; c < cols; c += p.box_cols) {
-          const int col0 = t.n0 + c;
-          uint8_t* box_out = warp_epi + box * (EPI_WARP_BYTES / 2);
-          uint8_t* box_pre = warp_epi + (box ^ 1) * (EPI_WARP_BYTES / 2);
-          if (tma_ok) {  // the stores that last read the box(es) have finished reading
-            if (lane == 0) {
-              if (p.pre_out != nullptr) kb::bulk_wait_group_read<0>();
-              else kb::bulk_wait_group_read<1>();
-            }
-            __syncwarp();
-          }
-#pragma unroll 1
-          for (int h = 0; h < p.box_cols; h += 32) {
-            uint32_t r[32];
-            if (kKind == CONTRACT && t.kb == 0) {  // an empty group: nothing was accumulated
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
+        const uint32_t acc = kHalves == 2 ? static_cast<uint32_t>(hb) : it & 1u;
+        const uint32_t aph = (kHalves == 2 ? it : it >> 1) & 1u;
+        if (*abort_flag == 0 && !kb::mbar_wait_bounded(&tfull[acc], aph, p.limit_ns, 2000)) {
+          kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, SITE_TFULL, (uint32_t)pos, 0);
+          *abort_flag = 1;
+        }
+        kb::tc_fence_after_sync();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * ACC_COLS;
+        const int gr0 = t.row0 + hb * BM + q * 32;
+        const int row = gr0 + lane;
+        const bool row_ok = row < t.row_end;
+        auto release = [&]() {  // this warp has read its share of the accumulator
+          kb::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            if constexpr (kPair) {
+              if (leader) kb::mbar_arrive(&tempty[acc]);
+              else kb::mbar_arrive_cluster(kb::map_to_cta(kb::smem_u32(&tempty[acc]), lead));
             } else {
-              kb::tmem_ld_32x32(taddr + c + h, r);
-              kb::tmem_ld_wait();
+              kb::mbar_arrive(&tempty[acc]);
             }
+          }
+        };
+        const int last = gr0 < t.row_end ? cols : 0;
+        if (turn * 64 >= last) release();
+#pragma unroll 1
+        for (int c = turn * 64; c < last; c += 128) {
+          const bool two = c + 32 < last;
+          uint32_t r[2][32];
+          if (kKind == CONTRACT && t.kb == 0) {  // an empty group: nothing was accumulated
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int col = col0 + h + 8 * i;
-              const Out8 o = finish8(p, reinterpret_cast<const float*>(r) + 8 * i, row, col, row_ok && col < p.N);
-              if (tma_ok) {
-                // 16-byte chunk j of the row at position j ^ (row & 7) of its 128 bytes (64-byte rows: j ^ ((row / 2) & 3))
-                const int j = h / 8 + i;
-                const int at = p.box_cols == 64 ? lane * 128 + ((j ^ (lane & 7)) * 16) : lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16);
-                *reinterpret_cast<uint4*>(box_out + at) = o.out;
-                if (p.pre_out != nullptr) *reinterpret_cast<uint4*>(box_pre + at) = o.pre;
-              } else if (row_ok && col < p.N) {
-                const size_t at = static_cast<size_t>(row) * p.N + col;
-                *reinterpret_cast<uint4*>(p.out + at) = o.out;
-                if (p.pre_out != nullptr) *reinterpret_cast<uint4*>(p.pre_out + at) = o.pre;
+            for (int i = 0; i < 32; ++i) r[0][i] = r[1][i] = 0u;
+          } else {
+            kb::tmem_ld_32x32(taddr + c, r[0]);
+            if (two) kb::tmem_ld_32x32(taddr + c + 32, r[1]);
+            kb::tmem_ld_wait();
+          }
+          if (c + 128 >= last) release();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (h == 1 && !two) break;
+            float f[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[h][i]);
+            uint4 o[4], pre[4];
+            const int col = t.n0 + c + 32 * h;
+            finish32<kEpi>(p, f, row, col, row_ok, o, pre);
+            if (row_ok) {
+              const size_t at = out0 + static_cast<size_t>(row) * p.N + col;
+              store_row32(p.out, at, col, p.N, p.wide != 0, o);
+              if constexpr (kEpi == EPI_ACT) {
+                if (p.pre_out != nullptr) store_row32(p.pre_out, at, col, p.N, p.wide != 0, pre);
               }
             }
           }
-          if (tma_ok) {
-            kb::fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              kb::tma_store_3d(&p.tmOut, box_out, col0, gr0, oz);
-              if (p.pre_out != nullptr) kb::tma_store_3d(&p.tmPre, box_pre, col0, gr0, oz);
-              kb::bulk_commit_group();
-            }
-            box ^= 1;
-          }
         }
-      }
-      kb::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (kPair) {
-          if (leader) kb::mbar_arrive(&tempty[acc]);
-          else kb::mbar_arrive_cluster(kb::map_to_cta(kb::smem_u32(&tempty[acc]), lead));
-        } else {
-          kb::mbar_arrive(&tempty[acc]);
-        }
-      }
       }
     }
-    if (lane == 0) kb::bulk_wait_group<0>();  // the boxes are read and the output is written before the CTA leaves
   } else if (warp == 4 && p.split > 1) {
     // The members of a cluster work on one tile each: wait here until this CTA's partial is complete.
     if (!kb::mbar_wait_bounded(&tfull[0], 0u, p.limit_ns, 1000)) {
@@ -552,21 +586,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     if (p.split > 1) {
       // ------------------------------------------- exchange of the partials ----
       // Chunk c of 32 columns belongs to member c * split / chunks.  Slot (chunk,
-      // source) of the owner's operand ring holds 128 rows x 32 columns as
+      // source) of the owner's operand ring holds slot_rows x 32 columns as
       // [4-column group][row] float4: neighbouring lanes write neighbouring 16 bytes.
       __syncthreads();
       kb::cluster_sync_all();  // every member's MMAs have finished: all operand rings are free
       kb::tc_fence_after_sync();
+      const uint32_t tmem_base = *tmem_slot;  // the producer warp did not wait for it
       const Tile t = tile_at(sched_id);
       const int chunks = p.bn / CHUNK_COLS;
       const int q = warp & 3;            // TMEM lane quadrant of this warp
       const int gr0 = t.row0 + q * 32;
       const int row = gr0 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-      constexpr int SLOT = BM * CHUNK_COLS * 4;
+      const int slot_bytes = p.slot_rows * CHUNK_COLS * 4;
       const bool live = gr0 < t.row_end;
       if (live) {
-        for (int c = warp >> 2; c < chunks; c += 2) {
+        for (int c = warp >> 2; c < chunks; c += THREADS / 128) {
           const int owner = c * p.split / chunks;
           if (owner == member || t.n0 + c * CHUNK_COLS >= p.N) continue;
           const int first = (owner * chunks + p.split - 1) / p.split;  // the owner's first chunk
@@ -574,48 +609,50 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
           uint32_t r[32];
           kb::tmem_ld_32x32(taddr + c * CHUNK_COLS, r);
           kb::tmem_ld_wait();
-          const uint32_t to = kb::map_to_cta(kb::smem_u32(base + ((c - first) * (p.split - 1) + src) * SLOT),
+          const uint32_t to = kb::map_to_cta(kb::smem_u32(base + ((c - first) * (p.split - 1) + src) * slot_bytes),
                                              static_cast<uint32_t>(owner) * (kPair ? 2u : 1u) + half);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            kb::st_shared_cluster_v4(to + (i * BM + q * 32 + lane) * 16, r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+            kb::st_shared_cluster_v4(to + (i * p.slot_rows + q * 32 + lane) * 16, r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
           }
         }
       }
       kb::cluster_sync_all();  // the partials are in place
       if (live) {
-        for (int c = warp >> 2; c < chunks; c += 2) {
+        for (int c = warp >> 2; c < chunks; c += THREADS / 128) {
           const int col0 = t.n0 + c * CHUNK_COLS;
           if (c * p.split / chunks != member || col0 >= p.N) continue;
           const int first = (member * chunks + p.split - 1) / p.split;
           uint32_t r[32];
           kb::tmem_ld_32x32(taddr + c * CHUNK_COLS, r);
+          float f[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] = 0.f;
+          const uint32_t from = kb::smem_u32(base) + (q * 32 + lane) * 16;
           kb::tmem_ld_wait();
+#pragma unroll 1
+          for (int m = 0; m < p.split; ++m) {  // ascending member order
+            if (m == member) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float f[8];
+              for (int i = 0; i < 32; ++i) f[i] += __uint_as_float(r[i]);
+            } else {
+              const uint32_t slot = from + ((c - first) * (p.split - 1) + (m < member ? m : m - 1)) * slot_bytes;
+              float4 v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = 0.f;
-            for (int m = 0; m < p.split; ++m) {  // ascending member order
-              if (m == member) {
+              for (int i = 0; i < 8; ++i) v[i] = kb::ld_shared_v4(slot + i * p.slot_rows * 16);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] += __uint_as_float(r[8 * i + e]);
-                continue;
-              }
-              const uint8_t* slot = base + ((c - first) * (p.split - 1) + (m < member ? m : m - 1)) * SLOT;
-#pragma unroll
-              for (int g = 0; g < 2; ++g) {
-                const float4 v = *reinterpret_cast<const float4*>(slot + ((2 * i + g) * BM + q * 32 + lane) * 16);
-                f[4 * g] += v.x; f[4 * g + 1] += v.y; f[4 * g + 2] += v.z; f[4 * g + 3] += v.w;
+              for (int i = 0; i < 8; ++i) {
+                f[4 * i] += v[i].x; f[4 * i + 1] += v[i].y; f[4 * i + 2] += v[i].z; f[4 * i + 3] += v[i].w;
               }
             }
-            const int col = col0 + 8 * i;
-            const bool ok = row < t.row_end && col < p.N;
-            const Out8 o = finish8(p, f, row, col, ok);
-            if (ok) {
-              const size_t at = static_cast<size_t>(row) * p.N + col;
-              *reinterpret_cast<uint4*>(p.out + at) = o.out;
-              if (p.pre_out != nullptr) *reinterpret_cast<uint4*>(p.pre_out + at) = o.pre;
+          }
+          uint4 o[4], pre[4];
+          finish32<kEpi>(p, f, row, col0, row < t.row_end, o, pre);
+          if (row < t.row_end) {
+            const size_t at = static_cast<size_t>(row) * p.N + col0;
+            store_row32(p.out, at, col0, p.N, p.wide != 0, o);
+            if constexpr (kEpi == EPI_ACT) {
+              if (p.pre_out != nullptr) store_row32(p.pre_out, at, col0, p.N, p.wide != 0, pre);
             }
           }
         }

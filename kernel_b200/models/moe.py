@@ -78,6 +78,17 @@ def _expert_major_rows(counts_h: torch.Tensor, cap: int):
     return idx, c.sum(0).tolist()
 
 
+def _pad8_t(rows: torch.Tensor) -> torch.Tensor:
+    """``rows[n, A]`` -> contiguous ``[A, n8]`` (n rounded up to a multiple of 8 with
+    zero columns): the K-major operand layout of a GEMM that contracts over rows, for
+    callers of ``ops.gemm.gemm``; the layers here contract rows where they lie."""
+    n, A = rows.shape
+    n8 = (n + 7) // 8 * 8
+    out = rows.new_zeros((A, n8))
+    out[:, :n] = rows.t()
+    return out
+
+
 def _all_local(a2a: MoEAllToAll, x: torch.Tensor) -> bool:
     """One rank on a GPU: no row leaves it, so the layer permutes rows instead of
     sending them, and no count has to reach the host."""
