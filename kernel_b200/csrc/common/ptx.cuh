@@ -109,9 +109,6 @@ __device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uin
 
 // 16-byte accesses to this CTA's shared memory by address (a pointer that went through
 // integer arithmetic has lost its address space and would be accessed generically).
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint4& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 __device__ __forceinline__ float4 ld_shared_v4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -131,22 +128,29 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
       ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// 3-D forms (innermost coordinate x, then y, z).  kPair: the completion is counted on
-// the mbarrier at cluster address `bar` (the leader of a CTA pair); otherwise `bar` is
-// the shared-memory address of one of this CTA's own barriers.
+// 3-D form (innermost coordinate x, then y, z), called by a converged warp: one elected
+// lane issues.  kPair: the completion is counted on the mbarrier at cluster address
+// `bar` (the leader of a CTA pair); otherwise `bar` is the shared-memory address of one
+// of this CTA's own barriers.
 template <bool kPair>
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y, int32_t z) {
+__device__ __forceinline__ void tma_load_3d_warp(uint32_t smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y, int32_t z) {
   if constexpr (kPair) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
         : "memory");
   } else {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
         : "memory");
   }
+}
+__device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+               "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
@@ -437,6 +441,11 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
+}
+
+// Loads 16 bytes of read-only data and drops them: the line is in L1 afterwards.
+__device__ __forceinline__ void touch_nc(const void* p) {
+  asm volatile("{\n\t.reg .b32 a, b, c, d;\n\tld.global.nc.v4.u32 {a, b, c, d}, [%0];\n\t}" ::"l"(p));
 }
 
 // Device-scope counterparts for words that only threads of this GPU touch.

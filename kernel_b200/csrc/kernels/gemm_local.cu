@@ -1,6 +1,7 @@
 // Host side of the single-GPU tcgen05 GEMM family (device code: gemm_local.cuh).
 #include "gemm_local.cuh"
 
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -52,6 +53,7 @@ struct Config {
   bool pair;
   int bn, split;
   bool tall = false;  // pair with 256 rows per CTA
+  int rows = 128;     // ROWS, one CTA: rows of a tile
 };
 
 // Ring stages of a configuration and whether the partial tiles of a split fit the ring.
@@ -129,6 +131,59 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
     }
   }
   return best;
+}
+
+// Grouped rows.  The counts stay on the device, so the number of row blocks is an
+// estimate from the average group: one if it fits a tile with two standard deviations
+// to spare, else half a block of padding per group.  The rest is the model of the dense
+// products.  With few rows the weights are the traffic and every shape that keeps the
+// SMs loading is near the memory time; the second-order term breaks such ties.
+//   64 experts, 2048 x 1024, 3 rows each: 32 x 256 tiles 45 us, 32 x 64 (first version) 68 us
+//   64 experts, 128 rows each: 128 x 192 tiles 61 us;  8 experts, 1000 rows of 4096 x 4096: pairs 198 us, one CTA 218 us
+Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape) {
+  Config best;
+  best.bn = b_mn ? 128 : 256;
+  best.pair = shape > 0;
+  best.split = 1;
+  double best_t = 1e30;
+  const int KB = ceil_div(K, BK);
+  const double n = static_cast<double>(M) / groups;
+  const double used = n < 1.0 ? n : 1.0;  // share of groups that have rows
+  const double memory = 2.0 * (used * groups * N * static_cast<double>(K) + static_cast<double>(M) * (N + K)) / 6500.0 + 6600.0;
+  for (int s = 0; s < 4; ++s) {
+    const bool pair = s == 3;
+    if (shape >= 0 ? pair != (shape > 0) : pair && sms < 2) continue;
+    const int rows = pair ? 256 : 32 << s;
+    const double blocks = n + 2.0 * sqrt(n) <= rows ? used : n / rows + 0.5;
+    for (int bn = 64; bn <= 256; bn += 64) {
+      if (!bn_ok(bn, pair, b_mn)) continue;
+      const double tiles = groups * blocks * ceil_div(N, bn);
+      const double units = pair ? sms / 2 : sms;
+      const double waves = tiles <= units ? 1.0 : tiles / units + 0.5;
+      const double mma = 300.0 * (bn < 190 ? 190 : bn) / 256.0 * (pair ? 1.0 : 1.33);
+      const double load = 128.0 * ((pair ? 128 : rows) + (pair ? bn / 2 : bn)) / 95.0 * (b_mn ? 1.07 : 1.0);
+      const double t = 2000.0 + waves * (KB * (mma > load ? mma : load) + 2000.0) + 2000.0 * bn / 256.0 + (pair ? 1000.0 : 0.0);
+      const double cost = t > memory ? t + 0.1 * memory : memory + 0.1 * t;
+      if (cost < best_t) {
+        best_t = cost;
+        best.pair = pair;
+        best.bn = bn;
+        best.rows = pair ? 128 : rows;
+      }
+    }
+  }
+  return best;
+}
+
+// Contractions over a group's rows are short (a few k blocks), the outputs are the
+// traffic: the widest tile of one CTA (64 experts, 128 rows, 2048 x 1024: 79 us, pair 98 us).
+Config contract_config(int M, int N, int shape) {
+  (void)M;
+  Config c;
+  c.pair = shape > 0;
+  c.bn = N <= 64 && !c.pair ? 64 : N <= 128 ? 128 : 256;
+  c.split = 1;
+  return c;
 }
 
 int device_info(int* dev_out, int* sms_out) {
@@ -310,14 +365,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &c);
     if (rc != KB_OK) return rc;
   } else {
-    // Rows per group decide: with fewer than about 1.5 tiles of 256 rows per group a pair
-    // would work mostly on padding.
-    const double per_group = contract ? a->M : static_cast<double>(a->M) / groups;
-    c.pair = shape < 0 ? per_group >= 384 : shape > 0;
-    // few rows per group: the weights are the traffic, narrow tiles spread them evenly over the SMs
-    c.bn = a->kind == KB_LOCAL_ROWS && per_group <= 64 ? 64 : a->N <= 64 ? 64 : a->N <= 128 ? 128 : 256;
-    c.split = 1;
-    if (!bn_ok(c.bn, c.pair, b_mn)) c.bn = 128;
+    c = contract ? contract_config(a->M, a->N, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape);
   }
   if (a->bn > 0) c.bn = a->bn;
   if (a->split > 0) c.split = a->split;
@@ -334,11 +382,10 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.K = a->K;
   // A single CTA whose rows are few brings in only those: the MMA reads 128 rows of
   // shared memory, what lies behind the box only reaches accumulator rows that are not
-  // stored.  Groups: 32 or 64 rows per tile when the average group fits it comfortably.
+  // stored.
   p.a_rows = c.tall ? 256 : 128;
   if (a->kind == KB_LOCAL_ROWS && !c.pair) {
-    const int avg = a->M / groups;
-    p.a_rows = avg <= 20 ? 32 : avg <= 48 ? 64 : 128;
+    p.a_rows = c.rows;
   } else if (!c.pair && !a_mn && a->M < 128) {
     p.a_rows = ceil_div(a->M, 8) * 8;
   }

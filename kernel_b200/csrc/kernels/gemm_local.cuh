@@ -152,12 +152,12 @@ __device__ __forceinline__ void slope32(const uint4* at, float* f) {
 }
 
 // 32 accumulator values of one row -> bf16: (+ bias, one rounding), then the activation
-// of the rounded value, or the product with the slope at `pre_in`.  A scheduler has two
+// of the rounded value, or the product with the slope at the saved value `at`.  A scheduler has two
 // epilogue warps at most, so latency counts: all loads of the 32 columns are issued
 // together and the arithmetic is straight-line, branches are taken once per 32 columns
 // (branching per 8 values cost 250 cycles each: 11000 cycles for a 128 x 256 tile).
 template <Epi kEpi>
-__device__ __forceinline__ void finish32(const Params& p, float* f, int row, int col, bool row_ok, uint4* out, uint4* pre) {
+__device__ __forceinline__ void finish32(const Params& p, float* f, int col, const uint4* at, uint4* out, uint4* pre) {
   if (p.bias != nullptr) {
     uint4 b[4];
 #pragma unroll
@@ -171,10 +171,6 @@ __device__ __forceinline__ void finish32(const Params& p, float* f, int row, int
     }
   }
   if constexpr (kEpi == EPI_SLOPE) {
-    uint4 at[4];
-    const uint4* src = reinterpret_cast<const uint4*>(p.pre_in + static_cast<size_t>(row) * p.N + col);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) at[i] = row_ok && col + 8 * i < p.N ? src[i] : make_uint4(0, 0, 0, 0);
     if (p.act == ACT_SILU) slope32<ACT_SILU>(at, f);
     else if (p.act == ACT_GELU) slope32<ACT_GELU>(at, f);
     else slope32<ACT_RELU>(at, f);
@@ -190,10 +186,10 @@ __device__ __forceinline__ void finish32(const Params& p, float* f, int row, int
 }
 // 32 values of a lane's row, straight from the registers.  A lane's 32-byte store is a
 // whole L2 sector, so the 32 rows a warp touches per instruction cost no partial
-// writes; against staging through shared memory and TMA stores this saves a fence, a
-// store issue and the wait for the store engine to read the box (about 1000 cycles per
-// box with two epilogue warps per scheduler), and the staging memory is another
-// pipeline stage.
+// writes.  Staging through shared memory (for TMA stores, or to let eight lanes store
+// a row's 128 bytes) moves twice the tile through a memory whose bandwidth a pair's
+// mainloop uses up: operands in and out are 128 bytes per cycle.  It also costs a
+// pipeline stage; 8 groups of 1000 rows, 4096 x 4096: 198 us stored from registers, 207 staged.
 __device__ __forceinline__ void store_row32(bf16* base, size_t at, int col, int n, bool wide, const uint4* v) {
   if (wide && col + 32 <= n) {
     kb::st_global_v8(base + at, v[0], v[1]);
@@ -384,12 +380,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      int s = 0;
+    // Converged like the MMA issuer: with few rows a stage is small and has to leave
+    // every 350 cycles to keep the memory busy.
+    {
+      uint32_t s = 0;
       uint32_t ph = 0;
       bool ok = true;
       const uint32_t a_bytes = static_cast<uint32_t>(p.a_rows) * BK * 2;
       const uint32_t stage_bytes = a_bytes + static_cast<uint32_t>(b_cols) * BK * 2;
+      const uint32_t a0 = kb::smem_u32(sm_a), b0 = kb::smem_u32(sm_b), full0 = kb::smem_u32(full);
+      // a pair's bytes are counted on the leader's barrier, which expects the sum
+      const uint32_t bar0 = kPair ? kb::map_to_cta(full0, lead) : full0;
       for (int pos = sched_id; ok && pos < total_tiles; pos += sched_n) {
         const Tile t = tile_at(pos);
         int k0, k1;
@@ -403,31 +404,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
             ok = false;
             break;
           }
-          uint8_t* da = sm_a + s * p.a_slot;
-          uint8_t* db = sm_b + s * p.b_slot;
-          uint32_t bar = kb::smem_u32(&full[s]);
-          if constexpr (kPair) {
-            if (leader) kb::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
-            bar = kb::map_to_cta(bar, lead);  // both CTAs' bytes are counted on the leader's barrier
-          } else {
-            kb::mbar_arrive_expect_tx(&full[s], stage_bytes);
-          }
+          const uint32_t da = a0 + s * p.a_slot, db = b0 + s * p.b_slot, bar = bar0 + 8 * s;
+          if (leader) kb::mbar_expect_tx_warp(full0 + 8 * s, kPair ? 2 * stage_bytes : stage_bytes);
           if constexpr (kAMn) {
 #pragma unroll
             for (int i = 0; i < CTA_ROWS / 64; ++i) {
-              kb::tma_load_3d<kPair>(da + i * MN_BLOCK_BYTES, &p.tmA, bar, t.row0 + i * 64, t.k_row + k * BK, 0);
+              kb::tma_load_3d_warp<kPair>(da + i * MN_BLOCK_BYTES, &p.tmA, bar, t.row0 + i * 64, t.k_row + k * BK, 0);
             }
           } else {
-            kb::tma_load_3d<kPair>(da, &p.tmA, bar, k * BK, t.row0, 0);
+            kb::tma_load_3d_warp<kPair>(da, &p.tmA, bar, k * BK, t.row0, 0);
           }
           if constexpr (kBMn) {
             for (int i = 0; i < b_cols / 64; ++i) {
-              kb::tma_load_3d<kPair>(db + i * MN_BLOCK_BYTES, &p.tmB, bar, nrow + i * 64, t.k_row + k * BK, bz);
+              kb::tma_load_3d_warp<kPair>(db + i * MN_BLOCK_BYTES, &p.tmB, bar, nrow + i * 64, t.k_row + k * BK, bz);
             }
           } else {
-            kb::tma_load_3d<kPair>(db, &p.tmB, bar, k * BK, nrow, bz);
+            kb::tma_load_3d_warp<kPair>(db, &p.tmB, bar, k * BK, nrow, bz);
           }
-          if (++s == p.stages) {
+          if (++s == static_cast<uint32_t>(p.stages)) {
             s = 0;
             ph ^= 1u;
           }
@@ -511,6 +505,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     uint32_t it = 0;
     for (int pos = sched_id; pos < total_tiles; pos += sched_n, ++it) {
       const Tile t = tile_at(pos);
+      if (p.bias != nullptr) {
+        // brings the tile's bias into L1 while the accumulator is not ready yet: eight values per lane
+        const int col = t.n0 + 8 * lane;
+        if (8 * lane < p.bn && col < p.N) kb::touch_nc(p.bias + col);
+      }
       const size_t out0 = kKind == CONTRACT ? static_cast<size_t>(t.group) * p.M * p.N : 0;
       const int cols = min(p.bn, p.N - t.n0);
 #pragma unroll 1
@@ -543,6 +542,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
 #pragma unroll 1
         for (int c = turn * 64; c < last; c += 128) {
           const bool two = c + 32 < last;
+          const int col = t.n0 + c;
+          const size_t at0 = out0 + static_cast<size_t>(row) * p.N + col;
+          uint4 at[8];
+          if constexpr (kEpi == EPI_SLOPE) {  // fetched before the accumulator is read
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              at[i] = make_uint4(0u, 0u, 0u, 0u);
+              if (row_ok && c + 8 * i < last) at[i] = kb::ld_nc_v4(p.pre_in + at0 + 8 * i);
+            }
+          }
           uint32_t r[2][32];
           if (kKind == CONTRACT && t.kb == 0) {  // an empty group: nothing was accumulated
 #pragma unroll
@@ -560,13 +569,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[h][i]);
             uint4 o[4], pre[4];
-            const int col = t.n0 + c + 32 * h;
-            finish32<kEpi>(p, f, row, col, row_ok, o, pre);
+            finish32<kEpi>(p, f, col + 32 * h, at + 4 * h, o, pre);
             if (row_ok) {
-              const size_t at = out0 + static_cast<size_t>(row) * p.N + col;
-              store_row32(p.out, at, col, p.N, p.wide != 0, o);
+              store_row32(p.out, at0 + 32 * h, col + 32 * h, p.N, p.wide != 0, o);
               if constexpr (kEpi == EPI_ACT) {
-                if (p.pre_out != nullptr) store_row32(p.pre_out, at, col, p.N, p.wide != 0, pre);
+                if (p.pre_out != nullptr) store_row32(p.pre_out, at0 + 32 * h, col + 32 * h, p.N, p.wide != 0, pre);
               }
             }
           }
@@ -593,6 +600,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       kb::tc_fence_after_sync();
       const uint32_t tmem_base = *tmem_slot;  // the producer warp did not wait for it
       const Tile t = tile_at(sched_id);
+      if (p.bias != nullptr) {
+        const int col = t.n0 + 8 * lane;
+        if (8 * lane < p.bn && col < p.N) kb::touch_nc(p.bias + col);
+      }
       const int chunks = p.bn / CHUNK_COLS;
       const int q = warp & 3;            // TMEM lane quadrant of this warp
       const int gr0 = t.row0 + q * 32;
@@ -647,7 +658,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
             }
           }
           uint4 o[4], pre[4];
-          finish32<kEpi>(p, f, row, col0, row < t.row_end, o, pre);
+          uint4 at4[4];
+          if constexpr (kEpi == EPI_SLOPE) {
+            const uint4* src = reinterpret_cast<const uint4*>(p.pre_in + static_cast<size_t>(row) * p.N + col0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) at4[i] = row < t.row_end && col0 + 8 * i < p.N ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+          }
+          finish32<kEpi>(p, f, col0, at4, o, pre);
           if (row < t.row_end) {
             const size_t at = static_cast<size_t>(row) * p.N + col0;
             store_row32(p.out, at, col0, p.N, p.wide != 0, o);
