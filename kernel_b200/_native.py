@@ -15,7 +15,7 @@ KB_OK, KB_ERR_CUDA, KB_ERR_ARG, KB_ERR_TIMEOUT, KB_ERR_IO, KB_ERR_UNSUPPORTED = 
 BACKEND_HOST, BACKEND_VMM, BACKEND_IPC = 0, 1, 2
 GEMM_PLAIN, GEMM_RS, GEMM_AG = 0, 1, 2
 LOCAL_DENSE, LOCAL_ROWS, LOCAL_CONTRACT = 0, 1, 2
-ACTS = {None: 0, "gelu": 1, "relu": 2, "silu": 3}
+ACTS = {"gelu": 1, "relu": 2, "silu": 3}  # no activation: 0
 
 DEV_CODES = {0: "ok", 1: "pipeline barrier timeout", 2: "peer flag timeout", 3: "index out of bounds"}
 
@@ -158,6 +158,8 @@ def _declare(lib: C.CDLL) -> None:
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
         "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
         "kb_gemm_local_config": (i, [i, i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
+        "kb_col_sum_parts": (i, [i, i]),
+        "kb_col_sum": (i, [vp, i, i, vp, vp, vp]),
         "kb_moe_permute": (i, [vp, vp, i, i, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
         "kb_moe_combine": (i, [vp, vp, vp, i, i, i, vp, vp]),
         "kb_moe_grad_rows": (i, [vp, vp, vp, vp, i, i, i, i, vp, vp, vp, vp, vp, vp]),

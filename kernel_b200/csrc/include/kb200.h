@@ -161,6 +161,11 @@ uint64_t kb_gemm_ag_data_bytes(int M, int K);
 uint64_t kb_gemm_ag_flag_bytes(int M, int world);
 uint64_t kb_gemm_ag_counter_bytes(int M, int world);
 
+// Column sums in fp32 of a bf16 matrix (kernels/col_sum.cu): out[cols] bf16; `partial`: fp32
+// [kb_col_sum_parts(rows, cols)][cols], may be NULL when that is 1.
+int kb_col_sum_parts(int rows, int cols);
+int kb_col_sum(const void* x, int rows, int cols, float* partial, void* out, void* stream);
+
 // ---- MoE rows on one rank (kernels/moe_rows.cu), bf16 rows of `hidden` elements ----
 // permute: copy of token t for its choice j -> rows[slots[t*k + j]], experts in ascending order, an expert's rows in
 // token order, each expert starting at a multiple of `pad` rows (the rows in between are zeroed).

@@ -14,7 +14,10 @@ from typing import Optional
 
 import torch
 
+from .._native import ACTS
+from ..ops.autograd import ColumnParallelLinear, LocalMLPFn, RowParallelLinear
 from ..ops.gemm import AGGemm, GemmRS
+from ..ops.local import product
 from ..parallel.symm import _dist_info
 
 
@@ -47,6 +50,10 @@ class SequenceParallelMLP:
         raise ValueError(f"unknown activation {self.activation!r}")
 
     def __call__(self, x_local: torch.Tensor) -> torch.Tensor:
+        if x_local.is_cuda and self.world == 1 and self.activation in ACTS:
+            self.up.check(x_local, self.w1)
+            h = product(x_local, self.w1, self.b1, act=self.activation)   # the activation in the product's epilogue
+            return self.down(h, self.w2, self.b2)
         h = self.up(x_local, self.w1, self.b1)           # [tokens, ffn/world]
         h = self._act(h)
         return self.down(h, self.w2, self.b2)            # [tokens/world, hidden]
@@ -77,13 +84,15 @@ class TrainableSequenceParallelMLP(torch.nn.Module):
     def __init__(self, tokens: int, hidden: int, ffn_local: int, bias: bool = True, activation: str = "gelu", group=None,
                  device: Optional[torch.device] = None):
         super().__init__()
-        from ..ops.autograd import ColumnParallelLinear, RowParallelLinear
-
         self.up = ColumnParallelLinear(tokens, hidden, ffn_local, bias=bias, group=group, device=device)
         self.down = RowParallelLinear(tokens, ffn_local, hidden, bias=bias, group=group, device=device)
         self.activation = activation
 
     def forward(self, x_local: torch.Tensor) -> torch.Tensor:
+        up, down = self.up, self.down
+        if x_local.is_cuda and up.world == 1 and self.activation in ACTS:
+            up.fwd.check(x_local.contiguous(), up.weight)
+            return LocalMLPFn.apply(x_local, up.weight, up.bias, down.weight, down.bias, self.activation)
         h = self.up(x_local)
         if self.activation == "gelu":
             h = torch.nn.functional.gelu(h, approximate="tanh")

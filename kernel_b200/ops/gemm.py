@@ -396,14 +396,18 @@ class AGGemm:
         elif self.native:
             self.status = torch.zeros(8, dtype=torch.int32, device=device or torch.device("cuda", torch.cuda.current_device()))
 
-    def __call__(self, a_local: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def check(self, a_local: torch.Tensor, w: torch.Tensor) -> None:
+        """Raises unless the operands fit this context."""
         _check_bf16_2d(a_local, "a_local")
         _check_bf16_2d(w, "w")
         rows, K = a_local.shape
         if rows * self.world != self.M or K != self.K or w.shape[1] != K:
             raise ValueError("shape does not match this AGGemm context")
-        Nl = w.shape[0]
+
+    def __call__(self, a_local: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        self.check(a_local, w)
+        Nl, K = w.shape
         if not a_local.is_cuda and self.host_heap:
             if out is None:
                 out = torch.empty((self.M, Nl), dtype=torch.bfloat16)

@@ -66,10 +66,10 @@ def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
     G.launch_count += 1
 
 
-def product(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = False, act: Optional[str] = None,
-            pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
+def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, *, a_t: bool = False, b_t: bool = False,
+            act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``A @ B^T`` in bf16 with fp32 accumulation, ``A`` being ``a[M, K]`` (``a_t``: ``a[K, M]``)
+    """``A @ B^T (+ bias)`` in bf16 with fp32 accumulation, ``A`` being ``a[M, K]`` (``a_t``: ``a[K, M]``)
     and ``B`` being ``b[N, K]`` (``b_t``: ``b[K, N]``); ``a_t`` needs ``b_t``.
 
     ``act``: the activation of the rounded product, which ``pre_out`` also receives;
@@ -78,16 +78,31 @@ def product(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = 
     Nn = b.shape[1] if b_t else b.shape[0]
     if not a.is_cuda:
         A, B = a.float(), b.float()
-        return _finish((A.t() if a_t else A) @ (B if b_t else B.t()), act, pre_out, pre_in, out)
+        res = (A.t() if a_t else A) @ (B if b_t else B.t())
+        return _finish(res if bias is None else res + bias.float(), act, pre_out, pre_in, out)
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
     args = N.LocalGemmArgs()
     args.kind, args.M, args.N, args.K = N.LOCAL_DENSE, M, Nn, K
     args.a_mn, args.b_mn = a_t, b_t
+    args.bias, args.bias_scale = _ptr(bias), 1.0
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.act, args.pre_out, args.pre_in = N.ACTS[act], _ptr(pre_out), _ptr(pre_in)
+    args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
     args.pair = -1
     _launch(args, a.device)
+    return out
+
+
+def col_sum(x: torch.Tensor) -> torch.Tensor:
+    """``x[R, C].sum(0)`` accumulated in fp32, in bf16 (bias gradients)."""
+    R, Cn = x.shape
+    if not x.is_cuda or x.dtype != torch.bfloat16 or R == 0 or Cn % 8:
+        return x.float().sum(0).to(x.dtype)
+    lib = N.lib()
+    parts = lib.kb_col_sum_parts(R, Cn)
+    partial = torch.empty((parts, Cn), dtype=torch.float32, device=x.device) if parts > 1 else None
+    out = torch.empty(Cn, dtype=torch.bfloat16, device=x.device)
+    N.check(lib.kb_col_sum(x.data_ptr(), R, Cn, _ptr(partial), out.data_ptr(), _stream(x.device)))
     return out
 
 
@@ -116,7 +131,7 @@ def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: t
     args.b_mn, args.groups = b_t, E
     args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.act, args.pre_out, args.pre_in = N.ACTS[act], _ptr(pre_out), _ptr(pre_in)
+    args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
     args.pair = -1
     _launch(args, a.device)
     return out
