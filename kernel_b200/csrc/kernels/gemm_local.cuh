@@ -122,11 +122,9 @@ __device__ __forceinline__ float act_slope(float x) {
   if constexpr (kAct == ACT_GELU) {
     const float s = sigmoid(GELU_C * x * (1.0f + GELU_A * x * x));
     return s + x * s * (1.0f - s) * GELU_C * (1.0f + 3.0f * GELU_A * x * x);
-  } else if constexpr (kAct == ACT_SILU) {
+  } else {
     const float s = sigmoid(x);
     return s * (1.0f + x * (1.0f - s));
-  } else {
-    return x > 0.0f ? 1.0f : 0.0f;
   }
 }
 template <int kAct>
@@ -147,7 +145,11 @@ __device__ __forceinline__ void slope32(const uint4* at, float* f) {
     float s[8];
     unpack8(at[i], s);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[8 * i + e] *= act_slope<kAct>(s[e]);
+    for (int e = 0; e < 8; ++e) {
+      // ReLU selects: an infinite gradient where it is off is zero, a NaN passes the gradient on
+      if constexpr (kAct == ACT_RELU) f[8 * i + e] = s[e] <= 0.0f ? 0.0f : f[8 * i + e];
+      else f[8 * i + e] *= act_slope<kAct>(s[e]);
+    }
   }
 }
 

@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <initializer_list>
+
 #include "../common/host_util.h"
 #include "../common/ptx.cuh"
 #include "../include/kb200.h"
@@ -288,6 +290,23 @@ int check_sizes(int T, int k, int E, int hidden) {
   return KB_OK;
 }
 
+// Rows are moved in 16-byte vectors, tables and weights in 4-byte words.
+int check_pointers(std::initializer_list<const void*> rows, std::initializer_list<const void*> words) {
+  for (const void* q : rows) {
+    if ((reinterpret_cast<uintptr_t>(q) & 15u) != 0) {
+      kb::set_error("moe rows: row buffers must be 16-byte aligned");
+      return KB_ERR_ARG;
+    }
+  }
+  for (const void* q : words) {
+    if ((reinterpret_cast<uintptr_t>(q) & 3u) != 0) {
+      kb::set_error("moe rows: tables and weights must be 4-byte aligned");
+      return KB_ERR_ARG;
+    }
+  }
+  return KB_OK;
+}
+
 }  // namespace
 
 extern "C" int kb_moe_permute(const void* x, const int32_t* indices, int T, int k, int experts, int hidden, int pad, void* rows,
@@ -296,6 +315,8 @@ extern "C" int kb_moe_permute(const void* x, const int32_t* indices, int T, int 
   int rc = check_sizes(T, k, experts, hidden);
   if (rc != KB_OK) return rc;
   if (pad < 1) return KB_ERR_ARG;
+  rc = check_pointers({x, rows}, {indices, slots, row_start, row_count, row_padded});
+  if (rc != KB_OK) return rc;
   int sms = 0;
   rc = sm_count(&sms);
   if (rc != KB_OK) return rc;
@@ -329,6 +350,8 @@ extern "C" int kb_moe_permute(const void* x, const int32_t* indices, int T, int 
 extern "C" int kb_moe_combine(const void* y, const int32_t* slots, const float* weights, int T, int k, int hidden, void* out, void* stream) {
   int rc = check_sizes(T, k, 1, hidden);
   if (rc != KB_OK || T == 0) return rc;
+  rc = check_pointers({y, out}, {slots, weights});
+  if (rc != KB_OK) return rc;
   int sms = 0;
   rc = sm_count(&sms);
   if (rc != KB_OK) return rc;
@@ -343,6 +366,8 @@ extern "C" int kb_moe_grad_rows(const void* dy, const void* y, const int32_t* sl
                                 int hidden, void* dyr, float* dw, const int32_t* row_start, const int32_t* row_count,
                                 const int32_t* row_padded, void* stream) {
   int rc = check_sizes(T, k, experts, hidden);
+  if (rc != KB_OK) return rc;
+  rc = check_pointers({dy, y, dyr}, {slots, weights, dw});
   if (rc != KB_OK) return rc;
   GradParams p = {T, k, experts, hidden / 8, static_cast<const uint4*>(dy), static_cast<const uint4*>(y), slots, weights,
                   static_cast<uint4*>(dyr), dw, row_start, row_count, row_padded};

@@ -52,7 +52,7 @@ class SequenceParallelMLP:
     def __call__(self, x_local: torch.Tensor) -> torch.Tensor:
         if x_local.is_cuda and self.world == 1 and self.activation in ACTS:
             self.up.check(x_local, self.w1)
-            h = product(x_local, self.w1, self.b1, act=self.activation)   # the activation in the product's epilogue
+            h = product(x_local, self.w1, self.b1, act=self.activation, status=self.up.status)   # the activation in the product's epilogue
             return self.down(h, self.w2, self.b2)
         h = self.up(x_local, self.w1, self.b1)           # [tokens, ffn/world]
         h = self._act(h)
@@ -75,6 +75,12 @@ class SequenceParallelMLP:
                 ctx.heap.close()
 
 
+def _plain(layer: torch.nn.Module, kind: type) -> bool:
+    """One rank, and nothing (a replacement, hooks) asks for the layer to be called by itself."""
+    return type(layer) is kind and layer.world == 1 and not (
+        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
+
+
 class TrainableSequenceParallelMLP(torch.nn.Module):
     """The same block as ``SequenceParallelMLP`` with parameters and a backward
     pass: ``ColumnParallelLinear`` (all-gather fused forward, reduce-scatter fused
@@ -90,9 +96,10 @@ class TrainableSequenceParallelMLP(torch.nn.Module):
 
     def forward(self, x_local: torch.Tensor) -> torch.Tensor:
         up, down = self.up, self.down
-        if x_local.is_cuda and up.world == 1 and self.activation in ACTS:
+        if (x_local.is_cuda and self.activation in ACTS and _plain(up, ColumnParallelLinear) and _plain(down, RowParallelLinear)
+                and down.weight.dtype == torch.bfloat16 and down.weight.shape == (down.fwd.N, up.weight.shape[0])):
             up.fwd.check(x_local.contiguous(), up.weight)
-            return LocalMLPFn.apply(x_local, up.weight, up.bias, down.weight, down.bias, self.activation)
+            return LocalMLPFn.apply(x_local, up.weight, up.bias, down.weight, down.bias, self.activation, up.fwd.status)
         h = self.up(x_local)
         if self.activation == "gelu":
             h = torch.nn.functional.gelu(h, approximate="tanh")

@@ -115,33 +115,34 @@ class LocalMLPFn(torch.autograd.Function):
     elementwise pass: both were 40 % of a step at 8192 x 8192 x 29568."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, act):
+    def forward(ctx, x, w1, b1, w2, b2, act, status):
         x, w1, w2 = x.contiguous(), w1.contiguous(), w2.contiguous()
         pre = torch.empty((x.shape[0], w1.shape[0]), dtype=x.dtype, device=x.device)
-        h = product(x, w1, b1, act=act, pre_out=pre)
-        ctx.act = act
+        h = product(x, w1, b1, act=act, pre_out=pre, status=status)
+        ctx.act, ctx.status = act, status
         ctx.save_for_backward(x, w1, w2, pre, h)
-        return product(h, w2, b2)
+        return product(h, w2, b2, status=status)
 
     @staticmethod
     def backward(ctx, dy):
         x, w1, w2, pre, h = ctx.saved_tensors
-        need_x, need_w1, need_b1, need_w2, need_b2, _ = ctx.needs_input_grad
+        status = ctx.status
+        need_x, need_w1, need_b1, need_w2, need_b2 = ctx.needs_input_grad[:5]
         dy = dy.contiguous()
         dx = dw1 = db1 = dw2 = db2 = None
         if need_w2:
-            dw2 = product(dy, h, a_t=True, b_t=True)
+            dw2 = product(dy, h, a_t=True, b_t=True, status=status)
         if need_b2:
             db2 = col_sum(dy)
         if need_x or need_w1 or need_b1:
-            dpre = product(dy, w2, b_t=True, act=ctx.act, pre_in=pre)
+            dpre = product(dy, w2, b_t=True, act=ctx.act, pre_in=pre, status=status)
             if need_w1:
-                dw1 = product(dpre, x, a_t=True, b_t=True)
+                dw1 = product(dpre, x, a_t=True, b_t=True, status=status)
             if need_b1:
                 db1 = col_sum(dpre)
             if need_x:
-                dx = product(dpre, w1, b_t=True)
-        return dx, dw1, db1, dw2, db2, None
+                dx = product(dpre, w1, b_t=True, status=status)
+        return dx, dw1, db1, dw2, db2, None, None
 
 
 class ColumnParallelLinear(torch.nn.Module):

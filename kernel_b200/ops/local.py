@@ -17,6 +17,7 @@ from typing import Optional
 import torch
 
 from .. import _native as N
+from . import gemm as G
 
 ROW_ALIGN = 64  # rows of a group in a table made for contract_product start at multiples of the kernel's k block
 
@@ -57,9 +58,14 @@ def _stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
 
 
-def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
-    from . import gemm as G  # launch accounting of the GEMM front-ends
+def _args(kind: int, M: int, Nn: int, K: int, status: Optional[torch.Tensor]) -> N.LocalGemmArgs:
+    args = N.LocalGemmArgs()
+    args.kind, args.M, args.N, args.K, args.pair = kind, M, Nn, K, -1
+    args.status, args.wait_limit_ns = _ptr(status), G._WAIT_LIMIT_NS
+    return args
 
+
+def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
     code = N.lib().kb_gemm_local(C.byref(args), _stream(device))
     if code:
         N.check(code)
@@ -68,7 +74,7 @@ def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
 
 def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, *, a_t: bool = False, b_t: bool = False,
             act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
-            out: Optional[torch.Tensor] = None) -> torch.Tensor:
+            out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``A @ B^T (+ bias)`` in bf16 with fp32 accumulation, ``A`` being ``a[M, K]`` (``a_t``: ``a[K, M]``)
     and ``B`` being ``b[N, K]`` (``b_t``: ``b[K, N]``); ``a_t`` needs ``b_t``.
 
@@ -82,13 +88,11 @@ def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = Non
         return _finish(res if bias is None else res + bias.float(), act, pre_out, pre_in, out)
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
-    args = N.LocalGemmArgs()
-    args.kind, args.M, args.N, args.K = N.LOCAL_DENSE, M, Nn, K
+    args = _args(N.LOCAL_DENSE, M, Nn, K, status)
     args.a_mn, args.b_mn = a_t, b_t
     args.bias, args.bias_scale = _ptr(bias), 1.0
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
-    args.pair = -1
     _launch(args, a.device)
     return out
 
@@ -96,7 +100,7 @@ def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = Non
 def col_sum(x: torch.Tensor) -> torch.Tensor:
     """``x[R, C].sum(0)`` accumulated in fp32, in bf16 (bias gradients)."""
     R, Cn = x.shape
-    if not x.is_cuda or x.dtype != torch.bfloat16 or R == 0 or Cn % 8:
+    if not x.is_cuda or x.dtype != torch.bfloat16 or R == 0 or Cn % 8 or x.data_ptr() % 16:
         return x.float().sum(0).to(x.dtype)
     lib = N.lib()
     parts = lib.kb_col_sum_parts(R, Cn)
@@ -108,7 +112,7 @@ def col_sum(x: torch.Tensor) -> torch.Tensor:
 
 def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor, *, b_t: bool = False,
                  act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
-                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Rows ``start[e] .. start[e] + count[e]`` of ``a[R, K]`` times ``b[e]`` transposed
     (``b[E, N, K]``, ``b_t``: ``b[E, K, N]``).  Rows outside every group are left alone."""
     R, K = a.shape
@@ -126,18 +130,17 @@ def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: t
                 _finish(a[sl].float() @ (B if b_t else B.t()), act, None if pre_out is None else pre_out[sl],
                         None if pre_in is None else pre_in[sl], out[sl])
         return out
-    args = N.LocalGemmArgs()
-    args.kind, args.M, args.N, args.K = N.LOCAL_ROWS, R, Nn, K
+    args = _args(N.LOCAL_ROWS, R, Nn, K, status)
     args.b_mn, args.groups = b_t, E
     args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
-    args.pair = -1
     _launch(args, a.device)
     return out
 
 
-def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor) -> torch.Tensor:
+def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor,
+                     status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[e] = a[rows of e]^T @ b[rows of e]`` for ``a[R, M]``, ``b[R, N]``.  Groups start at
     multiples of ``ROW_ALIGN``; rows between a group's last and the next multiple are
     zero in one operand and finite in the other."""
@@ -148,12 +151,10 @@ def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, coun
             out[e] = (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)
         return out
     out = torch.empty((E, M, Nn), dtype=torch.bfloat16, device=a.device)
-    args = N.LocalGemmArgs()
-    args.kind, args.M, args.N, args.K = N.LOCAL_CONTRACT, M, Nn, R
+    args = _args(N.LOCAL_CONTRACT, M, Nn, R, status)
     args.groups = E
     args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.pair = -1
     _launch(args, a.device)
     return out
 
@@ -167,14 +168,24 @@ class ExpertRows:
 
     def __init__(self, x: torch.Tensor, indices: torch.Tensor, experts: int, pad: int = 1, status: Optional[torch.Tensor] = None):
         (T, H), k, dev = x.shape, indices.shape[1], x.device
-        self.T, self.k, self.E, self.H = T, k, experts, H
-        self.rows = torch.empty((T * k + experts * (pad - 1), H), dtype=torch.bfloat16, device=dev)
-        table = torch.empty(3 * experts + T * k, dtype=torch.int32, device=dev)
-        self.start, self.count, self.padded = table[:experts], table[experts:2 * experts], table[2 * experts:3 * experts]
-        self.slots = table[3 * experts:].view(T, k)
+        rows = torch.empty((T * k + experts * (pad - 1), H), dtype=torch.bfloat16, device=dev)
+        self._set(rows, torch.empty(3 * experts + T * k, dtype=torch.int32, device=dev), T, k, experts)
         N.check(N.lib().kb_moe_permute(x.data_ptr(), indices.data_ptr(), T, k, experts, H, pad, self.rows.data_ptr(),
                                        self.slots.data_ptr(), self.start.data_ptr(), self.count.data_ptr(), self.padded.data_ptr(),
                                        _ptr(status), _stream(dev)))
+
+    def _set(self, rows: torch.Tensor, table: torch.Tensor, T: int, k: int, experts: int) -> None:
+        self.T, self.k, self.E, self.H = T, k, experts, rows.shape[1]
+        self.rows, self.table = rows, table
+        self.start, self.count, self.padded = table[:experts], table[experts:2 * experts], table[2 * experts:3 * experts]
+        self.slots = table[3 * experts:].view(T, k)
+
+    @classmethod
+    def saved(cls, rows: torch.Tensor, table: torch.Tensor, T: int, k: int, experts: int) -> "ExpertRows":
+        """The rows and tables an earlier instance made (``rows``, ``table``), for a backward pass."""
+        er = cls.__new__(cls)
+        er._set(rows, table, T, k, experts)
+        return er
 
     def combine(self, y: torch.Tensor, weights: Optional[torch.Tensor]) -> torch.Tensor:
         """``out[t] = sum_j weights[t, j] * y[slots[t, j]]`` (``None``: unit weights)."""

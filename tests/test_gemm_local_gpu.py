@@ -1,0 +1,249 @@
+"""Products of one GPU (``ops/local.py``) at the edges of their tiles, against plain fp32 torch.
+
+Operands are small integers: every product and sum is exact in fp32 in any order, so a
+result differs from the reference only if a value is wrong, and the comparison is
+exact.  Activations are compared within two bf16 roundings (2 ** -8 each)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _ints(*shape, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.randint(-2, 3, shape, device=DEV, generator=g).to(torch.bfloat16)
+
+
+def _clean(status):
+    torch.cuda.synchronize()
+    assert status.cpu().tolist()[0] == 0, status.cpu().tolist()
+
+
+def _status():
+    return torch.zeros(8, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (7, 72, 72), (127, 256, 64), (128, 264, 136), (129, 512, 200), (257, 1000, 584),
+                                   (513, 320, 1032), (64, 2048, 4104), (300, 136, 8200), (1025, 2056, 264)])
+@pytest.mark.parametrize("layout", ["tn", "nn", "nt"])
+def test_dense_product(M, N, K, layout):
+    from kernel_b200.ops.local import product
+
+    a_t, b_t = layout == "nt", layout != "tn"
+    if a_t:
+        M, K = (M + 7) // 8 * 8, K + 3  # contiguous along M: whole 16-byte units there, any K
+    a, b, bias = _ints(M, K, seed=1), _ints(N, K, seed=2), _ints(N, seed=3)
+    st = _status()
+    out = product(a.t().contiguous() if a_t else a, b.t().contiguous() if b_t else b, bias, a_t=a_t, b_t=b_t, status=st)
+    _clean(st)
+    assert torch.equal(out, (a.float() @ b.float().t() + bias.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("pair,bn,split", [(0, 32, 1), (0, 96, 8), (0, 256, 5), (1, 64, 4), (1, 160, 3), (1, 256, 2), (2, 256, 1)])
+def test_dense_configurations(pair, bn, split):
+    """Every tile shape the launcher can pick gives the same numbers, also where the last tile is mostly padding."""
+    from kernel_b200 import _native as N
+    from kernel_b200.ops import local as L
+
+    M, Nn, K = 264, 296, 2120  # k blocks for eight members of a split
+    a, b = _ints(M, K, seed=4), _ints(Nn, K, seed=5)
+    out = torch.full((M, Nn), 7.0, dtype=torch.bfloat16, device=DEV)
+    st = _status()
+    args = L._args(N.LOCAL_DENSE, M, Nn, K, st)
+    args.bias_scale, args.A, args.B, args.out = 1.0, a.data_ptr(), b.data_ptr(), out.data_ptr()
+    args.pair, args.bn, args.split = pair, bn, split
+    L._launch(args, a.device)
+    _clean(st)
+    assert torch.equal(out, (a.float() @ b.float().t()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
+@pytest.mark.parametrize("M,N,K", [(5, 72, 64), (200, 264, 328), (600, 520, 128)])
+def test_activation_and_slope_in_the_epilogue(act, M, N, K):
+    from kernel_b200.ops.local import _ACTS, _slope, product
+
+    a, b = _ints(M, K, seed=6), (_ints(N, K, seed=7).float() / K ** 0.5).to(torch.bfloat16)
+    st = _status()
+    pre = torch.empty((M, N), dtype=torch.bfloat16, device=DEV)
+    out = product(a, b, act=act, pre_out=pre, status=st)
+    g = product(a, b.t().contiguous(), b_t=True, act=act, pre_in=pre, status=st)
+    _clean(st)
+    full = a.float() @ b.float().t()
+    assert (pre.float() - full).abs().max() <= 2 ** -8 * full.abs().max()
+    want = _ACTS[act](pre.float())
+    assert ((out.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+    want = full * _slope(act, pre)
+    assert ((g.float() - want).abs() <= 2 ** -7 * want.abs() + 1e-4 * full.abs()).all()
+
+
+def test_relu_slope_selects():
+    """Where ReLU is off an infinite gradient is zero; a NaN input passes the gradient on (as torch does)."""
+    from kernel_b200.ops.local import product
+
+    a = torch.zeros((8, 8), dtype=torch.bfloat16, device=DEV)
+    a[:, 0] = float("inf")
+    b = torch.zeros((8, 8), dtype=torch.bfloat16, device=DEV)
+    b[0] = 1.0
+    pre = torch.tensor([-1.0, 0.0, 1.0, float("nan")] * 2, device=DEV).to(torch.bfloat16).repeat(8, 1).contiguous()
+    out = product(a, b, b_t=True, act="relu", pre_in=pre).float()
+    assert out.cpu().tolist()[0] == [0.0, 0.0, float("inf"), float("inf")] * 2
+
+
+COUNTS = [[0, 1, 33, 0, 128, 300, 64], [0, 0, 0], [5], [257, 0, 255, 256], [1] * 40]
+
+
+def _table(counts, pad):
+    n = torch.tensor(counts)
+    padded = (n + pad - 1) // pad * pad
+    start = padded.cumsum(0) - padded
+    return start.int().to(DEV), n.int().to(DEV), max(1, int(padded.sum()))
+
+
+def _force(monkeypatch, pair):
+    """Tile shape of the products made through ``ops.local``."""
+    from kernel_b200.ops import local as L
+
+    made = L._args
+
+    def forced(*a):
+        args = made(*a)
+        args.pair = pair
+        return args
+
+    monkeypatch.setattr(L, "_args", forced)
+    return L
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("b_t", [False, True])
+@pytest.mark.parametrize("N,K", [(264, 72), (64, 520)])
+@pytest.mark.parametrize("pair", [-1, 0, 1])
+def test_rows_product(counts, b_t, N, K, pair, monkeypatch):
+    L = _force(monkeypatch, pair)
+    start, count, R = _table(counts, 1)
+    a, b = _ints(R, K, seed=8), _ints(len(counts), N, K, seed=9)
+    st = _status()
+    out = torch.full((R, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    L.rows_product(a, b.transpose(1, 2).contiguous() if b_t else b, start, count, b_t=b_t, out=out, status=st)
+    _clean(st)
+    want = torch.full((R, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        want[s:s + n] = (a[s:s + n].float() @ b[e].float().t()).to(torch.bfloat16)
+    assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("M,N", [(136, 72), (64, 264), (520, 128)])
+@pytest.mark.parametrize("pair", [-1, 0, 1])
+def test_contract_product(counts, M, N, pair, monkeypatch):
+    L = _force(monkeypatch, pair)
+    start, count, R = _table(counts, L.ROW_ALIGN)
+    a, b = torch.zeros((R, M), dtype=torch.bfloat16, device=DEV), torch.zeros((R, N), dtype=torch.bfloat16, device=DEV)
+    for s, n in zip(start.tolist(), count.tolist()):
+        a[s:s + n], b[s:s + n] = _ints(n, M, seed=10 + s), _ints(n, N, seed=11 + s)
+    st = _status()
+    out = L.contract_product(a, b, start, count, status=st)
+    _clean(st)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        assert torch.equal(out[e], (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)), e
+
+
+@pytest.mark.parametrize("R,Cn", [(1, 8), (63, 264), (65, 2048), (1000, 520), (8192, 72)])
+def test_col_sum(R, Cn):
+    from kernel_b200.ops.local import col_sum
+
+    x = _ints(R, Cn, seed=12)
+    assert torch.equal(col_sum(x), x.float().sum(0).to(torch.bfloat16))
+
+
+def test_col_sum_of_a_misaligned_matrix():
+    from kernel_b200.ops.local import col_sum
+
+    x = _ints(17 * 64 + 1, seed=13)[1:].view(17, 64)
+    assert torch.equal(col_sum(x), x.float().sum(0).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T,k,E,H,pad", [(0, 2, 8, 64, 1), (1, 1, 1, 8, 64), (3, 8, 256, 1032, 1), (130, 6, 64, 256, 64),
+                                         (777, 4, 1024, 72, 64), (40, 64, 100, 520, 1)])
+def test_expert_rows(T, k, E, H, pad):
+    """Row movement of a single-rank MoE layer: permutation, combine and its backward."""
+    from kernel_b200.ops.local import ExpertRows
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    idx = torch.rand((T, E), device=DEV, generator=g).argsort(1)[:, :k].to(torch.int32).contiguous()
+    x, w = _ints(T, H, seed=14), torch.randint(-3, 4, (T, k), device=DEV, generator=g).float()
+    st = _status()
+    er = ExpertRows(x, idx, E, pad=pad, status=st)
+    _clean(st)
+    count = torch.bincount(idx.reshape(-1).long(), minlength=E)
+    padded = (count + pad - 1) // pad * pad
+    assert torch.equal(er.count.long(), count) and torch.equal(er.padded.long(), padded)
+    assert torch.equal(er.start.long(), padded.cumsum(0) - padded)
+    slots = er.slots.long()
+    assert torch.equal(er.rows[slots], x.unsqueeze(1).expand(T, k, H))
+    real = torch.zeros(er.rows.shape[0], dtype=torch.bool, device=DEV)
+    real[slots.reshape(-1)] = True
+    used = int(padded.sum())
+    assert int(real.sum()) == T * k and not real[used:].any() and not er.rows[:used][~real[:used]].any()
+    y = _ints(er.rows.shape[0], H, seed=15)
+    assert torch.equal(er.combine(y, w), (y[slots].float() * w.unsqueeze(-1)).sum(1).to(torch.bfloat16))
+    assert torch.equal(er.combine(y, None), y[slots].float().sum(1).to(torch.bfloat16))
+    dy = _ints(T, H, seed=16)
+    dyr, dw = er.grad_rows(dy, y, w)
+    assert torch.equal(dyr[slots], (dy.unsqueeze(1).float() * w.unsqueeze(-1)).to(torch.bfloat16))
+    assert not dyr[:used][~real[:used]].any()
+    assert torch.equal(dw, (dy.unsqueeze(1).float() * y[slots].float()).sum(-1))
+
+
+def test_expert_rows_out_of_range_id_is_reported_and_skipped():
+    from kernel_b200.ops.local import ExpertRows
+
+    x, idx = _ints(4, 64, seed=17), torch.tensor([[0, 5], [1, -1], [2, 3], [3, 0]], dtype=torch.int32, device=DEV)
+    st = _status()
+    er = ExpertRows(x, idx, 4, status=st)
+    torch.cuda.synchronize()
+    assert st.cpu().tolist()[0] != 0
+    assert er.slots.cpu().tolist() == [[0, -1], [2, -1], [3, 4], [5, 1]]
+    assert torch.equal(er.combine(er.rows, None), torch.stack([x[0], x[1], 2 * x[2], 2 * x[3]]))
+
+
+@pytest.mark.parametrize("E,k,H,T", [(8, 2, 8, 1), (64, 6, 1032, 33), (256, 8, 7168, 300), (128, 4, 2880, 2048), (64, 33, 520, 70)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mode):
+    """Bit for bit; a traced call runs the general kernels."""
+    from kernel_b200.ops.dispatch_combine import MoEAllToAll
+
+    g = torch.Generator(device=DEV).manual_seed(H)
+    ctx = MoEAllToAll(E, k, H, T, dtype=dtype, device=torch.device(DEV))
+    x = torch.randn((T, H), device=DEV, generator=g).to(dtype)
+    idx = torch.rand((T, E), device=DEV, generator=g).argsort(1)[:, :k].to(torch.int32).contiguous()
+    w = torch.softmax(torch.randn((T, k), device=DEV, generator=g), -1)
+    out = ctx.dispatch_scale_combine(x, idx, w, mode)
+    ctx.enable_trace()
+    general = ctx.dispatch_scale_combine(x, idx, w, mode)
+    torch.cuda.synchronize()
+    ctx.heap.check_status()
+    assert torch.equal(out, general)
+    ctx.heap.close()
+
+
+@pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
+def test_mlp_with_hooks_equals_the_fused_block(activation):
+    """Hooks on the two linear layers run: the block then takes the general path."""
+    from kernel_b200.models import TrainableSequenceParallelMLP
+
+    torch.manual_seed(0)
+    mlp = TrainableSequenceParallelMLP(72, 136, 264, activation=activation, device=torch.device(DEV))
+    x = torch.randn(72, 136, device=DEV).to(torch.bfloat16)
+    fused = mlp(x)
+    seen = []
+    handle = mlp.up.register_forward_hook(lambda mod, inp, out: seen.append(out.shape))
+    plain = mlp(x)
+    handle.remove()
+    assert seen == [(72, 264)]
+    # the fused block's gelu and silu differ from torch's by at most one bf16 rounding of the hidden value
+    assert (fused.float() - plain.float()).norm() <= 2 ** -8 * plain.float().norm()
+    mlp.close()

@@ -69,3 +69,62 @@ def test_schedule_refuses_bad_problem():
     assert lib.kb_gemm_schedule(N.GEMM_RS, 100, 256, 0, 3, 0, 0, C.byref(blk), C.byref(nb)) == -1    # M % world
     assert lib.kb_gemm_schedule(N.GEMM_RS, 256, 256, 2, 2, 0, 0, C.byref(blk), C.byref(nb)) == -1    # rank out of range
     assert lib.kb_gemm_schedule(N.GEMM_AG, 256, 256, 0, 2, 1, 0, C.byref(blk), C.byref(nb)) == -1    # pairs need 256-row shards
+
+
+def _local(**kw):
+    a = N.LocalGemmArgs()
+    buf = C.create_string_buffer(4096 + 16)
+    base = (C.addressof(buf) + 15) & ~15
+    a.kind, a.M, a.N, a.K, a.pair = N.LOCAL_DENSE, 128, 256, 64, -1
+    a.A = a.B = a.out = base
+    for k, v in kw.items():
+        setattr(a, k, base + v if k in ("A", "bias", "pre_out", "pre_in") else v)
+    a._keepalive = buf
+    return a
+
+
+@pytest.mark.parametrize("kw,needle", [
+    (dict(M=0), "M,N,K > 0"),
+    (dict(K=60), "multiples of 8"),
+    (dict(N=100), "multiples of 8"),
+    (dict(a_mn=1, b_mn=1, M=100), "multiples of 8"),
+    (dict(a_mn=1), "only with B contiguous along N"),
+    (dict(kind=3), "unknown kind"),
+    (dict(act=4), "unknown kind"),
+    (dict(pre_in=0), "belong to an activation"),
+    (dict(kind=N.LOCAL_ROWS, groups=4), "bad groups"),
+    (dict(A=8), "16-byte aligned"),
+    (dict(bias=2), "16-byte aligned"),
+])
+def test_local_gemm_refuses_bad_problem(kw, needle):
+    a = _local(**kw)
+    assert N.lib().kb_gemm_local(C.byref(a), None) in (N.KB_ERR_ARG, N.KB_ERR_UNSUPPORTED)
+    assert needle in N.last_error()
+
+
+def test_moe_rows_refuse_misaligned_rows():
+    lib = N.lib()
+    buf = C.create_string_buffer(4096 + 16)
+    p = (C.addressof(buf) + 15) & ~15
+    assert lib.kb_moe_permute(p + 2, p, 1, 1, 4, 8, 1, p, p, p, p, p, p, None) == N.KB_ERR_ARG and "16-byte aligned" in N.last_error()
+    assert lib.kb_moe_permute(p, p + 2, 1, 1, 4, 8, 1, p, p, p, p, p, p, None) == N.KB_ERR_ARG and "4-byte aligned" in N.last_error()
+    assert lib.kb_moe_grad_rows(p + 2, p, p, p, 1, 1, 4, 8, p, p, p, p, p, None) == N.KB_ERR_ARG
+
+
+def test_local_gemm_tile_rule_gives_launchable_configurations():
+    """Whatever the sizes, the picked tile has a legal width for its layout, a pair has rows
+    for both CTAs and a split has k blocks for every member."""
+    import random
+
+    rng = random.Random(0)
+    lib = N.lib()
+    pair, bn, split = C.c_int(), C.c_int(), C.c_int()
+    for _ in range(3000):
+        M, Nn, K = (8 * int(2 ** rng.uniform(0, 12)) for _ in range(3))
+        a_mn, b_mn = rng.choice([(0, 0), (0, 1), (1, 1)])
+        sms = rng.choice([148, 132, 16, 2])
+        assert lib.kb_gemm_local_config(M, Nn, K, a_mn, b_mn, sms, C.byref(pair), C.byref(bn), C.byref(split)) == N.KB_OK
+        per_cta = bn.value // 2 if pair.value else bn.value
+        assert 64 <= bn.value <= 256 and (per_cta % 64 == 0 if b_mn else bn.value % 32 == 0)
+        assert pair.value == 0 or M > 128
+        assert 1 <= split.value <= (8, 4, 1)[pair.value] and split.value <= (K + 63) // 64
