@@ -152,6 +152,26 @@ __device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
+// One stage of a GEMM: the expected bytes (0: this CTA expects none) and the boxes of both
+// operands, issued by one elected lane.  One election instead of three: the issuing
+// warp is what bounds narrow tiles.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_ab_warp(uint32_t own_bar, uint32_t tx_bytes, uint32_t bar, uint32_t a_dst, const void* a_map, int32_t ax,
+                                                 int32_t ay, int32_t az, uint32_t b_dst, const void* b_map, int32_t bx, int32_t by, int32_t bz) {
+#define KB_LOAD_AB(GROUP)                                                                                                          \
+  asm volatile(                                                                                                                    \
+      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\t"                                                                   \
+      "setp.ne.and.u32 e, %1, 0, q;\n\t"                                                                                           \
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"                                                              \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4, {%5, %6, %7}], [%2];\n\t"    \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%8], [%9, {%10, %11, %12}], [%2];\n\t}" \
+      ::"r"(own_bar), "r"(tx_bytes), "r"(bar), "r"(a_dst), "l"(a_map), "r"(ax), "r"(ay), "r"(az), "r"(b_dst), "l"(b_map), "r"(bx), \
+      "r"(by), "r"(bz)                                                                                                             \
+      : "memory")
+  if constexpr (kPair) KB_LOAD_AB(".cta_group::2");
+  else KB_LOAD_AB("");
+#undef KB_LOAD_AB
+}
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
