@@ -192,6 +192,11 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, const void* smem_
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_src, int32_t x, int32_t y, int32_t z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 // Untiled bulk copies (the same engine as TMA, no tensor map): both addresses
 // 16-byte aligned, size a multiple of 16 bytes.  The load completes on an
 // mbarrier of this CTA; the store belongs to the issuing thread's bulk group.

@@ -399,7 +399,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.split = c.split;
   p.a_slot = p.a_rows * BK * 2;
   p.b_slot = (c.pair ? c.bn / 2 : c.bn) * BK * 2;
-  const int tables = grouped ? (3 * groups + 1) * 4 : 4;
+  const int tables = (grouped ? (3 * groups + 1) * 4 : 4) + (contract ? OUT_BYTES : 0);  // what the ring leaves room for
   p.stages = ring_stages(p.a_slot, p.b_slot, tables);
   // the last A slot is read up to 128 rows far: the B slots behind it cover that
   if (p.stages < 2 || p.stages * p.b_slot < 16384) {
@@ -432,6 +432,10 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   rc = b_mn ? make_tmap3(&p.tmB, a->B, a->N, a->K, bz, 64, BK)
             : make_tmap3(&p.tmB, a->B, a->K, a->N, bz, BK, c.pair ? c.bn / 2 : c.bn);
   if (rc != KB_OK) return rc;
+  if (contract) {
+    rc = make_tmap3(&p.tmOut, a->out, a->N, a->M, groups, 64, 32);
+    if (rc != KB_OK) return rc;
+  }
   const int cluster = (c.pair ? 2 : 1) * c.split;
   int grid;
   if (c.split > 1) {

@@ -52,6 +52,8 @@ constexpr int MAX_GROUPS = 1024;
 constexpr int BAR_BYTES = 256;
 constexpr int MN_BLOCK_BYTES = BK * 128;  // M/N-contiguous operand: one box of 64 k rows x 64 elements
 constexpr int SMEM_MAX = 232448;
+constexpr int OUT_BOX_BYTES = 32 * 128;   // contract: 32 rows x 64 columns, staged for a TMA store
+constexpr int OUT_BYTES = EPI_WARPS * 2 * OUT_BOX_BYTES;  // two boxes per epilogue warp
 constexpr int CHUNK_COLS = 32;            // split: columns are exchanged in chunks of 32
 
 enum Kind { DENSE = 0, ROWS = 1, CONTRACT = 2 };
@@ -62,6 +64,7 @@ enum Act { ACT_NONE = 0, ACT_GELU = 1, ACT_RELU = 2, ACT_SILU = 3 };
 
 struct alignas(64) Params {
   CUtensorMap tmA, tmB;
+  CUtensorMap tmOut;  // contract: the output, written with TMA stores
   int M, N, K;
   int MBQ, NB, KB;   // scheduling blocks (128 or 256 rows), column blocks, k blocks of the whole contraction
   int bn;            // tile columns
@@ -225,7 +228,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sm_a = base;
   uint8_t* sm_b = sm_a + p.stages * p.a_slot;
-  uint8_t* sm_bar = sm_b + p.stages * p.b_slot;
+  uint8_t* sm_out = sm_b + p.stages * p.b_slot;  // 1024-byte aligned: slots are multiples of eight 128-byte rows
+  uint8_t* sm_bar = sm_out + (kKind == CONTRACT ? OUT_BYTES : 0);
   uint64_t* full = reinterpret_cast<uint64_t*>(sm_bar);
   uint64_t* empty = full + MAX_STAGES;
   uint64_t* tfull = empty + MAX_STAGES;
@@ -514,6 +518,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     const int q = warp & 3;
     const int turn = (warp - 4) >> 2;
     uint32_t it = 0;
+    int box_no = 0;  // contract: staging boxes used by this warp
     for (int pos = sched_id; pos < total_tiles; pos += sched_n, ++it) {
       const Tile t = tile_at(pos);
       if (p.bias != nullptr) {
@@ -521,7 +526,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
         const int col = t.n0 + 8 * lane;
         if (8 * lane < p.bn && col < p.N) kb::touch_nc(p.bias + col);
       }
-      const size_t out0 = kKind == CONTRACT ? static_cast<size_t>(t.group) * p.M * p.N : 0;
       const int cols = min(p.bn, p.N - t.n0);
 #pragma unroll 1
       for (int hb = 0; hb < kHalves; ++hb) {
@@ -550,11 +554,48 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
         };
         const int last = gr0 < t.row_end ? cols : 0;
         if (turn * 64 >= last) release();
+        if constexpr (kKind == CONTRACT) {
+          // Few k blocks per tile: the output is the traffic.  Staged boxes leave as whole
+          // 128-byte lines while the epilogue goes on (rows and columns outside the tensor are
+          // clipped); unlike in a long contraction the mainloop leaves shared memory
+          // bandwidth for it.  64 experts, 128 rows, 2048 x 1024: 85 us stored from registers,
+          // 75 staged; writing 268 MB alone takes a memset 72.
+#pragma unroll 1
+          for (int c = turn * 64; c < last; c += 128) {
+            uint8_t* box = sm_out + ((warp - 4) * 2 + (box_no++ & 1)) * OUT_BOX_BYTES;
+            uint32_t r[2][32];
+            if (t.kb == 0) {  // an empty group: nothing was accumulated
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[0][i] = r[1][i] = 0u;
+            } else {
+              kb::tmem_ld_32x32(taddr + c, r[0]);
+              kb::tmem_ld_32x32(taddr + c + 32, r[1]);
+            }
+            if (lane == 0) kb::bulk_wait_group_read<1>();  // the box's previous store has read it
+            __syncwarp();
+            if (t.kb != 0) kb::tmem_ld_wait();
+            if (c + 128 >= last) release();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float f[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j >> 2][(j & 3) * 8 + e]);
+              *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) * 16)) = pack8(f);
+            }
+            kb::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              kb::tma_store_3d(&p.tmOut, box, t.n0 + c, gr0, t.group);
+              kb::bulk_commit_group();
+            }
+          }
+          continue;
+        }
 #pragma unroll 1
         for (int c = turn * 64; c < last; c += 128) {
           const bool two = c + 32 < last;
           const int col = t.n0 + c;
-          const size_t at0 = out0 + static_cast<size_t>(row) * p.N + col;
+          const size_t at0 = static_cast<size_t>(row) * p.N + col;
           uint4 at[8];
           if constexpr (kEpi == EPI_SLOPE) {  // fetched before the accumulator is read
 #pragma unroll
@@ -564,14 +605,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
             }
           }
           uint32_t r[2][32];
-          if (kKind == CONTRACT && t.kb == 0) {  // an empty group: nothing was accumulated
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[0][i] = r[1][i] = 0u;
-          } else {
-            kb::tmem_ld_32x32(taddr + c, r[0]);
-            if (two) kb::tmem_ld_32x32(taddr + c + 32, r[1]);
-            kb::tmem_ld_wait();
-          }
+          kb::tmem_ld_32x32(taddr + c, r[0]);
+          if (two) kb::tmem_ld_32x32(taddr + c + 32, r[1]);
+          kb::tmem_ld_wait();
           if (c + 128 >= last) release();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -591,6 +627,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
         }
       }
     }
+    if (kKind == CONTRACT && lane == 0) kb::bulk_wait_group<0>();
   } else if (warp == 4 && p.split > 1) {
     // The members of a cluster work on one tile each: wait here until this CTA's partial is complete.
     if (!kb::mbar_wait_bounded(&tfull[0], 0u, p.limit_ns, 1000)) {
