@@ -175,12 +175,15 @@ Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shap
   return best;
 }
 
-// Contractions over a group's rows are short (a few k blocks), the outputs are the
-// traffic: the widest tile of one CTA (64 experts, 128 rows, 2048 x 1024: 79 us, pair 98 us).
-Config contract_config(int M, int N, int shape) {
-  (void)M;
+// Contractions over a group's rows.  A few k blocks: the outputs are the traffic, the widest
+// tile of one CTA, a pair's hand-overs cost more than its smaller operand traffic saves.
+// More: pairs.  The row capacity holds up to 63 padding rows per group; the line lies between
+//   64 experts, 128 rows, 2048 x 1024:   one CTA 76 us, pair 90
+//   32 experts, 512 rows, 2048 x 2048:   one CTA 155 us, pair 130
+//   8 experts, 500 rows, 4096 x 4096:    one CTA 151 us, pair 125
+Config contract_config(int M, int N, int K, int groups, int shape) {
   Config c;
-  c.pair = shape > 0;
+  c.pair = shape >= 0 ? shape > 0 : M > 128 && K / groups >= 352;
   c.bn = N <= 64 && !c.pair ? 64 : N <= 128 ? 128 : 256;
   c.split = 1;
   return c;
@@ -365,7 +368,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &c);
     if (rc != KB_OK) return rc;
   } else {
-    c = contract ? contract_config(a->M, a->N, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape);
+    c = contract ? contract_config(a->M, a->N, a->K, groups, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape);
   }
   if (a->bn > 0) c.bn = a->bn;
   if (a->split > 0) c.split = a->split;
