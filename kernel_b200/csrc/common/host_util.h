@@ -39,6 +39,26 @@ void* driver_fn(const char* name);
   } while (0)
 
 #ifdef __CUDACC__
+// Launch attribute of a kernel that begins with wait_for_previous_launch() (ptx.cuh): it may
+// be set up while the previous kernel of the stream still runs.
+inline cudaLaunchAttribute overlap_launch() {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+template <typename... Args>
+cudaError_t launch_after(void (*kernel)(Args...), dim3 grid, dim3 block, void* stream, Args... args) {
+  cudaLaunchAttribute attr = overlap_launch();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // First failure wins; later ones are dropped so the host sees the root cause.
 __device__ __forceinline__ void report_status(uint32_t* status, uint32_t code, uint32_t site, uint32_t what,
                                               uint32_t epoch) {

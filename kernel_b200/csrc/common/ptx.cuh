@@ -468,6 +468,15 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   return v;
 }
 
+// Start of a kernel launched with the overlap_launch attribute: waits until the previous
+// kernel of the stream has ended and its writes are visible, then lets the next one be set up.
+// Nothing that another kernel may write, and no output, is touched before it.  Without the
+// attribute the wait returns at once.
+__device__ __forceinline__ void wait_for_previous_launch() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Loads 16 bytes of read-only data and drops them: the line is in L1 afterwards.
 __device__ __forceinline__ void touch_nc(const void* p) {
   asm volatile("{\n\t.reg .b32 a, b, c, d;\n\tld.global.nc.v4.u32 {a, b, c, d}, [%0];\n\t}" ::"l"(p));

@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     kb::tma_prefetch_desc(&p.tmA);
     kb::tma_prefetch_desc(&p.tmB);
   }
+  kb::wait_for_previous_launch();  // barriers, tensor memory and descriptors are set up under the end of that one
   if constexpr (kKind != DENSE) {
     for (int e = tid; e < p.groups; e += THREADS) {
       g_start[e] = p.row_start[e];

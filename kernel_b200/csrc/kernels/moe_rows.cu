@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(PERM_THREADS) moe_permute_kernel(const MoePara
   __shared__ int32_t start[MAX_EXPERTS];
   __shared__ int32_t ent_e[MAX_ENT], ent_slot[MAX_ENT];
   __shared__ int32_t s_warp[PERM_WARPS];
+  kb::wait_for_previous_launch();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = min(static_cast<int>(blockIdx.x) * p.tok_per_cta, p.T);
   const int t1 = min(t0 + p.tok_per_cta, p.T);
@@ -190,6 +191,7 @@ struct CombineParams {
 
 // One CTA: one token and 1/splits of its row; a thread keeps eight rows' loads in flight.
 __global__ void __launch_bounds__(128) moe_combine_kernel(const CombineParams p) {
+  kb::wait_for_previous_launch();
   const int t = blockIdx.x / p.splits;
   const int part = blockIdx.x - t * p.splits;
   const int per = (p.vecs + p.splits - 1) / p.splits;
@@ -240,6 +242,7 @@ struct GradParams {
 // One CTA per token; the CTAs behind the last token zero-fill the padding rows of dyr, four
 // per expert (one: 17.7 us for 1024 tokens of 4 KB, top-8 of 64; four: 14.0).
 __global__ void __launch_bounds__(THREADS) moe_grad_rows_kernel(const GradParams p) {
+  kb::wait_for_previous_launch();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (static_cast<int>(blockIdx.x) >= p.T) {
     for (int u = blockIdx.x - p.T; u < 4 * p.E; u += gridDim.x - p.T) {
@@ -363,8 +366,7 @@ extern "C" int kb_moe_permute(const void* x, const int32_t* indices, int T, int 
   if (per > MAX_ENT / k) per = MAX_ENT / k;
   p.tok_per_cta = per;
   const int grid = T > 0 ? (T + per - 1) / per : 1;
-  moe_permute_kernel<<<grid, PERM_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  KB_CUDA_OK(cudaGetLastError());
+  KB_CUDA_OK(kb::launch_after(moe_permute_kernel, grid, PERM_THREADS, stream, p));
   return KB_OK;
 }
 
@@ -378,8 +380,7 @@ extern "C" int kb_moe_combine(const void* y, const int32_t* slots, const float* 
   if (rc != KB_OK) return rc;
   CombineParams p = {T, k, hidden / 8, 1, static_cast<const uint4*>(y), slots, weights, static_cast<uint4*>(out)};
   while (T * p.splits < 4 * sms && p.vecs > 32 * p.splits) p.splits *= 2;  // few tokens: spread a row over several CTAs
-  moe_combine_kernel<<<T * p.splits, 128, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  KB_CUDA_OK(cudaGetLastError());
+  KB_CUDA_OK(kb::launch_after(moe_combine_kernel, T * p.splits, 128, stream, p));
   return KB_OK;
 }
 
@@ -392,7 +393,6 @@ extern "C" int kb_moe_grad_rows(const void* dy, const void* y, const int32_t* sl
   if (rc != KB_OK) return rc;
   GradParams p = {T, k, experts, hidden / 8, static_cast<const uint4*>(dy), static_cast<const uint4*>(y), slots, weights,
                   static_cast<uint4*>(dyr), dw, row_start, row_count, row_padded};
-  moe_grad_rows_kernel<<<T + 4 * (experts < 64 ? experts : 64), THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  KB_CUDA_OK(cudaGetLastError());
+  KB_CUDA_OK(kb::launch_after(moe_grad_rows_kernel, T + 4 * (experts < 64 ? experts : 64), THREADS, stream, p));
   return KB_OK;
 }

@@ -230,6 +230,47 @@ def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mo
     ctx.heap.close()
 
 
+def test_overlapped_launches_keep_their_order_eagerly_and_in_a_graph():
+    """A chain in which every kernel reads what the one before wrote, also across a fork and a
+    join of streams, with torch kernels and copies in between."""
+    from kernel_b200.ops.local import product
+
+    a, eye = _ints(256, 512, seed=20), torch.eye(512, dtype=torch.bfloat16, device=DEV)
+    side = torch.cuda.Stream()
+    w = torch.zeros(512, 512, dtype=torch.bfloat16, device=DEV)
+    res = torch.zeros(256, 512, dtype=torch.bfloat16, device=DEV)
+    other = torch.zeros(256, 512, dtype=torch.bfloat16, device=DEV)
+
+    def chain():
+        cur = torch.cuda.current_stream()
+        w.zero_()
+        w.copy_(eye)                     # read by the next product
+        y = a
+        for _ in range(6):
+            y = product(y, w)            # each reads the one before
+        w.mul_(2.0)                      # after the last read, before the next
+        side.wait_stream(cur)
+        with torch.cuda.stream(side):
+            other.copy_(product(a, w))
+        y = product(y, w)
+        cur.wait_stream(side)
+        res.copy_(product(other, eye))   # first kernel behind the join
+        res.add_(y)
+
+    chain()
+    torch.cuda.synchronize()
+    assert torch.equal(res, 4 * a)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for _ in range(3):
+        res.zero_()
+        other.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(res, 4 * a)
+
+
 @pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
 def test_mlp_with_hooks_equals_the_fused_block(activation):
     """Hooks on the two linear layers run: the block then takes the general path."""
