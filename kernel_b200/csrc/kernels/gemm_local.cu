@@ -139,8 +139,12 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
 // products.  With few rows the weights are the traffic and every shape that keeps the
 // SMs loading is near the memory time; the second-order term breaks such ties.
 //   64 experts, 2048 x 1024, 3 rows each: 32 x 256 tiles 45 us, 32 x 64 (first version) 68 us
+// The epilogue that reads saved values back costs a pair more than one CTA (a pair's
+// accumulators are free only when both have stored): pairs from about 400 rows per group on.
+//   64 experts, 128 rows, 2048 x 1024:  pair 90 us, one CTA 79;  32 experts, 256 rows, 2048 x 2048: 114 and 103
+//   8 experts, 500 rows, 4096 x 4096:   pair 124 us, one CTA 131
 //   64 experts, 128 rows each: 128 x 192 tiles 61 us;  8 experts, 1000 rows of 4096 x 4096: pairs 198 us, one CTA 218 us
-Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape) {
+Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape, bool slope) {
   Config best;
   best.bn = b_mn ? 128 : 256;
   best.pair = shape > 0;
@@ -152,7 +156,7 @@ Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shap
   const double memory = 2.0 * (used * groups * N * static_cast<double>(K) + static_cast<double>(M) * (N + K)) / 6500.0 + 6600.0;
   for (int s = 0; s < 4; ++s) {
     const bool pair = s == 3;
-    if (shape >= 0 ? pair != (shape > 0) : pair && sms < 2) continue;
+    if (shape >= 0 ? pair != (shape > 0) : pair && (sms < 2 || (slope && n < 448.0))) continue;
     const int rows = pair ? 256 : 32 << s;
     const double blocks = n + 2.0 * sqrt(n) <= rows ? used : n / rows + 0.5;
     for (int bn = 64; bn <= 256; bn += 64) {
@@ -368,7 +372,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &c);
     if (rc != KB_OK) return rc;
   } else {
-    c = contract ? contract_config(a->M, a->N, a->K, groups, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape);
+    c = contract ? contract_config(a->M, a->N, a->K, groups, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape, a->pre_in != nullptr);
   }
   if (a->bn > 0) c.bn = a->bn;
   if (a->split > 0) c.split = a->split;
