@@ -58,6 +58,38 @@ def _stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
 
 
+def _check_operand(t: torch.Tensor, name: str, dims: int, device: torch.device) -> None:
+    if t.dtype != torch.bfloat16 or t.dim() != dims or not t.is_contiguous() or t.device != device:
+        raise ValueError(f"{name} must be a contiguous {dims}-D bf16 tensor on {device}")
+
+
+def _check_results(shape, device: torch.device, *results: Optional[torch.Tensor]) -> None:
+    """Matrices that are read or written by their address, row for row like the product."""
+    for t in results:
+        if t is not None and (t.shape != shape or t.dtype != torch.bfloat16 or not t.is_contiguous() or t.device != device):
+            raise ValueError(f"results and saved values must be contiguous bf16 matrices of shape {tuple(shape)} on {device}")
+
+
+def _check_choices(t: torch.Tensor, name: str, dtype: torch.dtype, shape, device: torch.device) -> None:
+    if t.dtype != dtype or t.shape != shape or not t.is_contiguous() or t.device != device:
+        raise ValueError(f"{name} must be contiguous {dtype} of shape {tuple(shape)} on {device}")
+
+
+def _check_table(start: torch.Tensor, count: torch.Tensor, groups: int, device: torch.device) -> None:
+    for t in (start, count):
+        if t.dtype != torch.int32 or t.shape != (groups,) or not t.is_contiguous() or t.device != device:
+            raise ValueError(f"group tables must be contiguous int32 [{groups}] on {device}")
+
+
+def _expert_matrices(b: torch.Tensor) -> torch.Tensor:
+    """``b[E, ...]`` as one block.  Matrices that are contiguous one by one (every second
+    expert of a larger tensor, one matrix expanded over the experts) are gathered; a
+    transposed matrix is not an operand layout, ``b_t`` says which one is meant."""
+    if b.dim() == 3 and not b.is_contiguous() and b[:1].is_contiguous():
+        return b.contiguous()
+    return b
+
+
 def _args(kind: int, M: int, Nn: int, K: int, status: Optional[torch.Tensor]) -> N.LocalGemmArgs:
     args = N.LocalGemmArgs()
     args.kind, args.M, args.N, args.K, args.pair = kind, M, Nn, K, -1
@@ -80,8 +112,13 @@ def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = Non
 
     ``act``: the activation of the rounded product, which ``pre_out`` also receives;
     with ``pre_in`` the product is multiplied by the activation's slope there."""
+    _check_operand(a, "a", 2, a.device)
+    _check_operand(b, "b", 2, a.device)
     K, M = a.shape if a_t else a.shape[::-1]
-    Nn = b.shape[1] if b_t else b.shape[0]
+    Kb, Nn = b.shape if b_t else b.shape[::-1]
+    if Kb != K:
+        raise ValueError("inner dimensions differ")
+    _check_results((M, Nn), a.device, out, pre_out, pre_in)
     if not a.is_cuda:
         A, B = a.float(), b.float()
         res = (A.t() if a_t else A) @ (B if b_t else B.t())
@@ -115,9 +152,16 @@ def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: t
                  out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Rows ``start[e] .. start[e] + count[e]`` of ``a[R, K]`` times ``b[e]`` transposed
     (``b[E, N, K]``, ``b_t``: ``b[E, K, N]``).  Rows outside every group are left alone."""
+    b = _expert_matrices(b)
+    _check_operand(a, "a", 2, a.device)
+    _check_operand(b, "b", 3, a.device)
     R, K = a.shape
     E = b.shape[0]
-    Nn = b.shape[2] if b_t else b.shape[1]
+    Kb, Nn = b.shape[1:] if b_t else (b.shape[2], b.shape[1])
+    if Kb != K:
+        raise ValueError("inner dimensions differ")
+    _check_table(start, count, E, a.device)
+    _check_results((R, Nn), a.device, out, pre_out, pre_in)
     if out is None:
         out = torch.empty((R, Nn), dtype=torch.bfloat16, device=a.device)
     if R == 0:
@@ -144,7 +188,12 @@ def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, coun
     """``out[e] = a[rows of e]^T @ b[rows of e]`` for ``a[R, M]``, ``b[R, N]``.  Groups start at
     multiples of ``ROW_ALIGN``; rows between a group's last and the next multiple are
     zero in one operand and finite in the other."""
+    _check_operand(a, "a", 2, a.device)
+    _check_operand(b, "b", 2, a.device)
     (R, M), Nn, E = a.shape, b.shape[1], start.shape[0]
+    if b.shape[0] != R:
+        raise ValueError("a and b have different numbers of rows")
+    _check_table(start, count, E, a.device)
     if not a.is_cuda or R == 0:
         out = torch.zeros((E, M, Nn), dtype=torch.bfloat16, device=a.device)
         for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
@@ -167,7 +216,9 @@ class ExpertRows:
     ``R`` is the capacity ``T * k + E * (pad - 1)``: no count travels to the host."""
 
     def __init__(self, x: torch.Tensor, indices: torch.Tensor, experts: int, pad: int = 1, status: Optional[torch.Tensor] = None):
+        _check_operand(x, "x", 2, x.device)
         (T, H), k, dev = x.shape, indices.shape[1], x.device
+        _check_choices(indices, "indices", torch.int32, (T, k), dev)
         rows = torch.empty((T * k + experts * (pad - 1), H), dtype=torch.bfloat16, device=dev)
         self._set(rows, torch.empty(3 * experts + T * k, dtype=torch.int32, device=dev), T, k, experts)
         N.check(N.lib().kb_moe_permute(x.data_ptr(), indices.data_ptr(), T, k, experts, H, pad, self.rows.data_ptr(),
@@ -187,8 +238,14 @@ class ExpertRows:
         er._set(rows, table, T, k, experts)
         return er
 
+    def _check(self, y: torch.Tensor, weights: Optional[torch.Tensor]) -> None:
+        _check_results(self.rows.shape, self.rows.device, y)
+        if weights is not None:
+            _check_choices(weights, "weights", torch.float32, (self.T, self.k), self.rows.device)
+
     def combine(self, y: torch.Tensor, weights: Optional[torch.Tensor]) -> torch.Tensor:
         """``out[t] = sum_j weights[t, j] * y[slots[t, j]]`` (``None``: unit weights)."""
+        self._check(y, weights)
         out = torch.empty((self.T, self.H), dtype=torch.bfloat16, device=y.device)
         N.check(N.lib().kb_moe_combine(y.data_ptr(), self.slots.data_ptr(), _ptr(weights), self.T, self.k, self.H, out.data_ptr(),
                                        _stream(y.device)))
@@ -196,6 +253,8 @@ class ExpertRows:
 
     def grad_rows(self, dy: torch.Tensor, y: torch.Tensor, weights: torch.Tensor):
         """Backward of ``combine``: ``(dY rows, d weights)``."""
+        self._check(y, weights)
+        _check_results((self.T, self.H), self.rows.device, dy)
         dyr = torch.empty_like(y)
         dw = torch.empty((self.T, self.k), dtype=torch.float32, device=dy.device)
         N.check(N.lib().kb_moe_grad_rows(dy.data_ptr(), y.data_ptr(), self.slots.data_ptr(), weights.data_ptr(), self.T, self.k, self.E,
