@@ -41,6 +41,13 @@ def _launch(args: N.GemmArgs, device: torch.device) -> None:
     launch_count += 1
 
 
+def _check_out(out: torch.Tensor, rows: int, cols: int, device: torch.device) -> None:
+    """The kernel writes ``rows x cols`` values from ``out``'s address on, whatever its shape
+    (a flat or a larger buffer is filled from its start)."""
+    if out.dtype != torch.bfloat16 or not out.is_contiguous() or out.device != device or out.numel() < rows * cols:
+        raise ValueError(f"out must be a contiguous bf16 tensor of at least {rows} x {cols} elements on {device}")
+
+
 def _local_args(status: Optional[torch.Tensor]) -> N.LocalGemmArgs:
     """Argument block of a product whose operands are all on this GPU."""
     args = N.LocalGemmArgs()
@@ -65,7 +72,8 @@ def _run_local(ctx, a: torch.Tensor, w: torch.Tensor, bias, bias_scale: float, o
     args = ctx._hot
     if args is None:
         args = ctx._hot = _local_args(ctx.status)
-    (args.M, args.K), args.N = a.shape, out.shape[1]
+    _check_out(out, a.shape[0], w.shape[0], a.device)
+    (args.M, args.K), args.N = a.shape, w.shape[0]
     args.A, args.B, args.out = a.data_ptr(), w.data_ptr(), out.data_ptr()
     args.bias = bias.data_ptr() if bias is not None else None
     args.bias_scale = bias_scale
@@ -198,6 +206,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
         return res
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
+    _check_out(out, M, Nn, a.device)
     args = _local_args(status)
     args.M, args.N, args.K = M, Nn, K
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()

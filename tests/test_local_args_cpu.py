@@ -113,3 +113,27 @@ def test_expert_rows_refuse_what_they_would_misread():
                    (_z(R, K), torch.zeros(R - 1, 2, dtype=torch.int32)), (_z(K, R).t(), torch.zeros(R, 2, dtype=torch.int32))]:
         with pytest.raises(ValueError):
             L.ExpertRows(x, idx, E)
+
+
+@pytest.mark.parametrize("shape", [(8, 24), (8 * 24,), (24, 8), (8, 64), (2, 8, 24)])
+def test_one_rank_product_takes_its_columns_from_the_weights(shape, monkeypatch):
+    """``out`` is an address: a flat or a larger buffer receives the same matrix."""
+    from types import SimpleNamespace
+
+    from kernel_b200.ops import gemm as G
+
+    seen = []
+    monkeypatch.setattr(G, "_launch_local", lambda args, device: seen.append((args.M, args.N, args.K)))
+    G._run_local(SimpleNamespace(_hot=None, status=None), _z(R, K), _z(Nn, K), None, 1.0, _z(*shape))
+    assert seen == [(R, Nn, K)]
+
+
+@pytest.mark.parametrize("out", [_z(R, Nn - 8), _z(R * Nn, dtype=torch.float16), _z(R, 2 * Nn)[:, :Nn], _z(1).expand(R, Nn)])
+def test_one_rank_product_refuses_out(out, monkeypatch):
+    from types import SimpleNamespace
+
+    from kernel_b200.ops import gemm as G
+
+    monkeypatch.setattr(G, "_launch_local", lambda args, device: None)
+    with pytest.raises(ValueError):
+        G._run_local(SimpleNamespace(_hot=None, status=None), _z(R, K), _z(Nn, K), None, 1.0, out)
