@@ -98,8 +98,7 @@ class TrainableSequenceParallelMLP(torch.nn.Module):
         up, down = self.up, self.down
         if (x_local.is_cuda and self.activation in ACTS and _plain(up, ColumnParallelLinear) and _plain(down, RowParallelLinear)
                 and down.weight.dtype == torch.bfloat16 and down.weight.shape == (down.fwd.N, up.weight.shape[0])):
-            up.fwd.check(x_local.contiguous(), up.weight)
-            return LocalMLPFn.apply(x_local, up.weight, up.bias, down.weight, down.bias, self.activation, up.fwd.status)
+            return LocalMLPFn.apply(x_local, up.weight, up.bias, down.weight, down.bias, self.activation, up.fwd)
         h = self.up(x_local)
         if self.activation == "gelu":
             h = torch.nn.functional.gelu(h, approximate="tanh")

@@ -112,11 +112,15 @@ class LocalMLPFn(torch.autograd.Function):
     """``act(x @ w1^T + b1) @ w2^T + b2`` on one GPU: two products forward, four backward,
     the activation in the first one's epilogue (which keeps the value before it), its
     slope in the epilogue of the hidden gradient's product.  No transposed copy and no
-    elementwise pass: both were 40 % of a step at 8192 x 8192 x 29568."""
+    elementwise pass: both were 40 % of a step at 8192 x 8192 x 29568.  ``up`` is the
+    ``AGGemm`` context whose shape ``x`` and ``w1`` have to fit; operands of other strides
+    are made contiguous first, as the two linear layers do."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, act, status):
+    def forward(ctx, x, w1, b1, w2, b2, act, up):
         x, w1, w2 = x.contiguous(), w1.contiguous(), w2.contiguous()
+        up.check(x, w1)
+        status = getattr(up, "status", None)  # CPU contexts have none
         pre = torch.empty((x.shape[0], w1.shape[0]), dtype=x.dtype, device=x.device)
         h = product(x, w1, b1, act=act, pre_out=pre, status=status)
         ctx.act, ctx.status = act, status

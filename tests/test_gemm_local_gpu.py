@@ -288,3 +288,17 @@ def test_mlp_with_hooks_equals_the_fused_block(activation):
     # the fused block's gelu and silu differ from torch's by at most one bf16 rounding of the hidden value
     assert (fused.float() - plain.float()).norm() <= 2 ** -8 * plain.float().norm()
     mlp.close()
+
+
+def test_mlp_with_strided_parameters():
+    """Transposed views as weights and input: the fused block gives what it gives for their copies."""
+    from kernel_b200.models import TrainableSequenceParallelMLP
+
+    torch.manual_seed(1)
+    mlp = TrainableSequenceParallelMLP(72, 136, 264, device=torch.device(DEV))
+    x = torch.randn(72, 136, device=DEV).to(torch.bfloat16)
+    want = mlp(x)
+    for t in (mlp.up.weight, mlp.down.weight):
+        t.data = t.data.t().contiguous().t()
+    assert torch.equal(mlp(x.t().contiguous().t()), want)
+    mlp.close()

@@ -137,3 +137,26 @@ def test_one_rank_product_refuses_out(out, monkeypatch):
     monkeypatch.setattr(G, "_launch_local", lambda args, device: None)
     with pytest.raises(ValueError):
         G._run_local(SimpleNamespace(_hot=None, status=None), _z(R, K), _z(Nn, K), None, 1.0, out)
+
+
+@pytest.mark.parametrize("which", ["x", "up", "down"])
+def test_fused_mlp_takes_operands_of_any_strides(which):
+    """The block of one GPU accepts what the two linear layers accept: a transposed view in
+    place of the input or of either weight, forward and backward."""
+    from kernel_b200.ops.autograd import LocalMLPFn
+    from kernel_b200.ops.gemm import AGGemm
+
+    g = torch.Generator().manual_seed(1)
+    make = lambda *shape: torch.randn(*shape, generator=g).to(torch.bfloat16)
+    x, w1, b1, w2, b2, dy = make(R, K), make(Nn, K), make(Nn), make(K, Nn), make(K), make(R, K)
+    grads = []
+    for strided in (False, True):
+        args = {"x": x, "up": w1, "down": w2}
+        if strided:
+            args[which] = args[which].t().contiguous().t()
+            assert not args[which].is_contiguous()
+        leaves = [args["x"], args["up"], b1, args["down"], b2]
+        leaves = [t.detach().requires_grad_(True) for t in leaves]
+        y = LocalMLPFn.apply(*leaves, "silu", AGGemm(R, K))
+        grads.append([y.detach(), *torch.autograd.grad(y, leaves, dy)])
+    assert all(torch.equal(p, q) for p, q in zip(*grads))
