@@ -13,6 +13,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from .._native import ACTS
 from ..ops.autograd import ColumnParallelLinear, LocalMLPFn, RowParallelLinear
@@ -49,8 +50,13 @@ class SequenceParallelMLP:
             return torch.nn.functional.silu(h)
         raise ValueError(f"unknown activation {self.activation!r}")
 
+    def _plain(self) -> bool:
+        """One rank, and the up-projection and the activation are the block's own."""
+        return (self.world == 1 and self.activation in ACTS and type(self.up) is AGGemm
+                and getattr(self._act, "__func__", None) is SequenceParallelMLP._act)
+
     def __call__(self, x_local: torch.Tensor) -> torch.Tensor:
-        if x_local.is_cuda and self.world == 1 and self.activation in ACTS:
+        if x_local.is_cuda and self._plain():
             self.up.check(x_local, self.w1)
             h = product(x_local, self.w1, self.b1, act=self.activation, status=self.up.status)   # the activation in the product's epilogue
             return self.down(h, self.w2, self.b2)
@@ -76,9 +82,10 @@ class SequenceParallelMLP:
 
 
 def _plain(layer: torch.nn.Module, kind: type) -> bool:
-    """One rank, and nothing (a replacement, hooks) asks for the layer to be called by itself."""
-    return type(layer) is kind and layer.world == 1 and not (
-        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
+    """One rank, and nothing (a replacement, a ``forward`` set on the instance, hooks of the
+    layer or of all modules) asks for the layer to be called by itself."""
+    return type(layer) is kind and layer.world == 1 and "forward" not in vars(layer) and not (
+        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks or _has_any_global_hook())
 
 
 class TrainableSequenceParallelMLP(torch.nn.Module):

@@ -70,3 +70,44 @@ def test_moe_layer_on_cpu_ranks_world3():
     from _mp import run_ranks
 
     assert all(run_ranks(_moe_layer_ranks, 3))
+
+
+def test_layers_that_are_asked_for_by_themselves_are_not_fused():
+    """The one-GPU block passes its linear layers by only when nothing could notice: no hook of a
+    layer or of all modules, no replaced layer, no ``forward`` set on the instance."""
+    from torch.nn.modules import module as M
+
+    from kernel_b200.models.tp_mlp import TrainableSequenceParallelMLP, _plain
+    from kernel_b200.ops.autograd import ColumnParallelLinear
+
+    up = TrainableSequenceParallelMLP(8, 16, 24).up
+    assert _plain(up, ColumnParallelLinear)
+    hook = lambda *a: None
+    for register in (up.register_forward_hook, up.register_forward_pre_hook, up.register_full_backward_hook, up.register_full_backward_pre_hook,
+                     M.register_module_forward_hook, M.register_module_forward_pre_hook, M.register_module_full_backward_hook,
+                     M.register_module_full_backward_pre_hook):
+        handle = register(hook)
+        assert not _plain(up, ColumnParallelLinear), register
+        handle.remove()
+        assert _plain(up, ColumnParallelLinear)
+    up.forward = lambda x: x
+    assert not _plain(up, ColumnParallelLinear)
+
+
+def test_inference_block_calls_what_was_put_in_place_of_its_parts():
+    from kernel_b200.models import SequenceParallelMLP
+
+    w1, w2 = torch.zeros(24, 16, dtype=torch.bfloat16), torch.zeros(16, 24, dtype=torch.bfloat16)
+    assert SequenceParallelMLP(8, 16, w1, w2)._plain()
+
+    class Clipped(SequenceParallelMLP):
+        def _act(self, h):
+            return super()._act(h).clamp(max=1.0)
+
+    assert not Clipped(8, 16, w1, w2)._plain()
+    mlp = SequenceParallelMLP(8, 16, w1, w2)
+    mlp.up = lambda x, w, b: x
+    assert not mlp._plain()
+    mlp = SequenceParallelMLP(8, 16, w1, w2)
+    mlp._act = torch.relu
+    assert not mlp._plain()
