@@ -47,9 +47,16 @@ def _wgrad(dy_full: torch.Tensor, x_full: torch.Tensor) -> torch.Tensor:
 
 
 def _one_gpu(layer, t: torch.Tensor) -> bool:
-    """Nothing to exchange: a gradient product reads the weights as they lie, instead of
-    a transposed copy for the fused kernel's operand layout."""
     return t.is_cuda and layer.world == 1
+
+
+def _input_grad(layer, dy: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``dy @ w`` through the layer's backward context.  On one GPU there is nothing to
+    exchange: the product reads the weights as they lie, instead of a transposed copy for
+    the fused kernel's operand layout, and reports a failed wait in the same status words."""
+    if _one_gpu(layer, dy):
+        return product(dy, w.contiguous(), b_t=True, status=layer.bwd.status)
+    return layer.bwd(dy, w.t().contiguous())
 
 
 class _ColumnParallelFn(torch.autograd.Function):
@@ -71,7 +78,7 @@ class _ColumnParallelFn(torch.autograd.Function):
             x_full = _gather_rows(x_local, layer.world, layer.group)
         if ctx.needs_input_grad[0]:
             # dx_local[M/world, K] = RS(dy[M, Nl] @ W[Nl, K]): contraction over the sharded Nl
-            dx = product(dy, w.contiguous(), b_t=True) if _one_gpu(layer, dy) else layer.bwd(dy, w.t().contiguous())
+            dx = _input_grad(layer, dy, w)
         if need_dw:
             dw = _wgrad(dy, x_full)
         if ctx.has_bias and ctx.needs_input_grad[2]:
@@ -98,7 +105,7 @@ class _RowParallelFn(torch.autograd.Function):
             dy_full = _gather_rows(dy_local, layer.world, layer.group)
         if ctx.needs_input_grad[0]:
             # dx[M, Kl] = AG(dy_local)[M, N] @ W[N, Kl]
-            dx = product(dy_local, w.contiguous(), b_t=True) if _one_gpu(layer, dy_local) else layer.bwd(dy_local, w.t().contiguous())
+            dx = _input_grad(layer, dy_local, w)
         if need_dw:
             dw = _wgrad(dy_full, x)
         if ctx.has_bias and ctx.needs_input_grad[2]:

@@ -160,3 +160,18 @@ def test_fused_mlp_takes_operands_of_any_strides(which):
         y = LocalMLPFn.apply(*leaves, "silu", AGGemm(R, K))
         grads.append([y.detach(), *torch.autograd.grad(y, leaves, dy)])
     assert all(torch.equal(p, q) for p, q in zip(*grads))
+
+
+@pytest.mark.parametrize("kind", ["ColumnParallelLinear", "RowParallelLinear"])
+def test_one_gpu_input_gradient_reports_to_the_layers_status(kind, monkeypatch):
+    from kernel_b200.ops import autograd as A
+
+    layer = getattr(A, kind)(R, K, Nn)
+    layer.bwd.status = torch.zeros(8, dtype=torch.int32)
+    seen = []
+    monkeypatch.setattr(A, "_one_gpu", lambda layer, t: True)
+    real = A.product
+    monkeypatch.setattr(A, "product", lambda *a, **kw: seen.append(kw) or real(*a, **kw))
+    x = _z(R, K).requires_grad_(True)
+    layer(x).sum().backward()
+    assert [kw["status"] for kw in seen if not kw.get("a_t")] == [layer.bwd.status]
