@@ -175,3 +175,14 @@ def test_one_gpu_input_gradient_reports_to_the_layers_status(kind, monkeypatch):
     x = _z(R, K).requires_grad_(True)
     layer(x).sum().backward()
     assert [kw["status"] for kw in seen if not kw.get("a_t")] == [layer.bwd.status]
+
+
+def test_round_trip_takes_token_rows_with_trailing_unit_dimensions():
+    from kernel_b200.ops.dispatch_combine import MoEAllToAll
+
+    ctx = MoEAllToAll(4, 2, 64, 4, dtype=torch.bfloat16, device=torch.device("cpu"))
+    x = torch.randn(3, 64, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
+    idx, w = torch.tensor([[0, 1], [2, 3], [1, 3]], dtype=torch.int32), torch.ones(3, 2)
+    want = ctx.dispatch_scale_combine(x, idx, w, 2)
+    assert torch.equal(ctx.dispatch_scale_combine(x[..., None], idx, w, 2), want[..., None])
+    ctx.heap.close()
