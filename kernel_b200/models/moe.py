@@ -33,9 +33,9 @@ class MoELayer:
             return self._dense(x, indices, weights)
         if _all_local(a2a, x):
             a2a._validate(x, indices, weights)
-            er = ExpertRows(x, indices, a2a.E, status=a2a.status)
+            er = ExpertRows(x.flatten(1), indices, a2a.E, status=a2a.status)
             h = rows_product(er.rows, self.w_up, er.start, er.count, act="silu", status=a2a.status)
-            return er.combine(rows_product(h, self.w_down, er.start, er.count, status=a2a.status), weights)
+            return er.combine(rows_product(h, self.w_down, er.start, er.count, status=a2a.status), weights).view(x.shape)
         counts, recv = a2a.dispatch(x, indices)
         # the segment lengths size the buffers (one sync per layer call); the rows of
         # one expert, from all sources, are gathered into one block per expert
@@ -116,24 +116,24 @@ class _LocalMoEFn(torch.autograd.Function):
     def forward(ctx, x, weights, w_up, w_down, layer, indices):
         a2a = layer.a2a
         a2a._validate(x, indices, weights)
-        er = ExpertRows(x, indices, a2a.E, pad=ROW_ALIGN, status=a2a.status)
+        er = ExpertRows(x.flatten(1), indices, a2a.E, pad=ROW_ALIGN, status=a2a.status)
         pre = torch.empty((er.rows.shape[0], w_up.shape[1]), dtype=x.dtype, device=x.device)
         h = rows_product(er.rows, w_up, er.start, er.padded, act="silu", pre_out=pre, status=a2a.status)
         Y = rows_product(h, w_down, er.start, er.padded, status=a2a.status)
         ctx.sizes, ctx.status = (er.T, er.k, er.E), a2a.status
         ctx.save_for_backward(weights, w_up, w_down, pre, h, Y, er.rows, er.table)
-        return er.combine(Y, weights)
+        return er.combine(Y, weights).view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
         weights, w_up, w_down, pre, h, Y, rows, table = ctx.saved_tensors
         er, status = ExpertRows.saved(rows, table, *ctx.sizes), ctx.status
-        dYs, dweights = er.grad_rows(dy.contiguous(), Y, weights)
+        dYs, dweights = er.grad_rows(dy.contiguous().flatten(1), Y, weights)
         dpre = rows_product(dYs, w_down, er.start, er.padded, b_t=True, act="silu", pre_in=pre, status=status)
         dw_down = contract_product(dYs, h, er.start, er.count, status=status)
         dw_up = contract_product(dpre, rows, er.start, er.count, status=status)
         dX = rows_product(dpre, w_up, er.start, er.padded, b_t=True, status=status)
-        return er.combine(dX, None), dweights, dw_up, dw_down, None, None
+        return er.combine(dX, None).view(dy.shape), dweights, dw_up, dw_down, None, None
 
 
 class _MoEFn(torch.autograd.Function):

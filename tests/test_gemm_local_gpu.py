@@ -302,3 +302,24 @@ def test_mlp_with_strided_parameters():
         t.data = t.data.t().contiguous().t()
     assert torch.equal(mlp(x.t().contiguous().t()), want)
     mlp.close()
+
+
+def test_moe_layers_take_token_rows_with_trailing_unit_dimensions():
+    from kernel_b200.models import MoELayer, TrainableMoELayer
+
+    torch.manual_seed(2)
+    E, k, H, F, T = 4, 2, 64, 128, 5
+    layer = TrainableMoELayer(E, k, H, F, 8, device=torch.device(DEV))
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    idx = torch.rand(T, E, device=DEV).argsort(1)[:, :k].to(torch.int32).contiguous()
+    w = torch.softmax(torch.randn(T, k, device=DEV), -1)
+    res = []
+    for shape in ((T, H), (T, H, 1)):
+        leaf = x.view(shape).requires_grad_(True)
+        y = layer(leaf, idx, w)
+        fixed = MoELayer(E, k, H, 8, layer.w_up.data, layer.w_down.data)
+        res.append([y.detach(), fixed(x.view(shape), idx, w), *torch.autograd.grad(y, leaf, torch.ones_like(y))])
+        assert all(t.shape == shape for t in res[-1])
+        fixed.a2a.heap.close()
+    assert all(torch.equal(p.view(T, H), q.view(T, H)) for p, q in zip(*res))
+    layer.close()
