@@ -468,6 +468,22 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   return v;
 }
 
+// The same without the non-coherent path, for kernels that begin before the previous kernel of the
+// stream has ended: what that one wrote is not read-only for the whole of this one, which
+// is what ld.global.nc (__ldg) asks for.  Volatile: stays behind wait_for_previous_launch().
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_global_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // Start of a kernel launched with the overlap_launch attribute: waits until the previous
 // kernel of the stream has ended and its writes are visible, then lets the next one be set up.
 // Nothing that another kernel may write, and no output, is touched before it.  Without the
@@ -477,9 +493,9 @@ __device__ __forceinline__ void wait_for_previous_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Loads 16 bytes of read-only data and drops them: the line is in L1 afterwards.
-__device__ __forceinline__ void touch_nc(const void* p) {
-  asm volatile("{\n\t.reg .b32 a, b, c, d;\n\tld.global.nc.v4.u32 {a, b, c, d}, [%0];\n\t}" ::"l"(p));
+// Loads 16 bytes and drops them: the line is in L1 afterwards.
+__device__ __forceinline__ void touch_global(const void* p) {
+  asm volatile("{\n\t.reg .b32 a, b, c, d;\n\tld.global.v4.u32 {a, b, c, d}, [%0];\n\t}" ::"l"(p));
 }
 
 // Device-scope counterparts for words that only threads of this GPU touch.

@@ -166,7 +166,7 @@ __device__ __forceinline__ void finish32(const Params& p, float* f, int col, con
   if (p.bias != nullptr) {
     uint4 b[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) b[i] = col + 8 * i < p.N ? __ldg(reinterpret_cast<const uint4*>(p.bias + col) + i) : make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < 4; ++i) b[i] = col + 8 * i < p.N ? kb::ld_global_v4(p.bias + col + 8 * i) : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float t[8];
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       if (p.bias != nullptr) {
         // brings the tile's bias into L1 while the accumulator is not ready yet: eight values per lane
         const int col = t.n0 + 8 * lane;
-        if (8 * lane < p.bn && col < p.N) kb::touch_nc(p.bias + col);
+        if (8 * lane < p.bn && col < p.N) kb::touch_global(p.bias + col);
       }
       const int cols = min(p.bn, p.N - t.n0);
 #pragma unroll 1
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               at[i] = make_uint4(0u, 0u, 0u, 0u);
-              if (row_ok && c + 8 * i < last) at[i] = kb::ld_nc_v4(p.pre_in + at0 + 8 * i);
+              if (row_ok && c + 8 * i < last) at[i] = kb::ld_stream_v4(p.pre_in + at0 + 8 * i);
             }
           }
           uint32_t r[2][32];
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       const Tile t = tile_at(sched_id);
       if (p.bias != nullptr) {
         const int col = t.n0 + 8 * lane;
-        if (8 * lane < p.bn && col < p.N) kb::touch_nc(p.bias + col);
+        if (8 * lane < p.bn && col < p.N) kb::touch_global(p.bias + col);
       }
       const int chunks = p.bn / CHUNK_COLS;
       const int q = warp & 3;            // TMEM lane quadrant of this warp

@@ -86,17 +86,17 @@ __global__ void __launch_bounds__(PERM_THREADS) moe_permute_kernel(const MoePara
     const uint4* src = p.x + static_cast<size_t>(t0 + i) * p.vecs;
 #pragma unroll
     for (int u = 0; u < PERM_VECS; ++u) {
-      if (v0 + u * 32 < p.vecs) val[u] = kb::ld_nc_v4(src + v0 + u * 32);
+      if (v0 + u * 32 < p.vecs) val[u] = kb::ld_stream_v4(src + v0 + u * 32);
     }
   };
   if (warp < tasks) fetch(warp);
-  for (int i = tid; i < n_ent; i += PERM_THREADS) ent_e[i] = __ldg(p.idx + t0 * p.k + i);
+  for (int i = tid; i < n_ent; i += PERM_THREADS) ent_e[i] = p.idx[t0 * p.k + i];
   for (int e = tid; e < p.E; e += PERM_THREADS) tot[e] = pre[e] = 0;
   __syncthreads();
   for (int i0 = tid; i0 < total; i0 += HIST * PERM_THREADS) {  // all fetched before any is counted
     int ev[HIST];
 #pragma unroll
-    for (int u = 0; u < HIST; ++u) ev[u] = i0 + u * PERM_THREADS < total ? __ldg(p.idx + i0 + u * PERM_THREADS) : 0;
+    for (int u = 0; u < HIST; ++u) ev[u] = i0 + u * PERM_THREADS < total ? p.idx[i0 + u * PERM_THREADS] : 0;
 #pragma unroll
     for (int u = 0; u < HIST; ++u) {
       const int i = i0 + u * PERM_THREADS;
@@ -209,10 +209,10 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const CombineParams p)
         u[j] = make_uint4(0u, 0u, 0u, 0u);
         wj[j] = 0.f;
         if (j0 + j < p.k) {
-          const int s = __ldg(ts + j0 + j);
+          const int s = ts[j0 + j];
           if (s >= 0) {
-            u[j] = __ldg(p.y + static_cast<size_t>(s) * p.vecs + v);
-            wj[j] = p.w != nullptr ? __ldg(p.w + static_cast<size_t>(t) * p.k + j0 + j) : 1.f;
+            u[j] = kb::ld_global_v4(p.y + static_cast<size_t>(s) * p.vecs + v);
+            wj[j] = p.w != nullptr ? p.w[static_cast<size_t>(t) * p.k + j0 + j] : 1.f;
           }
         }
       }
@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(THREADS) moe_grad_rows_kernel(const GradParams
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           if (v0 + 32 * u < p.vecs) {
-            a[u] = __ldg(dy + v0 + 32 * u);
-            b[u] = kb::ld_nc_v4(y + v0 + 32 * u);
+            a[u] = kb::ld_global_v4(dy + v0 + 32 * u);
+            b[u] = kb::ld_stream_v4(y + v0 + 32 * u);
           }
         }
 #pragma unroll

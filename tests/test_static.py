@@ -69,3 +69,12 @@ def test_build_for_sm100a_and_load():
     lib = _native.lib()
     assert lib.kb_gemm_rs_data_bytes(8192, 8192, 8) == 2 * 8192 * 8192 * 2
     assert lib.kb_a2a_rows_bytes(8, 256, 8, 7168, 2) == 8 * 2048 * 7168 * 2
+
+
+def test_overlapped_kernels_read_through_the_coherent_path():
+    """A kernel that begins before the previous one has ended must not read what that one wrote
+    with loads that are defined for data that is read-only for the whole kernel."""
+    files = [p for p in sorted((CSRC / "kernels").glob("*.cu*")) if "wait_for_previous_launch" in p.read_text()]
+    assert {p.name for p in files} >= {"gemm_local.cuh", "moe_rows.cu"}
+    for p in files:
+        assert not re.search(r"__ldg|ld_nc|touch_nc|global\.nc|__restrict__", p.read_text()), p.name
