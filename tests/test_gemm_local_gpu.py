@@ -304,6 +304,33 @@ def test_mlp_with_strided_parameters():
     mlp.close()
 
 
+def test_stamped_time_leaves_out_the_previous_kernel():
+    """``KB200_GEMM_TIMING`` (read once per process) stamps a product's own time, although the
+    product is set up while the one before it, on 64 of the SMs, still runs."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = """
+import torch
+from kernel_b200.ops.gemm import gemm
+a, b = (torch.zeros(8192, 8192, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+st = [torch.zeros(8, dtype=torch.int32, device="cuda") for _ in range(2)]
+small = torch.zeros(128, 128, dtype=torch.bfloat16, device="cuda")
+for _ in range(3):
+    for s in st: s.zero_()
+    gemm(a, b, status=st[0], num_ctas=64)
+    gemm(small, small, status=st[1])
+torch.cuda.synchronize()
+print(int(st[0][7]), int(st[1][7]))
+"""
+    out = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, KB200_GEMM_TIMING="1"), cwd=Path(__file__).parents[1], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    large, small = map(int, out.stdout.split())
+    assert large > 200 and small < large / 4, (large, small)
+
+
 def test_moe_layers_take_token_rows_with_trailing_unit_dimensions():
     from kernel_b200.models import MoELayer, TrainableMoELayer
 
