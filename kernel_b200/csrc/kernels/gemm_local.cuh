@@ -110,7 +110,15 @@ __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
   t = kb::unpack_bf16x2(v.w); f[6] = t.x; f[7] = t.y;
 }
 
-__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
+// exp(-|x|) cannot overflow, so the sigmoid of a negative number keeps its leading digits down to the smallest
+// fp32 value (1 / (1 + exp(-x)) with the fast division is 0 from -87.3 on).  The fast exponential and division
+// stay far inside the bf16 rounding that follows: over all finite bf16 inputs SiLU, GELU and their slopes round to the
+// nearest bf16 value except for 3 of 261120 (torch's own, with expf, tanhf and full division: 347).  expf and full
+// division here cost 10 us of a MoE layer's 104 (32 tokens) and 29 us of a training step's 519.
+__device__ __forceinline__ float sigmoid(float x) {
+  const float t = __expf(-fabsf(x));
+  return __fdividef(x < 0.0f ? t : 1.0f, 1.0f + t);
+}
 // tanh form of GELU: x * sigmoid(2u), u = sqrt(2/pi) * (x + 0.044715 x^3)
 constexpr float GELU_C = 2.0f * 0.7978845608028654f;
 constexpr float GELU_A = 0.044715f;

@@ -78,6 +78,29 @@ def test_activation_and_slope_in_the_epilogue(act, M, N, K):
     assert ((g.float() - want).abs() <= 2 ** -7 * want.abs() + 1e-4 * full.abs()).all()
 
 
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+def test_activation_and_slope_of_every_bf16_value(act):
+    """Against 64-bit arithmetic: one bf16 rounding (2 ** -9 relative, below the normal range half of the
+    spacing 2 ** -133) plus 110 ulp of the fast exponential (2 ** -16); the bound is twice that."""
+    from kernel_b200.ops.local import product
+
+    x = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = x[x.float().abs() < 1e12]   # the slope of gelu holds x ** 3
+    first = torch.zeros((x.numel(), 8), dtype=torch.bfloat16)
+    first[:, 0] = 1.0
+    ones = torch.zeros((8, 8), dtype=torch.bfloat16, device=DEV)
+    ones[:, 0] = 1.0
+    val = product((first * x[:, None]).to(DEV), ones, act=act)[:, 0].double().cpu()
+    slope = product(first.to(DEV), ones.t().contiguous(), b_t=True, act=act, pre_in=x[:, None].repeat(1, 8).to(DEV))[:, 0].double().cpu()
+    leaf = x.double().requires_grad_(True)
+    arg = leaf if act == "silu" else 2 * (2 / torch.pi) ** 0.5 * (leaf + 0.044715 * leaf ** 3)
+    want = leaf * torch.sigmoid(arg)
+    want_slope, = torch.autograd.grad(want.sum(), leaf)
+    for got, ref in ((val, want.detach()), (slope, want_slope)):
+        bad = (got - ref).abs() > 2 ** -8 * ref.abs() + 2 ** -133
+        assert not bad.any(), (x[bad], got[bad], ref[bad])
+
+
 def test_relu_slope_selects():
     """Where ReLU is off an infinite gradient is zero; a NaN input passes the gradient on (as torch does)."""
     from kernel_b200.ops.local import product
