@@ -213,13 +213,20 @@ class ExpertRows:
 
     ``rows[R, H]``; group table ``start``, ``count`` (``padded``: count rounded up to
     ``pad`` rows, zero rows in between); ``slots[T, k]`` maps a choice to its row.
-    ``R`` is the capacity ``T * k + E * (pad - 1)``: no count travels to the host."""
+    No count travels to the host, so ``R`` is a capacity: ``T * k`` rows and ``pad - 1`` for
+    every expert that can have one.  The price of staying off the host is memory: with
+    ``pad`` = 64 the activations of 64 tokens, top-8 of 1024 experts, take 32768 rows for 512
+    real ones (rows behind the last padded expert are neither written nor read)."""
+
+    @staticmethod
+    def capacity(T: int, k: int, experts: int, pad: int) -> int:
+        return T * k + min(experts, T * k) * (pad - 1)
 
     def __init__(self, x: torch.Tensor, indices: torch.Tensor, experts: int, pad: int = 1, status: Optional[torch.Tensor] = None):
         _check_operand(x, "x", 2, x.device)
         (T, H), k, dev = x.shape, indices.shape[1], x.device
         _check_choices(indices, "indices", torch.int32, (T, k), dev)
-        rows = torch.empty((T * k + experts * (pad - 1), H), dtype=torch.bfloat16, device=dev)
+        rows = torch.empty((self.capacity(T, k, experts, pad), H), dtype=torch.bfloat16, device=dev)
         self._set(rows, torch.empty(3 * experts + T * k, dtype=torch.int32, device=dev), T, k, experts)
         N.check(N.lib().kb_moe_permute(x.data_ptr(), indices.data_ptr(), T, k, experts, H, pad, self.rows.data_ptr(),
                                        self.slots.data_ptr(), self.start.data_ptr(), self.count.data_ptr(), self.padded.data_ptr(),

@@ -220,6 +220,35 @@ def test_expert_rows(T, k, E, H, pad):
     assert torch.equal(dw, (dy.unsqueeze(1).float() * y[slots].float()).sum(-1))
 
 
+@pytest.mark.parametrize("T,k,E", [(0, 2, 8), (1, 1, 256), (5, 2, 300), (150, 2, 4)])
+def test_moe_training_step_with_more_experts_than_rows(T, k, E):
+    """Gradients of every input where most experts have no row, and with no token at all."""
+    from kernel_b200.models import TrainableMoELayer
+
+    torch.manual_seed(T)
+    H, F = 64, 72
+    layer = TrainableMoELayer(E, k, H, F, max(T, 1), device=torch.device(DEV))
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16).requires_grad_(True)
+    w = torch.rand(T, k, device=DEV).requires_grad_(True)
+    idx = torch.rand(T, E, device=DEV).argsort(1)[:, :k].to(torch.int32).contiguous()
+    dy = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    y = layer(x, idx, w)
+    got = [y, *torch.autograd.grad(y, (x, w, layer.w_up, layer.w_down), dy)]
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, w, layer.w_up, layer.w_down)]
+    h = torch.nn.functional.silu(torch.einsum("th,tkfh->tkf", leaves[0], leaves[2][idx.long()]))
+    rows = torch.einsum("tkf,tkhf->tkh", h, leaves[3][idx.long()])
+    ref = (rows * leaves[1].unsqueeze(-1)).sum(1)
+    want = [ref, *torch.autograd.grad(ref, leaves, dy.double())]
+    for i, (p, q) in enumerate(zip(got, want)):
+        assert p.shape == q.shape
+        # at most four bf16 roundings (2 ** -9 each) between the inputs and a result; the error of a routing weight's
+        # gradient <dy, row> is relative to the lengths of both vectors (their product may cancel)
+        scale = (dy.double().norm(dim=1, keepdim=True) * rows.norm(dim=2)).norm() if i == 2 else q.norm()
+        assert (p.double() - q).norm() <= 4 * 2 ** -9 * scale
+    layer.a2a.heap.check_status()
+    layer.close()
+
+
 def test_expert_rows_out_of_range_id_is_reported_and_skipped():
     from kernel_b200.ops.local import ExpertRows
 

@@ -186,3 +186,19 @@ def test_round_trip_takes_token_rows_with_trailing_unit_dimensions():
     want = ctx.dispatch_scale_combine(x, idx, w, 2)
     assert torch.equal(ctx.dispatch_scale_combine(x[..., None], idx, w, 2), want[..., None])
     ctx.heap.close()
+
+
+def test_row_capacity_holds_every_routing_and_is_reached():
+    """The padded rows of any routing fit; the routing that spreads one row to as many experts as
+    it can and the rest so that each fills one more row than a multiple needs all of it."""
+    import itertools
+
+    for T, k, experts, pad in [(0, 2, 4, 64), (1, 2, 4, 64), (2, 1, 3, 4), (3, 2, 3, 2), (2, 2, 5, 3), (4, 1, 2, 3)]:
+        most = 0
+        for pick in itertools.product(range(experts), repeat=T * k):
+            n = torch.bincount(torch.tensor(pick, dtype=torch.long), minlength=experts)
+            most = max(most, int(((n + pad - 1) // pad * pad).sum()))
+        capacity = L.ExpertRows.capacity(T, k, experts, pad)
+        assert most <= capacity <= T * k + experts * (pad - 1)
+        if T * k <= experts:
+            assert most == capacity
