@@ -32,12 +32,20 @@ def _expected(x, idx, w, E, mode):
     return (y * w.unsqueeze(-1)).sum(1)
 
 
-@pytest.mark.parametrize("fused", ["1", "0"])
+def _select(monkeypatch, path):
+    """Kernels of the next context's round trips on one rank: "1" what a program gets (one pass over
+    the rows, no exchange), "0" three launches, "exchange" the one-launch kernels that several ranks
+    use (a traced call runs them on one rank too)."""
+    monkeypatch.setenv("KB200_A2A_FUSED", "0" if path == "0" else "1")
+    monkeypatch.setenv("KB200_TRACE", "1" if path == "exchange" else "0")
+
+
+@pytest.mark.parametrize("fused", ["1", "0", "exchange"])
 @pytest.mark.parametrize("E,k,H,T,dtype,mode", CASES)
 def test_round_trip_matches_fp32_reference(E, k, H, T, dtype, mode, fused, monkeypatch):
     from kernel_b200.ops.dispatch_combine import MoEAllToAll
 
-    monkeypatch.setenv("KB200_A2A_FUSED", fused)
+    _select(monkeypatch, fused)
     dev = torch.device("cuda")
     ctx = MoEAllToAll(E, k, H, max(T, 2), dtype=dtype, device=dev)
     x, idx, w = _inputs(E, k, H, T, dtype, dev)
@@ -88,9 +96,11 @@ def test_split_dispatch_expert_combine_api():
 def test_low_latency_path_equals_regular_path(T, dtype, monkeypatch):
     """Contexts of at most 32 tokens per rank take the flag-in-data kernel; its
     rounding points are those of the regular one-launch kernel, so the outputs are
-    equal bit for bit, call after call (the count lines alternate with the epoch)."""
+    equal bit for bit, call after call (the count lines alternate with the epoch).
+    Traced: on one rank an untraced call needs neither of the two."""
     from kernel_b200.ops.dispatch_combine import MoEAllToAll
 
+    _select(monkeypatch, "exchange")
     dev = torch.device("cuda")
     E, k, H = 64, 8, 7168
     x, idx, w = _inputs(E, k, H, T, dtype, dev, seed=T)
@@ -103,6 +113,7 @@ def test_low_latency_path_equals_regular_path(T, dtype, monkeypatch):
     for _ in range(3):
         got = ll.dispatch_scale_combine(x, idx, w, 2)
         assert torch.equal(got, want)
+    assert ll.read_trace()["total"] > 0 and regular.read_trace()["total"] > 0   # the exchange kernels ran: they stamp
     torch.cuda.synchronize()
     ll.heap.check_status()
     ref = _expected(x, idx, w, E, 2)
@@ -161,7 +172,7 @@ def test_sentinel_and_guard_rows_after_dispatch(monkeypatch):
     assert torch.isfinite(out.float()).all()
 
 
-@pytest.mark.parametrize("fused", ["1", "0"])
+@pytest.mark.parametrize("fused", ["1", "0", "exchange"])
 @pytest.mark.parametrize("E,k,T", [(2, 1, 3), (2, 2, 3), (4, 2, 2), (3, 3, 1)])
 def test_every_routing_of_tiny_cases(E, k, T, fused, monkeypatch):
     """All ordered picks of k distinct experts for every token, one call each on the
@@ -171,7 +182,7 @@ def test_every_routing_of_tiny_cases(E, k, T, fused, monkeypatch):
 
     from kernel_b200.ops.dispatch_combine import SCALE_EXPERT, MoEAllToAll, expert_scale_vector
 
-    monkeypatch.setenv("KB200_A2A_FUSED", fused)
+    _select(monkeypatch, fused)
     dev = torch.device("cuda")
     H = 64
     ctx = MoEAllToAll(E, k, H, 4, dtype=torch.float32, device=dev)

@@ -124,7 +124,7 @@ def _table(counts, pad):
     return start.int().to(DEV), n.int().to(DEV), max(1, int(padded.sum()))
 
 
-def _force(monkeypatch, pair):
+def _force(monkeypatch, pair, bn=0, split=0):
     """Tile shape of the products made through ``ops.local``."""
     from kernel_b200.ops import local as L
 
@@ -132,7 +132,7 @@ def _force(monkeypatch, pair):
 
     def forced(*a):
         args = made(*a)
-        args.pair = pair
+        args.pair, args.bn, args.split = pair, bn, split
         return args
 
     monkeypatch.setattr(L, "_args", forced)
@@ -155,6 +155,59 @@ def test_rows_product(counts, b_t, N, K, pair, monkeypatch):
     for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
         want[s:s + n] = (a[s:s + n].float() @ b[e].float().t()).to(torch.bfloat16)
     assert torch.equal(out, want)
+
+
+def _check_epilogues(act, full, pre, out, grad):
+    """``full`` is exact in fp32 (small integers times a power of two), so ``pre`` is its rounding;
+    value and slope: one bf16 rounding (2 ** -9) and some ulp of the fast exponential, of the factors where
+    the slope cancels.  The bounds are twice that."""
+    leaf = pre.double().requires_grad_(True)
+    arg = 2 * (2 / torch.pi) ** 0.5 * (leaf + 0.044715 * leaf ** 3)
+    want = torch.relu(leaf) if act == "relu" else leaf * torch.sigmoid(leaf if act == "silu" else arg)
+    slope, = torch.autograd.grad(want.sum(), leaf)
+    assert torch.equal(pre, full.to(torch.bfloat16))
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -133).all()
+    want = full.double() * slope
+    assert ((grad.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -16 * full.double().abs()).all()
+
+
+@pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
+@pytest.mark.parametrize("pair,bn,split,M,N,K", [
+    *((*shape, 520, 296, 2120) for shape in [(0, 64, 1), (0, 192, 1), (0, 128, 5), (0, 256, 8), (1, 128, 1), (1, 256, 1), (1, 128, 3),
+                                             (1, 256, 4), (2, 256, 1)]),
+    *((*shape, 40, 72, 1096) for shape in [(0, 64, 1), (0, 192, 1), (0, 128, 5), (0, 256, 8)])])
+def test_epilogues_of_every_tile_shape(act, pair, bn, split, M, N, K, monkeypatch):
+    """One CTA, pairs, 512-row tiles and the exchange of a split, with full and ragged tiles and (one CTA)
+    a matrix smaller than the tile."""
+    L = _force(monkeypatch, pair, bn, split)
+    a, b = _ints(M, K, seed=30), _ints(N, K, seed=31) * 2 ** -5
+    st = _status()
+    pre = torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = L.product(a, b, act=act, pre_out=pre, status=st)
+    grad = L.product(a, b.t().contiguous(), b_t=True, act=act, pre_in=pre, status=st)
+    _clean(st)
+    _check_epilogues(act, a.float() @ b.float().t(), pre, out, grad)
+
+
+@pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
+@pytest.mark.parametrize("pair,bn", [(0, 64), (0, 256), (1, 128), (1, 256)])
+@pytest.mark.parametrize("counts", COUNTS)
+def test_epilogues_of_grouped_rows(act, pair, bn, counts, monkeypatch):
+    L = _force(monkeypatch, pair, bn)
+    N, K = 264, 520
+    start, count, R = _table(counts, 1)
+    a, b = _ints(R, K, seed=32), _ints(len(counts), N, K, seed=33) * 2 ** -4
+    st = _status()
+    pre, out, grad = (torch.full((R, N), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3))
+    L.rows_product(a, b, start, count, act=act, pre_out=pre, out=out, status=st)
+    L.rows_product(a, b.transpose(1, 2).contiguous(), start, count, b_t=True, act=act, pre_in=pre, out=grad, status=st)
+    _clean(st)
+    inside = torch.zeros(R, dtype=torch.bool, device=DEV)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        inside[s:s + n] = True
+        sl = slice(s, s + n)
+        _check_epilogues(act, a[sl].float() @ b[e].float().t(), pre[sl], out[sl], grad[sl])
+    assert all((t[~inside] == 7.0).all() for t in (pre, out, grad))
 
 
 @pytest.mark.parametrize("counts", COUNTS)
@@ -321,6 +374,87 @@ def test_overlapped_launches_keep_their_order_eagerly_and_in_a_graph():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(res, 4 * a)
+
+
+def test_overlapped_row_kernels_keep_their_order_eagerly_and_in_a_graph():
+    """Permutation, grouped products, combine and its backward, each reading what the launch before
+    wrote, with the routing table, the weights and the tokens rewritten directly before they are read."""
+    from kernel_b200.ops.local import ExpertRows, contract_product, rows_product
+
+    T, k, E, H = 96, 2, 8, 128
+    g = torch.Generator(device=DEV).manual_seed(3)
+    tables = [torch.rand((T, E), device=DEV, generator=g).argsort(1)[:, :k].to(torch.int32).contiguous() for _ in range(2)]
+    tokens = [_ints(T, H, seed=40 + i) for i in range(2)]
+    eye = torch.eye(H, dtype=torch.bfloat16, device=DEV).repeat(E, 1, 1)
+    which = torch.zeros((), dtype=torch.int64, device=DEV)
+    x, idx, b, w = torch.zeros_like(tokens[0]), torch.zeros_like(tables[0]), torch.zeros_like(eye), torch.zeros((T, k), device=DEV)
+    both_tables, both_tokens, res = torch.stack(tables), torch.stack(tokens), {}
+
+    def chain():
+        b.copy_(eye * (1 + which))
+        w.copy_((2 + which).float().expand(T, k))
+        idx.copy_(both_tables.index_select(0, which.view(1))[0])
+        x.copy_(both_tokens.index_select(0, which.view(1))[0])
+        er = ExpertRows(x, idx, E, pad=64)                             # reads x and idx as just written
+        y = rows_product(er.rows, b, er.start, er.padded)              # reads b, the table and the rows
+        y = rows_product(y, b, er.start, er.padded, b_t=True)
+        res["out"] = er.combine(y, w)
+        dyr, res["dw"] = er.grad_rows(res["out"], y, w)                # reads what combine wrote
+        res["c"] = contract_product(dyr, er.rows, er.start, er.count)  # reads what grad_rows wrote
+        w.zero_()                                                      # after its last reader
+
+    def check(i):
+        s = (1 + i) ** 2
+        xi, wi = tokens[i].float(), float(2 + i)
+        out = (k * wi * s * xi).to(torch.bfloat16)
+        assert torch.equal(res["out"], out)
+        assert torch.equal(res["dw"], (out.float() * s * xi).sum(1, keepdim=True).expand(T, k))
+        for e in range(E):
+            rows = (tables[i] == e).any(1)
+            assert torch.equal(res["c"][e], ((wi * out[rows].float()).to(torch.bfloat16).float().t() @ xi[rows]).to(torch.bfloat16))
+
+    for i in (0, 1, 0):
+        which.fill_(i)
+        chain()
+        torch.cuda.synchronize()
+        check(i)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for i in (1, 0, 1):
+        which.fill_(i)
+        graph.replay()
+        torch.cuda.synchronize()
+        check(i)
+
+
+@pytest.mark.parametrize("hot", [1.0, 0.5])
+@pytest.mark.parametrize("T,k,E", [(300, 2, 64), (33, 4, 256)])
+def test_moe_layers_with_skewed_routing(hot, T, k, E):
+    """One expert receives every token, or every second one: the tile rule works from the average group."""
+    from kernel_b200.models import MoELayer, TrainableMoELayer
+
+    torch.manual_seed(4)
+    H, F = 128, 136
+    layer = TrainableMoELayer(E, k, H, F, T, device=torch.device(DEV))
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16).requires_grad_(True)
+    score = torch.rand(T, E, device=DEV)
+    score[torch.rand(T, device=DEV) < hot, E // 2] = -1.0
+    idx = score.argsort(1)[:, :k].to(torch.int32).contiguous()
+    w = torch.softmax(torch.randn(T, k, device=DEV), -1).requires_grad_(True)
+    dy = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    y = layer(x, idx, w)
+    got = [y, *torch.autograd.grad(y, (x, layer.w_up, layer.w_down), dy)]
+    fixed = MoELayer(E, k, H, T, layer.w_up.data, layer.w_down.data)
+    assert torch.equal(fixed(x.detach(), idx, w.detach()), y)
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, layer.w_up, layer.w_down)]
+    h = torch.nn.functional.silu(torch.einsum("th,tkfh->tkf", leaves[0], leaves[1][idx.long()]))
+    ref = (torch.einsum("tkf,tkhf->tkh", h, leaves[2][idx.long()]) * w.detach().double().unsqueeze(-1)).sum(1)
+    for p, q in zip(got, [ref, *torch.autograd.grad(ref, leaves, dy.double())]):
+        assert (p.double() - q).norm() <= 4 * 2 ** -9 * q.norm()   # at most four bf16 roundings on the way
+    layer.a2a.heap.check_status()
+    fixed.a2a.heap.close()
+    layer.close()
 
 
 @pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
