@@ -5,7 +5,7 @@
 // With one rank the dispatch would copy a token's row into a receive region, the
 // expert phase read it back and write a partial row, the combine read that: three
 // passes over memory and two grid-wide hand-offs for values that depend on one row of x
-// and k (expert, weight) pairs.  Here a CTA reads the row once, forms
+// and k (expert, weight) pairs.  Here a warp reads its part of the row once, forms
 //     out = sum_j  w_j * round(scale(e_j) * x)
 // in fp32 in ascending j with the rounding points of the general kernels (the expert's
 // output type, then the result's) and writes it once; outputs are equal to theirs bit
@@ -171,6 +171,6 @@ static int launch_local(const A2aParams& p, int sms, cudaStream_t st) {
   // half the values per vector, so twice the vectors (2048 tokens of 7168 values: bf16 31.0 -> 26.9 us, with unit scales
   // 22.8 -> 16.7; fp32 30.8 -> 24.9; 1500 tokens of 5000 bf16 values are unchanged at 16.5).
   if (static_cast<long long>(p.T) * p.vecs < 16ll * 32 * sms) return launch_local_as<T, 1, 8>(p, sms, st);
-  if (sizeof(T) == 4) return launch_local_as<T, 4, 4>(p, sms, st);
-  return launch_local_as<T, 2, 8>(p, sms, st);
+  if constexpr (sizeof(T) == 4) return launch_local_as<T, 4, 4>(p, sms, st);
+  else return launch_local_as<T, 2, 8>(p, sms, st);
 }

@@ -38,7 +38,6 @@ struct MoeParams {
   int pad;            // rows of an expert start at, and are zero-filled up to, multiples of this
   int tok_per_cta;
   const int32_t* idx;
-  const float* w;
   const uint4* x;
   uint4* rows;
   int32_t* slots;      // [T][k] row of a copy, or -1 (expert id out of range)
@@ -351,7 +350,6 @@ extern "C" int kb_moe_permute(const void* x, const int32_t* indices, int T, int 
   p.vecs = hidden / 8;
   p.pad = pad;
   p.idx = indices;
-  p.w = nullptr;
   p.x = static_cast<const uint4*>(x);
   p.rows = static_cast<uint4*>(rows);
   p.slots = slots;

@@ -2,7 +2,7 @@
 
 Where the reference simulates the experts with ``x * (1 + rank)``
 (``reference.py:262``), this layer runs a real two-matrix expert MLP on the rows
-each local expert received, with the tcgen05 GEMM, and writes the results row
+each local expert received, with the grouped tcgen05 products, and writes the results row
 for row into the buffer the combine kernel pulls from.  ``MoELayer`` is the
 forward-only block over given weights; ``TrainableMoELayer`` owns parameters and
 has a backward pass made of the same two exchange kernels.
@@ -80,8 +80,9 @@ def _expert_major_rows(counts_h: torch.Tensor, cap: int):
 
 def _pad8_t(rows: torch.Tensor) -> torch.Tensor:
     """``rows[n, A]`` -> contiguous ``[A, n8]`` (n rounded up to a multiple of 8 with
-    zero columns): the K-major operand layout of a GEMM that contracts over rows, for
-    callers of ``ops.gemm.gemm``; the layers here contract rows where they lie."""
+    zero columns): what ``ops.gemm.gemm``, whose operands are contiguous along K, needs to
+    contract over rows.  The layers here do not call it: ``contract_product`` reads rows where
+    they lie."""
     n, A = rows.shape
     n8 = (n + 7) // 8 * 8
     out = rows.new_zeros((A, n8))

@@ -1,8 +1,9 @@
 """Front-ends of the tcgen05 GEMM family: plain GEMM, GEMM + reduce-scatter and
 all-gather + GEMM.
 
-On CUDA tensors these always launch the hand-written sm_100a kernel
-(``csrc/kernels/gemm_sm100.cu``); there is no library fallback on a GPU.  CPU
+On CUDA tensors these always launch hand-written sm_100a kernels: the fused ones
+(``csrc/kernels/gemm_sm100.cu``) with several ranks, the product family of one GPU
+(``csrc/kernels/gemm_local.cu``) otherwise; there is no library fallback on a GPU.  CPU
 tensors take a torch reference path (``torch.matmul`` plus gloo collectives) so
 that host-side logic can be tested without a GPU; with more than one CPU rank the
 fused ops run the kernels' protocol over a host-backed symmetric heap.
