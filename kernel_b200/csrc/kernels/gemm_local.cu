@@ -95,9 +95,10 @@ struct Capacity {
 //             once, with 512-row tiles (no second accumulator) in every wave
 //   split     one barrier more and the exchange of (split - 1) / split of a tile
 //   memory    everything read and written once at 6.5 TB/s
-// The configurations differ most where few tiles leave SMs idle: 64 x 7168 x 18432 takes
-// 114 us with 256-column tiles and no split (28 of 148 SMs), 48 with the pick; 256 x 4096 x 14336 76
-// and 33 us; 2048 x 2880 x 2880 39 and 32 us.  512-row tiles move 25 % fewer operand bytes
+// The configurations differ most where few tiles leave SMs idle (GPU time, launches back to back
+// in a graph, three weights in turn; one CTA with 256 columns and no split against the pick):
+// 64 x 7168 x 18432 88.5 and 45.1 us, 256 x 4096 x 14336 85.1 and 30.5, 2048 x 2880 x 2880 (in the
+// L2) 35.1 and 24.4.  512-row tiles move 25 % fewer operand bytes
 // per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).
 Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape) {
   Config best = {false, 256, 1};
@@ -141,8 +142,14 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
 //   64 experts, 2048 x 1024, 3 rows each: 32 x 256 tiles 45 us, 32 x 64 (first version) 68 us
 // The epilogue that reads saved values back costs a pair more than one CTA (a pair's
 // accumulators are free only when both have stored): pairs from about 400 rows per group on.
-//   64 experts, 128 rows, 2048 x 1024:  pair 90 us, one CTA 79;  32 experts, 256 rows, 2048 x 2048: 114 and 103
-//   8 experts, 500 rows, 4096 x 4096:   pair 124 us, one CTA 131
+// Pair and one CTA in us, cold L2, equal groups (the line costs up to 10 % on its wrong sides, where N or K is
+// long below it and at 640 rows above it):
+//   rows per group            128         256         320         384         448         512         640
+//   64 of [2048, 1024]     102  84    113 107    158 125    147 135    153 152    161 161    212 192
+//   32 of [2048, 2048]     101  82    107 102    150 123    143 131    145 145    151 151    204 183
+//   8 of [4096, 4096]       80  75     84  88    120 111    121 113    121 133    125 139    173 164
+//   12 of [4096, 1536]      60  56     64  64     76  82     76  84     78  86     80  87     99 109
+// Without that epilogue the model decides; its pairs cost 6 to 10 % at 128 rows per group of [2048, 1024] (76 and 69 us):
 //   64 experts, 128 rows each: 128 x 192 tiles 61 us;  8 experts, 1000 rows of 4096 x 4096: pairs 198 us, one CTA 218 us
 Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape, bool slope) {
   Config best;
@@ -181,10 +188,14 @@ Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shap
 
 // Contractions over a group's rows.  A few k blocks: the outputs are the traffic, the widest
 // tile of one CTA, a pair's hand-overs cost more than its smaller operand traffic saves.
-// More: pairs.  The row capacity holds up to 63 padding rows per group; the line lies between
-//   64 experts, 128 rows, 2048 x 1024:   one CTA 76 us, pair 90
-//   32 experts, 512 rows, 2048 x 2048:   one CTA 155 us, pair 130
-//   8 experts, 500 rows, 4096 x 4096:    one CTA 151 us, pair 125
+// More: pairs.  The line is drawn on K / groups, which is the row capacity: up to 63 rows of padding per
+// group are in it.  One CTA and pair in us, cold L2, by the real rows of every group (a multiple of 64):
+//   rows                     128         192         256         320         384         512
+//   64 of 2048 x 1024      70  92      83  92     102  94     113  98     121 105     153 132
+//   32 of 2048 x 2048      72  91      84  90     102  92     113  94     121 102     152 125
+//   8 of 4096 x 4096       72  87      80  88     104  92     113  94     123 102     155 126
+//   128 of 1024 x 768      60  77      68  76      82  82      90  88      98  88     122 100
+// So pairs win from 256 rows on; groups of 256 to 288 rows still get one CTA (capacity below 352).
 Config contract_config(int M, int N, int K, int groups, int shape) {
   Config c;
   c.pair = shape >= 0 ? shape > 0 : M > 128 && K / groups >= 352;
@@ -481,8 +492,8 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     dim.val.clusterDim.z = 1;
   }
   // Set up under the end of the previous kernel, except the clusters of a split contraction:
-  // placed one by one as SMs fall free they leave SMs unused (64 x 7168 x 18432: 52 us
-  // launched in order, 60 overlapped).
+  // placed one by one as SMs fall free they leave SMs unused (64 x 7168 x 18432 back to back: 45.1 us
+  // launched in order, 51.7 overlapped).
   if (c.split == 1) attr[cfg.numAttrs++] = kb::overlap_launch();
   void* args[] = {&p};
   KB_CUDA_OK(cudaLaunchKernelExC(&cfg, fn, args));
