@@ -155,8 +155,9 @@ class MoEAllToAll:
         return out
 
     def _validate(self, x, indices, weights) -> None:
-        T = x.shape[0]
-        if x.dtype != self.dtype or x.shape[1] != self.H or not x.is_contiguous():
+        shape = x.shape  # every access builds the size anew
+        T = shape[0]
+        if x.dtype != self.dtype or shape[1] != self.H or not x.is_contiguous():
             raise ValueError("x must be contiguous [T, hidden] in the context dtype")
         Tk = (T, self.k)  # a torch.Size compares equal to a tuple
         if indices.dtype != torch.int32 or indices.shape != Tk or not indices.is_contiguous():
