@@ -8,12 +8,13 @@
 // and k (expert, weight) pairs.  Here a warp reads its part of the row once, forms
 //     out = sum_j  w_j * round(scale(e_j) * x)
 // in fp32 in ascending j with the rounding points of the general kernels (the expert's
-// output type, then the result's) and writes it once; outputs are equal to theirs bit
-// for bit.  Bound by memory (x in, out out) for many tokens, by the launch for few.
-// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 25 us a call, one token 12 -> 7 (3.6 us of GPU time).
+// output type, then the result's) and writes it once; outputs are equal to theirs value
+// for value.  Bound by memory (x in, out out) for many tokens, by the launch for few.
+// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 16.8 us, one token 12 -> 7 a call (1.5 us of GPU time).
 //
-// The arithmetic is next to the memory time (8 experts x 20 instructions per 16-byte
-// vector), hence two values per instruction (f32x2) where the type allows.
+// The arithmetic is next to the memory time (8 experts x 16 instructions per 16-byte vector, 6.5 us of issue slots;
+// 9.0 us to read and write the rows at the copy rate), hence two values per instruction, in fp32 (f32x2) and for the
+// scaling in the element type itself.
 
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
   uint64_t r;
@@ -51,101 +52,195 @@ __device__ __forceinline__ uint64_t round_f32x2<__half>(uint64_t v) {
   return pack_f32x2(f.x, f.y);
 }
 
+// Products of a pair in T itself.  Where the scale is a value of T this is one instruction for the product in fp32
+// and its rounding: a product of two 16-bit values has at most 22 significant bits and, with a scale of at least 1/1024,
+// no digit below the smallest fp32 value, so fp32 holds it exactly and both forms round the same number once.
+template <typename T>
+__device__ __forceinline__ uint32_t mul_t2(uint32_t a, uint32_t b);
+template <>
+__device__ __forceinline__ uint32_t mul_t2<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <>
+__device__ __forceinline__ uint32_t mul_t2<__half>(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ uint32_t both_t2(float v);  // v in both halves
+template <>
+__device__ __forceinline__ uint32_t both_t2<__nv_bfloat16>(float v) { return kb::pack_bf16x2(v, v); }
+template <>
+__device__ __forceinline__ uint32_t both_t2<__half>(float v) {
+  const __half2 h = __floats2half2_rn(v, v);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename T>
+__device__ __forceinline__ uint64_t widen_t2(uint32_t u);  // as a pair of fp32 values
+template <>
+__device__ __forceinline__ uint64_t widen_t2<__nv_bfloat16>(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+template <>
+__device__ __forceinline__ uint64_t widen_t2<__half>(uint32_t u) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u));
+  return pack_f32x2(f.x, f.y);
+}
+// Whether a scale is a value of T.
+template <typename T>
+__device__ __forceinline__ bool is_value_of(float v) {
+  if constexpr (sizeof(T) == 4) return true;
+  else {
+    float lo, hi;
+    unpack_f32x2(widen_t2<T>(both_t2<T>(v)), lo, hi);
+    return lo == v;
+  }
+}
+
 constexpr int LOCAL_WARPS = 4;  // of a CTA
 
-// A warp takes units of 32 * kVecs 16-byte vectors of one token's row, on its own: the (scale,
-// weight) pairs of the token go through its share of shared memory, the next unit's row
-// part and pairs are on their way while it computes.  (One CTA per row with a barrier between
-// the pairs and the arithmetic left the latency of the loads exposed seven times in a row:
-// 2048 tokens of 14 KB, bf16, 31 us.)
+// What a warp needs of one (token, choice): the routing weight twice, as an operand of the two-value instructions, and the
+// expert's scale as fp32 and as a pair of T.
+struct alignas(16) LocalChoice {
+  float w0, w1;
+  uint32_t scale2;
+  float scale;
+};
+
+// A warp takes a fixed part of the rows, 32 * kVecs 16-byte vectors, of every `step`-th token, on its own: the
+// choices of a token go through its share of shared memory, the next token's row part and choices are on their way while it
+// computes.  Issue slots are what bounds it (52 % of them at unit scales, 58 % with scales, at 37 % of the copy rate, in the
+// form before this one), so nothing is done per choice that can be done per token: entries out of range are left out
+// of the list instead of being skipped in the loop, operands are stored the way the instructions want them, and
+// parts that stay the same need no division.
 template <typename T, int kVecs, int kCtas>
-__global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(const A2aParams p, int parts, int units) {
-  __shared__ float2 s_sw[LOCAL_WARPS][64];  // topk <= 64; a negative scale marks an expert id out of range
+__global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(const A2aParams p, int parts, int step) {
+  __shared__ LocalChoice s_choice[LOCAL_WARPS][64];  // topk <= 64
+  kb::wait_for_previous_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float2* sw = s_sw[warp];
-  const int stride = gridDim.x * LOCAL_WARPS;
+  const int gw = blockIdx.x * LOCAL_WARPS + warp;
+  int t = gw / parts;
+  if (t >= step) return;
+  const int part = gw - t * parts;
+  LocalChoice* choice = s_choice[warp];
+  const int v0 = part * (32 * kVecs) + lane;
+  const bool whole = (part + 1) * (32 * kVecs) <= p.vecs;
+  const uint4* src = reinterpret_cast<const uint4*>(p.x) + v0;
+  uint4* dst = reinterpret_cast<uint4*>(p.out) + v0;
   uint4 in[kVecs];
   int e[2];
   float w[2];
-  auto fetch = [&](int unit) {
-    const int t = unit / parts;
-    const int v0 = (unit - t * parts) * (32 * kVecs) + lane;
-    const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(t) * p.row_bytes);
+  auto fetch = [&](int at) {
+    const uint4* row = src + static_cast<size_t>(at) * p.vecs;
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
-      if (v0 + 32 * u < p.vecs) in[u] = kb::ld_nc_v4(src + v0 + 32 * u);
+      if (whole || v0 + 32 * u < p.vecs) in[u] = kb::ld_stream_v4(row + 32 * u);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       if (lane + 32 * i < p.k) {
-        e[i] = __ldg(p.idx + static_cast<size_t>(t) * p.k + lane + 32 * i);
-        w[i] = __ldg(p.w + static_cast<size_t>(t) * p.k + lane + 32 * i);
+        e[i] = p.idx[static_cast<size_t>(at) * p.k + lane + 32 * i];
+        w[i] = p.w[static_cast<size_t>(at) * p.k + lane + 32 * i];
       }
     }
   };
-  int unit = blockIdx.x * LOCAL_WARPS + warp;
-  if (unit < units) fetch(unit);
-  for (; unit < units; unit += stride) {
-    const int t = unit / parts;
-    const int part = unit - t * parts;
-    bool differs = false;  // some scale is not 1
+#pragma unroll
+  for (int u = 0; u < kVecs; ++u) in[u] = make_uint4(0u, 0u, 0u, 0u);
+  if (t < p.T) fetch(t);
+  for (; t < p.T; t += step) {
+    bool differs = false, inexact = false;  // some scale is not 1, not a value of T
+    int n = 0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      if (lane + 32 * i >= p.k) continue;
-      float scale = 1.0f;
-      if (e[i] < 0 || e[i] >= p.E) {
-        if (part == 0) kb::report_status(p.status, KB_DEV_BAD_INDEX, SITE_DISP_IDX, (uint32_t)(t * p.k + lane + 32 * i), p.epoch);
-        scale = -1.0f;
-      } else if (p.scale_mode == 2) {
-        scale = static_cast<float>(e[i] + 1) / static_cast<float>(p.E);
+      if (32 * i >= p.k) break;
+      const bool mine = lane + 32 * i < p.k;
+      const bool valid = mine && e[i] >= 0 && e[i] < p.E;
+      if (mine && !valid && part == 0) kb::report_status(p.status, KB_DEV_BAD_INDEX, SITE_DISP_IDX, (uint32_t)(t * p.k + lane + 32 * i), p.epoch);
+      const float scale = valid && p.scale_mode == 2 ? static_cast<float>(e[i] + 1) / static_cast<float>(p.E) : 1.0f;
+      const uint32_t all = __ballot_sync(0xffffffffu, valid);
+      if (valid) {
+        LocalChoice c;
+        c.w0 = c.w1 = w[i];
+        c.scale2 = 0u;
+        if constexpr (sizeof(T) == 2) c.scale2 = both_t2<T>(scale);
+        c.scale = scale;
+        choice[n + __popc(all & ((1u << lane) - 1u))] = c;
+        differs |= scale != 1.0f;
+        inexact |= !is_value_of<T>(scale);
       }
-      sw[lane + 32 * i] = make_float2(scale, w[i]);
-      differs |= scale != 1.0f;
+      n += __popc(all);
     }
     const bool rounds = __any_sync(0xffffffffu, differs);
+    const bool exact = !__any_sync(0xffffffffu, inexact);
     constexpr int P = Vec16<T>::N / 2;
-    uint64_t xin[kVecs][P], acc[kVecs][P];
+    uint64_t acc[kVecs][P];
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
-      float f[Vec16<T>::N];
-      Vec16<T>::load(in[u], f);
 #pragma unroll
-      for (int i = 0; i < P; ++i) {
-        xin[u][i] = pack_f32x2(f[2 * i], f[2 * i + 1]);
-        acc[u][i] = 0ull;
-      }
+      for (int i = 0; i < P; ++i) acc[u][i] = 0ull;
     }
-    if (unit + stride < units) fetch(unit + stride);
-    __syncwarp();
-    for (int j = 0; j < p.k; ++j) {
-      const float2 c = sw[j];
-      if (c.x < 0.0f) continue;
-      const uint64_t w2 = pack_f32x2(c.y, c.y);
+    if (sizeof(T) == 2 && rounds && exact) {
+      if constexpr (sizeof(T) == 2) {
+        uint32_t xin[kVecs][P];
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u) xin[u][0] = in[u].x, xin[u][1] = in[u].y, xin[u][2] = in[u].z, xin[u][3] = in[u].w;
+        if (t + step < p.T) fetch(t + step);
+        __syncwarp();
+#pragma unroll 2
+        for (int j = 0; j < n; ++j) {
+          const LocalChoice c = choice[j];
+          const uint64_t w2 = pack_f32x2(c.w0, c.w1);
+#pragma unroll
+          for (int u = 0; u < kVecs; ++u) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) acc[u][i] = fma_f32x2(w2, widen_t2<T>(mul_t2<T>(xin[u][i], c.scale2)), acc[u][i]);
+          }
+        }
+      }
+    } else {
+      uint64_t xin[kVecs][P];
+#pragma unroll
+      for (int u = 0; u < kVecs; ++u) {
+        float f[Vec16<T>::N];
+        Vec16<T>::load(in[u], f);
+#pragma unroll
+        for (int i = 0; i < P; ++i) xin[u][i] = pack_f32x2(f[2 * i], f[2 * i + 1]);
+      }
+      if (t + step < p.T) fetch(t + step);
+      __syncwarp();
       if (rounds) {
-        const uint64_t s2 = pack_f32x2(c.x, c.x);
+#pragma unroll 2
+        for (int j = 0; j < n; ++j) {
+          const LocalChoice c = choice[j];
+          const uint64_t w2 = pack_f32x2(c.w0, c.w1), s2 = pack_f32x2(c.scale, c.scale);
 #pragma unroll
-        for (int u = 0; u < kVecs; ++u) {
+          for (int u = 0; u < kVecs; ++u) {
 #pragma unroll
-          for (int i = 0; i < P; ++i) acc[u][i] = fma_f32x2(w2, round_f32x2<T>(mul_f32x2(xin[u][i], s2)), acc[u][i]);
+            for (int i = 0; i < P; ++i) acc[u][i] = fma_f32x2(w2, round_f32x2<T>(mul_f32x2(xin[u][i], s2)), acc[u][i]);
+          }
         }
       } else {
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+          const uint64_t w2 = pack_f32x2(choice[j].w0, choice[j].w1);
 #pragma unroll
-        for (int u = 0; u < kVecs; ++u) {
+          for (int u = 0; u < kVecs; ++u) {
 #pragma unroll
-          for (int i = 0; i < P; ++i) acc[u][i] = fma_f32x2(w2, xin[u][i], acc[u][i]);
+            for (int i = 0; i < P; ++i) acc[u][i] = fma_f32x2(w2, xin[u][i], acc[u][i]);
+          }
         }
       }
     }
-    uint4* dst = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(t) * p.row_bytes);
-    const int v0 = part * (32 * kVecs) + lane;
+    uint4* row = dst + static_cast<size_t>(t) * p.vecs;
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
       float f[Vec16<T>::N];
 #pragma unroll
       for (int i = 0; i < P; ++i) unpack_f32x2(acc[u][i], f[2 * i], f[2 * i + 1]);
-      if (v0 + 32 * u < p.vecs) dst[v0 + 32 * u] = Vec16<T>::store(f);
+      if (whole || v0 + 32 * u < p.vecs) row[32 * u] = Vec16<T>::store(f);
     }
-    __syncwarp();  // the pairs may be overwritten
+    __syncwarp();  // the choices may be overwritten
   }
 }
 
@@ -154,23 +249,24 @@ static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
   const int parts = (p.vecs + 32 * kVecs - 1) / (32 * kVecs);
   const long long units = static_cast<long long>(p.T) * parts;
   if (units > 0x3fffffff) return KB_ERR_UNSUPPORTED;  // three launches of the general kernels
-  // as many rounds as the resident warps need, all warps with the same number of units
+  // All resident warps, though some then have a token more than others: as many warps as have the same number left
+  // every seventh SM a CTA short (2048 tokens of 14 KB 18.6 us against 16.8).
   const long long resident = static_cast<long long>(sms) * kCtas * LOCAL_WARPS;
-  const long long per_cta = (units + resident - 1) / resident * LOCAL_WARPS;
-  const int grid = static_cast<int>((units + per_cta - 1) / per_cta);
-  a2a_local_kernel<T, kVecs, kCtas><<<grid, 32 * LOCAL_WARPS, 0, st>>>(p, parts, static_cast<int>(units));
-  KB_CUDA_OK(cudaGetLastError());
+  const long long at_once = resident < parts ? 1 : resident / parts;  // tokens
+  const long long step = at_once < p.T ? at_once : p.T;
+  const int grid = static_cast<int>((step * parts + LOCAL_WARPS - 1) / LOCAL_WARPS);
+  KB_CUDA_OK(kb::launch_after(a2a_local_kernel<T, kVecs, kCtas>, grid, 32 * LOCAL_WARPS, st, p, parts, static_cast<int>(step)));
   return KB_OK;
 }
 
 template <typename T>
 static int launch_local(const A2aParams& p, int sms, cudaStream_t st) {
   if (p.T == 0) return KB_OK;
-  // Few tokens: one vector per lane spreads a row over more warps (up to about 80 tokens of
-  // 14 KB).  Many: what fits the registers without giving up resident warps; fp32 has
-  // half the values per vector, so twice the vectors (2048 tokens of 7168 values: bf16 31.0 -> 26.9 us, with unit scales
-  // 22.8 -> 16.7; fp32 30.8 -> 24.9; 1500 tokens of 5000 bf16 values are unchanged at 16.5).
+  // Few tokens: one vector per lane spreads a row over more warps (64 tokens of 14 KB 1.94 us of GPU time against 2.05 with four,
+  // 128 tokens 2.95 and 2.60: the line is at about 80).  Many: four, which do with the fewest instructions per value what
+  // the registers allow; back to back in a graph, three inputs in turn, 7168 values, us with 1 / 2 / 4 vectors:
+  //   2048 tokens bf16, scales exact  24.0 19.9 16.8    unit scales 19.9 15.6 13.2    scales not bf16 values 28.6 25.4 21.5
+  //   2048 tokens fp16                30.1 22.5 19.3    fp32 40.8 23.9 19.5           256 tokens bf16          4.6  4.2  3.8
   if (static_cast<long long>(p.T) * p.vecs < 16ll * 32 * sms) return launch_local_as<T, 1, 8>(p, sms, st);
-  if constexpr (sizeof(T) == 4) return launch_local_as<T, 4, 4>(p, sms, st);
-  else return launch_local_as<T, 2, 8>(p, sms, st);
+  return launch_local_as<T, 4, 4>(p, sms, st);
 }

@@ -59,6 +59,29 @@ def test_round_trip_matches_fp32_reference(E, k, H, T, dtype, mode, fused, monke
     assert torch.equal(out1, out2)  # fixed k order: bit-reproducible
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("E", [256, 512, 192])  # scales: values of bf16; of fp16 and some of bf16; of neither
+@pytest.mark.parametrize("H,T", [(7168, 700), (1048, 2048), (520, 3)])  # four vectors per lane, whole and ragged; one
+def test_one_pass_round_trip_equals_the_general_kernels(E, H, T, dtype, monkeypatch):
+    """Value for value, over every exponent of the type, infinities, NaN and zeros (of whose sign the general kernels'
+    additional sum over the ranks keeps nothing)."""
+    from kernel_b200.ops.dispatch_combine import MoEAllToAll
+
+    dev, k = torch.device("cuda"), 8
+    x, idx, w = _inputs(E, k, H, T, torch.float32, dev, seed=5)
+    info = torch.finfo(dtype)
+    span = torch.linspace(torch.log2(torch.tensor(info.smallest_normal)).item() - 12, torch.log2(torch.tensor(info.max)).item() - 3, H, device=dev)
+    x = (x.clamp(-4, 4) * torch.exp2(span)).to(dtype)
+    x[0, :4] = torch.tensor([float("inf"), float("-inf"), float("nan"), -0.0], device=dev, dtype=dtype)
+    out = []
+    for path in ("1", "exchange"):
+        _select(monkeypatch, path)
+        ctx = MoEAllToAll(E, k, H, T, dtype=dtype, device=dev)
+        out.append(ctx.dispatch_scale_combine(x, idx, w, 2))
+    differ = ((out[0] != out[1]) & ~(out[0].isnan() & out[1].isnan())).nonzero()
+    assert differ.numel() == 0, (differ[:8].tolist(), [t[tuple(differ[0].tolist())].item() for t in out])
+
+
 def test_split_dispatch_expert_combine_api():
     """dispatch -> user expert kernel on the received rows -> combine."""
     from kernel_b200.ops.dispatch_combine import MoEAllToAll
