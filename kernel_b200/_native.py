@@ -91,6 +91,9 @@ class LocalGemmArgs(C.Structure):
         ("pair", C.c_int),
         ("bn", C.c_int),
         ("split", C.c_int),
+        ("tok", C.c_int),
+        ("expect", C.c_int),
+        ("early", C.c_int),
     ]
 
 

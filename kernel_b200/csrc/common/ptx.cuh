@@ -152,6 +152,22 @@ __device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
+// The expected bytes (0: this CTA expects none) and one box, issued by one elected lane.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_expect_warp(uint32_t own_bar, uint32_t tx_bytes, uint32_t bar, uint32_t dst, const void* map, int32_t x,
+                                                     int32_t y, int32_t z) {
+#define KB_LOAD_EXPECT(GROUP)                                                                                                      \
+  asm volatile(                                                                                                                    \
+      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\t"                                                                   \
+      "setp.ne.and.u32 e, %1, 0, q;\n\t"                                                                                           \
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"                                                              \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4, {%5, %6, %7}], [%2];\n\t}" \
+      ::"r"(own_bar), "r"(tx_bytes), "r"(bar), "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z)                                          \
+      : "memory")
+  if constexpr (kPair) KB_LOAD_EXPECT(".cta_group::2");
+  else KB_LOAD_EXPECT("");
+#undef KB_LOAD_EXPECT
+}
 // One stage of a GEMM: the expected bytes (0: this CTA expects none) and the boxes of both
 // operands, issued by one elected lane.  One election instead of three: the issuing
 // warp is what bounds narrow tiles.
@@ -272,6 +288,12 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -476,6 +498,11 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_stream_v2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint4 ld_global_v4(const void* p) {

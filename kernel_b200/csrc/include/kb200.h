@@ -144,7 +144,11 @@ typedef struct KbLocalGemmArgs {
   uint32_t* status;
   uint64_t wait_limit_ns;
   int num_ctas;         // 0 = one per SM
-  int pair, bn, split;  // tile configuration; -1 / 0 / 0: chosen from the sizes (pair 2: 512-row tiles)
+  int pair, bn, split;  // tile configuration; -1 / 0 / 0: chosen from the sizes (pair 2: 512-row tiles; 3 and 4: exchanged
+                        // operands, one CTA and pair)
+  int tok;              // exchanged operands: most rows of a tile; 0: chosen from the sizes
+  int expect;           // grouped: rows expected in all groups together; 0: M (ROWS) or K (CONTRACT), which may be a capacity
+  int early;            // the weights and the row table were written before the previous launch of the stream began
 } KbLocalGemmArgs;
 int kb_gemm_local(const KbLocalGemmArgs* args, void* stream);
 // The configuration kb_gemm_local picks for a dense product on `sms` SMs (tests of the rule).

@@ -8,30 +8,12 @@
 #include <atomic>
 #include <mutex>
 
+#include "gemm_local_host.h"
+#include "gemm_swap.h"
+
 namespace {
 
 using namespace kbl;
-
-int ceil_div(int a, int b) { return (a + b - 1) / b; }
-
-// bf16 tensor [d2][d1][d0], contiguous, d0 innermost.
-int make_tmap3(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box0, uint32_t box1) {
-  static auto encode = KB_DRV(cuTensorMapEncodeTiled);
-  if (encode == nullptr) return KB_ERR_UNSUPPORTED;
-  cuuint64_t dims[3] = {d0, d1, d2};
-  cuuint64_t strides[2] = {d0 * 2, d0 * d1 * 2};
-  cuuint32_t box[3] = {box0, box1, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    kb::set_error("cuTensorMapEncodeTiled failed: CUresult %d (ptr %p dims %llu %llu %llu)", (int)r, ptr, (unsigned long long)d0,
-                  (unsigned long long)d1, (unsigned long long)d2);
-    return KB_ERR_CUDA;
-  }
-  return KB_OK;
-}
 
 // Environment switches, read once per process.
 struct Env {
@@ -100,9 +82,9 @@ struct Capacity {
 // 64 x 7168 x 18432 88.5 and 45.1 us, 256 x 4096 x 14336 85.1 and 30.5, 2048 x 2880 x 2880 (in the
 // L2) 35.1 and 24.4.  512-row tiles move 25 % fewer operand bytes
 // per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).
-Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape) {
+Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, double* cost = nullptr) {
   Config best = {false, 256, 1};
-  double best_t = 1e30;
+  double best_cost = 1e30;
   const int KB = ceil_div(K, BK);
   const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
   for (int s = 0; s < 3; ++s) {
@@ -123,16 +105,24 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 2000.0) + epilogue + (pair ? 1000.0 : 0.0);
         if (tall) t += 1.25 * waves * epilogue;
         if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
-        if (t < memory) t = memory;
-        if (t < best_t) {
-          best_t = t;
+        // launched behind the previous kernel instead of under its end
+        const int ctas = (pair ? 2 : 1) * split;
+        const double in_order = overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1]) ? 0.0 : 1500.0;
+        const double both = (t > memory ? t + 0.05 * memory : memory + 0.05 * t) + in_order;
+        if (both < best_cost) {
+          best_cost = both;
           best = {pair, bn, split, tall};
         }
       }
     }
   }
+  if (cost != nullptr) *cost = best_cost;
   return best;
 }
+
+// A tenth of the tensor time, ns, of all rows and columns computed, padding included: under the power cap the energy of
+// products of zeros and stale rows comes out of the clock.
+double mma_energy(double rows, double cols, double K) { return 0.1 * 2.0 * rows * cols * K / 1.6e6; }
 
 // Grouped rows.  The counts stay on the device, so the number of row blocks is an
 // estimate from the average group: one if it fits a tile with two standard deviations
@@ -151,7 +141,7 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
 //   12 of [4096, 1536]      60  56     64  64     76  82     76  84     78  86     80  87     99 109
 // Without that epilogue the model decides; its pairs cost 6 to 10 % at 128 rows per group of [2048, 1024] (76 and 69 us):
 //   64 experts, 128 rows each: 128 x 192 tiles 61 us;  8 experts, 1000 rows of 4096 x 4096: pairs 198 us, one CTA 218 us
-Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape, bool slope) {
+Config rows_plain_config(int M, int groups, int N, int K, bool b_mn, int sms, int shape, bool slope, double* cost_out) {
   Config best;
   best.bn = b_mn ? 128 : 256;
   best.pair = shape > 0;
@@ -177,6 +167,8 @@ Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shap
       const double cost = t > memory ? t + 0.1 * memory : memory + 0.1 * t;
       if (cost < best_t) {
         best_t = cost;
+        // the MMA computes 128 rows (256 for a pair) of every tile
+        *cost_out = cost + mma_energy(groups * blocks * (pair ? 256.0 : 128.0), static_cast<double>(ceil_div(N, bn)) * bn, K);
         best.pair = pair;
         best.bn = bn;
         best.rows = pair ? 128 : rows;
@@ -186,19 +178,101 @@ Config rows_config(int M, int groups, int N, int K, bool b_mn, int sms, int shap
   return best;
 }
 
+// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 per k block
+// (190 for a pair) however narrow the tile.
+double swap_k_block(bool pair, int w_cols, int tok, bool w_mn) {
+  const double mma = 300.0 * tok / 256.0 * (pair ? 1.0 : 1.33);
+  const double load = 128.0 * (w_cols + (pair ? tok / 2 : tok)) / 95.0 * (w_mn ? 1.07 : 1.0);
+  const double issue = pair ? 190.0 : 170.0;
+  const double t = mma > load ? mma : load;
+  return t > issue ? t : issue;
+}
+
+// Dense product with exchanged operands: rows in blocks of at most 256, columns and split so that the tiles fill the chip.
+double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shape, kbs::Config* best) {
+  double best_t = 1e30;
+  const int KB = ceil_div(K, BK), mb = ceil_div(M, 256);
+  const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
+  for (int s = 0; s < 2; ++s) {
+    const bool pair = s == 1;
+    if (shape >= 3 ? s != shape - 3 : pair && cap.clusters[2] < 1) continue;
+    const int step = pair ? 32 : 16;
+    const int tok = ceil_div(ceil_div(M, mb), step) * step;
+    for (int w_cols = w_mn ? 64 : 32; w_cols <= 128; w_cols += w_mn ? 64 : 8) {
+      const int bn = pair ? 2 * w_cols : w_cols;
+      const double tiles = static_cast<double>(mb) * ceil_div(N, bn);
+      const double k_block = swap_k_block(pair, w_cols, tok, w_mn);
+      for (int split = 1; split <= (pair ? 4 : 8); ++split) {
+        const int ctas = (pair ? 2 : 1) * split;
+        const int units = cap.clusters[ctas];
+        if (split > 1 && (tiles > units || KB < 4 * split)) continue;
+        const double waves = units > 0 ? static_cast<double>((static_cast<long long>(tiles) + units - 1) / units) : 1e9;
+        double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 1500.0) + 2000.0 * tok / 256.0 + (pair ? 1000.0 : 0.0);
+        if (split > 1) t += 800.0 + 2200.0 * tok / 256.0 * (split - 1) / split;
+        t = t > memory ? t + 0.05 * memory : memory + 0.05 * t;
+        if (split > 1 && !overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1])) t += 1500.0;
+        if (t < best_t) {
+          best_t = t;
+          best->pair = pair;
+          best->bn = bn;
+          best->tok = tok;
+          best->split = split;
+        }
+      }
+    }
+  }
+  return best_t;
+}
+
+// Grouped rows with exchanged operands; the same estimates.
+kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms, int shape, double* cost_out) {
+  kbs::Config best;
+  double best_t = 1e30;
+  const int KB = ceil_div(K, BK);
+  const double n = static_cast<double>(M) / groups;
+  const double used = n < 1.0 ? n : 1.0;  // share of groups that have rows
+  const double memory = 2.0 * (used * groups * N * static_cast<double>(K) + static_cast<double>(M) * (N + K)) / 6500.0 + 6600.0;
+  for (int s = 0; s < 2; ++s) {
+    const bool pair = s == 1;
+    if (shape >= 0 ? s != shape - 3 : pair && sms < 2) continue;
+    const int step = pair ? 32 : 16;
+    for (int tok = 64; tok <= 256; tok *= 2) {
+      const double fits = n + 2.0 * sqrt(n);
+      const double blocks = fits <= tok ? used : n / tok + 0.5;
+      const int cols = ceil_div(static_cast<int>(fits < tok ? fits : tok) + 1, step) * step;  // of a block
+      for (int w_cols = 64; w_cols <= 128; w_cols += 64) {
+        const int bn = pair ? 2 * w_cols : w_cols;
+        const double tiles = groups * blocks * ceil_div(N, bn);
+        const double units = pair ? sms / 2 : sms;
+        const double waves = tiles <= units ? 1.0 : tiles / units + 0.5;
+        const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, cols < tok ? cols : tok, w_mn) + 1000.0) + 2000.0 * cols / 256.0 +
+                         (pair ? 1000.0 : 0.0);
+        const double cost = t > memory ? t + 0.1 * memory : memory + 0.1 * t;
+        if (cost < best_t) {
+          best_t = cost;
+          *cost_out = cost + mma_energy(groups * blocks * cols, static_cast<double>(ceil_div(N, bn)) * (pair ? 256.0 : 128.0), K);
+          best.pair = pair;
+          best.bn = bn;
+          best.tok = tok;
+        }
+      }
+    }
+  }
+  return best;
+}
+
 // Contractions over a group's rows.  A few k blocks: the outputs are the traffic, the widest
 // tile of one CTA, a pair's hand-overs cost more than its smaller operand traffic saves.
-// More: pairs.  The line is drawn on K / groups, which is the row capacity: up to 63 rows of padding per
-// group are in it.  One CTA and pair in us, cold L2, by the real rows of every group (a multiple of 64):
+// More: pairs.  One CTA and pair in us, cold L2, by the real rows of every group (a multiple of 64):
 //   rows                     128         192         256         320         384         512
 //   64 of 2048 x 1024      70  92      83  92     102  94     113  98     121 105     153 132
 //   32 of 2048 x 2048      72  91      84  90     102  92     113  94     121 102     152 125
 //   8 of 4096 x 4096       72  87      80  88     104  92     113  94     123 102     155 126
 //   128 of 1024 x 768      60  77      68  76      82  82      90  88      98  88     122 100
-// So pairs win from 256 rows on; groups of 256 to 288 rows still get one CTA (capacity below 352).
-Config contract_config(int M, int N, int K, int groups, int shape) {
+// So pairs win from 256 rows on, and the line lies between that and 192.
+Config contract_config(int M, int N, int rows, int groups, int shape) {
   Config c;
-  c.pair = shape >= 0 ? shape > 0 : M > 128 && K / groups >= 352;
+  c.pair = shape >= 0 ? shape > 0 : M > 128 && rows / groups >= 224;
   c.bn = N <= 64 && !c.pair ? 64 : N <= 128 ? 128 : 256;
   c.split = 1;
   return c;
@@ -303,25 +377,75 @@ int device_capacity(int dev, int sms, Capacity* out) {
 
 // The choice depends on the sizes alone and a program calls with the same ones again
 // and again: a small table per thread remembers it (the search takes about 2 us).
-struct Remembered {
-  int M, N, K, key, dev;
+struct Choice {
+  bool swap;      // exchanged operands
   Config c;
+  kbs::Config s;
 };
-int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, Config* out) {
+struct Remembered {
+  int M, N, K, groups, key, dev;
+  Choice c;
+};
+Remembered& remembered(int M, int N, int K, int groups, int key) {
   thread_local Remembered table[64] = {};
-  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   const uint32_t h = (static_cast<uint32_t>(M) * 0x9e3779b1u) ^ (static_cast<uint32_t>(N) * 0x85ebca6bu) ^
-                     (static_cast<uint32_t>(K) * 0xc2b2ae35u) ^ static_cast<uint32_t>(key);
-  Remembered& e = table[(h ^ (h >> 15)) & 63u];
-  if (e.M != M || e.N != N || e.K != K || e.key != key || e.dev != dev) {
+                     (static_cast<uint32_t>(K) * 0xc2b2ae35u) ^ static_cast<uint32_t>(key + groups);
+  return table[(h ^ (h >> 15)) & 63u];
+}
+// Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy.  Near ties keep the rows
+// on the M side, whose epilogue stores wider vectors; with several blocks of rows the models tell less well what is one.
+// GPU time back to back, three weights in turn, us, M side and what is picked:
+//   1 x 8192 x 8192 28.3 26.3     40 x 2840 x 1392 8.2 7.5       64 x 7168 x 18432 47.7 47.2   100 x 4096 x 14336 28.7 26.7
+//   165 x 2920 x 1080 11.9 10.5   200 x 8192 x 8192 36.9 34.4    300 x 1024 x 1024 10.2 7.5    330 x 6296 x 1304 13.8 12.4
+//   400 x 25000 x 1504 38.8 34.7  90 x 1104 x 20000 18.4 15.4    weights along N: 64 x 4096 x 4096 12.3 11.0
+Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape) {
+  Choice r = {};
+  double plain = 0.0;
+  if (shape < 3) r.c = choose_config(M, N, K, a_mn, b_mn, cap, shape, &plain);
+  if (a_mn || (shape >= 0 && shape < 3)) return r;
+  const double other = choose_swap(M, N, K, b_mn, cap, shape, &r.s);
+  if (shape >= 3) {
+    r.swap = true;
+    return r;
+  }
+  const int tall = r.c.tall ? 512 : r.c.pair ? 256 : 128;
+  const int lanes = r.s.pair ? 256 : 128;
+  const double cost_m = plain + mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K);
+  const double cost_n = other + mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K);
+  r.swap = cost_n < (M <= 256 ? 0.97 : 0.92) * cost_m;
+  return r;
+}
+int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, Choice* out) {
+  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+  Remembered& e = remembered(M, N, K, 0, key);
+  if (e.M != M || e.N != N || e.K != K || e.groups != 0 || e.key != key || e.dev != dev) {
     Capacity have;
     const int rc = device_capacity(dev, sms, &have);
     if (rc != KB_OK) return rc;
     for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
-    e = {M, N, K, key, dev, choose_config(M, N, K, a_mn, b_mn, have, shape)};
+    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape)};
   }
   *out = e.c;
   return KB_OK;
+}
+// Grouped rows; `rows` of them are expected.
+Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int shape, bool slope) {
+  const int key = (slope ? 1 : 0) | (w_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+  Remembered& e = remembered(rows, N, K, groups, key);
+  if (e.M != rows || e.N != N || e.K != K || e.groups != groups || e.key != key) {
+    Choice r = {};
+    double plain = 1e30, other = 1e30;
+    if (shape < 3) r.c = rows_plain_config(rows, groups, N, K, w_mn, cap, shape, slope, &plain);
+    if (shape < 0 || shape >= 3) r.s = rows_swap_config(rows, groups, N, K, w_mn, cap, shape, &other);
+    // Groups of some blocks: little padding either way, and near ties go to the M side, unless its epilogue reads saved
+    // values back (each lane a row: it keeps the accumulator of a tile longer).  us, rows on the M side / exchanged:
+    //   rows per group, [N, K]        3, [1024, 2048]   3, [760, 2728]   128, [1024, 2048]   250, [4096, 4096]   717, [544, 3008]
+    //   forward with activation          47.6  45.5        99.5  89.4       75.3  67.7          98.5 101           25.3  26.7
+    //   slope                            56.6  56.0         145   144       90.8  75.4           116  94.4         36.5  31.5
+    r.swap = other < (rows >= 192ll * groups && !slope ? 0.85 : 0.97) * plain;
+    e = {rows, N, K, groups, key, 0, r};
+  }
+  return e.c;
 }
 
 }  // namespace
@@ -375,16 +499,27 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   const int cap = a->num_ctas > 0 && a->num_ctas < sms ? a->num_ctas : sms;
 
   const int groups = grouped ? a->groups : 1;
-  int shape = a->pair;  // -1: choose, 0: one CTA, 1: pair, 2: tall pair
-  if (cap < 2 || env().no_pair) shape = 0;
-  Config c;
-  if (a->kind == KB_LOCAL_DENSE) {
+  const int expect = a->expect > 0 ? a->expect : a->kind == KB_LOCAL_ROWS ? a->M : a->K;
+  int shape = a->pair;  // -1: choose, 0: one CTA, 1: pair, 2: tall pair, 3 and 4: exchanged operands
+  if (cap < 2 || env().no_pair) shape = shape >= 3 ? 3 : 0;
+  Choice pick = {};
+  if (a->kind == KB_LOCAL_ROWS) {
+    pick = pick_rows(cap, expect, groups, a->N, a->K, b_mn, shape, a->pre_in != nullptr);
+  } else if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &c);
+    rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &pick);
     if (rc != KB_OK) return rc;
+    if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
   } else {
-    c = contract ? contract_config(a->M, a->N, a->K, groups, shape) : rows_config(a->M, groups, a->N, a->K, b_mn, cap, shape, a->pre_in != nullptr);
+    pick.c = contract_config(a->M, a->N, expect, groups, shape);
   }
+  if (pick.swap) {
+    if (a->bn > 0) pick.s.bn = a->bn;
+    if (a->tok > 0) pick.s.tok = a->tok;
+    if (a->split > 0) pick.s.split = a->split;
+    return kbs::launch(*a, pick.s, dev, cap, env().timing, stream_v);
+  }
+  Config c = pick.c;
   if (a->bn > 0) c.bn = a->bn;
   if (a->split > 0) c.split = a->split;
   const int KB = ceil_div(a->K, BK);
@@ -477,25 +612,5 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
     if (dev >= 0 && dev < 64) attr_set[dev][shape_row][kernel_row] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_MAX;
-  cfg.stream = static_cast<cudaStream_t>(stream_v);
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
-  if (cluster > 1) {
-    cudaLaunchAttribute& dim = attr[cfg.numAttrs++];
-    dim.id = cudaLaunchAttributeClusterDimension;
-    dim.val.clusterDim.x = cluster;
-    dim.val.clusterDim.y = 1;
-    dim.val.clusterDim.z = 1;
-  }
-  // Set up under the end of the previous kernel, except the clusters of a split contraction:
-  // placed one by one as SMs fall free they leave SMs unused (64 x 7168 x 18432 back to back: 45.1 us
-  // launched in order, 51.7 overlapped).
-  if (c.split == 1) attr[cfg.numAttrs++] = kb::overlap_launch();
-  void* args[] = {&p};
-  KB_CUDA_OK(cudaLaunchKernelExC(&cfg, fn, args));
-  return KB_OK;
+  return launch_clusters(fn, grid, THREADS, cluster, cap, &p, stream_v);
 }

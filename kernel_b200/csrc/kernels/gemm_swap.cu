@@ -1,0 +1,123 @@
+// Host side of the products with exchanged operands (device code: gemm_swap.cuh).
+#include "gemm_swap.cuh"
+
+#include <math.h>
+#include <string.h>
+
+#include "gemm_local_host.h"
+#include "gemm_swap.h"
+
+namespace {
+
+using namespace kbs;
+using kbl::ceil_div;
+
+template <Kind kKind, bool kWMn, Epi kEpi>
+const void* kernel_of(bool pair) {
+  return pair ? (const void*)gemm_swap_kernel<kKind, true, kWMn, kEpi> : (const void*)gemm_swap_kernel<kKind, false, kWMn, kEpi>;
+}
+
+// An activation follows a product whose weights are contiguous along K (forward), a slope one
+// whose weights are contiguous along N (backward).
+const void* find_kernel(int kind, bool w_mn, int epi, bool pair, int* row) {
+  *row = (kind == KB_LOCAL_ROWS ? 4 : 0) + (w_mn ? 2 : 0) + (epi != EPI_PLAIN ? 1 : 0);
+  if (epi != EPI_PLAIN && (epi == EPI_SLOPE) != w_mn) return nullptr;
+  switch (*row) {
+    case 0: return kernel_of<DENSE, false, EPI_PLAIN>(pair);
+    case 1: return kernel_of<DENSE, false, EPI_ACT>(pair);
+    case 2: return kernel_of<DENSE, true, EPI_PLAIN>(pair);
+    case 3: return kernel_of<DENSE, true, EPI_SLOPE>(pair);
+    case 4: return kernel_of<ROWS, false, EPI_PLAIN>(pair);
+    case 5: return kernel_of<ROWS, false, EPI_ACT>(pair);
+    case 6: return kernel_of<ROWS, true, EPI_PLAIN>(pair);
+    case 7: return kernel_of<ROWS, true, EPI_SLOPE>(pair);
+  }
+  return nullptr;
+}
+
+}  // namespace
+
+namespace kbs {
+
+int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool timing, void* stream) {
+  const bool rows = a.kind == KB_LOCAL_ROWS, w_mn = a.b_mn != 0;
+  const int ctas = c.pair ? 2 : 1, step = c.pair ? 32 : 16;
+  const int w_cols = c.bn / ctas;
+  const int tok_cta = c.pair ? c.tok / 2 : c.tok;
+  Params p;
+  memset(&p, 0, sizeof(p));
+  p.KB = ceil_div(a.K, BK);
+  if (w_cols < 8 || w_cols > LANES || c.bn % (w_mn ? 64 * ctas : 8 * ctas) != 0 || c.tok < step || c.tok > 256 || c.tok % step != 0 ||
+      c.split < 1 || c.split > (c.pair ? 4 : 8) || c.split > p.KB || (rows && c.split > 1)) {
+    kb::set_error("kb_gemm_local: exchanged tile configuration pair=%d bn=%d tok=%d split=%d does not fit the problem", (int)c.pair, c.bn,
+                  c.tok, c.split);
+    return KB_ERR_ARG;
+  }
+  p.M = a.M;
+  p.N = a.N;
+  p.K = a.K;
+  p.NB = ceil_div(a.N, c.bn);
+  p.MB = ceil_div(a.M, c.tok);
+  p.bn = c.bn;
+  p.tok = c.tok;
+  // Grouped rows: most blocks are shorter than `tok`.  Boxes of half the expected block fetch little in vain and a warp issues
+  // two of them in the time the weights take (64 groups of 128 rows, 2048 x 1024: boxes of 32 rows 73.7 us, so 67.7).
+  p.xbox = tok_cta;
+  if (rows) {
+    const double n = static_cast<double>(a.expect > 0 ? a.expect : a.M) / a.groups, fits = n + 2.0 * sqrt(n);
+    const int expect = fits < c.tok ? (static_cast<int>(fits) / step + 1) * step / ctas : tok_cta;
+    p.xbox = ceil_div(expect, 16) * 8;
+    if (p.xbox < 16) p.xbox = 16;
+    if (p.xbox > tok_cta) p.xbox = tok_cta;
+  }
+  p.groups = rows ? a.groups : 0;
+  p.split = c.split;
+  p.w_slot = w_cols * BK * 2;
+  p.x_slot = ceil_div(tok_cta, p.xbox) * p.xbox * BK * 2;
+  const int room = kbl::SMEM_MAX - 1024 - BAR_BYTES - (rows ? (3 * a.groups + 1) * 4 : 4);
+  p.stages = room / (p.w_slot + p.x_slot);
+  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+  // the MMA reads 128 rows from the last slot of the weights on, of a narrower tile too: the token slots lie behind it
+  if (p.stages < 2 || p.stages * p.x_slot + p.w_slot < LANES * BK * 2 ||
+      (c.split > 1 && ceil_div(ceil_div(c.tok, CHUNK), c.split) * (c.split - 1) * LANES * CHUNK * 4 > p.stages * (p.w_slot + p.x_slot))) {
+    kb::set_error("kb_gemm_local: operand ring too small");
+    return KB_ERR_ARG;
+  }
+  p.act = a.act;
+  p.early = a.early != 0 ? 1 : 0;
+  p.bias = static_cast<const bf16*>(a.bias);
+  p.bias_scale = a.bias_scale;
+  p.out = static_cast<bf16*>(a.out);
+  p.pre_out = static_cast<bf16*>(a.pre_out);
+  p.pre_in = static_cast<const bf16*>(a.pre_in);
+  p.row_start = a.row_start;
+  p.row_count = a.row_count;
+  p.status = a.status;
+  p.limit_ns = a.wait_limit_ns ? a.wait_limit_ns : 2000000000ull;
+  p.timing = timing ? 1 : 0;
+  const uint64_t wz = rows ? a.groups : 1;
+  int rc = kbl::make_tmap3(&p.tmX, a.A, a.K, a.M, 1, BK, p.xbox);
+  if (rc != KB_OK) return rc;
+  rc = w_mn ? kbl::make_tmap3(&p.tmW, a.B, a.N, a.K, wz, 64, BK) : kbl::make_tmap3(&p.tmW, a.B, a.K, a.N, wz, BK, w_cols);
+  if (rc != KB_OK) return rc;
+
+  const int cluster = ctas * c.split;
+  const long long blocks = rows ? a.M / c.tok + static_cast<long long>(a.groups) : p.MB;  // rows: at most one partly filled block per group
+  long long grid = blocks * p.NB * cluster;
+  if (c.split == 1 && grid > cap / ctas * ctas) grid = cap / ctas * ctas;
+  const int epi = a.pre_in != nullptr ? EPI_SLOPE : a.act != kbl::ACT_NONE ? EPI_ACT : EPI_PLAIN;
+  int row = 0;
+  const void* fn = find_kernel(a.kind, w_mn, epi, c.pair, &row);
+  if (fn == nullptr) {
+    kb::set_error("kb_gemm_local: no kernel for kind %d, weights along N %d, epilogue %d", a.kind, (int)w_mn, epi);
+    return KB_ERR_UNSUPPORTED;
+  }
+  static bool attr_set[64][2][8] = {};
+  if (dev < 0 || dev >= 64 || !attr_set[dev][c.pair][row]) {
+    KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kbl::SMEM_MAX));
+    if (dev >= 0 && dev < 64) attr_set[dev][c.pair][row] = true;
+  }
+  return kbl::launch_clusters(fn, static_cast<int>(grid), THREADS, cluster, cap, &p, stream);
+}
+
+}  // namespace kbs

@@ -35,7 +35,8 @@ class MoELayer:
             a2a._validate(x, indices, weights)
             er = ExpertRows(x.flatten(1), indices, a2a.E, status=a2a.status)
             h = rows_product(er.rows, self.w_up, er.start, er.count, act="silu", status=a2a.status)
-            return er.combine(rows_product(h, self.w_down, er.start, er.count, status=a2a.status), weights).view(x.shape)
+            y = rows_product(h, self.w_down, er.start, er.count, status=a2a.status, early=True)
+            return er.combine(y, weights).view(x.shape)
         counts, recv = a2a.dispatch(x, indices)
         # the segment lengths size the buffers (one sync per layer call); the rows of
         # one expert, from all sources, are gathered into one block per expert
@@ -107,11 +108,17 @@ def _group_table(n_e, pad: int, device):
     return (start.to(torch.int32).to(device), padded.to(torch.int32).to(device), pos.to(device), int(padded.sum()))
 
 
+def _expected_rows(er: ExpertRows):
+    """Rows of all experts together, and with each expert padded by half an alignment on average."""
+    real = er.T * er.k
+    return real, real + min(er.E, real) * (ROW_ALIGN // 2)
+
+
 class _LocalMoEFn(torch.autograd.Function):
     """The block on one GPU: eight launches forward and backward together besides the
     two of the combine passes, none of which waits for the host.  Experts start at
     multiples of 64 rows with zero rows in between, so the weight gradients can
-    contract over whole k blocks."""
+    contract over whole k blocks; only what they contract over is computed for those rows."""
 
     @staticmethod
     def forward(ctx, x, weights, w_up, w_down, layer, indices):
@@ -119,8 +126,9 @@ class _LocalMoEFn(torch.autograd.Function):
         a2a._validate(x, indices, weights)
         er = ExpertRows(x.flatten(1), indices, a2a.E, pad=ROW_ALIGN, status=a2a.status)
         pre = torch.empty((er.rows.shape[0], w_up.shape[1]), dtype=x.dtype, device=x.device)
-        h = rows_product(er.rows, w_up, er.start, er.padded, act="silu", pre_out=pre, status=a2a.status)
-        Y = rows_product(h, w_down, er.start, er.padded, status=a2a.status)
+        real, padded = _expected_rows(er)
+        h = rows_product(er.rows, w_up, er.start, er.padded, act="silu", pre_out=pre, status=a2a.status, expect=padded)
+        Y = rows_product(h, w_down, er.start, er.count, status=a2a.status, early=True, expect=real)
         ctx.sizes, ctx.status = (er.T, er.k, er.E), a2a.status
         ctx.save_for_backward(weights, w_up, w_down, pre, h, Y, er.rows, er.table)
         return er.combine(Y, weights).view(x.shape)
@@ -130,10 +138,11 @@ class _LocalMoEFn(torch.autograd.Function):
         weights, w_up, w_down, pre, h, Y, rows, table = ctx.saved_tensors
         er, status = ExpertRows.saved(rows, table, *ctx.sizes), ctx.status
         dYs, dweights = er.grad_rows(dy.contiguous().flatten(1), Y, weights)
-        dpre = rows_product(dYs, w_down, er.start, er.padded, b_t=True, act="silu", pre_in=pre, status=status)
-        dw_down = contract_product(dYs, h, er.start, er.count, status=status)
-        dw_up = contract_product(dpre, rows, er.start, er.count, status=status)
-        dX = rows_product(dpre, w_up, er.start, er.padded, b_t=True, status=status)
+        real, padded = _expected_rows(er)
+        dpre = rows_product(dYs, w_down, er.start, er.padded, b_t=True, act="silu", pre_in=pre, status=status, early=True, expect=padded)
+        dw_down = contract_product(dYs, h, er.start, er.count, status=status, expect=real)
+        dw_up = contract_product(dpre, rows, er.start, er.count, status=status, expect=real)
+        dX = rows_product(dpre, w_up, er.start, er.count, b_t=True, status=status, early=True, expect=real)
         return er.combine(dX, None).view(dy.shape), dweights, dw_up, dw_down, None, None
 
 

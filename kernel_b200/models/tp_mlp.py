@@ -59,6 +59,8 @@ class SequenceParallelMLP:
         if x_local.is_cuda and self._plain():
             self.up.check(x_local, self.w1)
             h = product(x_local, self.w1, self.b1, act=self.activation, status=self.up.status)   # the activation in the product's epilogue
+            if type(self.down) is GemmRS and h.shape[0] == self.down.M and self.w2.shape[0] == self.down.N:
+                return product(h, self.w2, self.b2, status=self.down.status, early=True)
             return self.down(h, self.w2, self.b2)
         h = self.up(x_local, self.w1, self.b1)           # [tokens, ffn/world]
         h = self._act(h)

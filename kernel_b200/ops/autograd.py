@@ -132,7 +132,7 @@ class LocalMLPFn(torch.autograd.Function):
         h = product(x, w1, b1, act=act, pre_out=pre, status=status)
         ctx.act, ctx.status = act, status
         ctx.save_for_backward(x, w1, w2, pre, h)
-        return product(h, w2, b2, status=status)
+        return product(h, w2, b2, status=status, early=True)
 
     @staticmethod
     def backward(ctx, dy):
@@ -146,13 +146,13 @@ class LocalMLPFn(torch.autograd.Function):
         if need_b2:
             db2 = col_sum(dy)
         if need_x or need_w1 or need_b1:
-            dpre = product(dy, w2, b_t=True, act=ctx.act, pre_in=pre, status=status)
+            dpre = product(dy, w2, b_t=True, act=ctx.act, pre_in=pre, status=status, early=need_w2)  # else its weights may just have been copied
             if need_w1:
                 dw1 = product(dpre, x, a_t=True, b_t=True, status=status)
             if need_b1:
                 db1 = col_sum(dpre)
             if need_x:
-                dx = product(dpre, w1, b_t=True, status=status)
+                dx = product(dpre, w1, b_t=True, status=status, early=True)
         return dx, dw1, db1, dw2, db2, None, None
 
 

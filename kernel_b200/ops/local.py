@@ -106,12 +106,14 @@ def _launch(args: N.LocalGemmArgs, device: torch.device) -> None:
 
 def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, *, a_t: bool = False, b_t: bool = False,
             act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
-            out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
+            out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
     """``A @ B^T (+ bias)`` in bf16 with fp32 accumulation, ``A`` being ``a[M, K]`` (``a_t``: ``a[K, M]``)
     and ``B`` being ``b[N, K]`` (``b_t``: ``b[K, N]``); ``a_t`` needs ``b_t``.
 
     ``act``: the activation of the rounded product, which ``pre_out`` also receives;
-    with ``pre_in`` the product is multiplied by the activation's slope there."""
+    with ``pre_in`` the product is multiplied by the activation's slope there.
+    ``early``: the stream's previous launch is one of this module's kernels and did not write ``b``, so the product may
+    fetch it before that one has ended."""
     _check_operand(a, "a", 2, a.device)
     _check_operand(b, "b", 2, a.device)
     K, M = a.shape if a_t else a.shape[::-1]
@@ -126,7 +128,7 @@ def product(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = Non
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=a.device)
     args = _args(N.LOCAL_DENSE, M, Nn, K, status)
-    args.a_mn, args.b_mn = a_t, b_t
+    args.a_mn, args.b_mn, args.early = a_t, b_t, early
     args.bias, args.bias_scale = _ptr(bias), 1.0
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
@@ -149,10 +151,15 @@ def col_sum(x: torch.Tensor) -> torch.Tensor:
 
 def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor, *, b_t: bool = False,
                  act: Optional[str] = None, pre_out: Optional[torch.Tensor] = None, pre_in: Optional[torch.Tensor] = None,
-                 out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None, early: bool = False,
+                 expect: int = 0) -> torch.Tensor:
     """Rows ``start[e] .. start[e] + count[e]`` of ``a[R, K]`` times ``b[e]`` transposed
-    (``b[E, N, K]``, ``b_t``: ``b[E, K, N]``).  Rows outside every group are left alone."""
+    (``b[E, N, K]``, ``b_t``: ``b[E, K, N]``).  Rows outside every group are left alone.  ``early``: the stream's previous
+    launch is a kernel of this module and wrote neither ``b`` nor the table.  ``expect``: rows expected in all groups, where
+    ``R`` is a capacity (the choice of tiles depends on it, nothing else)."""
+    given = b
     b = _expert_matrices(b)
+    early = early and b is given  # else that launch is the copy
     _check_operand(a, "a", 2, a.device)
     _check_operand(b, "b", 3, a.device)
     R, K = a.shape
@@ -175,7 +182,7 @@ def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: t
                         None if pre_in is None else pre_in[sl], out[sl])
         return out
     args = _args(N.LOCAL_ROWS, R, Nn, K, status)
-    args.b_mn, args.groups = b_t, E
+    args.b_mn, args.groups, args.expect, args.early = b_t, E, expect, early
     args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     args.act, args.pre_out, args.pre_in = N.ACTS.get(act, 0), _ptr(pre_out), _ptr(pre_in)
@@ -184,7 +191,7 @@ def rows_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: t
 
 
 def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, count: torch.Tensor,
-                     status: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     status: Optional[torch.Tensor] = None, expect: int = 0) -> torch.Tensor:
     """``out[e] = a[rows of e]^T @ b[rows of e]`` for ``a[R, M]``, ``b[R, N]``.  Groups start at
     multiples of ``ROW_ALIGN``; rows between a group's last and the next multiple are
     zero in one operand and finite in the other."""
@@ -201,7 +208,7 @@ def contract_product(a: torch.Tensor, b: torch.Tensor, start: torch.Tensor, coun
         return out
     out = torch.empty((E, M, Nn), dtype=torch.bfloat16, device=a.device)
     args = _args(N.LOCAL_CONTRACT, M, Nn, R, status)
-    args.groups = E
+    args.groups, args.expect = E, expect
     args.row_start, args.row_count = start.data_ptr(), count.data_ptr()
     args.A, args.B, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
     _launch(args, a.device)

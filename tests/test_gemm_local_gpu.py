@@ -190,6 +190,66 @@ def test_epilogues_of_every_tile_shape(act, pair, bn, split, M, N, K, monkeypatc
 
 
 @pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
+@pytest.mark.parametrize("pair,bn,split", [(3, 64, 1), (3, 128, 1), (3, 64, 3), (3, 128, 8), (4, 128, 1), (4, 256, 1), (4, 128, 4), (4, 256, 2)])
+@pytest.mark.parametrize("M,N,K", [(1, 264, 2120), (64, 296, 1096), (165, 72, 520), (520, 264, 1096)])
+def test_epilogues_with_exchanged_operands(act, pair, bn, split, M, N, K, monkeypatch):
+    """Token rows on the MMA's N side: one token, whole and ragged blocks, several of them, columns that end inside a tile."""
+    L = _force(monkeypatch, pair, bn, split)
+    a, b = _ints(M, K, seed=34), _ints(N, K, seed=35) * 2 ** -5
+    st = _status()
+    pre = torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = L.product(a, b, act=act, pre_out=pre, status=st)
+    grad = L.product(a, b.t().contiguous(), b_t=True, act=act, pre_in=pre, status=st, early=True)
+    bias = _ints(N, seed=36)
+    plain = L.product(a, b, bias, status=st, early=True)
+    _clean(st)
+    full = a.float() @ b.float().t()
+    _check_epilogues(act, full, pre, out, grad)
+    assert torch.equal(plain, (full + bias.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("pair,bn", [(3, 64), (3, 128), (4, 128), (4, 256)])
+@pytest.mark.parametrize("counts", COUNTS)
+def test_grouped_rows_with_exchanged_operands(pair, bn, counts, monkeypatch):
+    L = _force(monkeypatch, pair, bn)
+    N, K = 264, 520
+    start, count, R = _table(counts, 1)
+    a, b = _ints(R, K, seed=37), _ints(len(counts), N, K, seed=38) * 2 ** -4
+    st = _status()
+    pre, out, grad, plain = (torch.full((R, N), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(4))
+    L.rows_product(a, b, start, count, act="silu", pre_out=pre, out=out, status=st)
+    L.rows_product(a, b.transpose(1, 2).contiguous(), start, count, b_t=True, act="silu", pre_in=pre, out=grad, status=st)
+    L.rows_product(a, b, start, count, out=plain, status=st, early=True, expect=len(counts))
+    _clean(st)
+    inside = torch.zeros(R, dtype=torch.bool, device=DEV)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        inside[s:s + n] = True
+        sl = slice(s, s + n)
+        full = a[sl].float() @ b[e].float().t()
+        _check_epilogues("silu", full, pre[sl], out[sl], grad[sl])
+        assert torch.equal(plain[sl], full.to(torch.bfloat16))
+    assert all((t[~inside] == 7.0).all() for t in (pre, out, grad, plain))
+
+
+def test_weights_fetched_early_are_those_of_the_call():
+    """The second product's weights change right before the block runs, call after call."""
+    from kernel_b200.models import SequenceParallelMLP
+
+    T, H, F = 24, 1032, 2056
+    w1, w2 = _ints(F, H, seed=39) * 2 ** -6, _ints(H, F, seed=40) * 2 ** -6
+    mlp = SequenceParallelMLP(T, H, w1, w2, activation="relu")
+    x = _ints(T, H, seed=41)
+    want = mlp(x)
+    for i in range(40):
+        mlp.w2.neg_()
+        want = -want
+        assert torch.equal(mlp(x), want), i
+    mlp.up.status.cpu()
+    _clean(mlp.up.status)
+    _clean(mlp.down.status)
+
+
+@pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
 @pytest.mark.parametrize("pair,bn", [(0, 64), (0, 256), (1, 128), (1, 256)])
 @pytest.mark.parametrize("counts", COUNTS)
 def test_epilogues_of_grouped_rows(act, pair, bn, counts, monkeypatch):
