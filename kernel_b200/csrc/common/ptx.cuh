@@ -148,6 +148,22 @@ __device__ __forceinline__ void tma_load_3d_warp(uint32_t smem_dst, const void* 
         : "memory");
   }
 }
+// The expected bytes (0: this CTA expects none) and one box of a 4-D map, issued by one elected lane.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_4d_expect_warp(uint32_t own_bar, uint32_t tx_bytes, uint32_t bar, uint32_t dst, const void* map, int32_t x,
+                                                        int32_t y, int32_t z, int32_t w) {
+#define KB_LOAD_EXPECT(GROUP)                                                                                                          \
+  asm volatile(                                                                                                                        \
+      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\t"                                                                       \
+      "setp.ne.and.u32 e, %1, 0, q;\n\t"                                                                                               \
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"                                                                  \
+      "@q cp.async.bulk.tensor.4d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4, {%5, %6, %7, %8}], [%2];\n\t}" \
+      ::"r"(own_bar), "r"(tx_bytes), "r"(bar), "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w)                                      \
+      : "memory")
+  if constexpr (kPair) KB_LOAD_EXPECT(".cta_group::2");
+  else KB_LOAD_EXPECT("");
+#undef KB_LOAD_EXPECT
+}
 __device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes) {
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");

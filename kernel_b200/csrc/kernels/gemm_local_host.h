@@ -29,6 +29,26 @@ inline int make_tmap3(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d
   return KB_OK;
 }
 
+// bf16 tensor [d2][d1][d0], d0 a multiple of 64, seen as [d2][d0 / 64][d1][64]: a box is `blocks` blocks of 64 elements
+// by `box1` rows, in shared memory block by block.
+inline int make_tmap4_blocks(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box1, uint32_t blocks) {
+  static auto encode = KB_DRV(cuTensorMapEncodeTiled);
+  if (encode == nullptr) return KB_ERR_UNSUPPORTED;
+  cuuint64_t dims[4] = {64, d1, d0 / 64, d2};
+  cuuint64_t strides[3] = {d0 * 2, 128, d0 * d1 * 2};
+  cuuint32_t box[4] = {64, box1, blocks, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    kb::set_error("cuTensorMapEncodeTiled failed: CUresult %d (ptr %p dims %llu %llu %llu)", (int)r, ptr, (unsigned long long)d0,
+                  (unsigned long long)d1, (unsigned long long)d2);
+    return KB_ERR_CUDA;
+  }
+  return KB_OK;
+}
+
 // Whether a launch of `grid` CTAs is set up under the end of the previous kernel of the stream.  Without that it starts up
 // to 2 us after the end of the one before.  Not so where clusters of an odd size fill the chip: placed one by one as SMs
 // fall free they leave some unused.  Launched in order and overlapped, us:

@@ -98,7 +98,10 @@ int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool tim
   const uint64_t wz = rows ? a.groups : 1;
   int rc = kbl::make_tmap3(&p.tmX, a.A, a.K, a.M, 1, BK, p.xbox);
   if (rc != KB_OK) return rc;
-  rc = w_mn ? kbl::make_tmap3(&p.tmW, a.B, a.N, a.K, wz, 64, BK) : kbl::make_tmap3(&p.tmW, a.B, a.K, a.N, wz, BK, w_cols);
+  // [groups][N / 64][K][64]: the two blocks of 64 columns in one load; otherwise two loads, clipped at N
+  p.w_whole = w_mn && a.N % 64 == 0 ? 1 : 0;
+  rc = p.w_whole ? kbl::make_tmap4_blocks(&p.tmW, a.B, a.N, a.K, wz, BK, w_cols / 64)
+       : w_mn ? kbl::make_tmap3(&p.tmW, a.B, a.N, a.K, wz, 64, BK) : kbl::make_tmap3(&p.tmW, a.B, a.K, a.N, wz, BK, w_cols);
   if (rc != KB_OK) return rc;
 
   const int cluster = ctas * c.split;

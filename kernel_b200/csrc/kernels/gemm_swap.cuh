@@ -51,6 +51,7 @@ struct alignas(64) Params {
   int xbox;            // rows of one box of X
   int groups, split;
   int stages, w_slot, x_slot;
+  int w_whole;         // weights contiguous along N, a multiple of 64 of them: one box of a 4-D map holds a stage's columns
   int act;
   int early;
   const bf16* bias;
@@ -331,7 +332,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
           s = 0;
           ph ^= 1u;
         }
-        // a pair's bytes are counted on the leader's barrier
+        // A pair's bytes are counted on the leader's barrier.  Weights along N: one load instead of two per k block (input
+        // gradients of 64 experts of 2048 x 1024, 3 rows each: 51.6 -> 44.8 us, 16 rows: 53.0 -> 50.1).
+        if (kWMn && p.w_whole) {
+          kb::tma_load_4d_expect_warp<kPair>(own, leader ? bytes : 0u, bar, dst, &p.tmW, 0, k * BK, col / 64, t.group);
+          continue;
+        }
         kb::tma_load_expect_warp<kPair>(own, leader ? bytes : 0u, bar, dst, &p.tmW, kWMn ? col : k * BK, kWMn ? k * BK : col, t.group);
         if constexpr (kWMn) {
           for (int i = 1; i < w_cols / 64; ++i) {
