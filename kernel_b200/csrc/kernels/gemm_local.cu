@@ -84,7 +84,7 @@ struct Capacity {
 // per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).
 Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, double* cost = nullptr) {
   Config best = {false, 256, 1};
-  double best_cost = 1e30;
+  double best_t = 1e30, best_cost = 1e30;
   const int KB = ceil_div(K, BK);
   const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
   for (int s = 0; s < 3; ++s) {
@@ -109,7 +109,9 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         const int ctas = (pair ? 2 : 1) * split;
         const double in_order = overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1]) ? 0.0 : 1500.0;
         const double both = (t > memory ? t + 0.05 * memory : memory + 0.05 * t) + in_order;
-        if (both < best_cost) {
+        t = (t > memory ? t : memory) + in_order;
+        if (t < best_t) {
+          best_t = t;
           best_cost = both;
           best = {pair, bn, split, tall};
         }

@@ -315,12 +315,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
     const uint32_t w_bytes = static_cast<uint32_t>(w_cols) * BK * 2;
     const uint32_t box_bytes = static_cast<uint32_t>(p.xbox) * BK * 2;
     uint32_t s = 0, ph = 0;
+    int ahead = p.early ? p.stages : -1;  // stages to fill before the previous launch has ended; then its end is no part of a bounded wait
     bool ok = true;
     for (int pos = sched_id; ok && pos < total_tiles; pos += sched_n) {
       const Tile t = tile_at(pos);
       const uint32_t bytes = (w_bytes + static_cast<uint32_t>(boxes_of(t)) * box_bytes) * (kPair ? 2 : 1);
       const int col = t.n0 + static_cast<int>(half) * w_cols;
       for (int k = k0; k < k1; ++k) {
+        if (ahead >= 0 && ahead-- == 0) kb::wait_for_previous_launch();
         if (!kb::mbar_wait_bounded(&empty[s], ph ^ 1u, p.limit_ns, 400)) {
           kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, kbl::SITE_EMPTY, (uint32_t)pos, 0);
           *abort_flag = 1;
