@@ -395,7 +395,8 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
   return table[(h ^ (h >> 15)) & 63u];
 }
 // Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy.  Near ties keep the rows
-// on the M side, whose epilogue stores wider vectors; with several blocks of rows the models tell less well what is one.
+// on the M side, whose epilogue stores wider vectors; from 129 rows on both kinds compute whole blocks and the models tell
+// less well what a tie is (195 x 26136 x 3200 in an MLP: ratio 0.94, 108.5 us for the block and 110.3 exchanged).
 // GPU time back to back, three weights in turn, us, M side and what is picked:
 //   1 x 8192 x 8192 28.3 26.3     40 x 2840 x 1392 8.2 7.5       64 x 7168 x 18432 47.7 47.2   100 x 4096 x 14336 28.7 26.7
 //   165 x 2920 x 1080 11.9 10.5   200 x 8192 x 8192 36.9 34.4    300 x 1024 x 1024 10.2 7.5    330 x 6296 x 1304 13.8 12.4
@@ -414,7 +415,7 @@ Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, in
   const int lanes = r.s.pair ? 256 : 128;
   const double cost_m = plain + mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K);
   const double cost_n = other + mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K);
-  r.swap = cost_n < (M <= 256 ? 0.97 : 0.92) * cost_m;
+  r.swap = cost_n < (M <= 128 ? 0.97 : M <= 256 ? 0.93 : 0.92) * cost_m;
   return r;
 }
 int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, Choice* out) {
