@@ -51,15 +51,16 @@ class SequenceParallelMLP:
         raise ValueError(f"unknown activation {self.activation!r}")
 
     def _plain(self) -> bool:
-        """One rank, and the up-projection and the activation are the block's own."""
-        return (self.world == 1 and self.activation in ACTS and type(self.up) is AGGemm
+        """One rank, and the up-projection and the activation are the block's own (a context put in
+        the projection's place may span several ranks)."""
+        return (self.world == 1 and self.activation in ACTS and type(self.up) is AGGemm and self.up.world == 1
                 and getattr(self._act, "__func__", None) is SequenceParallelMLP._act)
 
     def __call__(self, x_local: torch.Tensor) -> torch.Tensor:
         if x_local.is_cuda and self._plain():
             self.up.check(x_local, self.w1)
             h = product(x_local, self.w1, self.b1, act=self.activation, status=self.up.status)   # the activation in the product's epilogue
-            if type(self.down) is GemmRS and h.shape[0] == self.down.M and self.w2.shape[0] == self.down.N:
+            if type(self.down) is GemmRS and self.down.world == 1 and h.shape[0] == self.down.M and self.w2.shape[0] == self.down.N:
                 return product(h, self.w2, self.b2, status=self.down.status, early=True)
             return self.down(h, self.w2, self.b2)
         h = self.up(x_local, self.w1, self.b1)           # [tokens, ffn/world]

@@ -111,3 +111,38 @@ def test_inference_block_calls_what_was_put_in_place_of_its_parts():
     mlp = SequenceParallelMLP(8, 16, w1, w2)
     mlp._act = torch.relu
     assert not mlp._plain()
+
+
+def test_inference_block_leaves_the_exchange_to_parts_that_span_several_ranks(monkeypatch):
+    """A block of one rank whose down (or up) projection was replaced by a context over two ranks calls it: the
+    one-GPU product would return the unreduced sum (or a part of the rows)."""
+    from kernel_b200.models import SequenceParallelMLP, tp_mlp
+    from kernel_b200.ops.gemm import AGGemm, GemmRS
+
+    class OnGpu(torch.Tensor):
+        is_cuda = property(lambda self: True)
+
+    products, exchanged = [], []
+    monkeypatch.setattr(tp_mlp, "product", lambda a, b, *args, **kw: products.append(kw) or torch.zeros(a.shape[0], b.shape[0], dtype=a.dtype))
+    for kind in (AGGemm, GemmRS):
+        monkeypatch.setattr(kind, "__call__", lambda self, a, w, *args: exchanged.append(self) or torch.zeros(self.M, w.shape[0], dtype=a.dtype))
+    w1, w2 = torch.zeros(24, 16, dtype=torch.bfloat16), torch.zeros(16, 24, dtype=torch.bfloat16)
+
+    def block():
+        mlp = SequenceParallelMLP(8, 16, w1, w2)
+        mlp.up.status = mlp.down.status = None
+        return mlp
+
+    def call(mlp, rows=8):
+        products.clear()
+        exchanged.clear()
+        mlp(torch.zeros(rows, 16, dtype=torch.bfloat16).as_subclass(OnGpu))
+        return len(products), exchanged
+
+    assert call(block()) == (2, [])
+    mlp = block()
+    mlp.down.world = 2
+    assert call(mlp) == (1, [mlp.down])
+    mlp = block()
+    mlp.up.world = 2
+    assert call(mlp, rows=4) == (0, [mlp.up, mlp.down])
