@@ -97,6 +97,10 @@ class LocalGemmArgs(C.Structure):
     ]
 
 
+class LocalPick(C.Structure):
+    _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split")]
+
+
 class A2aArgs(C.Structure):
     _fields_ = [
         ("rank", C.c_int),
@@ -160,6 +164,7 @@ def _declare(lib: C.CDLL) -> None:
         "kb_device_barrier": (i, [C.POINTER(vp), u64, i, i, u32, u64, vp, vp]),
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
         "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
+        "kb_gemm_local_pick": (i, [C.POINTER(LocalGemmArgs), i, C.POINTER(LocalPick)]),
         "kb_gemm_local_config": (i, [i, i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
         "kb_col_sum_parts": (i, [i, i]),
         "kb_col_sum": (i, [vp, i, i, vp, vp, vp]),

@@ -151,7 +151,16 @@ typedef struct KbLocalGemmArgs {
   int early;            // the weights and the row table were written before the previous launch of the stream began
 } KbLocalGemmArgs;
 int kb_gemm_local(const KbLocalGemmArgs* args, void* stream);
-// The configuration kb_gemm_local picks for a dense product on `sms` SMs (tests of the rule).
+// The tile kb_gemm_local launches for these arguments on a B200 with `sms` SMs (tests of the rules; no pointer is read).
+// KB_ERR_UNSUPPORTED: one the kernel cannot run was asked for.
+typedef struct KbLocalPick {
+  int exchanged;  // token rows on the tensor cores' N side
+  int pair;       // CTA pairs; 2: 512-row tiles
+  int bn, rows;   // columns and (most) rows of a tile
+  int split;      // members of a cluster that share a tile's contraction
+} KbLocalPick;
+int kb_gemm_local_pick(const KbLocalGemmArgs* args, int sms, KbLocalPick* out);
+// The tile a dense product on `sms` SMs gets if its rows are on the M side.
 int kb_gemm_local_config(int M, int N, int K, int a_mn, int b_mn, int sms, int* pair, int* bn, int* split);
 // The fused modes (RS, AG) run by a CPU rank over a KB_BACKEND_HOST heap: same
 // schedule, staging layouts, flags and rounding points as the kernel (symm/gemm_host.cpp).

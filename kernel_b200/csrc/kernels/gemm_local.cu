@@ -208,6 +208,13 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
         const int ctas = (pair ? 2 : 1) * split;
         const int units = cap.clusters[ctas];
         if (split > 1 && (tiles > units || KB < 4 * split)) continue;
+        kbs::Config c;
+        c.pair = pair;
+        c.bn = bn;
+        c.tok = tok;
+        c.split = split;
+        kbs::Ring ring;
+        if (!kbs::ring_of(c, w_mn, K, 0, M, &ring)) continue;
         const double waves = units > 0 ? static_cast<double>((static_cast<long long>(tiles) + units - 1) / units) : 1e9;
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 1500.0) + 2000.0 * tok / 256.0 + (pair ? 1000.0 : 0.0);
         if (split > 1) t += 800.0 + 2200.0 * tok / 256.0 * (split - 1) / split;
@@ -215,10 +222,7 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
         if (split > 1 && !overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1])) t += 1500.0;
         if (t < best_t) {
           best_t = t;
-          best->pair = pair;
-          best->bn = bn;
-          best->tok = tok;
-          best->split = split;
+          *best = c;
         }
       }
     }
@@ -244,6 +248,12 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
       const int cols = ceil_div(static_cast<int>(fits < tok ? fits : tok) + 1, step) * step;  // of a block
       for (int w_cols = 64; w_cols <= 128; w_cols += 64) {
         const int bn = pair ? 2 * w_cols : w_cols;
+        kbs::Config c;
+        c.pair = pair;
+        c.bn = bn;
+        c.tok = tok;
+        kbs::Ring ring;
+        if (!kbs::ring_of(c, w_mn, K, groups, M, &ring)) continue;
         const double tiles = groups * blocks * ceil_div(N, bn);
         const double units = pair ? sms / 2 : sms;
         const double waves = tiles <= units ? 1.0 : tiles / units + 0.5;
@@ -253,9 +263,7 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
         if (cost < best_t) {
           best_t = cost;
           *cost_out = cost + mma_energy(groups * blocks * cols, static_cast<double>(ceil_div(N, bn)) * (pair ? 256.0 : 128.0), K);
-          best.pair = pair;
-          best.bn = bn;
-          best.tok = tok;
+          best = c;
         }
       }
     }
@@ -422,8 +430,8 @@ int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool 
   const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   Remembered& e = remembered(M, N, K, 0, key);
   if (e.M != M || e.N != N || e.K != K || e.groups != 0 || e.key != key || e.dev != dev) {
-    Capacity have;
-    const int rc = device_capacity(dev, sms, &have);
+    Capacity have = estimated_capacity(sms);
+    const int rc = dev < 0 ? KB_OK : device_capacity(dev, sms, &have);
     if (rc != KB_OK) return rc;
     for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
     e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape)};
@@ -462,22 +470,31 @@ extern "C" int kb_gemm_local_config(int M, int N, int K, int a_mn, int b_mn, int
   return KB_OK;
 }
 
-extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
+namespace {
+
+struct Layout {
+  bool contract, grouped, a_mn, b_mn;
+};
+
+// What does not depend on pointers or on a device.
+int check_problem(const KbLocalGemmArgs* a, Layout* l) {
   if (a == nullptr) return KB_ERR_ARG;
-  const bool contract = a->kind == KB_LOCAL_CONTRACT;
+  l->contract = a->kind == KB_LOCAL_CONTRACT;
   if (a->kind < 0 || a->kind > 2 || a->act < 0 || a->act > 3) {
     kb::set_error("kb_gemm_local: unknown kind %d or activation %d", a->kind, a->act);
     return KB_ERR_ARG;
   }
-  const bool a_mn = contract || a->a_mn, b_mn = contract || a->b_mn;
+  l->a_mn = l->contract || a->a_mn;
+  l->b_mn = l->contract || a->b_mn;
+  l->grouped = a->kind != KB_LOCAL_DENSE;
+  const bool a_mn = l->a_mn, b_mn = l->b_mn;
   // TMA rows are multiples of 16 bytes: the contiguous extent of every tensor is a multiple of 8.
   if (a->M <= 0 || a->N <= 0 || a->K <= 0 || a->N % 8 != 0 || (!a_mn && a->K % 8 != 0) || (!b_mn && a->K % 8 != 0) ||
       (a_mn && a->M % 8 != 0)) {
     kb::set_error("kb_gemm_local: need M,N,K > 0 and contiguous extents that are multiples of 8 (got %d %d %d)", a->M, a->N, a->K);
     return KB_ERR_ARG;
   }
-  const bool grouped = a->kind != KB_LOCAL_DENSE;
-  if (grouped && (a->groups < 1 || a->groups > MAX_GROUPS || a->row_start == nullptr || a->row_count == nullptr || a->bias != nullptr ||
+  if (l->grouped && (a->groups < 1 || a->groups > MAX_GROUPS || a->row_start == nullptr || a->row_count == nullptr || a->bias != nullptr ||
                   (a->kind == KB_LOCAL_ROWS && a_mn))) {
     kb::set_error("kb_gemm_local: bad groups (%d, at most %d, with row tables, without bias)", a->groups, MAX_GROUPS);
     return KB_ERR_ARG;
@@ -490,6 +507,88 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     kb::set_error("kb_gemm_local: pre_in and pre_out belong to an activation");
     return KB_ERR_ARG;
   }
+  return KB_OK;
+}
+
+// The tile a product gets: what is asked for, else what the sizes call for.
+int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int cap, Choice* out) {
+  const int groups = l.grouped ? a->groups : 1;
+  const int expect = a->expect > 0 ? a->expect : a->kind == KB_LOCAL_ROWS ? a->M : a->K;
+  int shape = a->pair;  // -1: choose, 0: one CTA, 1: pair, 2: tall pair, 3 and 4: exchanged operands
+  if (cap < 2 || env().no_pair) shape = shape >= 3 ? 3 : 0;
+  Choice pick = {};
+  if (a->kind == KB_LOCAL_ROWS) {
+    pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr);
+  } else if (a->kind == KB_LOCAL_DENSE) {
+    if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
+    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, &pick);
+    if (rc != KB_OK) return rc;
+    if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
+  } else {
+    pick.c = contract_config(a->M, a->N, expect, groups, shape);
+  }
+  int* bn = pick.swap ? &pick.s.bn : &pick.c.bn;
+  int* split = pick.swap ? &pick.s.split : &pick.c.split;
+  if (a->bn > 0) *bn = a->bn;
+  if (a->split > 0) *split = a->split;
+  if (a->tok > 0) pick.s.tok = a->tok;
+  *out = pick;
+  return KB_OK;
+}
+
+// Shared memory of a tile with the rows on the M side; false where the kernel cannot run it.
+struct Ring {
+  int a_rows, a_slot, b_slot, stages;
+  int slot_rows;  // of an exchange slot of a split
+};
+bool ring_of(const KbLocalGemmArgs* a, const Layout& l, const Config& c, Ring* r) {
+  if (c.bn < 32 || c.bn > 256 || !bn_ok(c.bn, c.pair, l.b_mn) || c.split < 1 || c.split > (c.pair ? 4 : 8) || c.split > ceil_div(a->K, BK) ||
+      ((l.grouped || c.tall) && c.split > 1)) {
+    return false;
+  }
+  // A single CTA whose rows are few brings in only those: the MMA reads 128 rows of
+  // shared memory, what lies behind the box only reaches accumulator rows that are not
+  // stored.
+  r->a_rows = c.tall ? 256 : 128;
+  if (a->kind == KB_LOCAL_ROWS && !c.pair) {
+    r->a_rows = c.rows;
+  } else if (!c.pair && !l.a_mn && a->M < 128) {
+    r->a_rows = ceil_div(a->M, 8) * 8;
+  }
+  r->a_slot = r->a_rows * BK * 2;
+  r->b_slot = (c.pair ? c.bn / 2 : c.bn) * BK * 2;
+  const int tables = (l.grouped ? (3 * a->groups + 1) * 4 : 4) + (l.contract ? OUT_BYTES : 0);  // what the ring leaves room for
+  r->stages = ring_stages(r->a_slot, r->b_slot, tables);
+  r->slot_rows = c.pair ? 128 : ceil_div(r->a_rows, 32) * 32;
+  // the last A slot is read up to 128 rows far: the B slots behind it cover that
+  return r->stages >= 2 && r->stages * r->b_slot >= 16384 && (c.split == 1 || exchange_fits(r->a_rows, c.pair, c.bn, c.split));
+}
+
+}  // namespace
+
+extern "C" int kb_gemm_local_pick(const KbLocalGemmArgs* a, int sms, KbLocalPick* out) {
+  if (a == nullptr || out == nullptr || sms < 1) return KB_ERR_ARG;
+  Layout l;
+  Choice pick;
+  int rc = check_problem(a, &l);
+  if (rc == KB_OK) rc = pick_tile(a, l, -1, sms, a->num_ctas > 0 && a->num_ctas < sms ? a->num_ctas : sms, &pick);
+  if (rc != KB_OK) return rc;
+  const Config& c = pick.c;
+  const kbs::Config& s = pick.s;
+  if (pick.swap) *out = {1, s.pair, s.bn, s.tok, s.split};
+  else *out = {0, c.tall ? 2 : c.pair, c.bn, c.tall ? 512 : c.pair ? 256 : a->kind == KB_LOCAL_ROWS ? c.rows : 128, c.split};
+  Ring ring;
+  kbs::Ring swap_ring;
+  const int expect = a->expect > 0 ? a->expect : a->M;
+  const bool fits = pick.swap ? kbs::ring_of(s, l.b_mn, a->K, l.grouped ? a->groups : 0, expect, &swap_ring) : ring_of(a, l, c, &ring);
+  return fits ? KB_OK : KB_ERR_UNSUPPORTED;
+}
+
+extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
+  Layout l;
+  int rc = check_problem(a, &l);
+  if (rc != KB_OK) return rc;
+  const bool contract = l.contract, grouped = l.grouped, a_mn = l.a_mn, b_mn = l.b_mn;
   auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) != 0; };
   if (a->A == nullptr || a->B == nullptr || a->out == nullptr || misaligned(a->A) || misaligned(a->B) || misaligned(a->out) ||
       misaligned(a->bias) || misaligned(a->pre_out) || misaligned(a->pre_in)) {
@@ -497,36 +596,18 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     return KB_ERR_ARG;
   }
   int dev = 0, sms = 0;
-  int rc = device_info(&dev, &sms);
+  rc = device_info(&dev, &sms);
   if (rc != KB_OK) return rc;
   const int cap = a->num_ctas > 0 && a->num_ctas < sms ? a->num_ctas : sms;
 
+  Choice pick;
+  rc = pick_tile(a, l, dev, sms, cap, &pick);
+  if (rc != KB_OK) return rc;
+  if (pick.swap) return kbs::launch(*a, pick.s, dev, cap, env().timing, stream_v);
+  const Config c = pick.c;
   const int groups = grouped ? a->groups : 1;
-  const int expect = a->expect > 0 ? a->expect : a->kind == KB_LOCAL_ROWS ? a->M : a->K;
-  int shape = a->pair;  // -1: choose, 0: one CTA, 1: pair, 2: tall pair, 3 and 4: exchanged operands
-  if (cap < 2 || env().no_pair) shape = shape >= 3 ? 3 : 0;
-  Choice pick = {};
-  if (a->kind == KB_LOCAL_ROWS) {
-    pick = pick_rows(cap, expect, groups, a->N, a->K, b_mn, shape, a->pre_in != nullptr);
-  } else if (a->kind == KB_LOCAL_DENSE) {
-    if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    rc = pick_config(dev, sms, cap, a->M, a->N, a->K, a_mn, b_mn, shape, &pick);
-    if (rc != KB_OK) return rc;
-    if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
-  } else {
-    pick.c = contract_config(a->M, a->N, expect, groups, shape);
-  }
-  if (pick.swap) {
-    if (a->bn > 0) pick.s.bn = a->bn;
-    if (a->tok > 0) pick.s.tok = a->tok;
-    if (a->split > 0) pick.s.split = a->split;
-    return kbs::launch(*a, pick.s, dev, cap, env().timing, stream_v);
-  }
-  Config c = pick.c;
-  if (a->bn > 0) c.bn = a->bn;
-  if (a->split > 0) c.split = a->split;
-  const int KB = ceil_div(a->K, BK);
-  if (c.bn < 32 || c.bn > 256 || !bn_ok(c.bn, c.pair, b_mn) || c.split > (c.pair ? 4 : 8) || c.split > KB || ((grouped || c.tall) && c.split > 1)) {
+  Ring ring;
+  if (!ring_of(a, l, c, &ring)) {
     kb::set_error("kb_gemm_local: tile configuration pair=%d bn=%d split=%d does not fit the problem", c.pair, c.bn, c.split);
     return KB_ERR_ARG;
   }
@@ -536,37 +617,19 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.M = a->M;
   p.N = a->N;
   p.K = a->K;
-  // A single CTA whose rows are few brings in only those: the MMA reads 128 rows of
-  // shared memory, what lies behind the box only reaches accumulator rows that are not
-  // stored.
-  p.a_rows = c.tall ? 256 : 128;
-  if (a->kind == KB_LOCAL_ROWS && !c.pair) {
-    p.a_rows = c.rows;
-  } else if (!c.pair && !a_mn && a->M < 128) {
-    p.a_rows = ceil_div(a->M, 8) * 8;
-  }
+  p.a_rows = ring.a_rows;
   const int tile_rows = c.tall ? 512 : c.pair ? 256 : a->kind == KB_LOCAL_ROWS ? p.a_rows : 128;
   p.MBQ = ceil_div(a->M, tile_rows);
   p.NB = ceil_div(a->N, c.bn);
-  p.KB = KB;
+  p.KB = ceil_div(a->K, BK);
   p.bn = c.bn;
   p.group = (c.tall ? 4096 : 2048) / tile_rows;
   p.groups = grouped ? groups : 0;
   p.split = c.split;
-  p.a_slot = p.a_rows * BK * 2;
-  p.b_slot = (c.pair ? c.bn / 2 : c.bn) * BK * 2;
-  const int tables = (grouped ? (3 * groups + 1) * 4 : 4) + (contract ? OUT_BYTES : 0);  // what the ring leaves room for
-  p.stages = ring_stages(p.a_slot, p.b_slot, tables);
-  // the last A slot is read up to 128 rows far: the B slots behind it cover that
-  if (p.stages < 2 || p.stages * p.b_slot < 16384) {
-    kb::set_error("kb_gemm_local: operand ring too small");
-    return KB_ERR_ARG;
-  }
-  p.slot_rows = c.pair ? 128 : ceil_div(p.a_rows, 32) * 32;
-  if (c.split > 1 && !exchange_fits(p.a_rows, c.pair, c.bn, c.split)) {
-    kb::set_error("kb_gemm_local: partial tiles do not fit the operand ring");
-    return KB_ERR_ARG;
-  }
+  p.a_slot = ring.a_slot;
+  p.b_slot = ring.b_slot;
+  p.stages = ring.stages;
+  p.slot_rows = ring.slot_rows;
   const int epi = a->pre_in != nullptr ? EPI_SLOPE : a->act != ACT_NONE ? EPI_ACT : EPI_PLAIN;
   auto wide = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0; };
   p.wide = a->N % 16 == 0 && wide(a->out) && wide(a->pre_out) ? 1 : 0;

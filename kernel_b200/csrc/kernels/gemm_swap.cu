@@ -39,50 +39,61 @@ const void* find_kernel(int kind, bool w_mn, int epi, bool pair, int* row) {
 
 namespace kbs {
 
-int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool timing, void* stream) {
-  const bool rows = a.kind == KB_LOCAL_ROWS, w_mn = a.b_mn != 0;
+bool ring_of(const Config& c, bool w_mn, int K, int groups, int rows, Ring* out) {
   const int ctas = c.pair ? 2 : 1, step = c.pair ? 32 : 16;
   const int w_cols = c.bn / ctas;
   const int tok_cta = c.pair ? c.tok / 2 : c.tok;
-  Params p;
-  memset(&p, 0, sizeof(p));
-  p.KB = ceil_div(a.K, BK);
   if (w_cols < 8 || w_cols > LANES || c.bn % (w_mn ? 64 * ctas : 8 * ctas) != 0 || c.tok < step || c.tok > 256 || c.tok % step != 0 ||
-      c.split < 1 || c.split > (c.pair ? 4 : 8) || c.split > p.KB || (rows && c.split > 1)) {
+      c.split < 1 || c.split > (c.pair ? 4 : 8) || c.split > ceil_div(K, BK) || (groups > 0 && c.split > 1)) {
+    return false;
+  }
+  // Grouped rows: most blocks are shorter than `tok`.  Boxes of half the expected block fetch little in vain and a warp issues
+  // two of them in the time the weights take (64 groups of 128 rows, 2048 x 1024: boxes of 32 rows 73.7 us, so 67.7).
+  out->xbox = tok_cta;
+  if (groups > 0) {
+    const double n = static_cast<double>(rows) / groups, fits = n + 2.0 * sqrt(n);
+    const int expect = fits < c.tok ? (static_cast<int>(fits) / step + 1) * step / ctas : tok_cta;
+    out->xbox = ceil_div(expect, 16) * 8;
+    if (out->xbox < 16) out->xbox = 16;
+    if (out->xbox > tok_cta) out->xbox = tok_cta;
+  }
+  out->w_slot = w_cols * BK * 2;
+  out->x_slot = ceil_div(tok_cta, out->xbox) * out->xbox * BK * 2;
+  const int room = kbl::SMEM_MAX - 1024 - BAR_BYTES - (groups > 0 ? (3 * groups + 1) * 4 : 4);
+  out->stages = room / (out->w_slot + out->x_slot);
+  if (out->stages > MAX_STAGES) out->stages = MAX_STAGES;
+  // The MMA reads 128 rows from the last slot of the weights on, of a narrower tile too: the token slots lie behind it.
+  // The partial tiles of a split are exchanged through the ring.
+  return out->stages >= 2 && out->stages * out->x_slot + out->w_slot >= LANES * BK * 2 &&
+         (c.split == 1 || ceil_div(ceil_div(c.tok, CHUNK), c.split) * (c.split - 1) * LANES * CHUNK * 4 <= out->stages * (out->w_slot + out->x_slot));
+}
+
+int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool timing, void* stream) {
+  const bool rows = a.kind == KB_LOCAL_ROWS, w_mn = a.b_mn != 0;
+  const int ctas = c.pair ? 2 : 1;
+  const int w_cols = c.bn / ctas;
+  Ring ring;
+  if (!ring_of(c, w_mn, a.K, rows ? a.groups : 0, a.expect > 0 ? a.expect : a.M, &ring)) {
     kb::set_error("kb_gemm_local: exchanged tile configuration pair=%d bn=%d tok=%d split=%d does not fit the problem", (int)c.pair, c.bn,
                   c.tok, c.split);
     return KB_ERR_ARG;
   }
+  Params p;
+  memset(&p, 0, sizeof(p));
   p.M = a.M;
   p.N = a.N;
   p.K = a.K;
+  p.KB = ceil_div(a.K, BK);
   p.NB = ceil_div(a.N, c.bn);
   p.MB = ceil_div(a.M, c.tok);
   p.bn = c.bn;
   p.tok = c.tok;
-  // Grouped rows: most blocks are shorter than `tok`.  Boxes of half the expected block fetch little in vain and a warp issues
-  // two of them in the time the weights take (64 groups of 128 rows, 2048 x 1024: boxes of 32 rows 73.7 us, so 67.7).
-  p.xbox = tok_cta;
-  if (rows) {
-    const double n = static_cast<double>(a.expect > 0 ? a.expect : a.M) / a.groups, fits = n + 2.0 * sqrt(n);
-    const int expect = fits < c.tok ? (static_cast<int>(fits) / step + 1) * step / ctas : tok_cta;
-    p.xbox = ceil_div(expect, 16) * 8;
-    if (p.xbox < 16) p.xbox = 16;
-    if (p.xbox > tok_cta) p.xbox = tok_cta;
-  }
   p.groups = rows ? a.groups : 0;
   p.split = c.split;
-  p.w_slot = w_cols * BK * 2;
-  p.x_slot = ceil_div(tok_cta, p.xbox) * p.xbox * BK * 2;
-  const int room = kbl::SMEM_MAX - 1024 - BAR_BYTES - (rows ? (3 * a.groups + 1) * 4 : 4);
-  p.stages = room / (p.w_slot + p.x_slot);
-  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
-  // the MMA reads 128 rows from the last slot of the weights on, of a narrower tile too: the token slots lie behind it
-  if (p.stages < 2 || p.stages * p.x_slot + p.w_slot < LANES * BK * 2 ||
-      (c.split > 1 && ceil_div(ceil_div(c.tok, CHUNK), c.split) * (c.split - 1) * LANES * CHUNK * 4 > p.stages * (p.w_slot + p.x_slot))) {
-    kb::set_error("kb_gemm_local: operand ring too small");
-    return KB_ERR_ARG;
-  }
+  p.xbox = ring.xbox;
+  p.w_slot = ring.w_slot;
+  p.x_slot = ring.x_slot;
+  p.stages = ring.stages;
   p.act = a.act;
   p.early = a.early != 0 ? 1 : 0;
   p.bias = static_cast<const bf16*>(a.bias);

@@ -11,6 +11,14 @@ struct Config {
   int split = 1;
 };
 
+// Shared memory of a configuration: rows of one box of X, bytes of a stage of the weights and of X, stages.
+struct Ring {
+  int xbox, w_slot, x_slot, stages;
+};
+// False where the kernel cannot run it: the choice of a tile skips such a configuration, the launcher refuses it.
+// `groups`: 0 for a dense product; `rows`: rows expected in all groups together.
+bool ring_of(const Config& c, bool w_mn, int K, int groups, int rows, Ring* out);
+
 // Launches a dense or grouped-rows product whose arguments kb_gemm_local has checked.
 int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool timing, void* stream);
 

@@ -128,3 +128,68 @@ def test_local_gemm_tile_rule_gives_launchable_configurations():
         assert 64 <= bn.value <= 256 and (per_cta % 64 == 0 if b_mn else bn.value % 32 == 0)
         assert pair.value == 0 or M > 128
         assert 1 <= split.value <= (8, 4, 1)[pair.value] and split.value <= (K + 63) // 64
+
+
+def _pick(sms, **kw):
+    """What ``kb_gemm_local`` launches: (exchanged operands, pair, columns, rows of a tile, split)."""
+    a, p = _local(**kw), N.LocalPick()
+    assert N.lib().kb_gemm_local_pick(C.byref(a), sms, C.byref(p)) == N.KB_OK, (kw, N.last_error())
+    return p.exchanged, p.pair, p.bn, p.rows, p.split
+
+
+def _exchanged_tile_runs(pair, bn, tok, split, K, w_mn, groups, rows):
+    """The limits of the exchanged-operand kernel, restated: 128 columns per CTA, blocks of at most 256 tokens, two stages and
+    the partial tiles of a split in 232448 bytes of shared memory."""
+    ctas, step = (2, 32) if pair else (1, 16)
+    w_cols, tok_cta = bn // ctas, tok // ctas
+    assert bn % ctas == 0 and 8 <= w_cols <= 128 and w_cols % (64 if w_mn else 8) == 0
+    assert step <= tok <= 256 and tok % step == 0
+    assert 1 <= split <= (4 if pair else 8) and split <= (K + 63) // 64 and (split == 1 or not groups)
+    box = tok_cta
+    if groups:  # boxes of half the block that most groups fit
+        most = rows / groups + 2 * (rows / groups) ** 0.5
+        block = (int(most) // step + 1) * step // ctas if most < tok else tok_cta
+        box = min(max((block + 15) // 16 * 8, 16), tok_cta)
+    stage = w_cols * 128 + -(-tok_cta // box) * box * 128
+    stages = min(16, (232448 - 1024 - 512 - 4 * (3 * groups + 1)) // stage)
+    assert box % 8 == 0 and stages >= 2
+    assert w_cols * 128 + stages * (stage - w_cols * 128) >= 128 * 128  # the MMA reads 128 rows from the last weight slot on
+    if split > 1:
+        chunks = -(-(tok // 8) // split)  # of the member that owns most
+        assert chunks * (split - 1) * 128 * 8 * 4 <= stages * stage
+
+
+def test_picked_tiles_are_launchable():
+    """Dense products with either operand layout and grouped rows, with few and many rows on few and many SMs: the tile
+    that is launched, whichever kind it is."""
+    import random
+
+    rng = random.Random(1)
+    seen = set()
+    for i in range(6000):
+        M, Nn, K = int(2 ** rng.uniform(0, 13)), 8 * int(2 ** rng.uniform(0, 12)), 8 * int(2 ** rng.uniform(0, 12))
+        sms = rng.choice([148, 148, 132, 16, 2, 1])
+        b_mn = rng.choice([0, 1])
+        kw = dict(M=M, N=Nn, K=K, b_mn=b_mn)
+        if i % 2:
+            groups = int(2 ** rng.uniform(0, 10))
+            kw.update(kind=N.LOCAL_ROWS, groups=groups, expect=rng.choice([0, 1 + M // 2]))
+            kw.update(row_start=16, row_count=16)  # not read
+        swap, pair, bn, rows, split = _pick(sms, **kw)
+        seen.add((i % 2, b_mn, swap, pair))
+        assert sms > 1 or not pair
+        if swap:
+            _exchanged_tile_runs(pair, bn, rows, split, K, b_mn, kw.get("groups", 0), kw.get("expect") or M)
+        else:
+            assert 32 <= bn <= 256 and ((bn // 2 if pair else bn) % 64 == 0 if b_mn else bn % 32 == 0)
+            assert 1 <= split <= (8, 4, 1)[pair] and split <= (K + 63) // 64 and (split == 1 or not i % 2)
+    # every kind of tile was picked for every kind of product
+    assert seen >= {(g, b, s, p) for g in (0, 1) for b in (0, 1) for s in (0, 1) for p in (0, 1)}, seen
+
+
+def test_tiles_that_no_kernel_runs_are_refused():
+    p = N.LocalPick()
+    for kw in (dict(pair=3, bn=136), dict(pair=4, bn=64, b_mn=1), dict(pair=3, bn=64, tok=24), dict(pair=3, bn=64, tok=272),
+               dict(pair=3, split=2), dict(pair=0, bn=40), dict(pair=1, bn=64, b_mn=1, M=256), dict(pair=0, bn=64, split=9)):
+        a = _local(**kw)
+        assert N.lib().kb_gemm_local_pick(C.byref(a), 148, C.byref(p)) == N.KB_ERR_UNSUPPORTED, kw
