@@ -523,10 +523,10 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
     const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, &pick);
     if (rc != KB_OK) return rc;
-    if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
   } else {
     pick.c = contract_config(a->M, a->N, expect, groups, shape);
   }
+  if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
   int* bn = pick.swap ? &pick.s.bn : &pick.c.bn;
   int* split = pick.swap ? &pick.s.split : &pick.c.split;
   if (a->bn > 0) *bn = a->bn;

@@ -193,3 +193,14 @@ def test_tiles_that_no_kernel_runs_are_refused():
                dict(pair=3, split=2), dict(pair=0, bn=40), dict(pair=1, bn=64, b_mn=1, M=256), dict(pair=0, bn=64, split=9)):
         a = _local(**kw)
         assert N.lib().kb_gemm_local_pick(C.byref(a), 148, C.byref(p)) == N.KB_ERR_UNSUPPORTED, kw
+
+
+def test_a_tile_that_is_asked_for_is_of_the_kind_with_rows_on_the_m_side():
+    """Columns (or a split) without a kind mean the M side, in grouped products as in dense ones."""
+    free = dict(kind=N.LOCAL_ROWS, M=192, N=1024, K=2048, groups=64, row_start=16, row_count=16)
+    assert _pick(148, **free)[0] == 1
+    for bn in (64, 128, 256):
+        assert _pick(148, **free, bn=bn)[:3:2] == (0, bn)
+    assert _pick(148, M=64, N=1104, K=20000)[0] == 1
+    assert _pick(148, M=64, N=1104, K=20000, bn=96)[:3:2] == (0, 96)
+    assert _pick(148, **free, pair=3, bn=64)[:3:2] == (1, 64)
