@@ -98,7 +98,7 @@ class LocalGemmArgs(C.Structure):
 
 
 class LocalPick(C.Structure):
-    _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split")]
+    _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split", "overlapped")]
 
 
 class A2aArgs(C.Structure):

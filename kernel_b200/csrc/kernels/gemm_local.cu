@@ -107,7 +107,7 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
         // launched behind the previous kernel instead of under its end
         const int ctas = (pair ? 2 : 1) * split;
-        const double in_order = overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1]) ? 0.0 : 1500.0;
+        const double in_order = overlaps(ctas, split, static_cast<int>(tiles) * ctas, cap.clusters[1], 2.0 * N * K) ? 0.0 : 1500.0;
         const double both = (t > memory ? t + 0.05 * memory : memory + 0.05 * t) + in_order;
         t = (t > memory ? t : memory) + in_order;
         if (t < best_t) {
@@ -219,7 +219,7 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 1500.0) + 2000.0 * tok / 256.0 + (pair ? 1000.0 : 0.0);
         if (split > 1) t += 800.0 + 2200.0 * tok / 256.0 * (split - 1) / split;
         t = t > memory ? t + 0.05 * memory : memory + 0.05 * t;
-        if (split > 1 && !overlaps(ctas, static_cast<int>(tiles) * ctas, cap.clusters[1])) t += 1500.0;
+        if (split > 1 && !overlaps(ctas, split, static_cast<int>(tiles) * ctas, cap.clusters[1], 2.0 * N * K)) t += 1500.0;
         if (t < best_t) {
           best_t = t;
           *best = c;
@@ -571,12 +571,15 @@ extern "C" int kb_gemm_local_pick(const KbLocalGemmArgs* a, int sms, KbLocalPick
   Layout l;
   Choice pick;
   int rc = check_problem(a, &l);
-  if (rc == KB_OK) rc = pick_tile(a, l, -1, sms, a->num_ctas > 0 && a->num_ctas < sms ? a->num_ctas : sms, &pick);
+  const int cap = a->num_ctas > 0 && a->num_ctas < sms ? a->num_ctas : sms;
+  if (rc == KB_OK) rc = pick_tile(a, l, -1, sms, cap, &pick);
   if (rc != KB_OK) return rc;
   const Config& c = pick.c;
   const kbs::Config& s = pick.s;
   if (pick.swap) *out = {1, s.pair, s.bn, s.tok, s.split};
   else *out = {0, c.tall ? 2 : c.pair, c.bn, c.tall ? 512 : c.pair ? 256 : a->kind == KB_LOCAL_ROWS ? c.rows : 128, c.split};
+  const int cluster = (out->pair ? 2 : 1) * out->split;
+  out->overlapped = overlaps(cluster, out->split, ceil_div(a->M, out->rows) * ceil_div(a->N, out->bn) * cluster, cap, 2.0 * a->N * a->K);
   Ring ring;
   kbs::Ring swap_ring;
   const int expect = a->expect > 0 ? a->expect : a->M;
@@ -678,5 +681,5 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
     KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
     if (dev >= 0 && dev < 64) attr_set[dev][shape_row][kernel_row] = true;
   }
-  return launch_clusters(fn, grid, THREADS, cluster, cap, &p, stream_v);
+  return launch_clusters(fn, grid, THREADS, cluster, overlaps(cluster, c.split, grid, cap, 2.0 * a->N * a->K), &p, stream_v);
 }

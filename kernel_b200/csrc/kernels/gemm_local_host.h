@@ -49,16 +49,23 @@ inline int make_tmap4_blocks(CUtensorMap* map, const void* ptr, uint64_t d0, uin
   return KB_OK;
 }
 
-// Whether a launch of `grid` CTAs is set up under the end of the previous kernel of the stream.  Without that it starts up
-// to 2 us after the end of the one before.  Not so where clusters of an odd size fill the chip: placed one by one as SMs
-// fall free they leave some unused.  Launched in order and overlapped, us:
-//   64 x 7168 x 18432   clusters of 2 on 112 SMs 48.4 46.9   of 4 on 128 49.1 46.9   of 3 on 114 47.9 46.2   of 3 on 135 47.6 50.2
-//   256 x 4096 x 14336  clusters of 6 on 132 SMs 32.9 30.2   of 4 on 128 32.9 30.6   of 3 on 114 36.8 35.2   of 3 on 132 34.9 37.0
-// Clusters of eight wait longest for SMs that are free together (195 x 3200 x 26136 on 120 SMs costs 1.8 us overlapped).
-inline bool overlaps(int cluster, int grid, int sms) { return cluster == 1 || (cluster < 8 && (cluster % 2 == 0 || grid * 100ll < sms * 88ll)); }
+// Whether a launch of `grid` CTAs is set up under the end of the previous kernel of the stream.  Without that it starts 2 to 3 us
+// after the end of the one before (a launch in order starts on a 2 us grid); 760 dense products back to back, three weights in
+// turn, each way.  Two kinds of launch lose by it:
+//   clusters of an odd size that fill the chip: placed one by one as SMs fall free they leave some unused.  26 clusters of five
+//     (130 CTAs) 23.1 us in order, 32.2 overlapped and 37.0 43.2; 25 of them 29.0 25.7; 45 of three 25.0 25.4, 43 of them 31.4 29.0;
+//     clusters of seven (105 CTAs) gain 2 us.
+//   a long read of weights by single CTAs in clusters of two on less than 9/10 of the SMs, which then stand closer together:
+//     64 clusters 81.7 us in order, 90.7 overlapped (91 x 8088 x 22632), 60 clusters of 198 MB + 13 %, 56 of 525 MB + 15 %;
+//     below 160 MB, or on more SMs, the gain is larger (72 clusters of 186 MB - 5 %, 64 of 96 MB - 7 %).
+// Over all of them the launch picked here takes 0.2 % more than the better one, 32 of 1236 more than 3 % (in order: 10 %).
+inline bool overlaps(int cluster, int split, int grid, int sms, double weight_bytes) {
+  if (cluster % 2 != 0) return cluster == 1 || grid * 8ll < sms * 7ll;
+  return cluster != 2 || split != 2 || weight_bytes < 160e6 || grid * 10ll >= sms * 9ll;
+}
 
 // One CTA per SM with all of its shared memory, in clusters of `cluster` CTAs.
-inline int launch_clusters(const void* fn, int grid, int threads, int cluster, int sms, void* params, void* stream) {
+inline int launch_clusters(const void* fn, int grid, int threads, int cluster, bool overlapped, void* params, void* stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -73,7 +80,7 @@ inline int launch_clusters(const void* fn, int grid, int threads, int cluster, i
     dim.val.clusterDim.y = 1;
     dim.val.clusterDim.z = 1;
   }
-  if (overlaps(cluster, grid, sms)) attr[cfg.numAttrs++] = kb::overlap_launch();
+  if (overlapped) attr[cfg.numAttrs++] = kb::overlap_launch();
   void* args[] = {params};
   KB_CUDA_OK(cudaLaunchKernelExC(&cfg, fn, args));
   return KB_OK;

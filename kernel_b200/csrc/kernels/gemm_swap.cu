@@ -131,7 +131,8 @@ int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool tim
     KB_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kbl::SMEM_MAX));
     if (dev >= 0 && dev < 64) attr_set[dev][c.pair][row] = true;
   }
-  return kbl::launch_clusters(fn, static_cast<int>(grid), THREADS, cluster, cap, &p, stream);
+  const bool overlapped = kbl::overlaps(cluster, c.split, static_cast<int>(grid), cap, 2.0 * a.N * a.K);
+  return kbl::launch_clusters(fn, static_cast<int>(grid), THREADS, cluster, overlapped, &p, stream);
 }
 
 }  // namespace kbs

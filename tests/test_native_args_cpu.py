@@ -204,3 +204,21 @@ def test_a_tile_that_is_asked_for_is_of_the_kind_with_rows_on_the_m_side():
     assert _pick(148, M=64, N=1104, K=20000)[0] == 1
     assert _pick(148, M=64, N=1104, K=20000, bn=96)[:3:2] == (0, 96)
     assert _pick(148, **free, pair=3, bn=64)[:3:2] == (1, 64)
+
+
+def test_which_launches_of_split_products_are_overlapped():
+    """All but clusters of an odd size that fill the chip and long reads of weights by clusters of two on less than 9/10 of
+    the SMs."""
+    def overlapped(pair, clusters, split, K):
+        a, p = _local(M=64, N=128 * clusters, K=K, pair=pair, bn=128, split=split), N.LocalPick()
+        assert N.lib().kb_gemm_local_pick(C.byref(a), 148, C.byref(p)) == N.KB_OK and (p.bn, p.split) == (128, split)
+        return p.overlapped
+
+    for pair in (0, 3):
+        assert [overlapped(pair, n, 3, 4096) for n in (43, 44, 45)] == [1, 0, 0]
+        assert [overlapped(pair, n, 5, 4096) for n in (20, 25, 26)] == [1, 1, 0]
+        assert [overlapped(pair, n, 7, 4096) for n in (10, 15)] == [1, 1]
+        for split in (4, 6, 8):
+            assert all(overlapped(pair, n, split, 20000) for n in range(8, 148 // split + 1))
+        assert [overlapped(pair, n, 2, 20000) for n in (40, 64, 66, 67, 74)] == [0, 0, 0, 1, 1]
+        assert [overlapped(pair, 64, 2, K) for K in (9600, 9768)] == [1, 0]   # 157, 160 MB
