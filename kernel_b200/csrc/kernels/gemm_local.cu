@@ -63,6 +63,11 @@ struct Capacity {
   int clusters[9];
 };
 
+// Operands in and results out at 6.5 TB/s behind the latency of a launch, ns.
+double memory_time(int M, int N, int K) {
+  return 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
+}
+
 // Picks the tile shape (one CTA, pair, 512-row pair), its columns and the split of K.
 //
 // Model of the kernel's time in ns, constants fitted to 190 shapes x all configurations
@@ -86,7 +91,7 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
   Config best = {false, 256, 1};
   double best_t = 1e30, best_cost = 1e30;
   const int KB = ceil_div(K, BK);
-  const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
+  const double memory = memory_time(M, N, K);
   for (int s = 0; s < 3; ++s) {
     if (shape >= 0 ? s != shape : s != 0 && (M <= 128 || cap.clusters[2] < 1)) continue;
     const bool pair = s > 0, tall = s == 2;
@@ -105,9 +110,11 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 2000.0) + epilogue + (pair ? 1000.0 : 0.0);
         if (tall) t += 1.25 * waves * epilogue;
         if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
-        // launched behind the previous kernel instead of under its end
+        // Launched behind the previous kernel instead of under its end.  Not so for the long reads that are launched in order
+        // because that is faster (4 x 14488 x 16616, weights along N: 86.6 us split in two, 104 unsplit).
         const int ctas = (pair ? 2 : 1) * split;
-        const double in_order = overlaps(ctas, split, static_cast<int>(tiles) * ctas, cap.clusters[1], 2.0 * N * K) ? 0.0 : 1500.0;
+        const bool late = ctas % 2 != 0 && !overlaps(ctas, split, static_cast<int>(tiles) * ctas, cap.clusters[1], 2.0 * N * K);
+        const double in_order = late ? 1500.0 : 0.0;
         const double both = (t > memory ? t + 0.05 * memory : memory + 0.05 * t) + in_order;
         t = (t > memory ? t : memory) + in_order;
         if (t < best_t) {
@@ -194,7 +201,7 @@ double swap_k_block(bool pair, int w_cols, int tok, bool w_mn) {
 double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shape, kbs::Config* best) {
   double best_t = 1e30;
   const int KB = ceil_div(K, BK), mb = ceil_div(M, 256);
-  const double memory = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * N) / 6500.0 + 6600.0;
+  const double memory = memory_time(M, N, K);
   for (int s = 0; s < 2; ++s) {
     const bool pair = s == 1;
     if (shape >= 3 ? s != shape - 3 : pair && cap.clusters[2] < 1) continue;
@@ -402,14 +409,17 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
                      (static_cast<uint32_t>(K) * 0xc2b2ae35u) ^ static_cast<uint32_t>(key + groups);
   return table[(h ^ (h >> 15)) & 63u];
 }
-// Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy.  Near ties keep the rows
-// on the M side, whose epilogue stores wider vectors; from 129 rows on both kinds compute whole blocks and the models tell
-// less well what a tie is (195 x 26136 x 3200 in an MLP: ratio 0.94, 108.5 us for the block and 110.3 exchanged).
-// GPU time back to back, three weights in turn, us, M side and what is picked:
-//   1 x 8192 x 8192 28.3 26.3     40 x 2840 x 1392 8.2 7.5       64 x 7168 x 18432 47.7 47.2   100 x 4096 x 14336 28.7 26.7
-//   165 x 2920 x 1080 11.9 10.5   200 x 8192 x 8192 36.9 34.4    300 x 1024 x 1024 10.2 7.5    330 x 6296 x 1304 13.8 12.4
-//   400 x 25000 x 1504 38.8 34.7  90 x 1104 x 20000 18.4 15.4    weights along N: 64 x 4096 x 4096 12.3 11.0
-Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape) {
+// Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy, plus what 2000 products (1 to
+// 8192 rows, all layouts and epilogues, three weights in turn) showed them to leave out: a split costs more than they say,
+// more so with many tokens, whose partial tiles are exchanged; tiles that are not split fall a little further short of the
+// memory's rate, exchanged ones of more than 128 rows too.  Constants fitted; those of either half of the products choose as well for
+// the other.  The picked kind takes 2.1 % more than the better one on average (always the M side 5.5 %, always exchanged
+// 5.1 %).  Near ties keep the rows on the M side, whose epilogue stores wider vectors, except with a slope, whose saved
+// values it reads back with a row per lane.  us, M side and exchanged, the picked one marked:
+//   1 x 8192 x 8192   27.2  26.4*   40 x 2840 x 1392    7.8   7.2*   64 x 7168 x 18432   47.2* 48.1    100 x 4096 x 14336   27.9* 28.3
+//   165 x 2920 x 1080 10.4* 12.0    200 x 8192 x 8192  33.8* 33.4    300 x 1024 x 1024    9.2*  9.9    330 x 6296 x 1304    14.0* 13.8
+//   400 x 25000 x 1504 35.1 31.2*   90 x 1104 x 20000  16.4  17.0*   195 x 26136 x 3200  38.9* 42.0    256 x 4096 x 14336   36.5* 46.0
+Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool slope) {
   Choice r = {};
   double plain = 0.0;
   if (shape < 3) r.c = choose_config(M, N, K, a_mn, b_mn, cap, shape, &plain);
@@ -421,20 +431,24 @@ Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, in
   }
   const int tall = r.c.tall ? 512 : r.c.pair ? 256 : 128;
   const int lanes = r.s.pair ? 256 : 128;
-  const double cost_m = plain + mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K);
-  const double cost_n = other + mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K);
-  r.swap = cost_n < (M <= 128 ? 0.97 : M <= 256 ? 0.93 : 0.92) * cost_m;
+  const double memory = memory_time(M, N, K);
+  const double exchange = 3900.0 * r.s.tok / 256.0 * (r.s.split - 1) / r.s.split;
+  const double cost_m = plain + 1.7 * mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K) +
+                        (r.c.split > 1 ? 2300.0 : 0.095 * memory);
+  const double cost_n = other + 1.7 * mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K) +
+                        (r.s.split > 1 ? 1600.0 + exchange : 0.13 * memory) + (M > 128 ? 0.07 * memory : 0.0);
+  r.swap = cost_n < (slope ? 1.03 : 0.96) * cost_m;
   return r;
 }
-int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, Choice* out) {
-  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool slope, Choice* out) {
+  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | (slope ? 1 << 29 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   Remembered& e = remembered(M, N, K, 0, key);
   if (e.M != M || e.N != N || e.K != K || e.groups != 0 || e.key != key || e.dev != dev) {
     Capacity have = estimated_capacity(sms);
     const int rc = dev < 0 ? KB_OK : device_capacity(dev, sms, &have);
     if (rc != KB_OK) return rc;
     for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
-    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape)};
+    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape, slope)};
   }
   *out = e.c;
   return KB_OK;
@@ -521,7 +535,7 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
     pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr);
   } else if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, &pick);
+    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->pre_in != nullptr, &pick);
     if (rc != KB_OK) return rc;
   } else {
     pick.c = contract_config(a->M, a->N, expect, groups, shape);

@@ -222,3 +222,22 @@ def test_which_launches_of_split_products_are_overlapped():
             assert all(overlapped(pair, n, split, 20000) for n in range(8, 148 // split + 1))
         assert [overlapped(pair, n, 2, 20000) for n in (40, 64, 66, 67, 74)] == [0, 0, 0, 1, 1]
         assert [overlapped(pair, 64, 2, K) for K in (9600, 9768)] == [1, 0]   # 157, 160 MB
+
+
+def test_kind_of_dense_products_whose_difference_was_measured():
+    """Products at least 10 % apart on a B200: the faster kind (us, rows on the M side / exchanged)."""
+    for M, Nn, K, b_mn in ((267, 4120, 1344, 0),     # 12.3 16.5
+                           (443, 3624, 2352, 0),     # 13.7 15.9
+                           (164, 3072, 1728, 0),     # 10.5 16.5
+                           (301, 1136, 1600, 0),     # 9.2 14.2
+                           (182, 7496, 1488, 1),     # 11.7 13.6
+                           (256, 4096, 14336, 0)):   # 36.5 46.0
+        assert _pick(148, M=M, N=Nn, K=K, b_mn=b_mn)[0] == 0, (M, Nn, K)
+    for M, Nn, K, b_mn in ((400, 25000, 1504, 0),    # 35.1 31.2
+                           (142, 1184, 23256, 0),    # 31.9 24.0
+                           (309, 8208, 23040, 0),    # 126 100
+                           (4, 1632, 6040, 1),       # 13.4 10.4
+                           (285, 4640, 5696, 0)):    # 24.2 19.3
+        assert _pick(148, M=M, N=Nn, K=K, b_mn=b_mn)[0] == 1, (M, Nn, K)
+    for M, Nn, K in ((285, 17576, 1712), (190, 12288, 3216), (1051, 4920, 4448)):   # with a slope: 51.4 30.9, 38.7 27.6, 89.9 65.6
+        assert _pick(148, M=M, N=Nn, K=K, b_mn=1, act=N.ACTS["silu"], pre_in=0)[0] == 1, (M, Nn, K)
