@@ -409,6 +409,11 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
                      (static_cast<uint32_t>(K) * 0xc2b2ae35u) ^ static_cast<uint32_t>(key + groups);
   return table[(h ^ (h >> 15)) & 63u];
 }
+// What the exchanged kernel gains, ns, by fetching weights under the end of the previous launch, which the other one does not
+// do.  500 MLPs of 1 to 1200 tokens: with 0, 1500 and 3000 the two products take 0.856, 0.852 and 0.854 of what they
+// took on the M side in order, and 4, none and 2 of them more than 3 % longer than that.
+constexpr double EARLY = 1500.0;
+
 // Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy, plus what 2000 products (1 to
 // 8192 rows, all layouts and epilogues, three weights in turn) showed them to leave out: a split costs more than they say,
 // more so with many tokens, whose partial tiles are exchanged; tiles that are not split fall a little further short of the
@@ -419,7 +424,7 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
 //   1 x 8192 x 8192   27.2  26.4*   40 x 2840 x 1392    7.8   7.2*   64 x 7168 x 18432   47.2* 48.1    100 x 4096 x 14336   27.9* 28.3
 //   165 x 2920 x 1080 10.4* 12.0    200 x 8192 x 8192  33.8* 33.4    300 x 1024 x 1024    9.2*  9.9    330 x 6296 x 1304    14.0* 13.8
 //   400 x 25000 x 1504 35.1 31.2*   90 x 1104 x 20000  16.4  17.0*   195 x 26136 x 3200  38.9* 42.0    256 x 4096 x 14336   36.5* 46.0
-Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool slope) {
+Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool slope, bool early) {
   Choice r = {};
   double plain = 0.0;
   if (shape < 3) r.c = choose_config(M, N, K, a_mn, b_mn, cap, shape, &plain);
@@ -437,18 +442,18 @@ Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, in
                         (r.c.split > 1 ? 2300.0 : 0.095 * memory);
   const double cost_n = other + 1.7 * mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K) +
                         (r.s.split > 1 ? 1600.0 + exchange : 0.13 * memory) + (M > 128 ? 0.07 * memory : 0.0);
-  r.swap = cost_n < (slope ? 1.03 : 0.96) * cost_m;
+  r.swap = cost_n - (early ? EARLY : 0.0) < (slope ? 1.03 : 0.96) * cost_m;
   return r;
 }
-int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool slope, Choice* out) {
-  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | (slope ? 1 << 29 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool slope, bool early, Choice* out) {
+  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | (slope ? 1 << 29 : 0) | (early ? 1 << 28 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   Remembered& e = remembered(M, N, K, 0, key);
   if (e.M != M || e.N != N || e.K != K || e.groups != 0 || e.key != key || e.dev != dev) {
     Capacity have = estimated_capacity(sms);
     const int rc = dev < 0 ? KB_OK : device_capacity(dev, sms, &have);
     if (rc != KB_OK) return rc;
     for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
-    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape, slope)};
+    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape, slope, early)};
   }
   *out = e.c;
   return KB_OK;
@@ -535,7 +540,7 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
     pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr);
   } else if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->pre_in != nullptr, &pick);
+    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->pre_in != nullptr, a->early != 0, &pick);
     if (rc != KB_OK) return rc;
   } else {
     pick.c = contract_config(a->M, a->N, expect, groups, shape);
