@@ -414,14 +414,15 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
 // took on the M side in order, and 4, none and 2 of them more than 3 % longer than that.
 constexpr double EARLY = 1500.0;
 
-// Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy, plus what 2000 products (1 to
+// Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy, plus what 2330 products (1 to
 // 8192 rows, all layouts and epilogues, three weights in turn) showed them to leave out: a split costs more than they say,
 // more so with many tokens, whose partial tiles are exchanged; tiles that are not split fall a little further short of the
-// memory's rate, exchanged ones of more than 128 rows too.  Constants fitted; those of either half of the products choose as well for
-// the other.  The picked kind takes 2.1 % more than the better one on average (always the M side 5.5 %, always exchanged
-// 5.1 %).  Near ties keep the rows on the M side, whose epilogue stores wider vectors, except with a slope, whose saved
-// values it reads back with a row per lane.  us, M side and exchanged, the picked one marked:
-//   1 x 8192 x 8192   27.2  26.4*   40 x 2840 x 1392    7.8   7.2*   64 x 7168 x 18432   47.2* 48.1    100 x 4096 x 14336   27.9* 28.3
+// memory's rate, exchanged ones of more than 128 rows too.  Constants fitted between 330 near ties repeated for 0.1 s each, at the
+// power cap, where the energy counts for most, and 2000 short bursts.  The picked kind takes 1.2 % and 1.6 % more than the better
+// one on average (always the M side 5.0 and 5.5 %, always exchanged 3.9 and 5.0 %).  Near ties keep the rows on the M side, whose
+// epilogue stores wider vectors, except with a slope, whose saved values it reads back with a row per lane.  Bursts, us, M side and
+// exchanged, the picked one marked:
+//   1 x 8192 x 8192   27.2  26.4*   40 x 2840 x 1392    7.8   7.2*   64 x 7168 x 18432   47.2  48.1*   100 x 4096 x 14336   27.9* 28.3
 //   165 x 2920 x 1080 10.4* 12.0    200 x 8192 x 8192  33.8* 33.4    300 x 1024 x 1024    9.2*  9.9    330 x 6296 x 1304    14.0* 13.8
 //   400 x 25000 x 1504 35.1 31.2*   90 x 1104 x 20000  16.4  17.0*   195 x 26136 x 3200  38.9* 42.0    256 x 4096 x 14336   36.5* 46.0
 Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool slope, bool early) {
@@ -437,12 +438,12 @@ Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, in
   const int tall = r.c.tall ? 512 : r.c.pair ? 256 : 128;
   const int lanes = r.s.pair ? 256 : 128;
   const double memory = memory_time(M, N, K);
-  const double exchange = 3900.0 * r.s.tok / 256.0 * (r.s.split - 1) / r.s.split;
-  const double cost_m = plain + 1.7 * mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K) +
-                        (r.c.split > 1 ? 2300.0 : 0.095 * memory);
-  const double cost_n = other + 1.7 * mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K) +
-                        (r.s.split > 1 ? 1600.0 + exchange : 0.13 * memory) + (M > 128 ? 0.07 * memory : 0.0);
-  r.swap = cost_n - (early ? EARLY : 0.0) < (slope ? 1.03 : 0.96) * cost_m;
+  const double exchange = 3700.0 * r.s.tok / 256.0 * (r.s.split - 1) / r.s.split;
+  const double cost_m = plain + 3.5 * mma_energy(static_cast<double>(ceil_div(M, tall)) * tall, static_cast<double>(ceil_div(N, r.c.bn)) * r.c.bn, K) +
+                        (r.c.split > 1 ? 3000.0 : 0.167 * memory);
+  const double cost_n = other + 3.5 * mma_energy(static_cast<double>(ceil_div(M, r.s.tok)) * r.s.tok, static_cast<double>(ceil_div(N, r.s.bn)) * lanes, K) +
+                        (r.s.split > 1 ? 2300.0 + exchange : 0.174 * memory) + (M > 128 ? 0.12 * memory : 0.0);
+  r.swap = cost_n - (early ? EARLY : 0.0) < (slope ? 1.05 : 0.97) * cost_m;
   return r;
 }
 int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool slope, bool early, Choice* out) {

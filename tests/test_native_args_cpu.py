@@ -244,7 +244,7 @@ def test_kind_of_dense_products_whose_difference_was_measured():
 
 
 def test_a_product_that_may_fetch_its_weights_early_is_exchanged_sooner():
-    """The down product of an MLP of 796 tokens, 4136 x 2432: 48.5 us for the block, 51.0 with it on the M side."""
-    assert _pick(148, M=796, N=4136, K=2432)[0] == 0
-    assert _pick(148, M=796, N=4136, K=2432, early=1)[0] == 1
+    """Near ties: the exchanged kernel alone fetches them under the previous launch."""
+    for M, Nn, K in ((128, 4096, 4096), (330, 6296, 1304), (672, 10008, 2040)):
+        assert [_pick(148, M=M, N=Nn, K=K, early=early)[0] for early in (0, 1)] == [0, 1], (M, Nn, K)
     assert _pick(148, M=256, N=4096, K=14336, early=1)[0] == 0   # 36.5 us, exchanged 46.0
