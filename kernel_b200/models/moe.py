@@ -109,9 +109,11 @@ def _group_table(n_e, pad: int, device):
 
 
 def _expected_rows(er: ExpertRows):
-    """Rows of all experts together, and with each expert padded by half an alignment on average."""
+    """Rows of all experts together, and with each expert padded: by half an alignment on average.  An expert with few rows has
+    one alignment of them; the tile rules allow two standard deviations beyond the average, 48 rows stand for 64 there."""
     real = er.T * er.k
-    return real, real + min(er.E, real) * (ROW_ALIGN // 2)
+    used = min(er.E, real)
+    return real, max(real + used * (ROW_ALIGN // 2), used * (ROW_ALIGN * 3 // 4))
 
 
 class _LocalMoEFn(torch.autograd.Function):

@@ -146,3 +146,20 @@ def test_inference_block_leaves_the_exchange_to_parts_that_span_several_ranks(mo
     mlp = block()
     mlp.up.world = 2
     assert call(mlp, rows=4) == (0, [mlp.up, mlp.down])
+
+
+def test_expected_rows_of_padded_experts():
+    """What the tile rules are told of a table that stays on the device.  An expert with any row has a whole alignment of them;
+    the rules take a tile that holds the average and two standard deviations: neither half an alignment nor two."""
+    from kernel_b200.models.moe import _expected_rows
+    from kernel_b200.ops.local import ROW_ALIGN, ExpertRows
+
+    er = ExpertRows.__new__(ExpertRows)
+    for er.E in (8, 64, 256):
+        for er.k in (1, 8):
+            for er.T in range(1, 2000, 7):
+                real, padded = _expected_rows(er)
+                assert real == er.T * er.k and real < padded <= ExpertRows.capacity(er.T, er.k, er.E, ROW_ALIGN)
+                n = padded / er.E
+                if er.E // 2 <= real < 16 * er.E:
+                    assert ROW_ALIGN // 2 < n + 2 * n ** 0.5 <= ROW_ALIGN, (er.E, er.k, er.T)
