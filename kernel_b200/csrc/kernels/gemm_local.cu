@@ -187,12 +187,12 @@ Config rows_plain_config(int M, int groups, int N, int K, bool b_mn, int sms, in
   return best;
 }
 
-// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 per k block
-// (190 for a pair) however narrow the tile.
-double swap_k_block(bool pair, int w_cols, int tok, bool w_mn) {
+// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 (190 for a pair) for
+// each box of the tokens, however narrow the tile.
+double swap_k_block(bool pair, int w_cols, int tok, bool w_mn, int boxes) {
   const double mma = 300.0 * tok / 256.0 * (pair ? 1.0 : 1.33);
   const double load = 128.0 * (w_cols + (pair ? tok / 2 : tok)) / 95.0 * (w_mn ? 1.07 : 1.0);
-  const double issue = pair ? 190.0 : 170.0;
+  const double issue = boxes * (pair ? 190.0 : 170.0);
   const double t = mma > load ? mma : load;
   return t > issue ? t : issue;
 }
@@ -210,7 +210,7 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
     for (int w_cols = w_mn ? 64 : 32; w_cols <= 128; w_cols += w_mn ? 64 : 8) {
       const int bn = pair ? 2 * w_cols : w_cols;
       const double tiles = static_cast<double>(mb) * ceil_div(N, bn);
-      const double k_block = swap_k_block(pair, w_cols, tok, w_mn);
+      const double k_block = swap_k_block(pair, w_cols, tok, w_mn, 1);
       for (int split = 1; split <= (pair ? 4 : 8); ++split) {
         const int ctas = (pair ? 2 : 1) * split;
         const int units = cap.clusters[ctas];
@@ -264,12 +264,18 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
         const double tiles = groups * blocks * ceil_div(N, bn);
         const double units = pair ? sms / 2 : sms;
         const double waves = tiles <= units ? 1.0 : tiles / units + 0.5;
-        const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, cols < tok ? cols : tok, w_mn) + 1000.0) + 2000.0 * cols / 256.0 +
-                         (pair ? 1000.0 : 0.0);
-        const double cost = t > memory ? t + 0.1 * memory : memory + 0.1 * t;
+        // The tile is chosen as if the tokens came in one box, its cost counts the boxes: 8 groups of 121 rows of [640, 2960], in
+        // pairs, take 15.9 us on the M side and 20.7 here.
+        const int block = cols < tok ? cols : tok;
+        auto cost_of = [&](int boxes) {
+          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 1000.0 : 0.0);
+          return t > memory ? t + 0.1 * memory : memory + 0.1 * t;
+        };
+        const double cost = cost_of(1);
         if (cost < best_t) {
           best_t = cost;
-          *cost_out = cost + mma_energy(groups * blocks * cols, static_cast<double>(ceil_div(N, bn)) * (pair ? 256.0 : 128.0), K);
+          *cost_out = cost_of(ceil_div(block, (pair ? 2 : 1) * ring.xbox)) +
+                      mma_energy(groups * blocks * cols, static_cast<double>(ceil_div(N, bn)) * (pair ? 256.0 : 128.0), K);
           best = c;
         }
       }
@@ -410,8 +416,8 @@ Remembered& remembered(int M, int N, int K, int groups, int key) {
   return table[(h ^ (h >> 15)) & 63u];
 }
 // What the exchanged kernel gains, ns, by fetching weights under the end of the previous launch, which the other one does not
-// do.  500 MLPs of 1 to 1200 tokens: with 0, 1500 and 3000 the two products take 0.856, 0.852 and 0.854 of what they
-// took on the M side in order, and 4, none and 2 of them more than 3 % longer than that.
+// do.  500 MLPs (1 to 1200 tokens) and 582 MoE layers: with 0, 1500 and 3000 a pair of products takes 0.856, 0.852 and 0.854 of what it
+// took on the M side in order (MLP), 0.919, 0.906 and 0.905 (MoE); 4, none and 2 MLPs take more than 3 % longer, 10, 24 and 32 layers.
 constexpr double EARLY = 1500.0;
 
 // Rows on the tensor cores' M side or on their N side: what the two models say, plus the energy, plus what 2330 products (1 to
@@ -460,20 +466,25 @@ int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool 
   return KB_OK;
 }
 // Grouped rows; `rows` of them are expected.
-Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int shape, bool slope) {
-  const int key = (slope ? 1 : 0) | (w_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int shape, bool slope, bool early) {
+  const int key = (slope ? 1 : 0) | (early ? 1 << 28 : 0) | (w_mn ? 2 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   Remembered& e = remembered(rows, N, K, groups, key);
   if (e.M != rows || e.N != N || e.K != K || e.groups != groups || e.key != key) {
     Choice r = {};
     double plain = 1e30, other = 1e30;
     if (shape < 3) r.c = rows_plain_config(rows, groups, N, K, w_mn, cap, shape, slope, &plain);
     if (shape < 0 || shape >= 3) r.s = rows_swap_config(rows, groups, N, K, w_mn, cap, shape, &other);
-    // Groups of some blocks: little padding either way, and near ties go to the M side, unless its epilogue reads saved
-    // values back (each lane a row: it keeps the accumulator of a tile longer).  us, rows on the M side / exchanged:
+    // Groups of some blocks: little padding either way.  A slope favours the N side: the M side's epilogue reads the saved values
+    // back with a row per lane and keeps the accumulator of a tile longer.  us, rows on the M side / exchanged:
     //   rows per group, [N, K]        3, [1024, 2048]   3, [760, 2728]   128, [1024, 2048]   250, [4096, 4096]   717, [544, 3008]
     //   forward with activation          47.6  45.5        99.5  89.4       75.3  67.7          98.5 101           25.3  26.7
     //   slope                            56.6  56.0         145   144       90.8  75.4           116  94.4         36.5  31.5
-    r.swap = other < (rows >= 192ll * groups && !slope ? 0.85 : 0.97) * plain;
+    // Limits from 3100 products of uniformly routed rows in bursts (8 to 128 groups of 0.1 to 1600 rows, N and K 512 to 4096) and 330
+    // near ties repeated at the power cap: those take 3.1 % more than the better kind on average (always the M side 9.5 %,
+    // always exchanged 1.9 %) and 14 are more than 2 % slower than on the M side (26 with 0.97 and 0.85 before the
+    // boxes were counted; 39 always exchanged).
+    const double limit = slope ? 1.25 : rows >= 192ll * groups ? 0.9 : rows >= 32ll * groups ? 0.99 : 0.97;
+    r.swap = other - (early ? EARLY : 0.0) < limit * plain;
     e = {rows, N, K, groups, key, 0, r};
   }
   return e.c;
@@ -538,7 +549,7 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
   if (cap < 2 || env().no_pair) shape = shape >= 3 ? 3 : 0;
   Choice pick = {};
   if (a->kind == KB_LOCAL_ROWS) {
-    pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr);
+    pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr, a->early != 0);
   } else if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
     const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->pre_in != nullptr, a->early != 0, &pick);

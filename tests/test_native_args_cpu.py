@@ -248,3 +248,19 @@ def test_a_product_that_may_fetch_its_weights_early_is_exchanged_sooner():
     for M, Nn, K in ((128, 4096, 4096), (330, 6296, 1304), (672, 10008, 2040)):
         assert [_pick(148, M=M, N=Nn, K=K, early=early)[0] for early in (0, 1)] == [0, 1], (M, Nn, K)
     assert _pick(148, M=256, N=4096, K=14336, early=1)[0] == 0   # 36.5 us, exchanged 46.0
+
+
+def test_kind_of_grouped_products_whose_difference_was_measured():
+    """At least 8 % apart on a B200 with uniformly routed rows (us, rows on the M side / exchanged)."""
+    def kind(groups, rows, Nn, K, **kw):
+        return _pick(148, kind=N.LOCAL_ROWS, M=rows, N=Nn, K=K, groups=groups, row_start=16, row_count=16, **kw)[0]
+
+    assert kind(8, 968, 640, 2960) == 0      # 15.9 20.7
+    assert kind(8, 446, 712, 1280) == 0      # 8.2 10.4
+    assert kind(16, 3400, 560, 864) == 0     # 12.0 11.1, but 8.0 with groups of one size
+    assert kind(64, 192, 760, 2728) == 1     # 99.5 89.4
+    assert kind(64, 8192, 1024, 2048) == 1   # 75.3 67.7
+    slope = dict(b_mn=1, act=N.ACTS["silu"], pre_in=0)
+    assert kind(64, 10240, 1024, 2048, **slope) == 1   # 90.8 75.4
+    assert kind(64, 4096, 2872, 552, **slope) == 1     # 50.0 35.3, 64 rows of padding and tokens in every group
+    assert kind(8, 4000, 4096, 4096, **slope) == 1     # 116 94.4
