@@ -164,6 +164,7 @@ def _declare(lib: C.CDLL) -> None:
         "kb_device_barrier": (i, [C.POINTER(vp), u64, i, i, u32, u64, vp, vp]),
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
         "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
+        "kb_a2a_local_vecs": (i, [i, i, i, i]),
         "kb_gemm_local_pick": (i, [C.POINTER(LocalGemmArgs), i, C.POINTER(LocalPick)]),
         "kb_gemm_local_config": (i, [i, i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
         "kb_col_sum_parts": (i, [i, i]),

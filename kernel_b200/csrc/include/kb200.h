@@ -233,6 +233,8 @@ uint64_t kb_a2a_flag_bytes(void);
 uint64_t kb_a2a_sync_bytes(void);
 int kb_a2a_flag_stride_words(void);
 // Posts this rank's y-ready flag of args->epoch on every rank (after the caller's own expert computation).
+// 16-byte vectors per lane that the round trip of a single rank takes on `sms` SMs (tests of the rule).
+int kb_a2a_local_vecs(int tokens, int hidden, int elem_bytes, int sms);
 int kb_a2a_post_ready(const KbA2aArgs* a, void* stream);
 int kb_a2a_dispatch(const KbA2aArgs* a, void* stream);
 int kb_a2a_expert_scale(const KbA2aArgs* a, void* stream);

@@ -1214,3 +1214,8 @@ extern "C" int kb_a2a_static_status(uint32_t* out8, int clear, void* stream) {
   if (clear) KB_CUDA_OK(cudaMemsetAsync(base + ST_STATUS_OFF, 0, 8 * sizeof(uint32_t), st));
   return KB_OK;
 }
+
+extern "C" int kb_a2a_local_vecs(int tokens, int hidden, int elem_bytes, int sms) {
+  if (tokens < 1 || hidden < 1 || (elem_bytes != 2 && elem_bytes != 4) || sms < 1) return KB_ERR_ARG;
+  return local_vecs(tokens, hidden * elem_bytes / 16, elem_bytes, sms);
+}

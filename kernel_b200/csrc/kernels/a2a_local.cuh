@@ -244,8 +244,11 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
   }
 }
 
-template <typename T, int kVecs, int kCtas>
+constexpr int LOCAL_CTAS[5] = {0, 8, 6, 0, 4};  // resident CTAs of an SM by vectors per lane
+
+template <typename T, int kVecs>
 static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
+  constexpr int kCtas = LOCAL_CTAS[kVecs];
   const int parts = (p.vecs + 32 * kVecs - 1) / (32 * kVecs);
   const long long units = static_cast<long long>(p.T) * parts;
   if (units > 0x3fffffff) return KB_ERR_UNSUPPORTED;  // three launches of the general kernels
@@ -259,14 +262,45 @@ static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
   return KB_OK;
 }
 
+// Vectors per lane.  Few tokens: one, which spreads a row over more warps (64 tokens of 14 KB 1.94 us of GPU time against 2.05
+// with four, 128 tokens 2.95 and 2.60: the line is at about 60).  Many: four, which do with the fewest instructions per value
+// what the registers allow; back to back in a graph, three inputs in turn, 7168 values, us with 1 / 2 / 4 vectors:
+//   2048 tokens bf16, scales exact  24.0 19.9 16.8    unit scales 19.9 15.6 13.2    scales not bf16 values 28.6 25.4 21.5
+//   2048 tokens fp16                30.1 22.5 19.3    fp32 40.8 23.9 19.5           256 tokens bf16          4.6  4.2  3.8
+// In between a wide form may need a round of the resident warps more for a few tokens, leave most of a row's last warp idle
+// or fill the SMs unevenly, so 16-bit rows count the rounds and the CTAs of an SM (constants fitted): bf16, scales not bf16
+// values, 1 / 2 / 4 vectors
+//   700 tokens of 1048   3.7  4.0  4.6    300 of 4104   4.4  4.2  4.9    2048 of 2056   10.6  9.6  11.7    2048 of 2560   11.7  9.7  11.8
+// Over 610 cases past the first line (200 to 2048 tokens of 1024 to 7168 values) 1.6 % above the best form on average, with four
+// always 9.5 %.
+inline int local_vecs(int tokens, int vecs, int elem_bytes, int sms) {
+  const long long all = static_cast<long long>(tokens) * vecs;
+  if (elem_bytes == 4) return all < 16ll * 32 * sms ? 1 : 4;
+  if (all < 12ll * 32 * sms) return 1;
+  int best = 1;
+  double best_cost = 1e30;
+  for (int v = 1; v <= 4; v *= 2) {
+    const int parts = (vecs + 32 * v - 1) / (32 * v);
+    const long long at_once = static_cast<long long>(sms) * LOCAL_CTAS[v] * LOCAL_WARPS / parts;  // tokens
+    const long long step = at_once < 1 ? 1 : at_once < tokens ? at_once : tokens;
+    const double per_sm = static_cast<double>(((step * parts + LOCAL_WARPS - 1) / LOCAL_WARPS + sms - 1) / sms);  // CTAs
+    const double rounds = static_cast<double>((tokens + step - 1) / step) + 2.6 * tokens / step;
+    const double cost = rounds * (per_sm * (v + 0.13) + 1.5) + (v == 1 ? 1.8 : v == 2 ? -3.4 : 0.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = v;
+    }
+  }
+  return best;
+}
+
 template <typename T>
 static int launch_local(const A2aParams& p, int sms, cudaStream_t st) {
   if (p.T == 0) return KB_OK;
-  // Few tokens: one vector per lane spreads a row over more warps (64 tokens of 14 KB 1.94 us of GPU time against 2.05 with four,
-  // 128 tokens 2.95 and 2.60: the line is at about 80).  Many: four, which do with the fewest instructions per value what
-  // the registers allow; back to back in a graph, three inputs in turn, 7168 values, us with 1 / 2 / 4 vectors:
-  //   2048 tokens bf16, scales exact  24.0 19.9 16.8    unit scales 19.9 15.6 13.2    scales not bf16 values 28.6 25.4 21.5
-  //   2048 tokens fp16                30.1 22.5 19.3    fp32 40.8 23.9 19.5           256 tokens bf16          4.6  4.2  3.8
-  if (static_cast<long long>(p.T) * p.vecs < 16ll * 32 * sms) return launch_local_as<T, 1, 8>(p, sms, st);
-  return launch_local_as<T, 4, 4>(p, sms, st);
+  switch (local_vecs(p.T, p.vecs, sizeof(T), sms)) {
+    case 1: return launch_local_as<T, 1>(p, sms, st);
+    case 2:
+      if constexpr (sizeof(T) == 2) return launch_local_as<T, 2>(p, sms, st);
+  }
+  return launch_local_as<T, 4>(p, sms, st);
 }

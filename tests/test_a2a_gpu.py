@@ -61,7 +61,7 @@ def test_round_trip_matches_fp32_reference(E, k, H, T, dtype, mode, fused, monke
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("E", [256, 512, 192])  # scales: values of bf16; of fp16 and some of bf16; of neither
-@pytest.mark.parametrize("H,T", [(7168, 700), (1048, 2048), (520, 3)])  # four vectors per lane, whole and ragged; one
+@pytest.mark.parametrize("H,T", [(4096, 2048), (4040, 2048), (2560, 2048), (2056, 2048), (1048, 700), (520, 3)])  # four vectors per lane (16-bit), whole and ragged; two; one
 def test_one_pass_round_trip_equals_the_general_kernels(E, H, T, dtype, monkeypatch):
     """Value for value, over every exponent of the type, infinities, NaN and zeros (of whose sign the general kernels'
     additional sum over the ranks keeps nothing)."""

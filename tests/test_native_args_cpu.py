@@ -264,3 +264,17 @@ def test_kind_of_grouped_products_whose_difference_was_measured():
     assert kind(64, 10240, 1024, 2048, **slope) == 1   # 90.8 75.4
     assert kind(64, 4096, 2872, 552, **slope) == 1     # 50.0 35.3, 64 rows of padding and tokens in every group
     assert kind(8, 4000, 4096, 4096, **slope) == 1     # 116 94.4
+
+
+def test_vectors_per_lane_of_the_round_trip():
+    """Where a form was at least 5 % faster than the others on a B200 (us with 1 / 2 / 4 vectors per lane)."""
+    vecs = lambda tokens, hidden, elem=2: N.lib().kb_a2a_local_vecs(tokens, hidden, elem, 148)
+    for tokens, hidden in ((2048, 7168), (2048, 4096), (300, 7168)):
+        assert vecs(tokens, hidden) == vecs(tokens, hidden, 4) == 4        # 28.6 25.4 21.5 for the first
+    for tokens, hidden in ((1, 7168), (60, 7168), (101, 2880), (130, 1024)):
+        assert vecs(tokens, hidden) == 1
+    for tokens, hidden in ((700, 1048), (700, 1280)):
+        assert vecs(tokens, hidden) == 1, (tokens, hidden)                 # 3.7 4.0 4.6 for the first
+    for tokens, hidden in ((2048, 2056), (2048, 2560), (300, 4104), (700, 1536)):
+        assert vecs(tokens, hidden) == 2, (tokens, hidden)                 # 10.6 9.6 11.7 for the first
+    assert vecs(2048, 2560, 4) == 4                                        # fp32: 14.4 14.4 11.8 for 2880 values
