@@ -39,6 +39,17 @@ void* driver_fn(const char* name);
   } while (0)
 
 #ifdef __CUDACC__
+// A driver call that wants a current context.  A thread that has made no runtime call yet has none (a fresh autograd
+// worker whose memory came from the allocator's cache): its device's is bound then.
+template <typename Call>
+CUresult with_context(Call&& call) {
+  const CUresult r = call();
+  if (r != CUDA_ERROR_INVALID_CONTEXT) return r;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return r;
+  return call();
+}
+
 // Launch attribute of a kernel that begins with wait_for_previous_launch() (ptx.cuh): it may
 // be set up while the previous kernel of the stream still runs.
 inline cudaLaunchAttribute overlap_launch() {

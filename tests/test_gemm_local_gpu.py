@@ -396,6 +396,33 @@ def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mo
     ctx.heap.close()
 
 
+def test_a_product_is_the_first_cuda_call_of_its_thread():
+    """As in an autograd worker whose memory comes from the allocator's cache: no runtime call has bound a context."""
+    import threading
+
+    from kernel_b200.ops.local import product
+
+    a, b, failed = _ints(136, 264, seed=18), _ints(72, 264, seed=19), []
+    outs = [torch.zeros(136, 72, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    product(a, b, out=outs[0])
+    torch.cuda.synchronize()
+
+    def work(i, *args, **kw):
+        try:
+            product(*args, out=outs[i], **kw)
+        except Exception as e:  # reported in the test's thread
+            failed.append(e)
+
+    for i, args, kw in ((1, (a, b), {}), (2, (a, b.t().contiguous()), dict(b_t=True))):
+        torch.cuda.synchronize()
+        t = threading.Thread(target=work, args=(i, *args), kwargs=kw)
+        t.start()
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    assert torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
+
+
 def test_overlapped_launches_keep_their_order_eagerly_and_in_a_graph():
     """A chain in which every kernel reads what the one before wrote, also across a fork and a
     join of streams, with torch kernels and copies in between."""
