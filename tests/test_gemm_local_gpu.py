@@ -124,7 +124,7 @@ def _table(counts, pad):
     return start.int().to(DEV), n.int().to(DEV), max(1, int(padded.sum()))
 
 
-def _force(monkeypatch, pair, bn=0, split=0):
+def _force(monkeypatch, pair, bn=0, split=0, tok=0):
     """Tile shape of the products made through ``ops.local``."""
     from kernel_b200.ops import local as L
 
@@ -132,7 +132,7 @@ def _force(monkeypatch, pair, bn=0, split=0):
 
     def forced(*a):
         args = made(*a)
-        args.pair, args.bn, args.split = pair, bn, split
+        args.pair, args.bn, args.split, args.tok = pair, bn, split, tok
         return args
 
     monkeypatch.setattr(L, "_args", forced)
@@ -196,23 +196,45 @@ def test_epilogues_with_exchanged_operands(act, pair, bn, split, M, N, K, monkey
     """Token rows on the MMA's N side: one token, whole and ragged blocks, several of them, columns that end inside a tile."""
     L = _force(monkeypatch, pair, bn, split)
     a, b = _ints(M, K, seed=34), _ints(N, K, seed=35) * 2 ** -5
+    bt, bias = b.t().contiguous(), _ints(N, seed=36)
     st = _status()
-    pre = torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
-    out = L.product(a, b, act=act, pre_out=pre, status=st)
-    grad = L.product(a, b.t().contiguous(), b_t=True, act=act, pre_in=pre, status=st, early=True)
-    bias = _ints(N, seed=36)
-    plain = L.product(a, b, bias, status=st, early=True)
+    pre, plain = (torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    out, grad = torch.empty_like(pre), torch.empty_like(pre)
+    torch.cuda.synchronize()
+    L.product(a, b, act=act, pre_out=pre, out=out, status=st)
+    L.product(a, bt, b_t=True, act=act, pre_in=pre, out=grad, status=st, early=True)   # behind a product that wrote neither weights
+    L.product(a, b, bias, out=plain, status=st, early=True)
     _clean(st)
     full = a.float() @ b.float().t()
     _check_epilogues(act, full, pre, out, grad)
     assert torch.equal(plain, (full + bias.float()).to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("pair,bn", [(3, 64), (3, 128), (4, 128), (4, 256)])
+@pytest.mark.parametrize("pair,bn,split", [(3, 32, 1), (3, 56, 2), (3, 80, 7), (3, 112, 5), (4, 80, 1), (4, 176, 2), (4, 208, 1), (4, 240, 3)])
+@pytest.mark.parametrize("M,N,K,tok", [(1, 264, 2120, 0), (64, 480, 1096, 32), (165, 72, 520, 0), (520, 264, 1096, 96), (300, 1664, 520, 256)])
+def test_exchanged_tiles_that_end_inside_a_warp(pair, bn, split, M, N, K, tok, monkeypatch):
+    """Weights along K come in tiles of any multiple of 8 columns per CTA: whole tiles and cut ones, splits that do not divide the
+    k blocks, token blocks of a chosen height."""
+    L = _force(monkeypatch, pair, bn, split, tok)
+    a, b, bias = _ints(M, K, seed=46), _ints(N, K, seed=47), _ints(N, seed=48)
+    st = _status()
+    pre, out, plain = (torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3))
+    torch.cuda.synchronize()
+    L.product(a, b, act="relu", pre_out=pre, out=out, status=st)
+    L.product(a, b, bias, out=plain, status=st, early=True)
+    _clean(st)
+    full = a.float() @ b.float().t()
+    assert torch.equal(pre, full.to(torch.bfloat16)) and torch.equal(out, torch.relu(full).to(torch.bfloat16))
+    assert torch.equal(plain, (full + bias.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("pair,bn,tok", [(3, 64, 0), (3, 128, 0), (4, 128, 0), (4, 256, 0), (3, 128, 16), (3, 64, 48), (3, 128, 256), (4, 256, 32), (4, 128, 96),
+                                         (4, 256, 256)])
 @pytest.mark.parametrize("counts", COUNTS)
 @pytest.mark.parametrize("N", [264, 320])  # 320: a multiple of 64, weights along N come in whole boxes, the last tile ends inside
-def test_grouped_rows_with_exchanged_operands(N, pair, bn, counts, monkeypatch):
-    L = _force(monkeypatch, pair, bn)
+def test_grouped_rows_with_exchanged_operands(N, pair, bn, tok, counts, monkeypatch):
+    """``tok``: most rows of a block; groups of several uneven blocks."""
+    L = _force(monkeypatch, pair, bn, tok=tok)
     K = 520
     start, count, R = _table(counts, 1)
     a, b = _ints(R, K, seed=37), _ints(len(counts), N, K, seed=38) * 2 ** -4
@@ -248,6 +270,72 @@ def test_weights_fetched_early_are_those_of_the_call():
     mlp.up.status.cpu()
     _clean(mlp.up.status)
     _clean(mlp.down.status)
+
+
+@pytest.mark.parametrize("pair", [3, 4])
+def test_moe_weights_fetched_early_are_those_of_the_call(pair, monkeypatch):
+    """Rewritten directly before the inference block, and between a forward pass and its backward pass (the block reads the
+    parameters themselves): the output is odd in the second matrix, the token gradient in each of them."""
+    from kernel_b200.models import MoELayer, TrainableMoELayer
+
+    _force(monkeypatch, pair)
+    torch.manual_seed(6)
+    E, k, H, F, T = 16, 2, 1024, 1032, 96
+    layer = TrainableMoELayer(E, k, H, F, T, device=torch.device(DEV))
+    fixed = MoELayer(E, k, H, T, layer.w_up.data.clone(), layer.w_down.data.clone())
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16).requires_grad_(True)
+    idx = torch.rand(T, E, device=DEV).argsort(1)[:, :k].to(torch.int32).contiguous()
+    w = torch.softmax(torch.randn(T, k, device=DEV), -1)
+    dy = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    want = fixed(x.detach(), idx, w)
+    grad, = torch.autograd.grad(layer(x, idx, w), x, dy)
+    for i in range(10):
+        fixed.w_down.neg_()
+        want = -want
+        assert torch.equal(fixed(x.detach(), idx, w), want), i
+        y = layer(x, idx, w)
+        for weights in ((layer.w_down,), (layer.w_up,), (layer.w_up, layer.w_down)):
+            for p in weights:
+                p.data.neg_()
+            got, = torch.autograd.grad(y, x, dy, retain_graph=True)
+            assert torch.equal(got, grad if len(weights) == 2 else -grad), i
+            for p in weights:
+                p.data.neg_()
+    layer.a2a.heap.check_status()
+    fixed.a2a.heap.close()
+    layer.close()
+
+
+@pytest.mark.parametrize("pair", [3, 4])
+def test_mlp_gradients_fetch_the_weights_of_the_call(pair, monkeypatch):
+    """As above: the token gradient is odd in each weight matrix."""
+    from kernel_b200.models import TrainableSequenceParallelMLP
+    from kernel_b200.ops import local as L
+
+    launch = L._launch
+
+    def exchanged(args, device):
+        if not args.a_mn:
+            args.pair = pair
+        launch(args, device)
+
+    monkeypatch.setattr(L, "_launch", exchanged)
+    torch.manual_seed(7)
+    mlp = TrainableSequenceParallelMLP(48, 1032, 4104, activation="relu", device=torch.device(DEV))
+    x = torch.randn(48, 1032, device=DEV).to(torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(48, 1032, device=DEV).to(torch.bfloat16)
+    leaves = (x, mlp.down.weight)          # with the second one the hidden gradient follows a product of this module
+    grad, dw2 = torch.autograd.grad(mlp(x), leaves, dy)
+    for i in range(10):
+        y = mlp(x)
+        for weights in ((mlp.down.weight,), (mlp.up.weight,)):
+            for p in weights:
+                p.data.neg_()
+            got = torch.autograd.grad(y, leaves, dy, retain_graph=True)
+            assert torch.equal(got[0], -grad) and torch.equal(got[1], dw2), i
+            for p in weights:
+                p.data.neg_()
+    mlp.close()
 
 
 @pytest.mark.parametrize("act", ["gelu", "relu", "silu"])
