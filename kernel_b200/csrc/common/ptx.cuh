@@ -529,8 +529,9 @@ __device__ __forceinline__ uint4 ld_global_v4(const void* p) {
 
 // Start of a kernel launched with the overlap_launch attribute: waits until the previous
 // kernel of the stream has ended and its writes are visible, then lets the next one be set up.
-// Nothing that another kernel may write, and no output, is touched before it.  Without the
-// attribute the wait returns at once.
+// Nothing that the previous kernel may write, and no output, is touched before it.  What was written before
+// that kernel began may be read earlier if that kernel passes its own wait before it lets this one start, as all kernels that call
+// this do (`early` in gemm_swap.cuh).  Without the attribute the wait returns at once.
 __device__ __forceinline__ void wait_for_previous_launch() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -399,7 +399,7 @@ int device_capacity(int dev, int sms, Capacity* out) {
 }
 
 // The choice depends on the sizes alone and a program calls with the same ones again
-// and again: a small table per thread remembers it (the search takes about 2 us).
+// and again: a small table per thread, dense and grouped products together, remembers it (a search takes 0.3 to 1.7 us).
 struct Choice {
   bool swap;      // exchanged operands
   Config c;

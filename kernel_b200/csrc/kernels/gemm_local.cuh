@@ -19,7 +19,8 @@
 //
 // A tile has 128 rows (one CTA) or 256 rows (CTA pair, cta_group::2) and `bn`
 // columns, a runtime multiple of 32 up to 256: what the launcher picks so that
-// the tiles fill the chip (see choose_config in gemm_local.cu).
+// the tiles fill the chip (see choose_config in gemm_local.cu; choose
+// weighs it against exchanged operands, gemm_swap.cuh).
 //
 // Split contraction (dense, few tiles): `split` CTAs (or pairs) form one cluster
 // and share a tile, each with its part of K.  The fp32 partial tiles are exchanged

@@ -188,8 +188,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
     """``out[M,N] = a[M,K] @ b[N,K]^T (+ bias_scale * bias)`` in bf16 with fp32 accumulation.
 
     ``pair=True`` uses clusters of two CTAs sharing 256x256 tiles (``cta_group::2``,
-    more than 128 rows), ``pair=False`` tiles of one CTA, ``None`` lets the launcher pick
-    the tile shape from the sizes (``choose_config`` in ``csrc/kernels/gemm_local.cu``)."""
+    more than 128 rows), ``pair=False`` tiles of one CTA, both with the rows on the tensor cores' M side;
+    ``None`` lets the launcher pick the side and the tile from the sizes (``choose`` in ``csrc/kernels/gemm_local.cu``)."""
     _check_bf16_2d(a, "a")
     _check_bf16_2d(b, "b")
     M, K = a.shape
