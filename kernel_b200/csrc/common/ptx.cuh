@@ -148,6 +148,22 @@ __device__ __forceinline__ void tma_load_3d_warp(uint32_t smem_dst, const void* 
         : "memory");
   }
 }
+template <bool kPair>
+__device__ __forceinline__ void tma_load_4d_warp(uint32_t smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y, int32_t z, int32_t w) {
+  if constexpr (kPair) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+  }
+}
 // The expected bytes (0: this CTA expects none) and one box of a 4-D map, issued by one elected lane.
 template <bool kPair>
 __device__ __forceinline__ void tma_load_4d_expect_warp(uint32_t own_bar, uint32_t tx_bytes, uint32_t bar, uint32_t dst, const void* map, int32_t x,

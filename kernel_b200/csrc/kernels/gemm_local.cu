@@ -680,10 +680,14 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.timing = env().timing ? 1 : 0;
 
   const uint64_t bz = a->kind == KB_LOCAL_ROWS ? groups : 1;
-  rc = a_mn ? make_tmap3(&p.tmA, a->A, a->M, a->K, 1, 64, BK) : make_tmap3(&p.tmA, a->A, a->K, a->M, 1, BK, p.a_rows);
+  p.a_whole = a_mn && a->M % 64 == 0 ? 1 : 0;
+  p.b_whole = b_mn && a->N % 64 == 0 ? 1 : 0;
+  const int b_cols = c.pair ? c.bn / 2 : c.bn;
+  rc = p.a_whole ? make_tmap4_blocks(&p.tmA, a->A, a->M, a->K, 1, BK, p.a_rows / 64)
+       : a_mn ? make_tmap3(&p.tmA, a->A, a->M, a->K, 1, 64, BK) : make_tmap3(&p.tmA, a->A, a->K, a->M, 1, BK, p.a_rows);
   if (rc != KB_OK) return rc;
-  rc = b_mn ? make_tmap3(&p.tmB, a->B, a->N, a->K, bz, 64, BK)
-            : make_tmap3(&p.tmB, a->B, a->K, a->N, bz, BK, c.pair ? c.bn / 2 : c.bn);
+  rc = p.b_whole ? make_tmap4_blocks(&p.tmB, a->B, a->N, a->K, bz, BK, b_cols / 64)
+       : b_mn ? make_tmap3(&p.tmB, a->B, a->N, a->K, bz, 64, BK) : make_tmap3(&p.tmB, a->B, a->K, a->N, bz, BK, b_cols);
   if (rc != KB_OK) return rc;
   if (contract) {
     rc = make_tmap3(&p.tmOut, a->out, a->N, a->M, groups, 64, 32);

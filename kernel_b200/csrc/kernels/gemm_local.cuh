@@ -73,6 +73,7 @@ struct alignas(64) Params {
   int groups;
   int split;         // members of a cluster that share a tile
   int stages, a_slot, b_slot;  // operand ring: bytes per stage
+  int a_whole, b_whole;  // M/N-contiguous operand whose extent is a multiple of 64: one box of a 4-D map holds a stage's share
   int a_rows;        // rows of A a stage brings in (128 per half, or fewer when M or the groups are smaller)
   int slot_rows;     // split: rows of an exchange slot (128, or fewer when M is smaller)
   int wide;          // rows of the output start at multiples of 32 bytes: whole-sector stores
@@ -431,15 +432,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
             continue;
           }
           if (leader) kb::mbar_expect_tx_warp(own, tx_bytes);
+          // M/N-contiguous operands in one load each instead of one per 64 columns: issuing six loads per stage is what
+          // held the producer back where a tile has few k blocks (weight gradients of 64 experts of 2048 x 1024, 128 rows:
+          // 73.8 -> 70.8 us, on 32 SMs alone 276 -> 237).
           if constexpr (kAMn) {
+            if (p.a_whole) {
+              kb::tma_load_4d_warp<kPair>(da, &p.tmA, bar, 0, t.k_row + k * BK, t.row0 / 64, 0);
+            } else {
 #pragma unroll
-            for (int i = 0; i < CTA_ROWS / 64; ++i) {
-              kb::tma_load_3d_warp<kPair>(da + i * MN_BLOCK_BYTES, &p.tmA, bar, t.row0 + i * 64, t.k_row + k * BK, 0);
+              for (int i = 0; i < CTA_ROWS / 64; ++i) {
+                kb::tma_load_3d_warp<kPair>(da + i * MN_BLOCK_BYTES, &p.tmA, bar, t.row0 + i * 64, t.k_row + k * BK, 0);
+              }
             }
           } else {
             kb::tma_load_3d_warp<kPair>(da, &p.tmA, bar, k * BK, t.row0, 0);
           }
           if constexpr (kBMn) {
+            if (p.b_whole) {
+              kb::tma_load_4d_warp<kPair>(db, &p.tmB, bar, 0, t.k_row + k * BK, nrow / 64, bz);
+              continue;
+            }
             for (int i = 0; i < b_cols / 64; ++i) {
               kb::tma_load_3d_warp<kPair>(db + i * MN_BLOCK_BYTES, &p.tmB, bar, nrow + i * 64, t.k_row + k * BK, bz);
             }

@@ -375,6 +375,25 @@ def test_contract_product(counts, M, N, pair, monkeypatch):
         assert torch.equal(out[e], (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)), e
 
 
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("M,N", [(192, 320), (64, 576), (320, 72), (136, 192)])
+@pytest.mark.parametrize("pair,bn", [(0, 64), (0, 256), (1, 128), (1, 256)])
+def test_contractions_whose_columns_come_in_one_box(counts, M, N, pair, bn, monkeypatch):
+    """Extents that are multiples of 64 (one box per operand and stage) and end inside a tile, both, one or the other operand."""
+    L = _force(monkeypatch, pair, bn)
+    start, count, R = _table(counts, L.ROW_ALIGN)
+    a, b = torch.zeros((R, M), dtype=torch.bfloat16, device=DEV), torch.zeros((R, N), dtype=torch.bfloat16, device=DEV)
+    for s, n in zip(start.tolist(), count.tolist()):
+        a[s:s + n], b[s:s + n] = _ints(n, M, seed=50 + s), _ints(n, N, seed=51 + s)
+    st = _status()
+    out = L.contract_product(a, b, start, count, status=st)
+    dense = L.product(a, b, a_t=True, b_t=True, status=st)
+    _clean(st)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        assert torch.equal(out[e], (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)), e
+    assert torch.equal(dense, (a.float().t() @ b.float()).to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("R,Cn", [(1, 8), (63, 264), (65, 2048), (1000, 520), (8192, 72)])
 def test_col_sum(R, Cn):
     from kernel_b200.ops.local import col_sum
