@@ -349,6 +349,11 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Without memory ordering: for arrivals that only say that tensor memory has been read (the values are in registers by then).  A
+// release at cluster scope waits until the thread's earlier stores have been performed, 2000 cycles behind an epilogue's.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // Each CTA of the pair loads its own box into its own shared memory; the bytes
 // are counted on the LEADER's mbarrier (`leader_bar` is a cluster address).
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t leader_bar, int32_t x,

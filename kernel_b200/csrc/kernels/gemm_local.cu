@@ -284,18 +284,17 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
   return best;
 }
 
-// Contractions over a group's rows.  A few k blocks: the outputs are the traffic, the widest
-// tile of one CTA, a pair's hand-overs cost more than its smaller operand traffic saves.
-// More: pairs.  One CTA and pair in us, cold L2, by the real rows of every group (a multiple of 64):
-//   rows                     128         192         256         320         384         512
-//   64 of 2048 x 1024      70  92      83  92     102  94     113  98     121 105     153 132
-//   32 of 2048 x 2048      72  91      84  90     102  92     113  94     121 102     152 125
-//   8 of 4096 x 4096       72  87      80  88     104  92     113  94     123 102     155 126
-//   128 of 1024 x 768      60  77      68  76      82  82      90  88      98  88     122 100
-// So pairs win from 256 rows on, and the line lies between that and 192.
+// Contractions over a group's rows.  About one k block: the outputs are all of the traffic, tiles of one CTA.  More: pairs, which
+// fetch a third fewer operand bytes for the same output.  One CTA and pair in us, three outputs in turn, Poisson row counts:
+//   rows per group           32          64          80          96         128         160         192         256
+//   64 of 2048 x 1024      57  58      56  59      61  61      63  61      69  64      78  73      85  79     101  94
+//   8 of 4096 x 4096       54  55      53  54      60  57      61  57      71  63      77  71      86  76     104  83
+//   128 of 1024 x 768      45  46      46  50      49  49      50  50      61  52      64  55      70  64      83  73
+//   32 of 2040 x 1000      35  37      40  36      42  39      44  39      48  43      53  46      58  50      67  57
+// (Before the second CTA's epilogue gave its accumulator back without a fence, a pair took 93, 86, 76 and 53 at 128 rows.)
 Config contract_config(int M, int N, int rows, int groups, int shape) {
   Config c;
-  c.pair = shape >= 0 ? shape > 0 : M > 128 && rows / groups >= 224;
+  c.pair = shape >= 0 ? shape > 0 : M > 128 && rows / groups >= 72;
   c.bn = N <= 64 && !c.pair ? 64 : N <= 128 ? 128 : 256;
   c.split = 1;
   return c;
@@ -680,8 +679,12 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.timing = env().timing ? 1 : 0;
 
   const uint64_t bz = a->kind == KB_LOCAL_ROWS ? groups : 1;
-  p.a_whole = a_mn && a->M % 64 == 0 ? 1 : 0;
-  p.b_whole = b_mn && a->N % 64 == 0 ? 1 : 0;
+  // A contraction over one k block waits for its stores, not for loads, and large boxes hold the stores up: 128 groups of 16 rows,
+  // 512 x 2048, 58 us with a load per 64 columns, 61 with one per operand.
+  const int expect = a->expect > 0 ? a->expect : a->K;
+  const bool whole = !contract || expect > 56ll * groups;
+  p.a_whole = whole && a_mn && a->M % 64 == 0 ? 1 : 0;
+  p.b_whole = whole && b_mn && a->N % 64 == 0 ? 1 : 0;
   const int b_cols = c.pair ? c.bn / 2 : c.bn;
   rc = p.a_whole ? make_tmap4_blocks(&p.tmA, a->A, a->M, a->K, 1, BK, p.a_rows / 64)
        : a_mn ? make_tmap3(&p.tmA, a->A, a->M, a->K, 1, 64, BK) : make_tmap3(&p.tmA, a->A, a->K, a->M, 1, BK, p.a_rows);

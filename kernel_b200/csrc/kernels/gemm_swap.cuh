@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
           if (lane == 0) {
             if constexpr (kPair) {
               if (leader) kb::mbar_arrive(&tempty[acc]);
-              else kb::mbar_arrive_cluster(kb::map_to_cta(kb::smem_u32(&tempty[acc]), lead));
+              else kb::mbar_arrive_cluster_relaxed(kb::map_to_cta(kb::smem_u32(&tempty[acc]), lead));
             } else {
               kb::mbar_arrive(&tempty[acc]);
             }
