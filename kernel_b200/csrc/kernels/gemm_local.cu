@@ -658,6 +658,9 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.bn = c.bn;
   p.group = (c.tall ? 4096 : 2048) / tile_rows;
   p.groups = grouped ? groups : 0;
+  p.per = Div::by(contract ? p.MBQ * p.NB : grouped ? p.NB : p.group * p.NB);
+  p.first = Div::by(contract ? p.MBQ : p.group);
+  p.last = Div::by(p.MBQ % p.group);
   p.split = c.split;
   p.a_slot = ring.a_slot;
   p.b_slot = ring.b_slot;

@@ -57,6 +57,22 @@ constexpr int OUT_BOX_BYTES = 32 * 128;   // contract: 32 rows x 64 columns, sta
 constexpr int OUT_BYTES = EPI_WARPS * 2 * OUT_BOX_BYTES;  // two boxes per epilogue warp
 constexpr int CHUNK_COLS = 32;            // split: columns are exchanged in chunks of 32
 
+// Division of 0 <= n < 2^31 by a number that is the same for a whole launch: every role of the kernel turns schedule positions
+// into tiles, and two divisions by variables take it 500 cycles per tile.
+struct Div {
+  uint32_t mul, shift;  // mul 0: division by one
+  __host__ static Div by(int d) {  // mul = ceil(2^(31 + l) / d), 2^(l - 1) < d <= 2^l: mul * d exceeds 2^(31 + l) by less than 2^l
+    if (d <= 1) return {0u, 0u};
+    uint32_t l = 1;
+    while ((1ull << l) < static_cast<uint64_t>(d)) ++l;
+    return {static_cast<uint32_t>(((1ull << (31 + l)) + d - 1) / d), l - 1};
+  }
+  __host__ __device__ int of(int n) const {
+    if (mul == 0u) return n;
+    return static_cast<int>(static_cast<uint32_t>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> 32) >> shift);
+  }
+};
+
 enum Kind { DENSE = 0, ROWS = 1, CONTRACT = 2 };
 // What the epilogue does besides the bias: nothing; the activation (runtime kind), with
 // the value before it kept if asked for; the product with the activation's slope.
@@ -70,6 +86,7 @@ struct alignas(64) Params {
   int MBQ, NB, KB;   // scheduling blocks (128 or 256 rows), column blocks, k blocks of the whole contraction
   int bn;            // tile columns
   int group;         // scheduling blocks swept together (rasterisation)
+  Div per, first, last;  // dense: by group * NB, group and the size of the last group; rows: by NB; contract: by MBQ * NB and MBQ
   int groups;
   int split;         // members of a cluster that share a tile
   int stages, a_slot, b_slot;  // operand ring: bytes per stage
@@ -351,17 +368,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     t.k_row = 0;
     t.kb = p.KB;
     if constexpr (kKind == DENSE) {
-      const int per_group = p.group * p.NB;
-      const int g = pos / per_group;
-      const int r = pos - g * per_group;
+      const int g = p.per.of(pos);
+      const int r = pos - g * p.group * p.NB;
       const int gs = min(p.MBQ - g * p.group, p.group);
-      nb = r / gs;
+      nb = (gs == p.group ? p.first : p.last).of(r);
       mbq = g * p.group + (r - nb * gs);
       t.group = 0;
       t.row0 = mbq * TILE_ROWS + static_cast<int>(half) * CTA_ROWS;
       t.row_end = p.M;
     } else if constexpr (kKind == ROWS) {
-      const int block = pos / p.NB;  // counts row blocks: group e holds blocks pref[e] .. pref[e + 1] - 1
+      const int block = p.per.of(pos);  // counts row blocks: group e holds blocks pref[e] .. pref[e + 1] - 1
       int lo = 0, hi = p.groups - 1;
       while (lo < hi) {  // last group with pref <= block: it is not empty
         const int mid = (lo + hi + 1) >> 1;
@@ -370,16 +386,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       }
       const int blocks = pref[lo + 1] - pref[lo];
       const int r = pos - pref[lo] * p.NB;
-      nb = r / blocks;
+      nb = blocks == 1 ? r : r / blocks;
       mbq = r - nb * blocks;
       t.group = lo;
       t.row0 = g_start[lo] + mbq * block_rows + static_cast<int>(half) * CTA_ROWS;
       t.row_end = min(g_start[lo] + g_count[lo], t.row0 + (kPair ? CTA_ROWS : block_rows));
     } else {
-      const int per = p.MBQ * p.NB;
-      t.group = pos / per;
-      const int r = pos - t.group * per;
-      nb = r / p.MBQ;
+      t.group = p.per.of(pos);
+      const int r = pos - t.group * p.MBQ * p.NB;
+      nb = p.first.of(r);
       mbq = r - nb * p.MBQ;
       t.row0 = mbq * TILE_ROWS + static_cast<int>(half) * CTA_ROWS;
       t.row_end = p.M;
@@ -390,9 +405,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     return t;
   };
   // k blocks [k0, k1) of a tile that this member works on
+  // (at most 2^25 of them and eight members: 32 bits hold the products)
   auto k_range = [&](const Tile& t, int& k0, int& k1) {
-    k0 = static_cast<int>(static_cast<long long>(t.kb) * member / p.split);
-    k1 = static_cast<int>(static_cast<long long>(t.kb) * (member + 1) / p.split);
+    k0 = 0;
+    k1 = t.kb;
+    if (kKind == DENSE && p.split > 1) {
+      k0 = static_cast<int>(static_cast<uint32_t>(t.kb * member) / static_cast<uint32_t>(p.split));
+      k1 = static_cast<int>(static_cast<uint32_t>(t.kb * (member + 1)) / static_cast<uint32_t>(p.split));
+    }
   };
 
   if (warp == 0) {
