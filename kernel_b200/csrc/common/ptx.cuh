@@ -164,6 +164,20 @@ __device__ __forceinline__ void tma_load_4d_warp(uint32_t smem_dst, const void* 
         : "memory");
   }
 }
+// Two boxes of a 3-D map, at rows y0 and y1, for one election.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_3d_two_warp(uint32_t dst0, uint32_t dst1, const void* tmap, uint32_t bar, int32_t x, int32_t y0, int32_t y1, int32_t z) {
+#define KB_LOAD_TWO(GROUP)                                                                                                           \
+  asm volatile(                                                                                                                      \
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"                                                                       \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%4, %5, %7}], [%3];\n\t"    \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {%4, %6, %7}], [%3];\n\t}"   \
+      ::"r"(dst0), "r"(dst1), "l"(tmap), "r"(bar), "r"(x), "r"(y0), "r"(y1), "r"(z)                                                  \
+      : "memory")
+  if constexpr (kPair) KB_LOAD_TWO(".cta_group::2");
+  else KB_LOAD_TWO("");
+#undef KB_LOAD_TWO
+}
 // The expected bytes (0: this CTA expects none) and one box of a 4-D map, issued by one elected lane.
 template <bool kPair>
 __device__ __forceinline__ void tma_load_4d_expect_warp(uint32_t own_bar, uint32_t tx_bytes, uint32_t bar, uint32_t dst, const void* map, int32_t x,

@@ -86,6 +86,7 @@ int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool tim
   p.KB = ceil_div(a.K, BK);
   p.NB = ceil_div(a.N, c.bn);
   p.MB = ceil_div(a.M, c.tok);
+  p.per = kbl::Div::by(rows ? p.NB : p.MB);
   p.bn = c.bn;
   p.tok = c.tok;
   p.groups = rows ? a.groups : 0;
