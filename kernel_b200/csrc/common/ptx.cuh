@@ -532,6 +532,13 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint4& a, const uint
                : "memory");
 }
 
+// 32 bytes per thread; the address is a multiple of 32.
+__device__ __forceinline__ void ld_stream_v8(const void* p, uint4& a, uint4& b) {
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(p));
+}
+
 // Streaming read of data that is read-only for the whole kernel.
 __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   uint4 v;
@@ -572,6 +579,10 @@ __device__ __forceinline__ void wait_for_previous_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Brings `bytes` (a multiple of 16, 16-byte aligned) into the L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 // Loads 16 bytes and drops them: the line is in L1 afterwards.
 __device__ __forceinline__ void touch_global(const void* p) {
   asm volatile("{\n\t.reg .b32 a, b, c, d;\n\tld.global.v4.u32 {a, b, c, d}, [%0];\n\t}" ::"l"(p));

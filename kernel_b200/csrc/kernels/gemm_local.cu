@@ -86,8 +86,13 @@ double memory_time(int M, int N, int K) {
 // in a graph, three weights in turn; one CTA with 256 columns and no split against the pick):
 // 64 x 7168 x 18432 88.5 and 45.1 us, 256 x 4096 x 14336 85.1 and 30.5, 2048 x 2880 x 2880 (in the
 // L2) 35.1 and 24.4.  512-row tiles move 25 % fewer operand bytes
-// per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).
-Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, double* cost = nullptr) {
+// per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).  An activation, with the value
+// before it kept, or a slope takes their epilogue 11 us longer in every wave, where a pair's runs under the next tile's products;
+// pairs and 512-row tiles, us:
+//                           plain        gelu, value kept     slope of gelu
+//   8192 x 14336 x 4096    678   708        731   850           762   855
+//   8192 x 29568 x 8192   2830  2858       2831  3163          3068  3113
+Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool act, double* cost = nullptr) {
   Config best = {false, 256, 1};
   double best_t = 1e30, best_cost = 1e30;
   const int KB = ceil_div(K, BK);
@@ -108,7 +113,7 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         if (split > 1 && (tiles > units || KB < 4 * split || !exchange_fits(rows, pair, bn, split))) continue;
         const double waves = units > 0 ? static_cast<double>((static_cast<long long>(tiles) + units - 1) / units) : 1e9;
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 2000.0) + epilogue + (pair ? 1000.0 : 0.0);
-        if (tall) t += 1.25 * waves * epilogue;
+        if (tall) t += waves * (1.25 * epilogue + (act ? 10000.0 : 0.0));
         if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
         // Launched behind the previous kernel instead of under its end.  Not so for the long reads that are launched in order
         // because that is faster (4 x 14488 x 16616, weights along N: 86.6 us split in two, 104 unsplit).
@@ -430,10 +435,10 @@ constexpr double EARLY = 1500.0;
 //   1 x 8192 x 8192   27.2  26.4*   40 x 2840 x 1392    7.8   7.2*   64 x 7168 x 18432   47.2  48.1*   100 x 4096 x 14336   27.9* 28.3
 //   165 x 2920 x 1080 10.4* 12.0    200 x 8192 x 8192  33.8* 33.4    300 x 1024 x 1024    9.2*  9.9    330 x 6296 x 1304    14.0* 13.8
 //   400 x 25000 x 1504 35.1 31.2*   90 x 1104 x 20000  16.4  17.0*   195 x 26136 x 3200  38.9* 42.0    256 x 4096 x 14336   36.5* 46.0
-Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool slope, bool early) {
+Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool act, bool slope, bool early) {
   Choice r = {};
   double plain = 0.0;
-  if (shape < 3) r.c = choose_config(M, N, K, a_mn, b_mn, cap, shape, &plain);
+  if (shape < 3) r.c = choose_config(M, N, K, a_mn, b_mn, cap, shape, act, &plain);
   if (a_mn || (shape >= 0 && shape < 3)) return r;
   const double other = choose_swap(M, N, K, b_mn, cap, shape, &r.s);
   if (shape >= 3) {
@@ -451,15 +456,15 @@ Choice choose(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, in
   r.swap = cost_n - (early ? EARLY : 0.0) < (slope ? 1.05 : 0.97) * cost_m;
   return r;
 }
-int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool slope, bool early, Choice* out) {
-  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | (slope ? 1 << 29 : 0) | (early ? 1 << 28 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
+int pick_config(int dev, int sms, int cap, int M, int N, int K, bool a_mn, bool b_mn, int shape, bool act, bool slope, bool early, Choice* out) {
+  const int key = (a_mn ? 1 : 0) | (b_mn ? 2 : 0) | (act ? 1 << 27 : 0) | (slope ? 1 << 29 : 0) | (early ? 1 << 28 : 0) | ((shape + 1) << 2) | (cap << 5) | (1 << 30);
   Remembered& e = remembered(M, N, K, 0, key);
   if (e.M != M || e.N != N || e.K != K || e.groups != 0 || e.key != key || e.dev != dev) {
     Capacity have = estimated_capacity(sms);
     const int rc = dev < 0 ? KB_OK : device_capacity(dev, sms, &have);
     if (rc != KB_OK) return rc;
     for (int i = 1; i < 9; ++i) have.clusters[i] = have.clusters[i] * i <= cap ? have.clusters[i] : cap / i;
-    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape, slope, early)};
+    e = {M, N, K, 0, key, dev, choose(M, N, K, a_mn, b_mn, have, shape, act, slope, early)};
   }
   *out = e.c;
   return KB_OK;
@@ -493,7 +498,7 @@ Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int sha
 
 extern "C" int kb_gemm_local_config(int M, int N, int K, int a_mn, int b_mn, int sms, int* pair, int* bn, int* split) {
   if (M <= 0 || N <= 0 || K <= 0 || sms < 2 || !pair || !bn || !split) return KB_ERR_ARG;
-  const Config c = choose_config(M, N, K, a_mn != 0, b_mn != 0, estimated_capacity(sms), -1);
+  const Config c = choose_config(M, N, K, a_mn != 0, b_mn != 0, estimated_capacity(sms), -1, false);
   *pair = c.tall ? 2 : c.pair ? 1 : 0;
   *bn = c.bn;
   *split = c.split;
@@ -551,7 +556,7 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
     pick = pick_rows(cap, expect, groups, a->N, a->K, l.b_mn, shape, a->pre_in != nullptr, a->early != 0);
   } else if (a->kind == KB_LOCAL_DENSE) {
     if (shape == 1 && a->M <= 128) shape = 0;  // a pair's second CTA would hold padding only
-    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->pre_in != nullptr, a->early != 0, &pick);
+    const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->act != ACT_NONE, a->pre_in != nullptr, a->early != 0, &pick);
     if (rc != KB_OK) return rc;
   } else {
     pick.c = contract_config(a->M, a->N, expect, groups, shape);
@@ -668,7 +673,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.slot_rows = ring.slot_rows;
   const int epi = a->pre_in != nullptr ? EPI_SLOPE : a->act != ACT_NONE ? EPI_ACT : EPI_PLAIN;
   auto wide = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0; };
-  p.wide = a->N % 16 == 0 && wide(a->out) && wide(a->pre_out) ? 1 : 0;
+  p.wide = a->N % 16 == 0 && wide(a->out) && wide(a->pre_out) && wide(a->pre_in) ? 1 : 0;
   p.act = a->act;
   p.bias = static_cast<const bf16*>(a->bias);
   p.bias_scale = a->bias_scale;

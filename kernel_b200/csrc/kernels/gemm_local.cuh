@@ -234,6 +234,20 @@ __device__ __forceinline__ void store_row32(bf16* base, size_t at, int col, int 
   }
 }
 
+// Saved values of 32 columns from `c` on of a tile's row; `last`: columns that exist.
+__device__ __forceinline__ void fetch32(const Params& p, const bf16* row, int c, int last, uint4* at) {
+  if (p.wide && c + 32 <= last) {
+    kb::ld_stream_v8(row + c, at[0], at[1]);
+    kb::ld_stream_v8(row + c + 16, at[2], at[3]);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    at[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (c + 8 * i < last) at[i] = kb::ld_stream_v4(row + c + 8 * i);
+  }
+}
+
 // Shared-memory descriptor of an M/N-contiguous operand with the 128-byte swizzle:
 // blocks of 64 elements x 64 k rows (one TMA box, 8 KB), next block MN_BLOCK_BYTES
 // further (leading offset), next eight k rows 1024 bytes further (stride offset).
@@ -563,6 +577,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     int box_no = 0;  // contract: staging boxes used by this warp
     for (int pos = sched_id; pos < total_tiles; pos += sched_n, ++it) {
       const Tile t = tile_at(pos);
+      if constexpr (kEpi == EPI_SLOPE) {
+        // The tile's saved values are on their way from memory while its products are made: a lane's row of it, 64 columns in turn
+        // as below.
+        for (int hb = 0; hb < kHalves; ++hb) {
+          const int row = t.row0 + hb * BM + q * 32 + lane;
+          for (int c = turn * 64; c < p.bn && row < t.row_end && t.n0 + c < p.N; c += 128) {
+            kb::prefetch_l2(p.pre_in + static_cast<size_t>(row) * p.N + t.n0 + c, min(64, p.N - t.n0 - c) * 2);
+          }
+        }
+      }
       if (p.bias != nullptr) {
         // brings the tile's bias into L1 while the accumulator is not ready yet: eight values per lane
         const int col = t.n0 + 8 * lane;
@@ -596,6 +620,33 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
         };
         const int last = gr0 < t.row_end ? cols : 0;
         if (turn * 64 >= last) release();
+        if constexpr (kEpi == EPI_SLOPE) {
+          // 32 columns at a time, the saved values one step ahead.
+          uint4 at[4], next[4];
+          const bf16* saved = p.pre_in + static_cast<size_t>(row) * p.N + t.n0;
+          const int mine = row_ok ? last : 0;
+          fetch32(p, saved, turn * 64, mine, at);
+#pragma unroll 1
+          for (int s = 0; s < 4; ++s) {  // columns turn * 64 + 0, 32, 128, 160
+            const int c = turn * 64 + (s >> 1) * 128 + (s & 1) * 32;
+            if (c >= last) break;
+            const int c1 = c + ((s & 1) ? 96 : 32);
+            if (s < 3) fetch32(p, saved, c1, mine, next);
+            uint32_t r[32];
+            kb::tmem_ld_32x32(taddr + c, r);
+            kb::tmem_ld_wait();
+            if (s == 3 || c1 >= last) release();
+            float f[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[i]);
+            uint4 o[4], pre[4];
+            finish32<kEpi>(p, f, t.n0 + c, at, o, pre);
+            if (row_ok) store_row32(p.out, static_cast<size_t>(row) * p.N + t.n0 + c, t.n0 + c, p.N, p.wide != 0, o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) at[i] = next[i];
+          }
+          continue;
+        }
         if constexpr (kKind == CONTRACT) {
           // Few k blocks per tile: the output is the traffic.  Staged boxes leave as whole
           // 128-byte lines while the epilogue goes on (rows and columns outside the tensor are
@@ -638,14 +689,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
           const bool two = c + 32 < last;
           const int col = t.n0 + c;
           const size_t at0 = static_cast<size_t>(row) * p.N + col;
-          uint4 at[8];
-          if constexpr (kEpi == EPI_SLOPE) {  // fetched before the accumulator is read
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              at[i] = make_uint4(0u, 0u, 0u, 0u);
-              if (row_ok && c + 8 * i < last) at[i] = kb::ld_stream_v4(p.pre_in + at0 + 8 * i);
-            }
-          }
           uint32_t r[2][32];
           kb::tmem_ld_32x32(taddr + c, r[0]);
           if (two) kb::tmem_ld_32x32(taddr + c + 32, r[1]);
@@ -658,7 +701,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[h][i]);
             uint4 o[4], pre[4];
-            finish32<kEpi>(p, f, col + 32 * h, at + 4 * h, o, pre);
+            finish32<kEpi>(p, f, col + 32 * h, nullptr, o, pre);
             if (row_ok) {
               store_row32(p.out, at0 + 32 * h, col + 32 * h, p.N, p.wide != 0, o);
               if constexpr (kEpi == EPI_ACT) {
