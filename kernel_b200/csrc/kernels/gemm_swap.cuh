@@ -462,6 +462,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
         const int vcol = q * 32 + (lane & ~3);  // first of the four columns this lane stores
         const bool col_ok = vcol < w_cols && col0 + vcol < p.N;
         const bool live = q * 32 < w_cols && col0 + q * 32 < p.N;
+        const int last = live ? t.rows : 0;
+        uint2 saved[8];
+        if constexpr (kEpi == EPI_SLOPE) {
+          // The saved values are on their way while the tile's products are made: a token per thread into the L2, this warp's first
+          // tokens into registers.  Fetched when the accumulator was ready they took the last tile's epilogue 8 us.
+          const int token = (warp - 4) * 32 + lane;
+          if (token < t.rows && col0 < p.N) {
+            kb::prefetch_l2(p.pre_in + static_cast<size_t>(t.row0 + token) * p.N + col0, static_cast<uint32_t>(min(w_cols, p.N - col0)) * 2);
+          }
+          if (turn * 32 < last) fetch_saved<16>(p, static_cast<size_t>(t.row0 + turn * 32) * p.N + col0 + vcol, t.rows - turn * 32, col_ok, lane, saved);
+        }
         if (*abort_flag == 0 && !kb::mbar_wait_bounded(&tfull[acc], (it >> 1) & 1u, p.limit_ns, 2000)) {
           kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, kbl::SITE_TFULL, (uint32_t)pos, 0);
           *abort_flag = 1;
@@ -480,13 +491,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
             }
           }
         };
-        const int last = live ? t.rows : 0;
         if (turn * 32 >= last) release();
 #pragma unroll 1
         for (int c = turn * 32; c < last; c += 64) {
           const size_t at = static_cast<size_t>(t.row0 + c) * p.N + col0 + vcol;
-          uint2 saved[8];
-          if constexpr (kEpi == EPI_SLOPE) fetch_saved<16>(p, at, t.rows - c, col_ok, lane, saved);
+          uint2 now[8];
+          if constexpr (kEpi == EPI_SLOPE) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) now[i] = saved[i];
+            if (c + 64 < last) fetch_saved<16>(p, at + static_cast<size_t>(64) * p.N, t.rows - c - 64, col_ok, lane, saved);
+          }
           uint32_t r[32];
           kb::tmem_ld_32x32(taddr + c, r);
           kb::tmem_ld_wait();
@@ -494,7 +508,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
           float f[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[i]);
-          finish<kEpi, 16>(p, f, bias, saved, at, t.rows - c, col_ok, lane);
+          finish<kEpi, 16>(p, f, bias, now, at, t.rows - c, col_ok, lane);
         }
       }
     } else if (warp == 4 && p.split > 1) {
