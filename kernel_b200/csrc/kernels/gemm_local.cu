@@ -677,6 +677,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   p.act = a->act;
   p.bias = static_cast<const bf16*>(a->bias);
   p.bias_scale = a->bias_scale;
+  p.w = prefetches(*a) ? static_cast<const bf16*>(a->B) : nullptr;
   p.out = static_cast<bf16*>(a->out);
   p.pre_out = static_cast<bf16*>(a->pre_out);
   p.pre_in = static_cast<const bf16*>(a->pre_in);

@@ -97,6 +97,7 @@ struct alignas(64) Params {
   int act;           // applied to the rounded result, or, with pre_in, its derivative at pre_in
   const bf16* bias;
   float bias_scale;
+  const bf16* w;       // the weights where the first of them may be prefetched, or null
   bf16* out;
   bf16* pre_out;       // value before the activation, or null
   const bf16* pre_in;  // saved value before the activation (backward), or null
@@ -261,6 +262,21 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
   return d;
 }
 
+// Weights on their way into the L2 before the previous launch has ended: the first k blocks of `cols` columns from `col` on,
+// by 256 threads.  Nothing is read by it, so it does not matter that someone may still write them.  `w`: [N][K] or (kMn) [K][N].
+constexpr int AHEAD = 12;  // k blocks, 30 MB on 148 SMs: with 6 half of the gain, with 20 and 32 no more
+template <bool kMn>
+__device__ __forceinline__ void prefetch_weights(const bf16* w, int N, int K, int col, int cols, int k0, int k1, int thread) {
+  const int k = k0 * BK, ks = min(min(k1 - k0, AHEAD) * BK, K - k);
+  const int cs = min(cols, N - col);
+  if (cs <= 0 || ks <= 0) return;
+  if constexpr (kMn) {
+    for (int i = thread; i < ks; i += 256) kb::prefetch_l2(w + static_cast<size_t>(k + i) * N + col, static_cast<uint32_t>(cs) * 2);
+  } else {
+    for (int i = thread; i < cs; i += 256) kb::prefetch_l2(w + static_cast<size_t>(col + i) * K + k, static_cast<uint32_t>(ks) * 2);
+  }
+}
+
 // kHalves: 128-row blocks per CTA and tile.  2 (pairs only): a 512-row tile whose two
 // halves fill both accumulators.
 template <Kind kKind, bool kPair, bool kAMn, bool kBMn, int kHalves, Epi kEpi>
@@ -298,79 +314,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
   // rows of one scheduling block: groups with few rows get low tiles (one CTA, 32 or 64 of the MMA's 128 rows)
   const int block_rows = (kKind == ROWS && !kPair) ? p.a_rows : TILE_ROWS;
   const int b_cols = kPair ? p.bn / 2 : p.bn;  // columns of B this CTA stages
-
-  if (warp == 0) {
-    if (lane < p.stages) {
-      kb::mbar_init(&full[lane], 1);
-      kb::mbar_init(&empty[lane], 1);
-    }
-    if (lane < 2) {
-      kb::mbar_init(&tfull[lane], 1);
-      kb::mbar_init(&tempty[lane], kPair ? 2 * EPI_WARPS : EPI_WARPS);
-    }
-    if (lane == 0) *abort_flag = 0;
-    kb::mbar_fence_init();
-    __syncwarp();
-  }
-  if (warp == 2) {
-    if constexpr (kPair) {
-      kb::tmem_alloc_pair(tmem_slot, TMEM_COLS);
-      kb::tmem_relinquish_pair();
-    } else {
-      kb::tmem_alloc(tmem_slot, TMEM_COLS);
-      kb::tmem_relinquish();
-    }
-  }
-  if (warp == 3 && lane == 0) {
-    kb::tma_prefetch_desc(&p.tmA);
-    kb::tma_prefetch_desc(&p.tmB);
-  }
-  kb::wait_for_previous_launch();  // barriers, tensor memory and descriptors are set up under the end of that one
-  const uint64_t t_start = p.timing ? kb::globaltimer_ns() : 0;  // the product's own time
-  if constexpr (kKind != DENSE) {
-    for (int e = tid; e < p.groups; e += THREADS) {
-      g_start[e] = p.row_start[e];
-      g_count[e] = p.row_count[e];
-    }
-    if constexpr (kKind == ROWS) {
-      __syncthreads();
-      if (warp == 0) {  // exclusive prefix of the groups' row blocks
-        int carry = 0;
-        for (int e0 = 0; e0 < p.groups; e0 += 32) {
-          const int e = e0 + lane;
-          int v = e < p.groups ? (g_count[e] + block_rows - 1) / block_rows : 0;
-          const int mine = v;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int n = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += n;
-          }
-          if (e < p.groups) pref[e] = carry + v - mine;
-          carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) pref[p.groups] = carry;
-      }
-    }
-  }
-  // A pair's CTAs signal each other's barriers: both must have initialised theirs.
-  // Otherwise the producer warp, which needs only the barriers it has just made,
-  // goes ahead: its first loads are under way while the tensor memory is allocated.
-  if constexpr (kPair) {
-    kb::tc_fence_before_sync();
-    __syncthreads();
-    kb::cluster_sync_all();
-    kb::tc_fence_after_sync();
-  } else if (kKind == DENSE && warp == 0) {
-    asm volatile("bar.arrive 1, %0;" ::"n"(THREADS) : "memory");
-  } else {
-    kb::tc_fence_before_sync();
-    if constexpr (kKind == DENSE) asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
-    else __syncthreads();
-    kb::tc_fence_after_sync();
-  }
-  const uint32_t tmem_base = (kPair || kKind != DENSE || warp != 0) ? *tmem_slot : 0u;
-
-  const int total_tiles = kKind == DENSE ? p.MBQ * p.NB : kKind == ROWS ? pref[p.groups] * p.NB : p.groups * p.MBQ * p.NB;
 
   // Position in the static schedule -> tile.  Dense: groups of `group` row blocks
   // are swept column by column, so that the tiles in flight share few panels of A
@@ -428,6 +371,85 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       k1 = static_cast<int>(static_cast<uint32_t>(t.kb * (member + 1)) / static_cast<uint32_t>(p.split));
     }
   };
+
+  if (warp == 0) {
+    if (lane < p.stages) {
+      kb::mbar_init(&full[lane], 1);
+      kb::mbar_init(&empty[lane], 1);
+    }
+    if (lane < 2) {
+      kb::mbar_init(&tfull[lane], 1);
+      kb::mbar_init(&tempty[lane], kPair ? 2 * EPI_WARPS : EPI_WARPS);
+    }
+    if (lane == 0) *abort_flag = 0;
+    kb::mbar_fence_init();
+    __syncwarp();
+  }
+  if (warp == 2) {
+    if constexpr (kPair) {
+      kb::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+      kb::tmem_relinquish_pair();
+    } else {
+      kb::tmem_alloc(tmem_slot, TMEM_COLS);
+      kb::tmem_relinquish();
+    }
+  }
+  if (warp == 3 && lane == 0) {
+    kb::tma_prefetch_desc(&p.tmA);
+    kb::tma_prefetch_desc(&p.tmB);
+  }
+  if (kKind == DENSE && !kAMn && warp >= 4 && p.w != nullptr) {
+    const Tile t = tile_at(sched_id);
+    int k0, k1;
+    k_range(t, k0, k1);
+    prefetch_weights<kBMn>(p.w, p.N, p.K, t.n0 + static_cast<int>(half) * b_cols, b_cols, k0, k1, tid - 128);
+  }
+  kb::wait_for_previous_launch();  // barriers, tensor memory and descriptors are set up under the end of that one
+  const uint64_t t_start = p.timing ? kb::globaltimer_ns() : 0;  // the product's own time
+  if constexpr (kKind != DENSE) {
+    for (int e = tid; e < p.groups; e += THREADS) {
+      g_start[e] = p.row_start[e];
+      g_count[e] = p.row_count[e];
+    }
+    if constexpr (kKind == ROWS) {
+      __syncthreads();
+      if (warp == 0) {  // exclusive prefix of the groups' row blocks
+        int carry = 0;
+        for (int e0 = 0; e0 < p.groups; e0 += 32) {
+          const int e = e0 + lane;
+          int v = e < p.groups ? (g_count[e] + block_rows - 1) / block_rows : 0;
+          const int mine = v;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += n;
+          }
+          if (e < p.groups) pref[e] = carry + v - mine;
+          carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) pref[p.groups] = carry;
+      }
+    }
+  }
+  // A pair's CTAs signal each other's barriers: both must have initialised theirs.
+  // Otherwise the producer warp, which needs only the barriers it has just made,
+  // goes ahead: its first loads are under way while the tensor memory is allocated.
+  if constexpr (kPair) {
+    kb::tc_fence_before_sync();
+    __syncthreads();
+    kb::cluster_sync_all();
+    kb::tc_fence_after_sync();
+  } else if (kKind == DENSE && warp == 0) {
+    asm volatile("bar.arrive 1, %0;" ::"n"(THREADS) : "memory");
+  } else {
+    kb::tc_fence_before_sync();
+    if constexpr (kKind == DENSE) asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    else __syncthreads();
+    kb::tc_fence_after_sync();
+  }
+  const uint32_t tmem_base = (kPair || kKind != DENSE || warp != 0) ? *tmem_slot : 0u;
+
+  const int total_tiles = kKind == DENSE ? p.MBQ * p.NB : kKind == ROWS ? pref[p.groups] * p.NB : p.groups * p.MBQ * p.NB;
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer ----

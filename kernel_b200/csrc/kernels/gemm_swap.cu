@@ -99,6 +99,7 @@ int launch(const KbLocalGemmArgs& a, const Config& c, int dev, int cap, bool tim
   p.early = a.early != 0 ? 1 : 0;
   p.bias = static_cast<const bf16*>(a.bias);
   p.bias_scale = a.bias_scale;
+  p.w = kbl::prefetches(a) ? static_cast<const bf16*>(a.B) : nullptr;
   p.out = static_cast<bf16*>(a.out);
   p.pre_out = static_cast<bf16*>(a.pre_out);
   p.pre_in = static_cast<const bf16*>(a.pre_in);

@@ -57,6 +57,7 @@ struct alignas(64) Params {
   int early;
   const bf16* bias;
   float bias_scale;
+  const bf16* w;       // the weights where the first of them may be prefetched, or null
   bf16* out;
   bf16* pre_out;
   const bf16* pre_in;
@@ -213,6 +214,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
   constexpr int STEP = kPair ? 32 : 16;        // MMA columns come in multiples of this
   const int w_cols = kPair ? p.bn / 2 : p.bn;  // output columns of this CTA
 
+  int k0 = 0, k1 = p.KB;  // this member's part (32 bits: at most 2^25 k blocks, eight members)
+  if (kKind == DENSE && p.split > 1) {
+    k0 = static_cast<int>(static_cast<uint32_t>(p.KB * member) / static_cast<uint32_t>(p.split));
+    k1 = static_cast<int>(static_cast<uint32_t>(p.KB * (member + 1)) / static_cast<uint32_t>(p.split));
+  }
   if (warp == 0) {
     if (lane < p.stages) {
       kb::mbar_init(&full[lane], 1);
@@ -238,6 +244,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
   if (warp == 3 && lane == 0) {
     kb::tma_prefetch_desc(&p.tmW);
     kb::tma_prefetch_desc(&p.tmX);
+  }
+  if (kKind == DENSE && warp >= 4 && p.w != nullptr) {
+    kbl::prefetch_weights<kWMn>(p.w, p.N, p.K, p.per.of(sched_id) * p.bn + static_cast<int>(half) * w_cols, w_cols, k0, k1, tid - 128);
   }
   if (!p.early) kb::wait_for_previous_launch();
   uint64_t t_start = p.timing ? kb::globaltimer_ns() : 0;  // the product's own time
@@ -303,11 +312,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
     t.cols = (t.rows + STEP - 1) / STEP * STEP;
     return t;
   };
-  int k0 = 0, k1 = p.KB;  // this member's part (32 bits: at most 2^25 k blocks, eight members)
-  if (kKind == DENSE && p.split > 1) {
-    k0 = static_cast<int>(static_cast<uint32_t>(p.KB * member) / static_cast<uint32_t>(p.split));
-    k1 = static_cast<int>(static_cast<uint32_t>(p.KB * (member + 1)) / static_cast<uint32_t>(p.split));
-  }
   auto boxes_of = [&](const Tile& t) { return ((kPair ? t.cols >> 1 : t.cols) + p.xbox - 1) / p.xbox; };
 
   if (warp == 0) {
