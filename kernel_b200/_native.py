@@ -97,6 +97,21 @@ class LocalGemmArgs(C.Structure):
     ]
 
 
+class GemmStreamArgs(C.Structure):
+    _fields_ = [
+        ("product", LocalGemmArgs),
+        ("a_host", C.c_void_p),
+        ("out_host", C.c_void_p),
+        ("pieces", C.c_int),
+        ("rows", C.c_void_p),
+        ("again", C.c_int),
+        ("stream", C.c_void_p),
+        ("inward", C.c_void_p),
+        ("outward", C.c_void_p),
+        ("events", C.c_void_p),
+    ]
+
+
 class LocalPick(C.Structure):
     _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split", "overlapped")]
 
@@ -164,6 +179,12 @@ def _declare(lib: C.CDLL) -> None:
         "kb_device_barrier": (i, [C.POINTER(vp), u64, i, i, u32, u64, vp, vp]),
         "kb_gemm": (i, [C.POINTER(GemmArgs), vp]),
         "kb_gemm_local": (i, [C.POINTER(LocalGemmArgs), vp]),
+        "kb_gemm_stream_events": (i, [i]),
+        "kb_events_create": (i, [i, C.POINTER(vp)]),
+        "kb_events_destroy": (i, [i, C.POINTER(vp)]),
+        "kb_gemm_stream_begin": (i, [C.POINTER(GemmStreamArgs)]),
+        "kb_gemm_stream_run": (i, [C.POINTER(GemmStreamArgs)]),
+        "kb_gemm_stream_end": (i, [C.POINTER(GemmStreamArgs)]),
         "kb_a2a_local_vecs": (i, [i, i, i, i]),
         "kb_gemm_local_pick": (i, [C.POINTER(LocalGemmArgs), i, C.POINTER(LocalPick)]),
         "kb_gemm_local_config": (i, [i, i, i, i, i, i, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),

@@ -151,6 +151,25 @@ typedef struct KbLocalGemmArgs {
   int early;            // the weights and the row table were written before the previous launch of the stream began
 } KbLocalGemmArgs;
 int kb_gemm_local(const KbLocalGemmArgs* args, void* stream);
+// A dense product of rows in (pinned) host memory, its result there too (kernels/gemm_stream.cu).  The copy of the first piece's
+// rows, between _begin and _run on stream `in`, and that of the last piece's result, between _run and _end on stream `out`, are
+// the caller's: so its allocator of pinned memory learns which streams use the buffers.
+typedef struct KbGemmStreamArgs {
+  KbLocalGemmArgs product;  // A, out: device buffers of all M rows
+  const void* a_host;       // bf16 [M,K]
+  void* out_host;           // bf16 [M,N]
+  int pieces;
+  const int32_t* rows;      // host [pieces]: together M
+  int again;                // 0 for a first call, then kept by _end: the events have been through a call
+  void *stream, *in, *out;  // the caller's stream; both others are its own
+  void** events;            // kb_gemm_stream_events(pieces) of kb_events_create
+} KbGemmStreamArgs;
+int kb_gemm_stream_events(int pieces);
+int kb_events_create(int n, void** events);
+int kb_events_destroy(int n, void** events);
+int kb_gemm_stream_begin(const KbGemmStreamArgs* args);
+int kb_gemm_stream_run(const KbGemmStreamArgs* args);
+int kb_gemm_stream_end(KbGemmStreamArgs* args);
 // The tile kb_gemm_local launches for these arguments on a B200 with `sms` SMs (tests of the rules; no pointer is read).
 // KB_ERR_UNSUPPORTED: one the kernel cannot run was asked for.
 typedef struct KbLocalPick {

@@ -170,6 +170,104 @@ class _HostPipeline:
             self.cur.wait_stream(self.d2h)
 
 
+def _pieces(M: int, Nn: int, K: int, most: int) -> list:
+    """Rows of the pieces of a product on one GPU whose rows come from the host: the fewest microseconds by a model of the three
+    stages (53 GB/s each way and 10 for every copy; a product reads its weights at 5.5 TB/s or makes 1200 TFLOP/s) and of
+    the host, which takes 30 for a call and 11 for a piece.  Beside a direction that is by far the longer one sizes fall (way in)
+    or rise (way out) by a constant ratio, so that little of the other one is exposed: 8192 x 8192 x 1024 2565 us in
+    four equal pieces, 2511 in these; 4096 x 1024 x 8192 1312 and 1270.  Where both directions are busy most of the time they slow
+    each other down and unequal pieces gain nothing (2048 x 4096 x 7168: 692 and 719; two, eight and sixteen equal ones 756, 735
+    and 862).  Whole tiles of 64 rows."""
+    best, rows = None, [M]
+    blocks = -(-M // 64)
+    ratios = (1.0,) if 5 * K < 12 * Nn and 5 * Nn < 12 * K else (1.0, 0.8, 0.65, 0.5, 0.4, 0.3) if K > Nn else (1.0, 1.25, 1.5, 2.0, 2.5, 3.3)
+    for n in range(1, min(most, blocks) + 1):
+        for ratio in ratios if n > 1 else (1.0,):
+            share = [ratio ** i for i in range(n)]
+            cut = [round(blocks * sum(share[:i]) / sum(share)) * 64 for i in range(n)] + [M]
+            r = [b - a for a, b in zip(cut, cut[1:])]
+            if min(r) <= 0:
+                continue
+            there = made = back = 0.0
+            for m in r:
+                there += 2 * m * K / 53e3 + 10
+                made = max(made, there) + max(2 * m * Nn * K / 1.2e9, 2 * Nn * K / 5.5e6) + 4
+                back = max(back, made) + 2 * m * Nn / 53e3 + 10
+            t = max(back, 30 + 11 * n)
+            if best is None or t < best:
+                best, rows = t, r
+    return rows
+
+
+class _OneGpuStream:
+    """Device buffers, side streams and events of ``run_from_host`` on one GPU (``csrc/kernels/gemm_stream.cu``)."""
+
+    def __init__(self, device: torch.device, M: int, Nn: int, K: int, chunks: int, status: torch.Tensor):
+        self.rows = _pieces(M, Nn, K, max(1, min(chunks, 64)))
+        self.inp = torch.empty((M, K), dtype=torch.bfloat16, device=device)
+        self.out = torch.empty((M, Nn), dtype=torch.bfloat16, device=device)
+        self.inward, self.outward = torch.cuda.Stream(device), torch.cuda.Stream(device)
+        self.inp.record_stream(self.inward)
+        self.out.record_stream(self.outward)
+        args = self.args = N.GemmStreamArgs()
+        args.product = _local_args(status)
+        args.product.M, args.product.N, args.product.K = M, Nn, K
+        args.product.A, args.product.out = self.inp.data_ptr(), self.out.data_ptr()
+        args.pieces = len(self.rows)
+        self.table = (C.c_int32 * args.pieces)(*self.rows)
+        args.rows = C.addressof(self.table)
+        args.inward, args.outward = self.inward.cuda_stream, self.outward.cuda_stream
+        self.count = N.lib().kb_gemm_stream_events(args.pieces)
+        self.events = (C.c_void_p * self.count)()
+        self.destroy = N.lib().kb_events_destroy  # at hand when the interpreter has let go of the module
+        N.check(N.lib().kb_events_create(self.count, self.events))
+        args.events = C.addressof(self.events)
+
+    def run(self, a_host: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], bias_scale: float, out_host: torch.Tensor) -> None:
+        global launch_count
+        lib, args, index = N.lib(), self.args, w.device.index
+        args.product.B, args.product.bias, args.product.bias_scale = w.data_ptr(), bias.data_ptr() if bias is not None else None, bias_scale
+        args.a_host, args.out_host = a_host.data_ptr(), out_host.data_ptr()
+        args.stream = torch._C._cuda_getCurrentRawStream(index)
+        rows, last = self.rows[0], a_host.shape[0] - self.rows[-1]
+        N.check(lib.kb_gemm_stream_begin(C.byref(args)))
+        # torch's copies make its allocator of pinned memory wait for the side streams before it hands out a buffer again
+        self._copy(self.inward, index, self.inp[:rows], a_host[:rows])
+        N.check(lib.kb_gemm_stream_run(C.byref(args)))
+        self._copy(self.outward, index, out_host[last:], self.out[last:])
+        N.check(lib.kb_gemm_stream_end(C.byref(args)))
+        launch_count += args.pieces
+
+    @staticmethod
+    def _copy(stream: torch.cuda.Stream, index: int, dst: torch.Tensor, src: torch.Tensor) -> None:
+        """On ``stream``: what ``with torch.cuda.stream(stream)`` does on the current device, in a tenth of its time."""
+        current = torch._C._cuda_getCurrentStream(index)
+        torch._C._cuda_setStream(stream_id=stream.stream_id, device_index=stream.device_index, device_type=stream.device_type)
+        try:
+            dst.copy_(src, non_blocking=True)
+        finally:
+            torch._C._cuda_setStream(stream_id=current[0], device_index=current[1], device_type=current[2])
+
+    def __del__(self):
+        events, destroy = getattr(self, "events", None), getattr(self, "destroy", None)
+        if events is not None and destroy is not None:
+            destroy(self.count, events)
+
+
+def _from_host_on_one_gpu(ctx, a_host: torch.Tensor, w: torch.Tensor, bias, bias_scale: float, out_host: torch.Tensor, chunks: int) -> bool:
+    """``run_from_host`` where nothing is exchanged and the weights are on the current device; False elsewhere."""
+    if ctx.world != 1 or not ctx.native or not w.is_cuda or w.device.index != torch._C._cuda_getDevice():
+        return False
+    (M, K), Nn = a_host.shape, w.shape[0]
+    states = ctx.__dict__.setdefault("_one_gpu_streams", {})
+    st = states.get((chunks, Nn, K, w.device.index))
+    if st is None:
+        st = states[chunks, Nn, K, w.device.index] = _OneGpuStream(w.device, M, Nn, K, chunks, ctx.status)
+    st.run(a_host, w, bias, bias_scale, out_host)
+    ctx.epoch += 1
+    return True
+
+
 def _host_buffer(shape) -> torch.Tensor:
     t = torch.empty(shape, dtype=torch.bfloat16)
     return t.pin_memory() if torch.cuda.is_available() else t
@@ -178,7 +276,7 @@ def _host_buffer(shape) -> torch.Tensor:
 def _check_pinned(t: torch.Tensor, name: str, shape) -> None:
     if t.is_cuda or t.dtype != torch.bfloat16 or tuple(t.shape) != tuple(shape) or not t.is_contiguous():
         raise ValueError(f"{name} must be a contiguous bf16 host tensor of shape {tuple(shape)}")
-    if torch.cuda.is_available() and not t.is_pinned() and not os.environ.get("KB200_ALLOW_PAGEABLE"):
+    if not os.environ.get("KB200_ALLOW_PAGEABLE") and torch.cuda.is_available() and not t.is_pinned():
         raise ValueError(f"{name} must be in pinned host memory (tensor.pin_memory()), or the copies cannot overlap the kernel")
 
 
@@ -325,13 +423,14 @@ class GemmRS:
         of all owners forms a problem of ``M/chunks`` rows that runs through the
         same fused kernel, while piece i+1 is on its way in and the result of
         piece i-1 on its way out (one ``cudaMemcpyAsync`` per contiguous block), so
-        the PCIe transfers overlap the kernel instead of bracketing it.  Returns
+        the PCIe transfers overlap the kernel instead of bracketing it.  On one GPU, where
+        any rows can form a piece, there are at most ``chunks``, of the sizes that pay (``_pieces``).  Returns
         ``out_host``; the caller's stream is done when everything has arrived.
         Collective like ``__call__``.  The reference has no counterpart (its
         evaluator clones the inputs on the device inside its timed region,
         ``eval.py:358``)."""
         world, M, Nn = self.world, self.M, self.N
-        rows_rank = M // world
+        rows_rank, asked = M // world, chunks
         while chunks > 1 and (rows_rank % chunks or _rows_bad(rows_rank // chunks)):
             chunks -= 1
         rows = rows_rank // chunks
@@ -341,6 +440,12 @@ class GemmRS:
             out_host = _host_buffer((rows_rank, Nn))
         _check_pinned(out_host, "out_host", (rows_rank, Nn))
         dev = w.device
+        if world == 1 and dev.type == "cuda":
+            _check_bf16_2d(w, "w")
+            if w.shape[0] != Nn or w.shape[1] != K:
+                raise ValueError("shape does not match this GemmRS context")
+            if _from_host_on_one_gpu(self, a_host, w, bias, bias_scale, out_host, asked):
+                return out_host
         key = (chunks, K)
         st = self._stream_state.get(key) if hasattr(self, "_stream_state") else None
         if st is None:
@@ -371,6 +476,7 @@ class GemmRS:
             if sub is not self and sub.heap is not None:
                 sub.heap.close()
         self._stream_state = {}
+        self.__dict__.pop("_one_gpu_streams", None)
         if self.heap is not None:
             self.heap.close()
 
@@ -489,7 +595,7 @@ class AGGemm:
         piece i+1 coming in and of piece i-1's result going out (see
         ``GemmRS.run_from_host``).  Collective like ``__call__``."""
         world, M, K = self.world, self.M, self.K
-        rows_rank = M // world
+        rows_rank, asked = M // world, chunks
         while chunks > 1 and (rows_rank % chunks or _rows_bad(rows_rank // chunks)):
             chunks -= 1
         rows = rows_rank // chunks
@@ -499,6 +605,12 @@ class AGGemm:
             out_host = _host_buffer((M, Nl))
         _check_pinned(out_host, "out_host", (M, Nl))
         dev = w.device
+        if world == 1 and dev.type == "cuda":
+            _check_bf16_2d(w, "w")
+            if w.shape[1] != K:
+                raise ValueError("shape does not match this AGGemm context")
+            if _from_host_on_one_gpu(self, a_host, w, bias, 1.0, out_host, asked):
+                return out_host
         key = (chunks, Nl)
         st = self._stream_state.get(key) if hasattr(self, "_stream_state") else None
         if st is None:
@@ -529,5 +641,6 @@ class AGGemm:
             if sub is not self and sub.heap is not None:
                 sub.heap.close()
         self._stream_state = {}
+        self.__dict__.pop("_one_gpu_streams", None)
         if self.heap is not None:
             self.heap.close()

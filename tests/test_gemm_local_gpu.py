@@ -503,6 +503,53 @@ def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mo
     ctx.heap.close()
 
 
+@pytest.mark.parametrize("M,N,K,chunks", [(2, 8, 8, 4), (64, 72, 136, 4), (300, 264, 1032, 1), (515, 128, 2048, 7), (1024, 2048, 136, 4), (4096, 72, 2048, 4)])
+def test_rows_from_the_host_in_pieces(M, N, K, chunks):
+    """Sizes for which the pieces are one, equal, falling and rising, call after call with other rows, and on another stream."""
+    from kernel_b200.ops.gemm import AGGemm, GemmRS
+
+    w, bias = _ints(N, K, seed=60), _ints(N, seed=61)
+    rs, ag = GemmRS(M, N, device=torch.device(DEV)), AGGemm(M, K, device=torch.device(DEV))
+    side = torch.cuda.Stream()
+    for i in range(4):
+        a = _ints(M, K, seed=62 + i)
+        want = a.float() @ w.float().t() + bias.float()
+        host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
+        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
+            rs.run_from_host(host, w, bias, out_host=out, chunks=chunks)
+            got = ag.run_from_host(host, w, bias, chunks=chunks)
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), want.to(torch.bfloat16)) and torch.equal(got.to(DEV), want.to(torch.bfloat16))
+    _clean(rs.status)
+    rs.close()
+    ag.close()
+
+
+def test_rows_from_the_host_in_a_graph():
+    from kernel_b200.ops.gemm import GemmRS
+
+    M, N, K = 512, 264, 520
+    w, a = _ints(N, K, seed=66), _ints(M, K, seed=67)
+    ctx = GemmRS(M, N, device=torch.device(DEV))
+    host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
+    want = (a.float() @ w.float().t()).to(torch.bfloat16)
+    ctx.run_from_host(host, w, out_host=out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.run_from_host(host, w, out_host=out)
+    for sign in (-1, 1):
+        host.neg_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), sign * want)
+        ctx.run_from_host(host.neg_(), w, out_host=out)   # between two replays, outside of the graph
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), -sign * want)
+        host.neg_()
+    ctx.close()
+
+
 def test_a_product_is_the_first_cuda_call_of_its_thread():
     """As in an autograd worker whose memory comes from the allocator's cache: no runtime call has bound a context."""
     import threading

@@ -47,3 +47,36 @@ def test_gemm_rs_streamed_equals_whole(world, M, chunks):
 def test_ag_gemm_streamed_equals_whole(world, M, chunks):
     for same, _, shape in run_ranks(_ag, world, M, 136, 72, chunks):
         assert same and shape == (M, 136)
+
+
+def test_pieces_are_the_rows():
+    from kernel_b200.ops.gemm import _pieces
+
+    for M, N, K in [(1, 8, 8), (63, 8, 8192), (64, 4096, 4096), (65, 8192, 1024), (2047, 1024, 8192), (8192, 8192, 8192), (16384, 1024, 1024)]:
+        for most in (1, 2, 4, 7, 64):
+            rows = _pieces(M, N, K, most)
+            assert sum(rows) == M and min(rows) > 0 and len(rows) <= most
+            assert all(r % 64 == 0 for r in rows[:-1])
+    assert len(_pieces(256, 1024, 1024, 4)) == 1 and _pieces(2048, 4096, 7168, 4) == [512] * 4
+    assert _pieces(8192, 8192, 1024, 4) == sorted(_pieces(8192, 8192, 1024, 4)) and _pieces(4096, 1024, 8192, 4)[0] > 2048
+
+
+def test_stream_arguments_are_checked():
+    """Before anything is asked of the device."""
+    import ctypes as C
+
+    from kernel_b200 import _native as N
+
+    def code(rows, M=128, **kw):
+        table = (C.c_int32 * max(1, len(rows)))(*rows)
+        events = (C.c_void_p * 64)()
+        a = N.GemmStreamArgs()
+        a.product.M, a.product.N, a.product.K = M, 8, 8
+        a.pieces, a.rows, a.events, a.a_host, a.out_host = len(rows), C.addressof(table), C.addressof(events), 16, 16
+        for k, v in kw.items():
+            setattr(a, k, v)
+        return N.lib().kb_gemm_stream_run(C.byref(a))
+
+    for bad in (dict(rows=[]), dict(rows=[64, 63]), dict(rows=[128, 0]), dict(rows=[192, -64]), dict(rows=[2] * 65, M=130), dict(rows=[128], a_host=None),
+                dict(rows=[128], out_host=None), dict(rows=[128], events=None)):
+        assert code(**bad) == N.KB_ERR_ARG, bad
