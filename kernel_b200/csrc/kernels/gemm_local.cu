@@ -192,12 +192,12 @@ Config rows_plain_config(int M, int groups, int N, int K, bool b_mn, int sms, in
   return best;
 }
 
-// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 (190 for a pair) for
-// each box of the tokens, however narrow the tile.
+// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 (a pair's, whose boxes
+// mostly go by twos, 130) for each box of the tokens, however narrow the tile.
 double swap_k_block(bool pair, int w_cols, int tok, bool w_mn, int boxes) {
   const double mma = 300.0 * tok / 256.0 * (pair ? 1.0 : 1.33);
   const double load = 128.0 * (w_cols + (pair ? tok / 2 : tok)) / 95.0 * (w_mn ? 1.07 : 1.0);
-  const double issue = boxes * (pair ? 190.0 : 170.0);
+  const double issue = boxes * (pair ? 130.0 : 170.0);
   const double t = mma > load ? mma : load;
   return t > issue ? t : issue;
 }
@@ -273,7 +273,7 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
         // pairs, take 15.9 us on the M side and 20.7 here.
         const int block = cols < tok ? cols : tok;
         auto cost_of = [&](int boxes) {
-          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 1000.0 : 0.0);
+          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 2000.0 : 0.0);
           return t > memory ? t + 0.1 * memory : memory + 0.1 * t;
         };
         const double cost = cost_of(1);
@@ -483,11 +483,11 @@ Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int sha
     //   rows per group, [N, K]        3, [1024, 2048]   3, [760, 2728]   128, [1024, 2048]   250, [4096, 4096]   717, [544, 3008]
     //   forward with activation          47.6  45.5        99.5  89.4       75.3  67.7          98.5 101           25.3  26.7
     //   slope                            56.6  56.0         145   144       90.8  75.4           116  94.4         36.5  31.5
-    // Limits from 3100 products of uniformly routed rows in bursts (8 to 128 groups of 0.1 to 1600 rows, N and K 512 to 4096) and 330
-    // near ties repeated at the power cap: those take 3.1 % more than the better kind on average (always the M side 9.5 %,
-    // always exchanged 1.9 %) and 14 are more than 2 % slower than on the M side (26 with 0.97 and 0.85 before the
-    // boxes were counted; 39 always exchanged).
-    const double limit = slope ? 1.25 : rows >= 192ll * groups ? 0.9 : rows >= 32ll * groups ? 0.99 : 0.97;
+    // Limits, the time per box and a pair's 2000 ns fitted to 560 products in bursts (8 to 128 groups of 1 to 900 rows, Poisson
+    // counts, N and K 512 to 4096), after boxes came by twos and pairs handed their accumulators on without a fence: forward
+    // with activation, plain and slope take 1.4, 1.6 and 2.0 % more than the best tile of both kinds on average (before the fit 5.7, 3.6
+    // and 3.0; always exchanged 1.3, 1.9 and 1.4, always the M side 9.5, 4.5 and 17), 84 of 558 more than 3 % (179).
+    const double limit = slope ? 1.14 : rows >= 192ll * groups ? 1.02 : rows >= 32ll * groups ? 0.99 : 1.25;
     r.swap = other - (early ? EARLY : 0.0) < limit * plain;
     e = {rows, N, K, groups, key, 0, r};
   }
