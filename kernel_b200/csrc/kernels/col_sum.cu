@@ -3,8 +3,9 @@
 // Bound by memory: x is read once, 16 bytes per thread, 512 contiguous bytes per warp.
 // A CTA takes 256 columns and a contiguous range of rows; with several row ranges a
 // second, small launch adds their fp32 partials in ascending order, so the result does
-// not depend on timing.  8192 x 29568: 112 us (4.3 TB/s) with the second launch, against 804 us for a
-// cast to fp32, a library reduction and a cast back; 8192 x 8192 26.7 and 244, 256 x 4096 8.6 and 20.
+// not depend on timing.  8192 x 29568: 74 us (6.6 TB/s) with the second launch, against 804 us for a
+// cast to fp32, a library reduction and a cast back; 8192 x 8192 23 and 244.
+// One wave of the CTAs that fit: with eight CTAs asked for per SM, of which four fit, the last wave was mostly empty (116 and 28 us).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -17,10 +18,12 @@ namespace {
 constexpr int COLS = 256;   // columns of a CTA: 32 lanes x 8
 constexpr int WARPS = 8;
 constexpr int UNROLL = 8;   // rows in flight per warp
+constexpr int CTAS = 4;     // resident per SM
 
-__global__ void __launch_bounds__(32 * WARPS) col_sum_kernel(const __nv_bfloat16* __restrict__ x, int rows, int cols, int rows_per,
+__global__ void __launch_bounds__(32 * WARPS, CTAS) col_sum_kernel(const __nv_bfloat16* x, int rows, int cols, int rows_per,
                                                               float* partial, __nv_bfloat16* out) {
   __shared__ float s_sum[WARPS][COLS];
+  kb::wait_for_previous_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * COLS + lane * 8;
   const int r1 = min(rows, static_cast<int>(blockIdx.y + 1) * rows_per);
@@ -33,7 +36,7 @@ __global__ void __launch_bounds__(32 * WARPS) col_sum_kernel(const __nv_bfloat16
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
         const int row = r + u * WARPS;
-        v[u] = row < r1 ? kb::ld_nc_v4(x + static_cast<size_t>(row) * cols + c) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = row < r1 ? kb::ld_stream_v4(x + static_cast<size_t>(row) * cols + c) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
@@ -61,6 +64,7 @@ __global__ void __launch_bounds__(32 * WARPS) col_sum_kernel(const __nv_bfloat16
 }
 
 __global__ void __launch_bounds__(256) col_sum_finish_kernel(const float* partial, int parts, int cols, __nv_bfloat16* out) {
+  kb::wait_for_previous_launch();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= cols) return;
   float sum = 0.f;
@@ -70,10 +74,10 @@ __global__ void __launch_bounds__(256) col_sum_finish_kernel(const float* partia
 
 }  // namespace
 
-// Row ranges a matrix of this shape is cut into: about eight CTAs per SM, at least 64 rows each.
+// Row ranges a matrix of this shape is cut into, at least 64 rows each: as many CTAs as are resident on 148 SMs, in one wave.
 extern "C" int kb_col_sum_parts(int rows, int cols) {
   const int blocks = (cols + COLS - 1) / COLS;
-  int parts = (8 * 148 + blocks - 1) / blocks;
+  int parts = CTAS * 148 / blocks;
   if (parts > (rows + 63) / 64) parts = (rows + 63) / 64;
   return parts < 1 ? 1 : parts;
 }
@@ -83,7 +87,6 @@ extern "C" int kb_col_sum(const void* x, int rows, int cols, float* partial, voi
     kb::set_error("kb_col_sum: need rows > 0, columns a multiple of 8 and a 16-byte aligned matrix (got %d x %d)", rows, cols);
     return KB_ERR_ARG;
   }
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   const int parts = kb_col_sum_parts(rows, cols);
   if (parts > 1 && partial == nullptr) {
     kb::set_error("kb_col_sum: %d row ranges need a partial buffer", parts);
@@ -91,12 +94,11 @@ extern "C" int kb_col_sum(const void* x, int rows, int cols, float* partial, voi
   }
   const int rows_per = (rows + parts - 1) / parts;
   const dim3 grid((cols + COLS - 1) / COLS, parts);
-  col_sum_kernel<<<grid, 32 * WARPS, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, rows_per, parts > 1 ? partial : nullptr,
-                                                  static_cast<__nv_bfloat16*>(out));
-  KB_CUDA_OK(cudaGetLastError());
+  KB_CUDA_OK(kb::launch_after(col_sum_kernel, grid, 32 * WARPS, stream_v, static_cast<const __nv_bfloat16*>(x), rows, cols, rows_per,
+                              parts > 1 ? partial : nullptr, static_cast<__nv_bfloat16*>(out)));
   if (parts > 1) {
-    col_sum_finish_kernel<<<(cols + 255) / 256, 256, 0, stream>>>(partial, parts, cols, static_cast<__nv_bfloat16*>(out));
-    KB_CUDA_OK(cudaGetLastError());
+    KB_CUDA_OK(kb::launch_after(col_sum_finish_kernel, (cols + 255) / 256, 256, stream_v, static_cast<const float*>(partial), parts, cols,
+                                static_cast<__nv_bfloat16*>(out)));
   }
   return KB_OK;
 }
