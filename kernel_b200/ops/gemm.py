@@ -256,7 +256,7 @@ class _OneGpuStream:
 
 def _from_host_on_one_gpu(ctx, a_host: torch.Tensor, w: torch.Tensor, bias, bias_scale: float, out_host: torch.Tensor, chunks: int) -> bool:
     """``run_from_host`` where nothing is exchanged and the weights are on the current device; False elsewhere."""
-    if ctx.world != 1 or not ctx.native or not w.is_cuda or w.device.index != torch._C._cuda_getDevice():
+    if ctx.world != 1 or chunks < 1 or not ctx.native or not w.is_cuda or w.device.index != torch._C._cuda_getDevice():
         return False
     (M, K), Nn = a_host.shape, w.shape[0]
     states = ctx.__dict__.setdefault("_one_gpu_streams", {})
