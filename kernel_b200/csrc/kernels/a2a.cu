@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "../common/host_util.h"
 #include "../common/ptx.cuh"
 #include "../include/kb200.h"

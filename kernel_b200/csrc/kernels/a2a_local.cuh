@@ -10,7 +10,7 @@
 // in fp32 in ascending j with the rounding points of the general kernels (the expert's
 // output type, then the result's) and writes it once; outputs are equal to theirs value
 // for value.  Bound by memory (x in, out out) for many tokens, by the launch for few.
-// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 16.8 us, one token 12 -> 7 a call (1.5 us of GPU time).
+// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 15.6 us, one token 12 -> 7 a call (1.5 us of GPU time).
 //
 // The arithmetic is next to the memory time (8 experts x 16 instructions per 16-byte vector, 6.5 us of issue slots;
 // 9.0 us to read and write the rows at the copy rate), hence two values per instruction, in fp32 (f32x2) and for the
@@ -81,7 +81,12 @@ __device__ __forceinline__ uint32_t both_t2<__half>(float v) {
 template <typename T>
 __device__ __forceinline__ uint64_t widen_t2(uint32_t u);  // as a pair of fp32 values
 template <>
-__device__ __forceinline__ uint64_t widen_t2<__nv_bfloat16>(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ uint64_t widen_t2<__nv_bfloat16>(uint32_t u) {
+  // A byte permutation: a shift becomes a multiplication on the pipe that multiplies and adds already (16.6 -> 15.7 us).
+  uint32_t lo;
+  asm("prmt.b32 %0, %1, 0, 0x1044;" : "=r"(lo) : "r"(u));
+  return pack_f32x2(__uint_as_float(lo), __uint_as_float(u & 0xffff0000u));
+}
 template <>
 __device__ __forceinline__ uint64_t widen_t2<__half>(uint32_t u) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u));
@@ -100,6 +105,16 @@ __device__ __forceinline__ bool is_value_of(float v) {
 
 constexpr int LOCAL_WARPS = 4;  // of a CTA
 
+// What is known of the experts' scales before the launch: all are 1, all are values of T, nothing.  Each has a kernel of its own: with
+// the three loops in one, registers and schedule were those of the widest.  2048 tokens of 7168 bf16 values, top-8: scales of 1 13.2 -> 9.8
+// us (9.0 at the copy rate).
+enum Scales { UNIT, EXACT, ANY };
+// (e + 1) / E for all e: a power of two divides exactly, and e + 1 has the digits of T (8 of bf16, 11 of fp16)
+template <typename T>
+static bool exact_scales(int E) {
+  return (E & (E - 1)) == 0 && E <= (std::is_same<T, __half>::value ? 1024 : 256);
+}
+
 // What a warp needs of one (token, choice): the routing weight twice, as an operand of the two-value instructions, and the
 // expert's scale as fp32 and as a pair of T.
 struct alignas(16) LocalChoice {
@@ -114,7 +129,7 @@ struct alignas(16) LocalChoice {
 // form before this one), so nothing is done per choice that can be done per token: entries out of range are left out
 // of the list instead of being skipped in the loop, operands are stored the way the instructions want them, and
 // parts that stay the same need no division.
-template <typename T, int kVecs, int kCtas>
+template <typename T, int kVecs, int kCtas, Scales kScales>
 __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(const A2aParams p, int parts, int step) {
   __shared__ LocalChoice s_choice[LOCAL_WARPS][64];  // topk <= 64
   kb::wait_for_previous_launch();
@@ -157,7 +172,7 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
       const bool mine = lane + 32 * i < p.k;
       const bool valid = mine && e[i] >= 0 && e[i] < p.E;
       if (mine && !valid && part == 0) kb::report_status(p.status, KB_DEV_BAD_INDEX, SITE_DISP_IDX, (uint32_t)(t * p.k + lane + 32 * i), p.epoch);
-      const float scale = valid && p.scale_mode == 2 ? static_cast<float>(e[i] + 1) / static_cast<float>(p.E) : 1.0f;
+      const float scale = kScales != UNIT && valid ? static_cast<float>(e[i] + 1) / static_cast<float>(p.E) : 1.0f;
       const uint32_t all = __ballot_sync(0xffffffffu, valid);
       if (valid) {
         LocalChoice c;
@@ -171,8 +186,8 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
       }
       n += __popc(all);
     }
-    const bool rounds = __any_sync(0xffffffffu, differs);
-    const bool exact = !__any_sync(0xffffffffu, inexact);
+    const bool rounds = kScales == EXACT || (kScales == ANY && __any_sync(0xffffffffu, differs));
+    const bool exact = kScales == EXACT || (kScales == ANY && !__any_sync(0xffffffffu, inexact));
     constexpr int P = Vec16<T>::N / 2;
     uint64_t acc[kVecs][P];
 #pragma unroll
@@ -180,14 +195,14 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
 #pragma unroll
       for (int i = 0; i < P; ++i) acc[u][i] = 0ull;
     }
-    if (sizeof(T) == 2 && rounds && exact) {
-      if constexpr (sizeof(T) == 2) {
+    if (kScales != UNIT && sizeof(T) == 2 && rounds && exact) {
+      if constexpr (kScales != UNIT && sizeof(T) == 2) {
         uint32_t xin[kVecs][P];
 #pragma unroll
         for (int u = 0; u < kVecs; ++u) xin[u][0] = in[u].x, xin[u][1] = in[u].y, xin[u][2] = in[u].z, xin[u][3] = in[u].w;
         if (t + step < p.T) fetch(t + step);
         __syncwarp();
-#pragma unroll 2
+#pragma unroll 8
         for (int j = 0; j < n; ++j) {
           const LocalChoice c = choice[j];
           const uint64_t w2 = pack_f32x2(c.w0, c.w1);
@@ -198,7 +213,7 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
           }
         }
       }
-    } else {
+    } else if constexpr (kScales != EXACT) {
       uint64_t xin[kVecs][P];
 #pragma unroll
       for (int u = 0; u < kVecs; ++u) {
@@ -209,7 +224,7 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
       }
       if (t + step < p.T) fetch(t + step);
       __syncwarp();
-      if (rounds) {
+      if (kScales == ANY && rounds) {
 #pragma unroll 2
         for (int j = 0; j < n; ++j) {
           const LocalChoice c = choice[j];
@@ -244,11 +259,13 @@ __global__ void __launch_bounds__(32 * LOCAL_WARPS, kCtas) a2a_local_kernel(cons
   }
 }
 
-constexpr int LOCAL_CTAS[5] = {0, 8, 6, 0, 4};  // resident CTAs of an SM by vectors per lane
+// Resident CTAs of an SM by vectors per lane: what the registers allow.  fp32 rows have half the values per vector and need no widening:
+// five instead of four 21.7 -> 19.2 us with scales, 17.4 -> 15.7 without (2048 tokens of 7168, top-8 and top-6).
+constexpr int local_ctas(int vecs, int elem_bytes) { return vecs == 1 ? 8 : vecs == 2 ? 6 : elem_bytes == 4 ? 5 : 4; }
 
 template <typename T, int kVecs>
 static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
-  constexpr int kCtas = LOCAL_CTAS[kVecs];
+  constexpr int kCtas = local_ctas(kVecs, sizeof(T));
   const int parts = (p.vecs + 32 * kVecs - 1) / (32 * kVecs);
   const long long units = static_cast<long long>(p.T) * parts;
   if (units > 0x3fffffff) return KB_ERR_UNSUPPORTED;  // three launches of the general kernels
@@ -258,7 +275,11 @@ static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
   const long long at_once = resident < parts ? 1 : resident / parts;  // tokens
   const long long step = at_once < p.T ? at_once : p.T;
   const int grid = static_cast<int>((step * parts + LOCAL_WARPS - 1) / LOCAL_WARPS);
-  KB_CUDA_OK(kb::launch_after(a2a_local_kernel<T, kVecs, kCtas>, grid, 32 * LOCAL_WARPS, st, p, parts, static_cast<int>(step)));
+  auto* kernel = p.scale_mode == 2 ? a2a_local_kernel<T, kVecs, kCtas, ANY> : a2a_local_kernel<T, kVecs, kCtas, UNIT>;
+  if constexpr (sizeof(T) == 2) {
+    if (p.scale_mode == 2 && exact_scales<T>(p.E)) kernel = a2a_local_kernel<T, kVecs, kCtas, EXACT>;
+  }
+  KB_CUDA_OK(kb::launch_after(kernel, grid, 32 * LOCAL_WARPS, st, p, parts, static_cast<int>(step)));
   return KB_OK;
 }
 
@@ -267,6 +288,7 @@ static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
 // what the registers allow; back to back in a graph, three inputs in turn, 7168 values, us with 1 / 2 / 4 vectors:
 //   2048 tokens bf16, scales exact  24.0 19.9 16.8    unit scales 19.9 15.6 13.2    scales not bf16 values 28.6 25.4 21.5
 //   2048 tokens fp16                30.1 22.5 19.3    fp32 40.8 23.9 19.5           256 tokens bf16          4.6  4.2  3.8
+// (before each kind of scale had its own kernel; with four vectors now 15.6, 9.8, fp16 18.5)
 // In between a wide form may need a round of the resident warps more for a few tokens, leave most of a row's last warp idle
 // or fill the SMs unevenly, so 16-bit rows count the rounds and the CTAs of an SM (constants fitted): bf16, scales not bf16
 // values, 1 / 2 / 4 vectors
@@ -281,7 +303,7 @@ inline int local_vecs(int tokens, int vecs, int elem_bytes, int sms) {
   double best_cost = 1e30;
   for (int v = 1; v <= 4; v *= 2) {
     const int parts = (vecs + 32 * v - 1) / (32 * v);
-    const long long at_once = static_cast<long long>(sms) * LOCAL_CTAS[v] * LOCAL_WARPS / parts;  // tokens
+    const long long at_once = static_cast<long long>(sms) * local_ctas(v, elem_bytes) * LOCAL_WARPS / parts;  // tokens
     const long long step = at_once < 1 ? 1 : at_once < tokens ? at_once : tokens;
     const double per_sm = static_cast<double>(((step * parts + LOCAL_WARPS - 1) / LOCAL_WARPS + sms - 1) / sms);  // CTAs
     const double rounds = static_cast<double>((tokens + step - 1) / step) + 2.6 * tokens / step;

@@ -550,6 +550,34 @@ def test_rows_from_the_host_in_a_graph():
     ctx.close()
 
 
+@pytest.mark.parametrize("E", [256, 512, 100, 1024])  # bf16: exact scales, scales of more digits, no power of two; fp16: exact up to 1024
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("H,T,k", [(1032, 9, 1), (7168, 150, 8), (2056, 700, 3)])
+def test_round_trip_of_special_values_equals_the_general_kernels(E, dtype, H, T, k):
+    """Subnormal, infinite and undefined values, signed zeros, tokens whose scales are all 1: each kind of scale has a kernel of its own."""
+    from kernel_b200.ops.dispatch_combine import MoEAllToAll
+
+    g = torch.Generator(device=DEV).manual_seed(E + H)
+    ctx = MoEAllToAll(E, k, H, T, dtype=dtype, device=torch.device(DEV))
+    x = torch.randn((T, H), device=DEV, generator=g)
+    tiny, huge = torch.finfo(dtype).tiny, torch.finfo(dtype).max
+    special = torch.tensor([0.0, -0.0, tiny, -tiny, tiny / 2, tiny / 100, huge, -huge, float("inf"), float("-inf"), float("nan")], device=DEV)
+    x[:, ::7] = special[torch.randint(0, len(special), x[:, ::7].shape, device=DEV, generator=g)]
+    x = x.to(dtype)
+    idx = torch.rand((T, E), device=DEV, generator=g).argsort(1)[:, :k].to(torch.int32).contiguous()
+    idx[::3, 0] = E - 1   # scale 1 (and, for k = 1, nothing else)
+    w = torch.softmax(torch.randn((T, k), device=DEV, generator=g), -1)
+    for mode in (0, 2):
+        ctx.enable_trace(False)
+        out = ctx.dispatch_scale_combine(x, idx, w, mode)
+        ctx.enable_trace()
+        general = ctx.dispatch_scale_combine(x, idx, w, mode)
+        torch.cuda.synchronize()
+        ctx.heap.check_status()
+        assert torch.equal(out.isnan(), general.isnan()) and torch.equal(out.nan_to_num(), general.nan_to_num())
+    ctx.heap.close()
+
+
 def test_a_product_is_the_first_cuda_call_of_its_thread():
     """As in an autograd worker whose memory comes from the allocator's cache: no runtime call has bound a context."""
     import threading
