@@ -199,6 +199,11 @@ def _pieces(M: int, Nn: int, K: int, most: int) -> list:
     return rows
 
 
+# Rows and result of a `run_from_host` that one GPU holds whole.  Above it the buffers of two chunks of the general path: such a call
+# takes 80 ms on the link, beside which the 0.2 ms that the native calls save are nothing, and rows need not fit the GPU's memory.
+_WHOLE_ROWS_BYTES = 4 << 30
+
+
 class _OneGpuStream:
     """Device buffers, side streams and events of ``run_from_host`` on one GPU (``csrc/kernels/gemm_stream.cu``)."""
 
@@ -209,6 +214,7 @@ class _OneGpuStream:
         self.inward, self.outward = torch.cuda.Stream(device), torch.cuda.Stream(device)
         self.inp.record_stream(self.inward)
         self.out.record_stream(self.outward)
+        self.home = torch._C._cuda_getCurrentRawStream(device.index)
         args = self.args = N.GemmStreamArgs()
         args.product = _local_args(status)
         args.product.M, args.product.N, args.product.K = M, Nn, K
@@ -228,7 +234,11 @@ class _OneGpuStream:
         lib, args, index = N.lib(), self.args, w.device.index
         args.product.B, args.product.bias, args.product.bias_scale = w.data_ptr(), bias.data_ptr() if bias is not None else None, bias_scale
         args.a_host, args.out_host = a_host.data_ptr(), out_host.data_ptr()
-        args.stream = torch._C._cuda_getCurrentRawStream(index)
+        stream = args.stream = torch._C._cuda_getCurrentRawStream(index)
+        if stream != self.home:  # its products may still run when the buffers are freed
+            other = torch.cuda.current_stream(w.device)
+            self.inp.record_stream(other)
+            self.out.record_stream(other)
         rows, last = self.rows[0], a_host.shape[0] - self.rows[-1]
         N.check(lib.kb_gemm_stream_begin(C.byref(args)))
         # torch's copies make its allocator of pinned memory wait for the side streams before it hands out a buffer again
@@ -259,6 +269,8 @@ def _from_host_on_one_gpu(ctx, a_host: torch.Tensor, w: torch.Tensor, bias, bias
     if ctx.world != 1 or chunks < 1 or not ctx.native or not w.is_cuda or w.device.index != torch._C._cuda_getDevice():
         return False
     (M, K), Nn = a_host.shape, w.shape[0]
+    if 2 * M * (Nn + K) > _WHOLE_ROWS_BYTES:
+        return False
     states = ctx.__dict__.setdefault("_one_gpu_streams", {})
     st = states.get((chunks, Nn, K, w.device.index))
     if st is None:

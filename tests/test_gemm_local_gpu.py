@@ -525,6 +525,21 @@ def test_rows_from_the_host_in_pieces(M, N, K, chunks):
     ag.close()
 
 
+@pytest.mark.parametrize("above", [0, 1])  # the last size that is held whole and the first that is not
+def test_rows_from_the_host_that_are_too_many_to_hold(above, monkeypatch):
+    from kernel_b200.ops import gemm
+
+    M, N, K = 512, 264, 520
+    monkeypatch.setattr(gemm, "_WHOLE_ROWS_BYTES", 2 * M * (N + K) - above)
+    w, a = _ints(N, K, seed=68), _ints(M, K, seed=69)
+    want = (a.float() @ w.float().t()).to(torch.bfloat16)
+    for ctx in (gemm.GemmRS(M, N, device=torch.device(DEV)), gemm.AGGemm(M, K, device=torch.device(DEV))):
+        out = ctx.run_from_host(a.cpu().pin_memory(), w)
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), want) and ("_one_gpu_streams" in ctx.__dict__) == (not above)
+        ctx.close()
+
+
 def test_rows_from_the_host_in_a_graph():
     from kernel_b200.ops.gemm import GemmRS
 
