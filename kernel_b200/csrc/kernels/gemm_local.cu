@@ -192,17 +192,21 @@ Config rows_plain_config(int M, int groups, int N, int K, bool b_mn, int sms, in
   return best;
 }
 
-// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need 170 (a pair's, whose boxes
-// mostly go by twos, 130) for each box of the tokens, however narrow the tile.
-double swap_k_block(bool pair, int w_cols, int tok, bool w_mn, int boxes) {
+// Time of a k block of a tile with exchanged operands, ns: constants as above; the issuing warps need `box` for each box of the
+// tokens, however narrow the tile.
+double swap_k_block(bool pair, int w_cols, int tok, bool w_mn, int boxes, double box) {
   const double mma = 300.0 * tok / 256.0 * (pair ? 1.0 : 1.33);
   const double load = 128.0 * (w_cols + (pair ? tok / 2 : tok)) / 95.0 * (w_mn ? 1.07 : 1.0);
-  const double issue = boxes * (pair ? 130.0 : 170.0);
+  const double issue = boxes * box;
   const double t = mma > load ? mma : load;
   return t > issue ? t : issue;
 }
 
-// Dense product with exchanged operands: rows in blocks of at most 256, columns and split so that the tiles fill the chip.
+// Dense product with exchanged operands: rows in blocks of at most 256, columns and split so that the tiles fill the chip.  The rows of
+// a stage are one box, 170 ns in one CTA, 190 in a pair.  With the 130 of grouped rows' boxes, which a pair issues by twos, a quarter
+// of the products of at most 64 rows gets another tile; repeated, of 60 of them (and of 50, weights along N) 25 (29) take more than 3 %
+// longer, 8 (4) less:
+//   1 x 23464 x 1504 14.7 us, pairs 16.4    7 x 9592 x 7560 31.0 and 34.3    weights along N: 23 x 25792 x 7536 67.8 and 77.9
 double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shape, kbs::Config* best) {
   double best_t = 1e30;
   const int KB = ceil_div(K, BK), mb = ceil_div(M, 256);
@@ -215,7 +219,7 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
     for (int w_cols = w_mn ? 64 : 32; w_cols <= 128; w_cols += w_mn ? 64 : 8) {
       const int bn = pair ? 2 * w_cols : w_cols;
       const double tiles = static_cast<double>(mb) * ceil_div(N, bn);
-      const double k_block = swap_k_block(pair, w_cols, tok, w_mn, 1);
+      const double k_block = swap_k_block(pair, w_cols, tok, w_mn, 1, pair ? 190.0 : 170.0);
       for (int split = 1; split <= (pair ? 4 : 8); ++split) {
         const int ctas = (pair ? 2 : 1) * split;
         const int units = cap.clusters[ctas];
@@ -242,7 +246,7 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
   return best_t;
 }
 
-// Grouped rows with exchanged operands; the same estimates.
+// Grouped rows with exchanged operands; the same estimates.  A box takes 170 ns, a pair's, which mostly go by twos, 130.
 kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms, int shape, double* cost_out) {
   kbs::Config best;
   double best_t = 1e30;
@@ -273,7 +277,7 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
         // pairs, take 15.9 us on the M side and 20.7 here.
         const int block = cols < tok ? cols : tok;
         auto cost_of = [&](int boxes) {
-          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 2000.0 : 0.0);
+          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes, pair ? 130.0 : 170.0) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 2000.0 : 0.0);
           return t > memory ? t + 0.1 * memory : memory + 0.1 * t;
         };
         const double cost = cost_of(1);

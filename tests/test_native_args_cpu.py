@@ -243,6 +243,19 @@ def test_kind_of_dense_products_whose_difference_was_measured():
         assert _pick(148, M=M, N=Nn, K=K, b_mn=1, act=N.ACTS["silu"], pre_in=0)[0] == 1, (M, Nn, K)
 
 
+def test_tiles_of_few_rows_whose_difference_was_measured():
+    """At least 7 % apart on a B200, repeated (us, this tile / the one a shorter time per box of a pair gives)."""
+    slope = dict(b_mn=1, act=N.ACTS["gelu"], pre_in=16)
+    for (M, Nn, K), kw, want in (((1, 23464, 1504), {}, (1, 0, 80, 16, 1)),              # 14.7 16.4
+                                 ((1, 21248, 3704), {}, (1, 0, 72, 16, 1)),              # 30.6 32.9
+                                 ((7, 9592, 7560), {}, (1, 0, 72, 16, 1)),               # 31.0 34.3
+                                 ((23, 25792, 7536), dict(b_mn=1), (1, 1, 256, 32, 1)),  # 67.8 77.9
+                                 ((56, 24048, 14832), dict(b_mn=1), (1, 1, 256, 64, 1)), # 144 158
+                                 ((37, 27056, 3488), slope, (1, 1, 256, 64, 1)),         # 40.7 47.0
+                                 ((29, 22272, 12976), slope, (1, 1, 256, 32, 1))):       # 109 125
+        assert _pick(148, M=M, N=Nn, K=K, **kw)[:5] == want, (M, Nn, K)
+
+
 def test_a_product_that_may_fetch_its_weights_early_is_exchanged_sooner():
     """Near ties: the exchanged kernel alone fetches them under the previous launch."""
     for M, Nn, K in ((128, 4096, 4096), (330, 6296, 1304), (672, 10008, 2040)):
