@@ -86,12 +86,18 @@ double memory_time(int M, int N, int K) {
 // in a graph, three weights in turn; one CTA with 256 columns and no split against the pick):
 // 64 x 7168 x 18432 88.5 and 45.1 us, 256 x 4096 x 14336 85.1 and 30.5, 2048 x 2880 x 2880 (in the
 // L2) 35.1 and 24.4.  512-row tiles move 25 % fewer operand bytes
-// per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).  An activation, with the value
-// before it kept, or a slope takes their epilogue 11 us longer in every wave, where a pair's runs under the next tile's products;
-// pairs and 512-row tiles, us:
+// per flop and win where K is long (8192 x 8192 x 29568: 3030 and 2840 us under the power cap).  An activation or a slope takes
+// their epilogue longer in every wave, where a pair's runs under the next tile's products; pairs and 512-row tiles, us:
 //                           plain        gelu, value kept     slope of gelu
 //   8192 x 14336 x 4096    678   708        731   850           762   855
 //   8192 x 29568 x 8192   2830  2858       2831  3163          3068  3113
+// Not where K is an odd multiple of 8: rows along K then start inside a 32-byte sector, every 128 bytes of a box cost five
+// sectors, and the operand bytes that 512-row tiles save are worth more.  Products that get such a tile without the 10 us (gelu, silu,
+// relu; repeated), the picked tile above the better one on average without / with them; for the slope what replaces it against it:
+//                   45 each: value dropped   kept            70 with a slope
+//   K % 16 = 0               3.3  0.5 %      3.6   0.5 %     0.94
+//   K % 16 = 8               0.0 10.2 %      0.0  11.0 %     1.04
+// 8009 x 13128 x 8424 with gelu 1503 us, pairs 1852; 7974 x 21272 x 6984 with a slope 2423, exchanged pairs 2875.
 Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& cap, int shape, bool act, double* cost = nullptr) {
   Config best = {false, 256, 1};
   double best_t = 1e30, best_cost = 1e30;
@@ -113,7 +119,7 @@ Config choose_config(int M, int N, int K, bool a_mn, bool b_mn, const Capacity& 
         if (split > 1 && (tiles > units || KB < 4 * split || !exchange_fits(rows, pair, bn, split))) continue;
         const double waves = units > 0 ? static_cast<double>((static_cast<long long>(tiles) + units - 1) / units) : 1e9;
         double t = 2000.0 + waves * (ceil_div(KB, split) * k_block + 2000.0) + epilogue + (pair ? 1000.0 : 0.0);
-        if (tall) t += waves * (1.25 * epilogue + (act ? 10000.0 : 0.0));
+        if (tall) t += waves * (1.25 * epilogue + (act && K % 16 == 0 ? 10000.0 : 0.0));
         if (split > 1) t += 1300.0 + 2200.0 * bn / 256.0 * (split - 1) / split;
         // Launched behind the previous kernel instead of under its end.  Not so for the long reads that are launched in order
         // because that is faster (4 x 14488 x 16616, weights along N: 86.6 us split in two, 104 unsplit).

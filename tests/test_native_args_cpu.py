@@ -256,6 +256,25 @@ def test_tiles_of_few_rows_whose_difference_was_measured():
         assert _pick(148, M=M, N=Nn, K=K, **kw)[:5] == want, (M, Nn, K)
 
 
+def test_512_rows_with_an_activation():
+    """On a B200, repeated, at least 5 % apart (us, 512-row tiles / pairs): rows of odd multiples of 16 bytes want them, others do not."""
+    gelu = N.ACTS["gelu"]
+    for M, Nn, K, keep, want in ((8009, 13128, 8424, 0, 2),    # 1503 1852
+                                 (3032, 2496, 8504, 0, 2),     # 121 146
+                                 (7121, 25744, 8408, 1, 2),    # 2589 3322
+                                 (1570, 9032, 14968, 1, 2),    # 427 519
+                                 (7416, 17744, 5200, 0, 1),    # 1179 1016
+                                 (5626, 16064, 4192, 0, 1),    # 633 591
+                                 (8192, 14336, 4096, 1, 1),    # 850 731
+                                 (8083, 12864, 4528, 1, 1)):   # 839 794
+        assert _pick(148, M=M, N=Nn, K=K, act=gelu, **(dict(pre_out=16) if keep else {}))[:2] == (0, want), (M, Nn, K)
+    for M, Nn, K, want in ((7974, 21272, 6984, 2),    # 2423 2875 (exchanged pairs)
+                           (4799, 12416, 17208, 2),   # 1744 2070
+                           (4728, 4904, 4544, 1),     # 256 205
+                           (8192, 14336, 4096, 1)):   # 855 762
+        assert _pick(148, M=M, N=Nn, K=K, b_mn=1, act=gelu, pre_in=16)[1] == want, (M, Nn, K)
+
+
 def test_a_product_that_may_fetch_its_weights_early_is_exchanged_sooner():
     """Near ties: the exchanged kernel alone fetches them under the previous launch."""
     for M, Nn, K in ((128, 4096, 4096), (330, 6296, 1304), (672, 10008, 2040)):
