@@ -160,7 +160,7 @@ typedef struct KbGemmStreamArgs {
   void* out_host;           // bf16 [M,N]
   int pieces;
   const int32_t* rows;      // host [pieces]: together M
-  int again;                // 0 for a first call, then kept by _end: the events have been through a call
+  int again;                // 0 for a first call, set by _end of one outside of a capture: the last event has been recorded
   void *stream, *in, *out;  // the caller's stream; both others are its own
   void** events;            // kb_gemm_stream_events(pieces) of kb_events_create
 } KbGemmStreamArgs;

@@ -63,7 +63,8 @@ extern "C" int kb_events_destroy(int n, void** events) {
 extern "C" int kb_gemm_stream_begin(const KbGemmStreamArgs* s) {
   const int rc = check(s);
   if (rc != KB_OK) return rc;
-  // A call on another stream than the last one's finds that one's buffers in use.  A graph does not wait for calls before it.
+  // A call on another stream than the last one's finds that one's buffers in use.  A graph does not wait for
+  // calls before it, nor they for its replays: that order is the program's.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   KB_CUDA_OK(cudaStreamIsCapturing(stream(s->stream), &capturing));
   if (capturing == cudaStreamCaptureStatusNone && s->again) KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, finished_of(s->pieces)), 0));
@@ -108,9 +109,11 @@ extern "C" int kb_gemm_stream_end(KbGemmStreamArgs* s) {
   if (rc != KB_OK) return rc;
   KB_CUDA_OK(cudaEventRecord(event(s, left_of(s->pieces)), stream(s->out)));
   KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, left_of(s->pieces)), 0));
-  KB_CUDA_OK(cudaEventRecord(event(s, finished_of(s->pieces)), stream(s->stream)));
+  // An event of a graph is nothing to wait for outside of it: a captured call leaves the chain of the others as it was.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   KB_CUDA_OK(cudaStreamIsCapturing(stream(s->stream), &capturing));
-  s->again = capturing == cudaStreamCaptureStatusNone ? 1 : 0;  // an event of a graph is nothing to wait for outside of it
+  if (capturing != cudaStreamCaptureStatusNone) return KB_OK;
+  KB_CUDA_OK(cudaEventRecord(event(s, finished_of(s->pieces)), stream(s->stream)));
+  s->again = 1;
   return KB_OK;
 }

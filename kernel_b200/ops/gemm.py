@@ -438,6 +438,8 @@ class GemmRS:
         the PCIe transfers overlap the kernel instead of bracketing it.  On one GPU, where
         any rows can form a piece, there are at most ``chunks``, of the sizes that pay (``_pieces``).  Returns
         ``out_host``; the caller's stream is done when everything has arrived.
+        Calls of one context share device buffers; on one GPU a call waits for the one before it, also on another stream, but
+        replays of a graph that holds a call are for the program to order against other calls.
         Collective like ``__call__``.  The reference has no counterpart (its
         evaluator clones the inputs on the device inside its timed region,
         ``eval.py:358``)."""

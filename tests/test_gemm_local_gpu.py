@@ -565,6 +565,32 @@ def test_rows_from_the_host_in_a_graph():
     ctx.close()
 
 
+def test_rows_from_the_host_after_a_capture_wait_for_the_call_before_it():
+    """On a third stream, the first call still under way; the capture's own call comes out right as well."""
+    from kernel_b200.ops.gemm import GemmRS
+
+    M, N, K = 2048, 2048, 2048   # 160 us on the link each way
+    w, ctx = _ints(N, K, seed=70), GemmRS(M, N, device=torch.device(DEV))
+    hosts = [_ints(M, K, seed=71 + i).cpu().pin_memory() for i in range(3)]
+    outs = [torch.zeros((M, N), dtype=torch.bfloat16).pin_memory() for _ in hosts]
+    streams = [torch.cuda.Stream() for _ in hosts]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    for i, (host, out, stream) in enumerate(zip(hosts, outs, streams)):
+        with torch.cuda.stream(stream):
+            if i == 1:
+                graph.capture_begin(capture_error_mode="thread_local")
+            ctx.run_from_host(host, w, out_host=out)
+            if i == 1:
+                graph.capture_end()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for host, out in zip(hosts, outs):
+        assert torch.equal(out.to(DEV), (host.to(DEV).float() @ w.float().t()).to(torch.bfloat16))
+    ctx.close()
+
+
 @pytest.mark.parametrize("E", [256, 512, 100, 1024])  # bf16: exact scales, scales of more digits, no power of two; fp16: exact up to 1024
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("H,T,k", [(1032, 9, 1), (7168, 150, 8), (2056, 700, 3)])
