@@ -160,9 +160,9 @@ typedef struct KbGemmStreamArgs {
   void* out_host;           // bf16 [M,N]
   int pieces;
   const int32_t* rows;      // host [pieces]: together M
-  int again;                // 0 for a first call, set by _end of one outside of a capture: the last event has been recorded
+  int again;                // 0 for a first call, set by _end of one outside of a capture: the first event has been recorded
   void *stream, *in, *out;  // the caller's stream; both others are its own
-  void** events;            // kb_gemm_stream_events(pieces) of kb_events_create
+  void** events;            // at least kb_gemm_stream_events(pieces) of kb_events_create, the same from call to call
 } KbGemmStreamArgs;
 int kb_gemm_stream_events(int pieces);
 int kb_events_create(int n, void** events);

@@ -13,12 +13,10 @@
 namespace {
 
 constexpr int MAX_PIECES = 64;
-// events: the rows of piece i are there, its product is done, and three of the whole call
-int ready_of(int i) { return i; }
-int done_of(int pieces, int i) { return pieces + i; }
-int started_of(int pieces) { return 2 * pieces; }
-int left_of(int pieces) { return 2 * pieces + 1; }
-int finished_of(int pieces) { return 2 * pieces + 2; }
+// events: three of the whole call, then of piece i: its rows are there, its product is done
+constexpr int FINISHED = 0, STARTED = 1, LEFT = 2;
+int ready_of(int i) { return 3 + 2 * i; }
+int done_of(int i) { return 4 + 2 * i; }
 
 cudaEvent_t event(const KbGemmStreamArgs* s, int i) { return static_cast<cudaEvent_t>(s->events[i]); }
 cudaStream_t stream(void* p) { return static_cast<cudaStream_t>(p); }
@@ -67,9 +65,9 @@ extern "C" int kb_gemm_stream_begin(const KbGemmStreamArgs* s) {
   // calls before it, nor they for its replays: that order is the program's.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   KB_CUDA_OK(cudaStreamIsCapturing(stream(s->stream), &capturing));
-  if (capturing == cudaStreamCaptureStatusNone && s->again) KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, finished_of(s->pieces)), 0));
-  KB_CUDA_OK(cudaEventRecord(event(s, started_of(s->pieces)), stream(s->stream)));
-  KB_CUDA_OK(cudaStreamWaitEvent(stream(s->in), event(s, started_of(s->pieces)), 0));
+  if (capturing == cudaStreamCaptureStatusNone && s->again) KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, FINISHED), 0));
+  KB_CUDA_OK(cudaEventRecord(event(s, STARTED), stream(s->stream)));
+  KB_CUDA_OK(cudaStreamWaitEvent(stream(s->in), event(s, STARTED), 0));
   return KB_OK;
 }
 
@@ -94,8 +92,8 @@ extern "C" int kb_gemm_stream_run(const KbGemmStreamArgs* s) {
     a.out = out_dev + first * out_row;
     rc = kb_gemm_local(&a, s->stream);
     if (rc != KB_OK) return rc;
-    KB_CUDA_OK(cudaEventRecord(event(s, done_of(s->pieces, i)), cur));
-    KB_CUDA_OK(cudaStreamWaitEvent(out, event(s, done_of(s->pieces, i)), 0));
+    KB_CUDA_OK(cudaEventRecord(event(s, done_of(i)), cur));
+    KB_CUDA_OK(cudaStreamWaitEvent(out, event(s, done_of(i)), 0));
     if (i + 1 < s->pieces) {
       KB_CUDA_OK(cudaMemcpyAsync(static_cast<char*>(s->out_host) + first * out_row, out_dev + first * out_row, rows * out_row, cudaMemcpyDeviceToHost, out));
     }
@@ -107,13 +105,13 @@ extern "C" int kb_gemm_stream_run(const KbGemmStreamArgs* s) {
 extern "C" int kb_gemm_stream_end(KbGemmStreamArgs* s) {
   const int rc = check(s);
   if (rc != KB_OK) return rc;
-  KB_CUDA_OK(cudaEventRecord(event(s, left_of(s->pieces)), stream(s->out)));
-  KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, left_of(s->pieces)), 0));
+  KB_CUDA_OK(cudaEventRecord(event(s, LEFT), stream(s->out)));
+  KB_CUDA_OK(cudaStreamWaitEvent(stream(s->stream), event(s, LEFT), 0));
   // An event of a graph is nothing to wait for outside of it: a captured call leaves the chain of the others as it was.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   KB_CUDA_OK(cudaStreamIsCapturing(stream(s->stream), &capturing));
   if (capturing != cudaStreamCaptureStatusNone) return KB_OK;
-  KB_CUDA_OK(cudaEventRecord(event(s, finished_of(s->pieces)), stream(s->stream)));
+  KB_CUDA_OK(cudaEventRecord(event(s, FINISHED), stream(s->stream)));
   s->again = 1;
   return KB_OK;
 }

@@ -202,51 +202,96 @@ def _pieces(M: int, Nn: int, K: int, most: int) -> list:
 # Rows and result of a `run_from_host` that one GPU holds whole.  Above it the buffers of two chunks of the general path: such a call
 # takes 80 ms on the link, beside which the 0.2 ms that the native calls save are nothing, and rows need not fit the GPU's memory.
 _WHOLE_ROWS_BYTES = 4 << 30
+# Up to here they are held without a look at the memory that is left.
+_SMALL_ROWS_BYTES = 64 << 20
+
+
+def _room(device: torch.device) -> int:
+    """Bytes that a tensor can still get on the GPU."""
+    return torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
 
 class _OneGpuStream:
-    """Device buffers, side streams and events of ``run_from_host`` on one GPU (``csrc/kernels/gemm_stream.cu``)."""
+    """Device buffers, side streams and events of a context's ``run_from_host`` calls on one GPU (``csrc/kernels/gemm_stream.cu``):
+    one pair of buffers for all of them, as large as the largest so far."""
 
-    def __init__(self, device: torch.device, M: int, Nn: int, K: int, chunks: int, status: torch.Tensor):
-        self.rows = _pieces(M, Nn, K, max(1, min(chunks, 64)))
-        self.inp = torch.empty((M, K), dtype=torch.bfloat16, device=device)
-        self.out = torch.empty((M, Nn), dtype=torch.bfloat16, device=device)
+    def __init__(self, device: torch.device, status: torch.Tensor):
+        self.device = device
         self.inward, self.outward = torch.cuda.Stream(device), torch.cuda.Stream(device)
-        self.inp.record_stream(self.inward)
-        self.out.record_stream(self.outward)
-        self.home = torch._C._cuda_getCurrentRawStream(device.index)
+        self.inp = self.out = None
+        self.kept = []   # pairs that a graph may hold
+        self.plans = {}  # (chunks, N, K) -> rows of the pieces, the same for C
         args = self.args = N.GemmStreamArgs()
         args.product = _local_args(status)
-        args.product.M, args.product.N, args.product.K = M, Nn, K
-        args.product.A, args.product.out = self.inp.data_ptr(), self.out.data_ptr()
-        args.pieces = len(self.rows)
-        self.table = (C.c_int32 * args.pieces)(*self.rows)
-        args.rows = C.addressof(self.table)
         args.inward, args.outward = self.inward.cuda_stream, self.outward.cuda_stream
-        self.count = N.lib().kb_gemm_stream_events(args.pieces)
-        self.events = (C.c_void_p * self.count)()
+        self.count, self.events = 0, (C.c_void_p * N.lib().kb_gemm_stream_events(64))()
         self.destroy = N.lib().kb_events_destroy  # at hand when the interpreter has let go of the module
-        N.check(N.lib().kb_events_create(self.count, self.events))
         args.events = C.addressof(self.events)
 
-    def run(self, a_host: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], bias_scale: float, out_host: torch.Tensor) -> None:
+    def _allocate(self, count: int) -> torch.Tensor:
+        return torch.empty(count, dtype=torch.bfloat16, device=self.device)
+
+    def hold(self, a: int, o: int) -> bool:
+        """Buffers of at least ``a`` and ``o`` elements; False where they would take more than a quarter of the memory that is left."""
+        capturing = torch.cuda.is_current_stream_capturing()
+        if self.inp is None or self.inp.numel() < a or self.out.numel() < o:
+            had = (self.inp.numel(), self.out.numel()) if self.inp is not None else (0, 0)
+            self.inp = self.out = None  # frees the old pair, or leaves it to the graph that has it
+            sizes = max(a, had[0]), max(o, had[1])
+            if 2 * sum(sizes) > _WHOLE_ROWS_BYTES:
+                sizes = a, o
+            if not capturing and 2 * sum(sizes) > _SMALL_ROWS_BYTES and 8 * sum(sizes) > _room(self.device):
+                return False
+            try:
+                self.inp, self.out = self._allocate(sizes[0]), self._allocate(sizes[1])
+            except torch.OutOfMemoryError:
+                self.inp = self.out = None
+                return False
+            self.inp.record_stream(self.inward)
+            self.out.record_stream(self.outward)
+            self.home = torch._C._cuda_getCurrentRawStream(self.device.index)
+            self.args.product.A, self.args.product.out = self.inp.data_ptr(), self.out.data_ptr()
+        if capturing and all(pair[0] is not self.inp for pair in self.kept):
+            self.kept.append((self.inp, self.out))
+        return True
+
+    def _plan(self, M: int, Nn: int, K: int, chunks: int):
+        plan = self.plans.get((chunks, Nn, K))
+        if plan is None:
+            rows = _pieces(M, Nn, K, max(1, min(chunks, 64)))
+            events = N.lib().kb_gemm_stream_events(len(rows))
+            if events > self.count:
+                more = (C.c_void_p * (events - self.count)).from_buffer(self.events, self.count * C.sizeof(C.c_void_p))
+                N.check(N.lib().kb_events_create(events - self.count, more))
+                self.count = events
+            plan = self.plans[chunks, Nn, K] = (rows, (C.c_int32 * len(rows))(*rows))
+        return plan
+
+    def run(self, a_host: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], bias_scale: float, out_host: torch.Tensor, chunks: int) -> bool:
         global launch_count
-        lib, args, index = N.lib(), self.args, w.device.index
+        (M, K), Nn = a_host.shape, w.shape[0]
+        if not self.hold(M * K, M * Nn):
+            return False
+        lib, args, index = N.lib(), self.args, self.device.index
+        rows, table = self._plan(M, Nn, K, chunks)
+        args.product.M, args.product.N, args.product.K = M, Nn, K
         args.product.B, args.product.bias, args.product.bias_scale = w.data_ptr(), bias.data_ptr() if bias is not None else None, bias_scale
         args.a_host, args.out_host = a_host.data_ptr(), out_host.data_ptr()
+        args.pieces, args.rows = len(rows), C.addressof(table)
         stream = args.stream = torch._C._cuda_getCurrentRawStream(index)
         if stream != self.home:  # its products may still run when the buffers are freed
             other = torch.cuda.current_stream(w.device)
             self.inp.record_stream(other)
             self.out.record_stream(other)
-        rows, last = self.rows[0], a_host.shape[0] - self.rows[-1]
+        first, last = rows[0], M - rows[-1]
         N.check(lib.kb_gemm_stream_begin(C.byref(args)))
         # torch's copies make its allocator of pinned memory wait for the side streams before it hands out a buffer again
-        self._copy(self.inward, index, self.inp[:rows], a_host[:rows])
+        self._copy(self.inward, index, self.inp[:first * K], a_host[:first].view(-1))
         N.check(lib.kb_gemm_stream_run(C.byref(args)))
-        self._copy(self.outward, index, out_host[last:], self.out[last:])
+        self._copy(self.outward, index, out_host[last:].view(-1), self.out[last * Nn:M * Nn])
         N.check(lib.kb_gemm_stream_end(C.byref(args)))
         launch_count += args.pieces
+        return True
 
     @staticmethod
     def _copy(stream: torch.cuda.Stream, index: int, dst: torch.Tensor, src: torch.Tensor) -> None:
@@ -261,7 +306,7 @@ class _OneGpuStream:
     def __del__(self):
         events, destroy = getattr(self, "events", None), getattr(self, "destroy", None)
         if events is not None and destroy is not None:
-            destroy(self.count, events)
+            destroy(len(events), events)
 
 
 def _from_host_on_one_gpu(ctx, a_host: torch.Tensor, w: torch.Tensor, bias, bias_scale: float, out_host: torch.Tensor, chunks: int) -> bool:
@@ -272,10 +317,11 @@ def _from_host_on_one_gpu(ctx, a_host: torch.Tensor, w: torch.Tensor, bias, bias
     if 2 * M * (Nn + K) > _WHOLE_ROWS_BYTES:
         return False
     states = ctx.__dict__.setdefault("_one_gpu_streams", {})
-    st = states.get((chunks, Nn, K, w.device.index))
+    st = states.get(w.device.index)
     if st is None:
-        st = states[chunks, Nn, K, w.device.index] = _OneGpuStream(w.device, M, Nn, K, chunks, ctx.status)
-    st.run(a_host, w, bias, bias_scale, out_host)
+        st = states[w.device.index] = _OneGpuStream(w.device, ctx.status)
+    if not st.run(a_host, w, bias, bias_scale, out_host, chunks):
+        return False
     ctx.epoch += 1
     return True
 

@@ -591,6 +591,67 @@ def test_rows_from_the_host_after_a_capture_wait_for_the_call_before_it():
     ctx.close()
 
 
+def test_rows_from_the_host_of_several_widths_share_their_buffers():
+    """Nothing is held beside the largest rows and the largest result; a graph keeps those that it was captured with."""
+    from kernel_b200.ops.gemm import AGGemm
+
+    M, K = 1536, 1024
+    a = _ints(M, K, seed=74)
+    host, ctx = a.cpu().pin_memory(), AGGemm(M, K, device=torch.device(DEV))
+    ws = {N: _ints(N, K, seed=75) for N in (1024, 4096, 520, 4096, 8192)}
+    outs = {N: torch.zeros((M, N), dtype=torch.bfloat16).pin_memory() for N in ws}
+    want = {N: (a.float() @ w.float().t()).to(torch.bfloat16) for N, w in ws.items()}
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    before, most = torch.cuda.memory_allocated(), 0
+    for N, chunks in ((1024, 4), (4096, 4), (520, 1), (4096, 7), (1024, 2)):
+        most = max(most, N)
+        ctx.run_from_host(host, ws[N], out_host=outs[N], chunks=chunks)
+        torch.cuda.synchronize()
+        assert torch.equal(outs[N].to(DEV), want[N])
+        assert torch.cuda.memory_allocated() - before <= 2 * M * (K + most)
+    with torch.cuda.graph(graph):
+        ctx.run_from_host(host, ws[4096], out_host=outs[4096])
+    ctx.run_from_host(host, ws[8192], out_host=outs[8192])   # the others are too small for it
+    torch.cuda.synchronize()
+    taken = [torch.full((M * N,), -1.0, dtype=torch.bfloat16, device=DEV) for N in (K, 4096)]
+    outs[4096].zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(outs[4096].to(DEV), want[4096]) and torch.equal(outs[8192].to(DEV), want[8192])
+    assert all(bool((t == -1).all()) for t in taken)
+    ctx.close()
+
+
+@pytest.mark.parametrize("fault", ["room", "allocation"])
+def test_rows_from_the_host_that_cannot_be_held_go_in_chunks(fault, monkeypatch):
+    from kernel_b200.ops import gemm
+
+    M, N, K = 512, 264, 520
+    w, a = _ints(N, K, seed=76), _ints(M, K, seed=77)
+    want, host = (a.float() @ w.float().t()).to(torch.bfloat16), a.cpu().pin_memory()
+    for ctx in (gemm.GemmRS(M, N, device=torch.device(DEV)), gemm.AGGemm(M, K, device=torch.device(DEV))):
+        with monkeypatch.context() as patch:
+            if fault == "room":
+                patch.setattr(gemm, "_SMALL_ROWS_BYTES", 0)
+                patch.setattr(gemm, "_room", lambda device: 8 * M * (N + K) - 1)   # four times the buffers' bytes, but for one
+            else:
+                def full(self, count):
+                    raise torch.OutOfMemoryError("planted")
+                patch.setattr(gemm._OneGpuStream, "_allocate", full)
+            out = ctx.run_from_host(host, w)
+            torch.cuda.synchronize()
+            assert torch.equal(out.to(DEV), want) and hasattr(ctx, "_stream_state") and ctx._stream_state
+        ctx._stream_state.clear()
+        if fault == "room":
+            monkeypatch.setattr(gemm, "_room", lambda device: 8 * M * (N + K))
+            monkeypatch.setattr(gemm, "_SMALL_ROWS_BYTES", 0)
+        out = ctx.run_from_host(host, w)   # as soon as there is room
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), want) and not ctx._stream_state
+        ctx.close()
+
+
 @pytest.mark.parametrize("E", [256, 512, 100, 1024])  # bf16: exact scales, scales of more digits, no power of two; fp16: exact up to 1024
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("H,T,k", [(1032, 9, 1), (7168, 150, 8), (2056, 700, 3)])
