@@ -33,6 +33,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../common/host_util.h"
 #include "../common/ptx.cuh"
 #include "../include/kb200.h"
@@ -465,34 +467,37 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
       // a pair's bytes are counted on the leader's barrier, which expects the sum
       const uint32_t tx_bytes = kPair ? 2 * stage_bytes : stage_bytes;
       const uint32_t bar0 = kPair ? kb::map_to_cta(full0, lead) : full0;
-      for (int pos = sched_id; ok && pos < total_tiles; pos += sched_n) {
-        const Tile t = tile_at(pos);
-        int k0, k1;
-        k_range(t, k0, k1);
-        const int bz = kKind == ROWS ? t.group : 0;
-        const int nrow = t.n0 + static_cast<int>(half) * b_cols;
-        for (int k = k0; k < k1; ++k) {
-          if (!kb::mbar_wait_bounded(&empty[s], ph ^ 1u, p.limit_ns, 400)) {
-            kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, SITE_EMPTY, (uint32_t)pos, 0);
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
-          const uint32_t da = a0 + s * p.a_slot, db = b0 + s * p.b_slot, bar = bar0 + 8 * s, own = full0 + 8 * s;
-          if (++s == static_cast<uint32_t>(p.stages)) {
-            s = 0;
-            ph ^= 1u;
-          }
-          if constexpr (!kAMn && !kBMn) {
-            kb::tma_load_ab_warp<kPair>(own, leader ? tx_bytes : 0u, bar, da, &p.tmA, k * BK, t.row0, 0, db, &p.tmB, k * BK, nrow, bz);
-            continue;
-          }
-          if (leader) kb::mbar_expect_tx_warp(own, tx_bytes);
-          // M/N-contiguous operands in one load each instead of one per 64 columns: issuing six loads per stage is what
-          // held the producer back where a tile has few k blocks (weight gradients of 64 experts of 2048 x 1024, 128 rows:
-          // 73.8 -> 70.8 us, on 32 SMs alone 276 -> 237).
-          if constexpr (kAMn) {
-            if (p.a_whole) {
+      // M/N-contiguous operands in one load each instead of one per 64 columns where their extent allows it: issuing six loads per
+      // stage is what held the producer back where a tile has few k blocks (weight gradients of 64 experts of 2048 x 1024, 128 rows:
+      // 73.8 -> 70.8 us, on 32 SMs alone 276 -> 237).  Each kind of load has a loop of its own: with the choice inside it the loads per
+      // 64 columns took a pair 3 to 8 % longer (16 groups of 808 rows, 1296 x 2400: 105.7 us, 98.9 here).
+      auto produce = [&](auto a_whole, auto b_whole) {
+        for (int pos = sched_id; ok && pos < total_tiles; pos += sched_n) {
+          const Tile t = tile_at(pos);
+          int k0, k1;
+          k_range(t, k0, k1);
+          const int bz = kKind == ROWS ? t.group : 0;
+          const int nrow = t.n0 + static_cast<int>(half) * b_cols;
+          for (int k = k0; k < k1; ++k) {
+            if (!kb::mbar_wait_bounded(&empty[s], ph ^ 1u, p.limit_ns, 400)) {
+              kb::report_status(p.status, KB_DEV_TIMEOUT_MBAR, SITE_EMPTY, (uint32_t)pos, 0);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            const uint32_t da = a0 + s * p.a_slot, db = b0 + s * p.b_slot, bar = bar0 + 8 * s, own = full0 + 8 * s;
+            if (++s == static_cast<uint32_t>(p.stages)) {
+              s = 0;
+              ph ^= 1u;
+            }
+            if constexpr (!kAMn && !kBMn) {
+              kb::tma_load_ab_warp<kPair>(own, leader ? tx_bytes : 0u, bar, da, &p.tmA, k * BK, t.row0, 0, db, &p.tmB, k * BK, nrow, bz);
+              continue;
+            }
+            if (leader) kb::mbar_expect_tx_warp(own, tx_bytes);
+            if constexpr (!kAMn) {
+              kb::tma_load_3d_warp<kPair>(da, &p.tmA, bar, k * BK, t.row0, 0);
+            } else if constexpr (decltype(a_whole)::value) {
               kb::tma_load_4d_warp<kPair>(da, &p.tmA, bar, 0, t.k_row + k * BK, t.row0 / 64, 0);
             } else {
 #pragma unroll
@@ -500,21 +505,30 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
                 kb::tma_load_3d_warp<kPair>(da + i * MN_BLOCK_BYTES, &p.tmA, bar, t.row0 + i * 64, t.k_row + k * BK, 0);
               }
             }
-          } else {
-            kb::tma_load_3d_warp<kPair>(da, &p.tmA, bar, k * BK, t.row0, 0);
-          }
-          if constexpr (kBMn) {
-            if (p.b_whole) {
+            if constexpr (!kBMn) {
+              kb::tma_load_3d_warp<kPair>(db, &p.tmB, bar, k * BK, nrow, bz);
+            } else if constexpr (decltype(b_whole)::value) {
               kb::tma_load_4d_warp<kPair>(db, &p.tmB, bar, 0, t.k_row + k * BK, nrow / 64, bz);
-              continue;
+            } else {
+              for (int i = 0; i < b_cols / 64; ++i) {
+                kb::tma_load_3d_warp<kPair>(db + i * MN_BLOCK_BYTES, &p.tmB, bar, nrow + i * 64, t.k_row + k * BK, bz);
+              }
             }
-            for (int i = 0; i < b_cols / 64; ++i) {
-              kb::tma_load_3d_warp<kPair>(db + i * MN_BLOCK_BYTES, &p.tmB, bar, nrow + i * 64, t.k_row + k * BK, bz);
-            }
-          } else {
-            kb::tma_load_3d_warp<kPair>(db, &p.tmB, bar, k * BK, nrow, bz);
           }
         }
+      };
+      using Yes = std::true_type;
+      using No = std::false_type;
+      if constexpr (kAMn) {
+        if (p.a_whole && p.b_whole) produce(Yes{}, Yes{});
+        else if (p.a_whole) produce(Yes{}, No{});
+        else if (p.b_whole) produce(No{}, Yes{});
+        else produce(No{}, No{});
+      } else if constexpr (kBMn) {
+        if (p.b_whole) produce(No{}, Yes{});
+        else produce(No{}, No{});
+      } else {
+        produce(No{}, No{});
       }
     }
     __syncwarp();
