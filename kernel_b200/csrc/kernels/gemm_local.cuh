@@ -265,18 +265,13 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 }
 
 // Weights on their way into the L2 before the previous launch has ended: the first k blocks of `cols` columns from `col` on,
-// by 256 threads.  Nothing is read by it, so it does not matter that someone may still write them.  `w`: [N][K] or (kMn) [K][N].
+// by 256 threads.  Nothing is read by it, so it does not matter that someone may still write them.  `w`: [N][K].
 constexpr int AHEAD = 12;  // k blocks, 30 MB on 148 SMs: with 6 half of the gain, with 20 and 32 no more
-template <bool kMn>
 __device__ __forceinline__ void prefetch_weights(const bf16* w, int N, int K, int col, int cols, int k0, int k1, int thread) {
   const int k = k0 * BK, ks = min(min(k1 - k0, AHEAD) * BK, K - k);
   const int cs = min(cols, N - col);
-  if (cs <= 0 || ks <= 0) return;
-  if constexpr (kMn) {
-    for (int i = thread; i < ks; i += 256) kb::prefetch_l2(w + static_cast<size_t>(k + i) * N + col, static_cast<uint32_t>(cs) * 2);
-  } else {
-    for (int i = thread; i < cs; i += 256) kb::prefetch_l2(w + static_cast<size_t>(col + i) * K + k, static_cast<uint32_t>(ks) * 2);
-  }
+  if (ks <= 0) return;
+  for (int i = thread; i < cs; i += 256) kb::prefetch_l2(w + static_cast<size_t>(col + i) * K + k, static_cast<uint32_t>(ks) * 2);
 }
 
 // kHalves: 128-row blocks per CTA and tile.  2 (pairs only): a 512-row tile whose two
@@ -400,11 +395,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_local_kernel(const __grid_con
     kb::tma_prefetch_desc(&p.tmA);
     kb::tma_prefetch_desc(&p.tmB);
   }
-  if (kKind == DENSE && !kAMn && warp >= 4 && p.w != nullptr) {
+  if (kKind == DENSE && !kBMn && warp >= 4 && p.w != nullptr) {
     const Tile t = tile_at(sched_id);
     int k0, k1;
     k_range(t, k0, k1);
-    prefetch_weights<kBMn>(p.w, p.N, p.K, t.n0 + static_cast<int>(half) * b_cols, b_cols, k0, k1, tid - 128);
+    prefetch_weights(p.w, p.N, p.K, t.n0 + static_cast<int>(half) * b_cols, b_cols, k0, k1, tid - 128);
   }
   kb::wait_for_previous_launch();  // barriers, tensor memory and descriptors are set up under the end of that one
   const uint64_t t_start = p.timing ? kb::globaltimer_ns() : 0;  // the product's own time

@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_swap_kernel(const __grid_cons
     kb::tma_prefetch_desc(&p.tmW);
     kb::tma_prefetch_desc(&p.tmX);
   }
-  if (kKind == DENSE && warp >= 4 && p.w != nullptr) {
-    kbl::prefetch_weights<kWMn>(p.w, p.N, p.K, p.per.of(sched_id) * p.bn + static_cast<int>(half) * w_cols, w_cols, k0, k1, tid - 128);
+  if (kKind == DENSE && !kWMn && warp >= 4 && p.w != nullptr) {
+    kbl::prefetch_weights(p.w, p.N, p.K, p.per.of(sched_id) * p.bn + static_cast<int>(half) * w_cols, w_cols, k0, k1, tid - 128);
   }
   if (!p.early) kb::wait_for_previous_launch();
   uint64_t t_start = p.timing ? kb::globaltimer_ns() : 0;  // the product's own time
