@@ -307,10 +307,17 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
 //   128 of 1024 x 768      45  46      46  50      49  49      50  50      61  52      64  55      70  64      83  73
 //   32 of 2040 x 1000      35  37      40  36      42  39      44  39      48  43      53  46      58  50      67  57
 // (Before the second CTA's epilogue gave its accumulator back without a fence, a pair took 93, 86, 76 and 53 at 128 rows.)
-Config contract_config(int M, int N, int rows, int groups, int shape) {
+// Up to 224 rows that holds from three waves of pairs' tiles on, below six only if their taller tiles are no more than 1/16 padding.  One CTA
+// and pair: 8 groups of 171 rows, 832 x 1088 7.1 9.0, of 69, 640 x 1024 6.1 7.1; 16 of 74, 896 x 1408 12.4 13.5.  79 products (66 to 223
+// rows, 8 to 128 groups, M and N 512 to 4096): 0.4 % above the better tile on average and 2 more than 3 %; by the rows alone 2.4 % and 17.
+Config contract_config(int M, int N, int rows, int groups, int sms, int shape) {
   Config c;
-  c.pair = shape >= 0 ? shape > 0 : M > 128 && rows / groups >= 72;
-  c.bn = N <= 64 && !c.pair ? 64 : N <= 128 ? 128 : 256;
+  c.bn = N <= 128 ? 128 : 256;
+  const double wide = static_cast<double>(groups) * ceil_div(N, c.bn);
+  const double ones = wide * ceil_div(M, 128), pairs = wide * ceil_div(M, 256), wave = sms / 2;
+  const bool enough = pairs >= 6.0 * wave || (pairs >= 3.0 * wave && 32.0 * pairs <= 17.0 * ones);
+  c.pair = shape >= 0 ? shape > 0 : M > 128 && (rows / groups >= 224 || (rows / groups >= 72 && enough));
+  if (N <= 64 && !c.pair) c.bn = 64;
   c.split = 1;
   return c;
 }
@@ -569,7 +576,7 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
     const int rc = pick_config(dev, sms, cap, a->M, a->N, a->K, l.a_mn, l.b_mn, shape, a->act != ACT_NONE, a->pre_in != nullptr, a->early != 0, &pick);
     if (rc != KB_OK) return rc;
   } else {
-    pick.c = contract_config(a->M, a->N, expect, groups, shape);
+    pick.c = contract_config(a->M, a->N, expect, groups, cap, shape);
   }
   if (shape < 3 && (a->bn > 0 || a->split > 0)) pick.swap = false;  // a tile of the other kind is asked for
   int* bn = pick.swap ? &pick.s.bn : &pick.c.bn;

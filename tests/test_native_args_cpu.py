@@ -298,6 +298,27 @@ def test_kind_of_grouped_products_whose_difference_was_measured():
     assert kind(8, 4000, 4096, 4096, **slope) == 1     # 116 94.4
 
 
+def test_tiles_of_contractions_whose_difference_was_measured():
+    """At least 5 % apart on a B200 (us, one CTA / pair)."""
+    def pair(groups, rows, M, Nn):
+        return _pick(148, kind=N.LOCAL_CONTRACT, M=M, N=Nn, K=groups * (rows + 63), groups=groups, expect=groups * rows, row_start=16, row_count=16)[1]
+
+    for product in ((8, 171, 832, 1088),      # 7.1 9.0
+                    (8, 77, 616, 2384),       # 9.8 11.6
+                    (8, 69, 640, 1024),       # 6.1 7.1
+                    (16, 94, 608, 560),       # 6.8 7.7
+                    (16, 74, 896, 1408),      # 12.4 13.5
+                    (64, 32, 2048, 1024)):    # 57 58: one k block
+        assert pair(*product) == 0, product
+    for product in ((64, 128, 2048, 1024),    # 77.5 71.7
+                    (8, 180, 976, 1704),      # 14.0 12.9
+                    (16, 157, 1720, 584),     # 19.1 17.4
+                    (32, 97, 696, 1560),      # 28.8 26.5
+                    (128, 79, 704, 1480),     # 92.8 83.3
+                    (32, 242, 1160, 568)):    # 31.1 26.7
+        assert pair(*product) == 1, product
+
+
 def test_vectors_per_lane_of_the_round_trip():
     """Where a form was at least 5 % faster than the others on a B200 (us with 1 / 2 / 4 vectors per lane)."""
     vecs = lambda tokens, hidden, elem=2: N.lib().kb_a2a_local_vecs(tokens, hidden, elem, 148)
