@@ -252,7 +252,8 @@ double choose_swap(int M, int N, int K, bool w_mn, const Capacity& cap, int shap
   return best_t;
 }
 
-// Grouped rows with exchanged operands; the same estimates.  A box takes 170 ns, a pair's, which mostly go by twos, 130.
+// Grouped rows with exchanged operands; the same estimates.  A box takes 170 ns, a pair's 130 where there are several, which go by twos,
+// else 190 (16 groups of 0.2 rows, 832 x 3600: one CTA 14.3 us, pairs, which 130 would take, 16.4).
 kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms, int shape, double* cost_out) {
   kbs::Config best;
   double best_t = 1e30;
@@ -282,14 +283,15 @@ kbs::Config rows_swap_config(int M, int groups, int N, int K, bool w_mn, int sms
         // The tile is chosen as if the tokens came in one box, its cost counts the boxes: 8 groups of 121 rows of [640, 2960], in
         // pairs, take 15.9 us on the M side and 20.7 here.
         const int block = cols < tok ? cols : tok;
-        auto cost_of = [&](int boxes) {
-          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes, pair ? 130.0 : 170.0) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 2000.0 : 0.0);
+        const int boxes = ceil_div(block, (pair ? 2 : 1) * ring.xbox);
+        auto cost_of = [&](int boxes_counted) {
+          const double t = 2000.0 + waves * (KB * swap_k_block(pair, w_cols, block, w_mn, boxes_counted, !pair ? 170.0 : boxes > 1 ? 130.0 : 190.0) + 1000.0) + 2000.0 * cols / 256.0 + (pair ? 2000.0 : 0.0);
           return t > memory ? t + 0.1 * memory : memory + 0.1 * t;
         };
         const double cost = cost_of(1);
         if (cost < best_t) {
           best_t = cost;
-          *cost_out = cost_of(ceil_div(block, (pair ? 2 : 1) * ring.xbox)) +
+          *cost_out = cost_of(boxes) +
                       mma_energy(groups * blocks * cols, static_cast<double>(ceil_div(N, bn)) * (pair ? 256.0 : 128.0), K);
           best = c;
         }
@@ -503,8 +505,9 @@ Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int sha
     // Limits, the time per box and a pair's 2000 ns fitted to 560 products in bursts (8 to 128 groups of 1 to 900 rows, Poisson
     // counts, N and K 512 to 4096), after boxes came by twos and pairs handed their accumulators on without a fence: forward
     // with activation, plain and slope take 1.4, 1.6 and 2.0 % more than the best tile of both kinds on average (before the fit 5.7, 3.6
-    // and 3.0; always exchanged 1.3, 1.9 and 1.4, always the M side 9.5, 4.5 and 17), 84 of 558 more than 3 % (179).
-    const double limit = slope ? 1.14 : rows >= 192ll * groups ? 1.02 : rows >= 32ll * groups ? 0.99 : 1.25;
+    // and 3.0; always exchanged 1.3, 1.9 and 1.4, always the M side 9.5, 4.5 and 17), 84 of 558 more than 3 % (179).  That was with 1.25 below 32
+    // rows and 130 ns for a pair's single box; 563 others of 0.1 to 31 rows take 1.4 % more than the best kind so, 1.8 with those.
+    const double limit = slope ? 1.14 : rows >= 192ll * groups ? 1.02 : rows >= 32ll * groups ? 0.99 : 1.05;
     r.swap = other - (early ? EARLY : 0.0) < limit * plain;
     e = {rows, N, K, groups, key, 0, r};
   }

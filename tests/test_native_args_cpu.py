@@ -298,6 +298,21 @@ def test_kind_of_grouped_products_whose_difference_was_measured():
     assert kind(8, 4000, 4096, 4096, **slope) == 1     # 116 94.4
 
 
+def test_tiles_of_grouped_products_of_few_rows_whose_difference_was_measured():
+    """At least 8 % apart on a B200 (us, rows on the M side / exchanged, one CTA / exchanged pair)."""
+    def tile(groups, rows, Nn, K, **kw):
+        return _pick(148, kind=N.LOCAL_ROWS, M=rows, N=Nn, K=K, groups=groups, row_start=16, row_count=16, **kw)[:2]
+
+    silu = dict(act=N.ACTS["silu"])
+    assert tile(16, 4, 832, 3600, **silu) == (1, 0)          # 16.4 in pairs, 14.3 before them
+    assert tile(8, 2, 3816, 3632, **silu) == (1, 0)          # 18.3 15.6 17.1
+    assert tile(64, 12, 520, 3504, early=1) == (1, 0)        # 15.5 13.5 14.8
+    assert tile(32, 850, 672, 2016) == (0, 0)                # 18.8 24.1 23.5
+    assert tile(8, 168, 2456, 2144, b_mn=1) == (0, 0)        # 19.9 24.0 24.5
+    assert tile(8, 156, 2696, 2688, b_mn=1) == (0, 0)        # 25.8 30.1 30.9
+    assert tile(64, 192, 1024, 2048, **silu) == (1, 0)       # 47.6 45.5
+
+
 def test_tiles_of_contractions_whose_difference_was_measured():
     """At least 5 % apart on a B200 (us, one CTA / pair)."""
     def pair(groups, rows, M, Nn):
