@@ -503,23 +503,33 @@ def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mo
     ctx.heap.close()
 
 
-@pytest.mark.parametrize("M,N,K,chunks", [(2, 8, 8, 4), (64, 72, 136, 4), (300, 264, 1032, 1), (515, 128, 2048, 7), (1024, 2048, 136, 4), (4096, 72, 2048, 4)])
-def test_rows_from_the_host_in_pieces(M, N, K, chunks):
-    """Sizes for which the pieces are one, equal, falling and rising, call after call with other rows, and on another stream."""
-    from kernel_b200.ops.gemm import AGGemm, GemmRS
+@pytest.mark.parametrize("M,N,K,chunks,rows", [
+    (2, 8, 8, 4, [2]), (64, 72, 136, 4, [64]), (300, 264, 1032, 1, [300]), (4096, 72, 2048, 4, [4096]),
+    (515, 4096, 4096, 4, [192, 192, 131]), (2048, 2048, 2048, 4, [512] * 4), (1111, 1024, 8192, 4, [896, 215]), (1111, 8192, 1024, 4, [256, 855]),
+    (2000, 4096, 4096, 7, [320, 256, 320, 256, 320, 256, 272])])
+def test_rows_from_the_host_in_pieces(M, N, K, chunks, rows):
+    """One piece, equal, falling and rising ones: calls of one context queued behind each other on two streams, other rows in each."""
+    from kernel_b200.ops.gemm import AGGemm, GemmRS, _pieces
 
+    assert _pieces(M, N, K, chunks) == rows
     w, bias = _ints(N, K, seed=60), _ints(N, seed=61)
     rs, ag = GemmRS(M, N, device=torch.device(DEV)), AGGemm(M, K, device=torch.device(DEV))
-    side = torch.cuda.Stream()
-    for i in range(4):
-        a = _ints(M, K, seed=62 + i)
-        want = a.float() @ w.float().t() + bias.float()
-        host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
-        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
-            rs.run_from_host(host, w, bias, out_host=out, chunks=chunks)
-            got = ag.run_from_host(host, w, bias, chunks=chunks)
-        torch.cuda.synchronize()
-        assert torch.equal(out.to(DEV), want.to(torch.bfloat16)) and torch.equal(got.to(DEV), want.to(torch.bfloat16))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    host = [_ints(M, K, seed=62 + i).cpu().pin_memory() for i in range(6)]
+    out = [[torch.zeros((M, N), dtype=torch.bfloat16).pin_memory() for _ in host] for _ in (rs, ag)]
+    torch.cuda.synchronize()
+    for i in range(len(host)):
+        with torch.cuda.stream(streams[i % 2]):
+            rs.run_from_host(host[i], w, bias, out_host=out[0][i], chunks=chunks)
+            ag.run_from_host(host[i], w, bias, out_host=out[1][i], chunks=chunks)
+    torch.cuda.synchronize()
+    for i, a in enumerate(host):
+        want = (a.to(DEV).float() @ w.float().t() + bias.float()).to(torch.bfloat16)
+        assert torch.equal(out[0][i].to(DEV), want) and torch.equal(out[1][i].to(DEV), want), i
+    with torch.cuda.stream(streams[0]):   # all that a caller waits for is its own stream
+        got = rs.run_from_host(host[0], w, bias, out_host=torch.zeros((M, N), dtype=torch.bfloat16).pin_memory(), chunks=chunks)
+    streams[0].synchronize()
+    assert torch.equal(got, out[0][0])
     _clean(rs.status)
     rs.close()
     ag.close()
@@ -540,10 +550,11 @@ def test_rows_from_the_host_that_are_too_many_to_hold(above, monkeypatch):
         ctx.close()
 
 
-def test_rows_from_the_host_in_a_graph():
-    from kernel_b200.ops.gemm import GemmRS
+@pytest.mark.parametrize("M,N,K,pieces", [(512, 264, 520, 1), (515, 4096, 4096, 3)])
+def test_rows_from_the_host_in_a_graph(M, N, K, pieces):
+    from kernel_b200.ops.gemm import GemmRS, _pieces
 
-    M, N, K = 512, 264, 520
+    assert len(_pieces(M, N, K, 4)) == pieces
     w, a = _ints(N, K, seed=66), _ints(M, K, seed=67)
     ctx = GemmRS(M, N, device=torch.device(DEV))
     host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
@@ -609,7 +620,8 @@ def test_rows_from_the_host_of_several_widths_share_their_buffers():
         ctx.run_from_host(host, ws[N], out_host=outs[N], chunks=chunks)
         torch.cuda.synchronize()
         assert torch.equal(outs[N].to(DEV), want[N])
-        assert torch.cuda.memory_allocated() - before <= 2 * M * (K + most)
+        # torch's allocator splits a cached block only if more than 1 MB of it is left over
+        assert torch.cuda.memory_allocated() - before <= 2 * M * (K + most) + (2 << 20)
     with torch.cuda.graph(graph):
         ctx.run_from_host(host, ws[4096], out_host=outs[4096])
     ctx.run_from_host(host, ws[8192], out_host=outs[8192])   # the others are too small for it
@@ -676,7 +688,9 @@ def test_round_trip_of_special_values_equals_the_general_kernels(E, dtype, H, T,
         general = ctx.dispatch_scale_combine(x, idx, w, mode)
         torch.cuda.synchronize()
         ctx.heap.check_status()
-        assert torch.equal(out.isnan(), general.isnan()) and torch.equal(out.nan_to_num(), general.nan_to_num())
+        nan, bits = general.isnan(), torch.int32 if dtype == torch.float32 else torch.int16
+        assert torch.equal(out.isnan(), nan) and torch.equal(out.view(bits)[~nan], general.view(bits)[~nan])
+        assert (general == 0).any() and general.isinf().any() and nan.any() and not nan.all()
     ctx.heap.close()
 
 
