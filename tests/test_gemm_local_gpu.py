@@ -503,11 +503,33 @@ def test_single_rank_round_trip_equals_the_general_kernels(E, k, H, T, dtype, mo
     ctx.heap.close()
 
 
+@pytest.mark.parametrize("M,N,K,chunks", [(2, 8, 8, 4), (64, 72, 136, 4), (300, 264, 1032, 1), (515, 128, 2048, 7), (1024, 2048, 136, 4), (4096, 72, 2048, 4)])
+def test_rows_from_the_host_in_pieces(M, N, K, chunks):
+    """Sizes for which the pieces are one, equal, falling and rising, call after call with other rows, and on another stream."""
+    from kernel_b200.ops.gemm import AGGemm, GemmRS
+
+    w, bias = _ints(N, K, seed=60), _ints(N, seed=61)
+    rs, ag = GemmRS(M, N, device=torch.device(DEV)), AGGemm(M, K, device=torch.device(DEV))
+    side = torch.cuda.Stream()
+    for i in range(4):
+        a = _ints(M, K, seed=62 + i)
+        want = a.float() @ w.float().t() + bias.float()
+        host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
+        with torch.cuda.stream(side if i % 2 else torch.cuda.current_stream()):
+            rs.run_from_host(host, w, bias, out_host=out, chunks=chunks)
+            got = ag.run_from_host(host, w, bias, chunks=chunks)
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), want.to(torch.bfloat16)) and torch.equal(got.to(DEV), want.to(torch.bfloat16))
+    _clean(rs.status)
+    rs.close()
+    ag.close()
+
+
 @pytest.mark.parametrize("M,N,K,chunks,rows", [
     (2, 8, 8, 4, [2]), (64, 72, 136, 4, [64]), (300, 264, 1032, 1, [300]), (4096, 72, 2048, 4, [4096]),
     (515, 4096, 4096, 4, [192, 192, 131]), (2048, 2048, 2048, 4, [512] * 4), (1111, 1024, 8192, 4, [896, 215]), (1111, 8192, 1024, 4, [256, 855]),
     (2000, 4096, 4096, 7, [320, 256, 320, 256, 320, 256, 272])])
-def test_rows_from_the_host_in_pieces(M, N, K, chunks, rows):
+def test_rows_from_the_host_in_several_pieces_queued_on_two_streams(M, N, K, chunks, rows):
     """One piece, equal, falling and rising ones: calls of one context queued behind each other on two streams, other rows in each."""
     from kernel_b200.ops.gemm import AGGemm, GemmRS, _pieces
 
@@ -550,8 +572,33 @@ def test_rows_from_the_host_that_are_too_many_to_hold(above, monkeypatch):
         ctx.close()
 
 
+def test_rows_from_the_host_in_a_graph():
+    from kernel_b200.ops.gemm import GemmRS
+
+    M, N, K = 512, 264, 520
+    w, a = _ints(N, K, seed=66), _ints(M, K, seed=67)
+    ctx = GemmRS(M, N, device=torch.device(DEV))
+    host, out = a.cpu().pin_memory(), torch.zeros((M, N), dtype=torch.bfloat16).pin_memory()
+    want = (a.float() @ w.float().t()).to(torch.bfloat16)
+    ctx.run_from_host(host, w, out_host=out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.run_from_host(host, w, out_host=out)
+    for sign in (-1, 1):
+        host.neg_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), sign * want)
+        ctx.run_from_host(host.neg_(), w, out_host=out)   # between two replays, outside of the graph
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(DEV), -sign * want)
+        host.neg_()
+    ctx.close()
+
+
 @pytest.mark.parametrize("M,N,K,pieces", [(512, 264, 520, 1), (515, 4096, 4096, 3)])
-def test_rows_from_the_host_in_a_graph(M, N, K, pieces):
+def test_several_pieces_in_a_graph(M, N, K, pieces):
     from kernel_b200.ops.gemm import GemmRS, _pieces
 
     assert len(_pieces(M, N, K, 4)) == pieces
@@ -668,6 +715,34 @@ def test_rows_from_the_host_that_cannot_be_held_go_in_chunks(fault, monkeypatch)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("H,T,k", [(1032, 9, 1), (7168, 150, 8), (2056, 700, 3)])
 def test_round_trip_of_special_values_equals_the_general_kernels(E, dtype, H, T, k):
+    """Subnormal, infinite and undefined values, signed zeros, tokens whose scales are all 1: each kind of scale has a kernel of its own."""
+    from kernel_b200.ops.dispatch_combine import MoEAllToAll
+
+    g = torch.Generator(device=DEV).manual_seed(E + H)
+    ctx = MoEAllToAll(E, k, H, T, dtype=dtype, device=torch.device(DEV))
+    x = torch.randn((T, H), device=DEV, generator=g)
+    tiny, huge = torch.finfo(dtype).tiny, torch.finfo(dtype).max
+    special = torch.tensor([0.0, -0.0, tiny, -tiny, tiny / 2, tiny / 100, huge, -huge, float("inf"), float("-inf"), float("nan")], device=DEV)
+    x[:, ::7] = special[torch.randint(0, len(special), x[:, ::7].shape, device=DEV, generator=g)]
+    x = x.to(dtype)
+    idx = torch.rand((T, E), device=DEV, generator=g).argsort(1)[:, :k].to(torch.int32).contiguous()
+    idx[::3, 0] = E - 1   # scale 1 (and, for k = 1, nothing else)
+    w = torch.softmax(torch.randn((T, k), device=DEV, generator=g), -1)
+    for mode in (0, 2):
+        ctx.enable_trace(False)
+        out = ctx.dispatch_scale_combine(x, idx, w, mode)
+        ctx.enable_trace()
+        general = ctx.dispatch_scale_combine(x, idx, w, mode)
+        torch.cuda.synchronize()
+        ctx.heap.check_status()
+        assert torch.equal(out.isnan(), general.isnan()) and torch.equal(out.nan_to_num(), general.nan_to_num())
+    ctx.heap.close()
+
+
+@pytest.mark.parametrize("E", [256, 512, 100, 1024])  # bf16: exact scales, scales of more digits, no power of two; fp16: exact up to 1024
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("H,T,k", [(1032, 9, 1), (7168, 150, 8), (2056, 700, 3)])
+def test_round_trip_of_special_values_equals_the_general_kernels_bit_by_bit(E, dtype, H, T, k):
     """Subnormal, infinite and undefined values, signed zeros, tokens whose scales are all 1: each kind of scale has a kernel of its own."""
     from kernel_b200.ops.dispatch_combine import MoEAllToAll
 
