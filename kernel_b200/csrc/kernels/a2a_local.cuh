@@ -10,7 +10,7 @@
 // in fp32 in ascending j with the rounding points of the general kernels (the expert's
 // output type, then the result's) and writes it once; outputs are equal to theirs value
 // for value.  Bound by memory (x in, out out) for many tokens, by the launch for few.
-// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 15.6 us, one token 12 -> 7 a call (1.5 us of GPU time).
+// 7168 bf16 values, top-8, 256 experts: 2048 tokens 89 -> 16.1 us, one token 12 -> 7 a call (1.5 us of GPU time).
 //
 // The arithmetic is next to the memory time (8 experts x 16 instructions per 16-byte vector, 6.5 us of issue slots;
 // 9.0 us to read and write the rows at the copy rate), hence two values per instruction, in fp32 (f32x2) and for the
@@ -106,8 +106,8 @@ __device__ __forceinline__ bool is_value_of(float v) {
 constexpr int LOCAL_WARPS = 4;  // of a CTA
 
 // What is known of the experts' scales before the launch: all are 1, all are values of T, nothing.  Each has a kernel of its own: with
-// the three loops in one, registers and schedule were those of the widest.  2048 tokens of 7168 bf16 values, top-8: scales of 1 13.2 -> 9.8
-// us (9.0 at the copy rate).
+// the three loops in one, registers and schedule were those of the widest.  2048 tokens of 7168 bf16 values, top-8, inputs and outputs out of
+// the L2: scales of 1 14.7 -> 11.6 us (9.0 at the copy rate), exact ones 17.3 -> 16.2, others 23.1 -> 22.9.
 enum Scales { UNIT, EXACT, ANY };
 // (e + 1) / E for all e: a power of two divides exactly, and e + 1 has the digits of T (8 of bf16, 11 of fp16)
 template <typename T>
@@ -285,16 +285,15 @@ static int launch_local_as(const A2aParams& p, int sms, cudaStream_t st) {
 
 // Vectors per lane.  Few tokens: one, which spreads a row over more warps (64 tokens of 14 KB 1.94 us of GPU time against 2.05
 // with four, 128 tokens 2.95 and 2.60: the line is at about 60).  Many: four, which do with the fewest instructions per value
-// what the registers allow; back to back in a graph, three inputs in turn, 7168 values, us with 1 / 2 / 4 vectors:
-//   2048 tokens bf16, scales exact  24.0 19.9 16.8    unit scales 19.9 15.6 13.2    scales not bf16 values 28.6 25.4 21.5
-//   2048 tokens fp16                30.1 22.5 19.3    fp32 40.8 23.9 19.5           256 tokens bf16          4.6  4.2  3.8
-// (before each kind of scale had its own kernel; with four vectors now 15.6, 9.8, fp16 18.5)
+// what the registers allow; back to back in a graph, three inputs and outputs in turn, 7168 values, top-8, us with 1 / 2 / 4 vectors:
+//   2048 tokens bf16, scales exact  21.9 17.6 16.2    unit scales 17.2 12.7 11.6    scales not bf16 values 28.1 23.8 22.9
+//   2048 tokens fp16, exact         23.7 19.9 19.0    fp32 41.1  -   20.7           256 tokens bf16, exact  4.3  3.7  3.7
 // In between a wide form may need a round of the resident warps more for a few tokens, leave most of a row's last warp idle
-// or fill the SMs unevenly, so 16-bit rows count the rounds and the CTAs of an SM (constants fitted): bf16, scales not bf16
-// values, 1 / 2 / 4 vectors
-//   700 tokens of 1048   3.7  4.0  4.6    300 of 4104   4.4  4.2  4.9    2048 of 2056   10.6  9.6  11.7    2048 of 2560   11.7  9.7  11.8
-// Over 610 cases past the first line (200 to 2048 tokens of 1024 to 7168 values) 1.6 % above the best form on average, with four
-// always 9.5 %.
+// or fill the SMs unevenly, so 16-bit rows count the rounds and the CTAs of an SM: bf16, scales not bf16 values, 1 / 2 / 4 vectors
+//   700 tokens of 1048   3.4  3.7  4.2    300 of 4104   4.0  3.8  4.3    2048 of 2056   6.9  5.8  6.5    2048 of 2560   9.8  8.1  9.5
+// The constants were fitted when one kernel had all three kinds of scale.  Over 68 cases of each kind past the first line (64 to 2048
+// tokens of 1024 to 7168 16-bit values) the pick is 1.8 % above the best form on average with exact scales, 1.5 with others and 3.5 with
+// scales of 1; always four 8.3, 9.1 and 2.1.
 inline int local_vecs(int tokens, int vecs, int elem_bytes, int sms) {
   const long long all = static_cast<long long>(tokens) * vecs;
   if (elem_bytes == 4) return all < 16ll * 32 * sms ? 1 : 4;
