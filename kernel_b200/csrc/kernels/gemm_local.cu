@@ -591,6 +591,20 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
   return KB_OK;
 }
 
+// Contractions of groups that have about one k block.
+bool one_k_block(const KbLocalGemmArgs* a) { return (a->expect > 0 ? a->expect : a->K) <= 56ll * a->groups; }
+
+// Two stages of the ring instead of three: such a contraction waits for its stores, and loads that run ahead of them hold them up where the
+// output does not fit the L2 and its rows start inside a 32-byte sector, fill whole lines or are few and long.  us, three stages and two:
+//   64 groups of 22 rows, 3448 x 960   92.2  81.4    64 of 19, 3656 x 648   95.9  77.6    64 of 16, 2048 x 1024   56.1  51.5
+//   64 of 24, 2504 x 1432             143.5 118.9    32 of 22, 2064 x 2888 110.4  93.4    128 of 6, 656 x 2160    85.3  80.2
+// Elsewhere three: 32 of 24, 3792 x 1424 (rows of whole sectors) 63.9 and 72.1, 32 of 30, 2816 x 2848 94.2 and 103; 16 of 14, 792 x 1864 (47 MB) 15.0 and 15.6.  122 products of 4 to
+// 56 rows per group take 0.2 % more than with the better number on average; always three 2.3 %, always two 4.4 %.
+bool two_stages(const KbLocalGemmArgs* a, const Config& c) {
+  return one_k_block(a) && !c.pair && c.bn == 256 && 2.0 * a->groups * a->M * a->N > 180e6 &&
+         (a->N % 16 != 0 || a->N % 64 == 0 || a->N > 2 * a->M);
+}
+
 // Shared memory of a tile with the rows on the M side; false where the kernel cannot run it.
 struct Ring {
   int a_rows, a_slot, b_slot, stages;
@@ -614,6 +628,7 @@ bool ring_of(const KbLocalGemmArgs* a, const Layout& l, const Config& c, Ring* r
   r->b_slot = (c.pair ? c.bn / 2 : c.bn) * BK * 2;
   const int tables = (l.grouped ? (3 * a->groups + 1) * 4 : 4) + (l.contract ? OUT_BYTES : 0);  // what the ring leaves room for
   r->stages = ring_stages(r->a_slot, r->b_slot, tables);
+  if (l.contract && r->stages > 2 && two_stages(a, c)) r->stages = 2;
   r->slot_rows = c.pair ? 128 : ceil_div(r->a_rows, 32) * 32;
   // the last A slot is read up to 128 rows far: the B slots behind it cover that
   return r->stages >= 2 && r->stages * r->b_slot >= 16384 && (c.split == 1 || exchange_fits(r->a_rows, c.pair, c.bn, c.split));
@@ -639,6 +654,7 @@ extern "C" int kb_gemm_local_pick(const KbLocalGemmArgs* a, int sms, KbLocalPick
   kbs::Ring swap_ring;
   const int expect = a->expect > 0 ? a->expect : a->M;
   const bool fits = pick.swap ? kbs::ring_of(s, l.b_mn, a->K, l.grouped ? a->groups : 0, expect, &swap_ring) : ring_of(a, l, c, &ring);
+  out->stages = !fits ? 0 : pick.swap ? swap_ring.stages : ring.stages;
   return fits ? KB_OK : KB_ERR_UNSUPPORTED;
 }
 
@@ -710,8 +726,7 @@ extern "C" int kb_gemm_local(const KbLocalGemmArgs* a, void* stream_v) {
   const uint64_t bz = a->kind == KB_LOCAL_ROWS ? groups : 1;
   // A contraction over one k block waits for its stores, not for loads, and large boxes hold the stores up: 128 groups of 16 rows,
   // 512 x 2048, 58 us with a load per 64 columns, 61 with one per operand.
-  const int expect = a->expect > 0 ? a->expect : a->K;
-  const bool whole = !contract || expect > 56ll * groups;
+  const bool whole = !contract || !one_k_block(a);
   p.a_whole = whole && a_mn && a->M % 64 == 0 ? 1 : 0;
   p.b_whole = whole && b_mn && a->N % 64 == 0 ? 1 : 0;
   const int b_cols = c.pair ? c.bn / 2 : c.bn;

@@ -394,6 +394,23 @@ def test_contractions_whose_columns_come_in_one_box(counts, M, N, pair, bn, monk
     assert torch.equal(dense, (a.float().t() @ b.float()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("M,N", [(1000, 1416), (1104, 1344), (600, 2416)])
+def test_contractions_over_one_k_block_with_two_stages(M, N):
+    """Outputs of more than 180 MB, whose operand ring has two stages: empty groups, whole blocks and a group of several."""
+    from kernel_b200.ops import local as L
+
+    counts = ([0, 1, 17, 64, 5, 33, 0, 40] * 8)[:63] + [200]
+    start, count, R = _table(counts, L.ROW_ALIGN)
+    a, b = torch.zeros((R, M), dtype=torch.bfloat16, device=DEV), torch.zeros((R, N), dtype=torch.bfloat16, device=DEV)
+    for s, n in zip(start.tolist(), count.tolist()):
+        a[s:s + n], b[s:s + n] = _ints(n, M, seed=80 + s), _ints(n, N, seed=81 + s)
+    st = _status()
+    out = L.contract_product(a, b, start, count, status=st, expect=sum(counts))
+    _clean(st)
+    for e, (s, n) in enumerate(zip(start.tolist(), count.tolist())):
+        assert torch.equal(out[e], (a[s:s + n].float().t() @ b[s:s + n].float()).to(torch.bfloat16)), e
+
+
 @pytest.mark.parametrize("R,Cn", [(1, 8), (63, 264), (65, 2048), (1000, 520), (8192, 72)])
 def test_col_sum(R, Cn):
     from kernel_b200.ops.local import col_sum

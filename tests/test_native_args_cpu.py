@@ -334,6 +334,30 @@ def test_tiles_of_contractions_whose_difference_was_measured():
         assert pair(*product) == 1, product
 
 
+def test_ring_of_contractions_over_one_k_block():
+    """At least 5 % apart on a B200 (us, three stages / two)."""
+    def stages(groups, rows, M, Nn):
+        a, p = _local(kind=N.LOCAL_CONTRACT, M=M, N=Nn, K=groups * (rows + 63), groups=groups, expect=groups * rows, row_start=16, row_count=16), N.LocalPick()
+        assert N.lib().kb_gemm_local_pick(C.byref(a), 148, C.byref(p)) == N.KB_OK and p.pair == 0
+        return p.stages
+
+    for product in ((64, 22, 3448, 960),      # 92.2 81.4
+                    (64, 19, 3656, 648),      # 95.9 77.6
+                    (64, 5, 2320, 1752),      # 165 134
+                    (32, 22, 2064, 2888),     # 110 93.4
+                    (64, 16, 2048, 1024),     # 56.1 51.5
+                    (128, 6, 656, 2160)):     # 85.3 80.2
+        assert stages(*product) == 2, product
+    for product in ((32, 24, 3792, 1424),     # 63.9 72.1
+                    (64, 45, 3112, 1248),     # 88.9 96.9
+                    (128, 10, 1848, 624),     # 58.3 65.8
+                    (32, 24, 1128, 2416),     # 35.0 38.7
+                    (32, 30, 2816, 2848),     # 94.2 103
+                    (16, 29, 3744, 2960),     # 65.8 72.1
+                    (64, 64, 2048, 1024)):    # more than one k block
+        assert stages(*product) == 3, product
+
+
 def test_vectors_per_lane_of_the_round_trip():
     """Where a form was at least 5 % faster than the others on a B200 (us with 1 / 2 / 4 vectors per lane)."""
     vecs = lambda tokens, hidden, elem=2: N.lib().kb_a2a_local_vecs(tokens, hidden, elem, 148)
