@@ -113,7 +113,7 @@ class GemmStreamArgs(C.Structure):
 
 
 class LocalPick(C.Structure):
-    _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split", "overlapped", "stages")]
+    _fields_ = [(name, C.c_int) for name in ("exchanged", "pair", "bn", "rows", "split", "overlapped", "stages", "ahead")]
 
 
 class A2aArgs(C.Structure):

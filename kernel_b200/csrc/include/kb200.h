@@ -179,6 +179,7 @@ typedef struct KbLocalPick {
   int split;      // members of a cluster that share a tile's contraction
   int overlapped; // set up under the end of the previous launch (dense products)
   int stages;     // of the operand ring
+  int ahead;      // first weights into the L2 before the previous launch has ended
 } KbLocalPick;
 int kb_gemm_local_pick(const KbLocalGemmArgs* args, int sms, KbLocalPick* out);
 // The tile a dense product on `sms` SMs gets if its rows are on the M side.

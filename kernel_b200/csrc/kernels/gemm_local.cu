@@ -650,6 +650,7 @@ extern "C" int kb_gemm_local_pick(const KbLocalGemmArgs* a, int sms, KbLocalPick
   else *out = {0, c.tall ? 2 : c.pair, c.bn, c.tall ? 512 : c.pair ? 256 : a->kind == KB_LOCAL_ROWS ? c.rows : 128, c.split};
   const int cluster = (out->pair ? 2 : 1) * out->split;
   out->overlapped = overlaps(cluster, out->split, ceil_div(a->M, out->rows) * ceil_div(a->N, out->bn) * cluster, cap, 2.0 * a->N * a->K);
+  out->ahead = prefetches(*a);
   Ring ring;
   kbs::Ring swap_ring;
   const int expect = a->expect > 0 ? a->expect : a->M;

@@ -73,12 +73,14 @@ inline bool overlaps(int cluster, int split, int grid, int sms, double weight_by
 // with, back to back, three weights in turn:
 //   1 x 8192 x 8192  26.9  25.0    16 x 7168 x 18432  46.0  44.3    64 x 7168 x 18432  46.6  45.2    128 x 4096 x 4096  13.1  12.3
 // Not where `early` fills the ring itself by then, nor from more rows on, whose tensor work it only disturbs: an MLP of 256 tokens
-// 72.7 us without and 73.1 with, MoE layers of 32 tokens 94.0 and 94.5; nor for weights of a few MB, which are often in the L2
-// already: 64 x 2880 x 2880 7.7 us without and 7.9 with, 4 x 4096 x 4096 (34 MB) 9.4 and 8.7.  Nor for weights along N, which are 256
-// bytes of each of many rows: 24 to 60 MB 5 % longer with it on average (7 x 3376 x 5792 10.8 us without, 11.9 with), 60 to 100 MB
-// 2 %, more than that 1 %.
+// 72.7 us without and 73.1 with, MoE layers of 32 tokens 94.0 and 94.5; nor for weights along N, which are 256 bytes of each of
+// many rows: 24 to 60 MB 5 % longer with it on average (7 x 3376 x 5792 10.8 us without, 11.9 with), 60 to 100 MB 2 %, more than
+// that 1 %.  Nor for weights of up to 33 MB, of which the L2 holds four: weights that are there already take 4 to 7 % longer with it,
+// others gain the less the smaller they are.  us, one weight again and again, and eight in turn, without and with:
+//   16 x 2336 x 5544 (26 MB)  7.9 8.5   9.5  9.2    73 x 9200 x 1632 (30 MB)  8.5 9.1  10.6 10.1    8 x 4096 x 4096 (34 MB)  7.4 7.8  10.1 9.6
+//   16 x 4608 x 4608 (42 MB)  8.4 8.8  11.6 10.3    32 x 7168 x 4096 (59 MB) 10.0 10.4 14.2 12.8
 inline bool prefetches(const KbLocalGemmArgs& a) {
-  return a.kind == KB_LOCAL_DENSE && !a.b_mn && a.M <= 128 && a.early == 0 && 2.0 * a.N * a.K >= 24e6;
+  return a.kind == KB_LOCAL_DENSE && !a.b_mn && a.M <= 128 && a.early == 0 && 2.0 * a.N * a.K >= 33e6;
 }
 
 // One CTA per SM with all of its shared memory, in clusters of `cluster` CTAs.

@@ -334,6 +334,22 @@ def test_tiles_of_contractions_whose_difference_was_measured():
         assert pair(*product) == 1, product
 
 
+def test_weights_that_are_asked_for_ahead():
+    """Only where that gains more for weights in memory than it costs for weights in the L2 (us without / with, from the L2; from memory)."""
+    def ahead(M, Nn, K, **kw):
+        a, p = _local(M=M, N=Nn, K=K, **kw), N.LocalPick()
+        assert N.lib().kb_gemm_local_pick(C.byref(a), 148, C.byref(p)) == N.KB_OK
+        return p.ahead
+
+    for product in ((16, 2336, 5544), (38, 1712, 7840), (73, 9200, 1632)):   # 7.9 8.5, 9.5 9.2; 8.8 9.4, 10.4 10.1; 8.5 9.1, 10.6 10.1
+        assert ahead(*product) == 0, product
+    for product in ((8, 4096, 4096), (16, 4608, 4608), (32, 7168, 4096)):    # 7.4 7.8, 10.1 9.6; 8.4 8.8, 11.6 10.3; 10.0 10.4, 14.2 12.8
+        assert ahead(*product) == 1, product
+    for kw in (dict(b_mn=1), dict(early=1)):
+        assert ahead(32, 7168, 4096, **kw) == 0, kw
+    assert ahead(129, 7168, 4096) == 0
+
+
 def test_ring_of_contractions_over_one_k_block():
     """At least 5 % apart on a B200 (us, three stages / two)."""
     def stages(groups, rows, M, Nn):
