@@ -507,6 +507,8 @@ Choice pick_rows(int cap, int rows, int groups, int N, int K, bool w_mn, int sha
     // with activation, plain and slope take 1.4, 1.6 and 2.0 % more than the best tile of both kinds on average (before the fit 5.7, 3.6
     // and 3.0; always exchanged 1.3, 1.9 and 1.4, always the M side 9.5, 4.5 and 17), 84 of 558 more than 3 % (179).  That was with 1.25 below 32
     // rows and 130 ns for a pair's single box; 563 others of 0.1 to 31 rows take 1.4 % more than the best kind so, 1.8 with those.
+    // 2316 products of 0.2 to 1200 rows per group, in order of the three: 3.1, 4.2 and 3.3 % above the fastest of one CTA and pair of
+    // either kind (the fastest of five noisy times); kernels and rule before the fit took 9.7, 8.8 and 7.7 % more.
     const double limit = slope ? 1.14 : rows >= 192ll * groups ? 1.02 : rows >= 32ll * groups ? 0.99 : 1.05;
     r.swap = other - (early ? EARLY : 0.0) < limit * plain;
     e = {rows, N, K, groups, key, 0, r};
@@ -594,12 +596,14 @@ int pick_tile(const KbLocalGemmArgs* a, const Layout& l, int dev, int sms, int c
 // Contractions of groups that have about one k block.
 bool one_k_block(const KbLocalGemmArgs* a) { return (a->expect > 0 ? a->expect : a->K) <= 56ll * a->groups; }
 
-// Two stages of the ring instead of three: such a contraction waits for its stores, and loads that run ahead of them hold them up where the
-// output does not fit the L2 and its rows start inside a 32-byte sector, fill whole lines or are few and long.  us, three stages and two:
+// Two stages of the ring instead of three: such a contraction waits for its stores, and loads that run ahead of them hold them up
+// where the output does not fit the L2 and its rows start inside a 32-byte sector, fill whole lines or are few and long.  us, three
+// stages and two:
 //   64 groups of 22 rows, 3448 x 960   92.2  81.4    64 of 19, 3656 x 648   95.9  77.6    64 of 16, 2048 x 1024   56.1  51.5
 //   64 of 24, 2504 x 1432             143.5 118.9    32 of 22, 2064 x 2888 110.4  93.4    128 of 6, 656 x 2160    85.3  80.2
-// Elsewhere three: 32 of 24, 3792 x 1424 (rows of whole sectors) 63.9 and 72.1, 32 of 30, 2816 x 2848 94.2 and 103; 16 of 14, 792 x 1864 (47 MB) 15.0 and 15.6.  122 products of 4 to
-// 56 rows per group take 0.2 % more than with the better number on average; always three 2.3 %, always two 4.4 %.
+// Elsewhere three: 32 of 24, 3792 x 1424 (rows of whole sectors) 63.9 and 72.1, 32 of 30, 2816 x 2848 94.2 and 103; 16 of 14,
+// 792 x 1864 (47 MB) 15.0 and 15.6.  122 products of 4 to 56 rows per group take 0.2 % more than with the better number on average;
+// always three 2.3 %, always two 4.4 %.
 bool two_stages(const KbLocalGemmArgs* a, const Config& c) {
   return one_k_block(a) && !c.pair && c.bn == 256 && 2.0 * a->groups * a->M * a->N > 180e6 &&
          (a->N % 16 != 0 || a->N % 64 == 0 || a->N > 2 * a->M);
